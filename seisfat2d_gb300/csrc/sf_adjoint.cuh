@@ -476,12 +476,6 @@ __device__ __forceinline__ void gather_interior(const GatherStage& S, float* g, 
             }
 }
 
-__device__ __forceinline__ void cp_async16_cg(void* smem, const void* gmem)
-{
-    unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gmem) : "memory");
-}
-
 // Bounded wait of one thread until *p >= target (acquire); false after the
 // limit, with the error flag set.
 __device__ __forceinline__ bool wait_count(const unsigned* p, unsigned target, int* err, unsigned long long wait_ns)

@@ -102,19 +102,42 @@ __global__ void k_expand(const float* __restrict__ in, int nx, int nz, int nb, f
 
 // Checks fdiv_k against __fdiv_rn for b = divs[w] over all dividends of [1, 2)
 // (both signs follow by symmetry); rbs[w] = RN(1/b), bad bit w set on any
-// difference.
+// difference. Then (w = n) frcp_k on [1, 2), bad bit 5, and (w = n+1, n+2)
+// fsqrt_k on [1, 4), bad bit 4.
 __global__ void k_verify_div(const float* divs, int n, float* rbs, int* bad)
 {
-    const unsigned total = (unsigned)n << 23;
+    const unsigned total = (unsigned)(n + 3) << 23;
     for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
         const int w = t >> 23;
-        const float b = divs[w], rb = __frcp_rn(b);
-        if ((t & 0x7fffffu) == 0) rbs[w] = rb;
         const float a = __uint_as_float(0x3f800000u | (t & 0x7fffffu));
-        bool out_of_range = false;
-        if (__float_as_uint(fdiv_k<false>(a, b, rb, true, out_of_range)) != __float_as_uint(__fdiv_rn(a, b)))
-            atomicOr(bad, 1 << w);
+        float got, want;
+        int bit = w;
+        if (w < n) {
+            const float b = divs[w], rb = __frcp_rn(b);
+            if ((t & 0x7fffffu) == 0) rbs[w] = rb;
+            got = fdiv_k<false>(a, b, rb);
+            want = __fdiv_rn(a, b);
+        } else if (w == n) {
+            got = frcp_k(a);
+            want = __frcp_rn(a);
+            bit = 5;
+        } else {
+            const float v = (w == n + 1) ? a : 2.0f * a;
+            got = fsqrt_k<false>(v);
+            want = __fsqrt_rn(v);
+            bit = 4;
+        }
+        if (__float_as_uint(got) != __float_as_uint(want)) atomicOr(bad, 1 << bit);
     }
+}
+
+// Sets *flag when a slowness of the field lies outside in_fast_range.
+__global__ void k_check_range(const float* __restrict__ S, size_t n, float dx, float dz, int* flag)
+{
+    bool ok = true;
+    for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x)
+        ok &= in_fast_range(S[q], dx, dz);
+    if (!ok) *flag = 1;
 }
 
 // compute_seismogram on a device field (modeling.cu:161-194).
@@ -136,8 +159,9 @@ __global__ void k_picks(const float* __restrict__ T, int nzz, int ncols, int c0,
 
 size_t sf_fwd_smem_bytes(int warps, bool comp, bool tape)
 {
-    const int slots = tape ? FwdBlock<true>::RING : FwdBlock<false>::RING;
-    return ((sizeof(CtaShared) + 15) & ~size_t(15)) + (size_t)warps * (comp ? ring_bytes<true>(slots) : ring_bytes<false>(slots));
+    const size_t ring = tape ? (comp ? ring_bytes<true, true>() : ring_bytes<true, false>())
+                             : (comp ? ring_bytes<false, true>() : ring_bytes<false, false>());
+    return ((sizeof(CtaShared) + 15) & ~size_t(15)) + (size_t)warps * ring;
 }
 
 // ------------------------------------------------------------------ context
@@ -199,7 +223,7 @@ extern "C" int sf_ctx_destroy(sf_ctx* c)
     void* bufs[] = {c->d_S, c->d_flags, c->d_shots, c->d_T, c->d_rx, c->d_rz, c->d_picks, c->d_Sq,
                     c->d_tcode, c->d_tc1, c->d_tc2, c->d_model, c->d_cij_all, c->d_hand, c->d_ctr,
                     c->d_skern, c->d_upd, c->d_wav, c->d_mig, c->d_kgeo, c->d_kint, c->d_kpart,
-                    c->d_vfac, c->d_gcij, c->d_fuse, c->d_Tl};
+                    c->d_vfac, c->d_gcij, c->d_fuse, c->d_Tl, c->d_srange};
     for (void* b : bufs)
         if (b) cudaFree(b);
     delete c;
@@ -285,9 +309,10 @@ extern "C" int sf_get_launch(const sf_ctx* c, int* warps, int* gang_warps)
     return SF_OK;
 }
 
-// Warps per shot ("slots"): all strips of a shot on their own warp when the
-// device can hold every shot that way, else the largest divisor of the strip
-// count that keeps all shots resident at once (at least 1).
+// Warps per shot ("slots"). The solve of a shot is a list of 4 nstrips strip
+// tasks of which 2 nstrips can run at once (solve_window), so a shot gets up
+// to that many warps when the device holds every shot that way, else an equal
+// share of the device's warps (at least 1).
 int sf_gang_shape(sf_ctx* c, const void* kernel, size_t smem, int nshots, int nstrips, int gang_warps, int* G,
                   int* NG)
 {
@@ -298,10 +323,7 @@ int sf_gang_shape(sf_ctx* c, const void* kernel, size_t smem, int nshots, int ns
     int slots = gang_warps;
     if (slots <= 0) {
         const long long cap_warps = cap_ctas * c->warps;
-        slots = 1;
-        for (int d = 1; d <= nstrips; d++)
-            if (nstrips % d == 0 && (long long)d * nshots <= cap_warps) slots = d;
-        if ((long long)nstrips * std::max(1, nshots) <= cap_warps) slots = nstrips;
+        slots = (int)std::max(1LL, std::min<long long>(2LL * nstrips, cap_warps / std::max(1, nshots)));
     }
     int g = std::max(1, (slots + c->warps - 1) / c->warps);
     if (g > cap_ctas) g = (int)cap_ctas;
@@ -335,7 +357,7 @@ int sf_verify_divisors(sf_ctx* c)
     k.rdz = h_rb[1];
     k.rhyp = h_rb[2];
     k.rD = h_rb[3];
-    k.mflags = (~h_bad) & 0xf;
+    k.mflags = ((~h_bad) & 0x3f) | (range_ok(k.dx, k.dz) ? 0x40 : 0);
     return SF_OK;
 }
 
@@ -420,6 +442,18 @@ int sf_fwd_setup(sf_ctx* c)
 
 // ------------------------------------------------------------------ models
 
+// Checks the context's slowness for the fast form of the updates (d_flags[2],
+// read by the solves), on the legacy stream like the copies that set it.
+int sf_check_slowness(sf_ctx* c, cudaStream_t st)
+{
+    const size_t n = (size_t)c->nxx * c->nzz;
+    CK(cudaMemsetAsync(c->d_flags + 2, 0, sizeof(int), st));
+    k_check_range<<<(unsigned)std::min<size_t>((n + 255) / 256, (size_t)c->sms * 8), 256, 0, st>>>(c->d_S, n, c->dx, c->dz,
+                                                                                                 c->d_flags + 2);
+    CK(cudaGetLastError());
+    return SF_OK;
+}
+
 extern "C" int sf_set_slowness(sf_ctx* c, const float* s, int layout, int mem)
 {
     if (!c || !s) return SF_ERR_ARG;
@@ -428,7 +462,10 @@ extern "C" int sf_set_slowness(sf_ctx* c, const float* s, int layout, int mem)
     if (layout == SF_LAYOUT_PADDED) {
         CK(cudaMemcpy(c->d_S, s, npad * sizeof(float),
                       mem == SF_MEM_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice));
-        return SF_OK;
+        int rc = sf_check_slowness(c, nullptr);
+        // a host copy is finished when the call returns: so is its check
+        if (!rc && mem != SF_MEM_DEVICE) CK(cudaStreamSynchronize(nullptr));
+        return rc;
     }
     if (layout != SF_LAYOUT_MODEL) return sf_fail(c, SF_ERR_ARG, "unknown layout");
     const size_t nm = (size_t)c->nx * c->nz;
@@ -438,6 +475,8 @@ extern "C" int sf_set_slowness(sf_ctx* c, const float* s, int layout, int mem)
                   mem == SF_MEM_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice));
     k_expand<<<std::min<size_t>((npad + 255) / 256, 4096), 256>>>(c->d_model, c->nx, c->nz, c->nb, c->d_S);
     CK(cudaGetLastError());
+    int rc = sf_check_slowness(c, nullptr);
+    if (rc) return rc;
     CK(cudaDeviceSynchronize());
     return SF_OK;
 }
@@ -674,7 +713,7 @@ int sf_fwd_configure(sf_ctx* c, int nrec, bool per_shot_T, bool tape, int gang_w
         if (rc) return rc;
     }
     const size_t hand_bytes =
-        (size_t)NG * 4 * nstrips * c->batch_maxcols * sizeof(unsigned long long) * (comp ? 2 : 1);
+        (size_t)NG * hand_words(nstrips, c->batch_maxcols, comp ? 2 : 1) * sizeof(unsigned long long);
     rc = sf_dev_reserve_zero(c, (void**)&c->d_hand, &c->cap_hand, hand_bytes);
     if (rc) return rc;
     const size_t nctr = (size_t)NG;
@@ -707,6 +746,7 @@ int sf_fwd_configure(sf_ctx* c, int nrec, bool per_shot_T, bool tape, int gang_w
     p.wait_ns = c->wait_ns;
     p.hand = c->d_hand;
     p.bar = c->d_ctr;
+    p.srange = Sshots ? c->d_srange : c->d_flags + 2;
     if (tape) {
         p.tcode = c->d_tcode;
         p.tc1 = c->d_tc1;
@@ -781,6 +821,8 @@ int sf_qp_launch(sf_ctx* c, bool fact, cudaStream_t st)
     for (int k = 0; k < 6; k++) q.cij[k] = c->d_cij_all + k * npad;
     std::memcpy(q.mm, c->mm, sizeof(q.mm));
     q.Sq = c->d_Sq;
+    q.srange = c->d_srange;
+    CK(cudaMemsetAsync(c->d_srange, 0, c->hshots.size() * sizeof(int), st));
     q.vfac = fact ? c->d_vfac : nullptr;
     q.vfac_total = c->batch_q_cells;
     const bool comp = c->arith == SF_ARITH_COMPENSATED, ref = c->arith == SF_ARITH_REFERENCE;
@@ -807,6 +849,7 @@ int sf_launch_shots(sf_ctx* c, int ani, int nrec, float* d_picks, bool keep_tabl
         // eikonal_ani.cu:33-45: solve on S, qP pass, solve on the qP slowness;
         // every shot keeps its window between the launches
         rc = sf_dev_reserve(c, (void**)&c->d_Sq, &c->cap_Sq, (size_t)c->batch_q_cells * sizeof(float));
+        if (!rc) rc = sf_dev_reserve(c, (void**)&c->d_srange, &c->cap_srange, c->hshots.size() * sizeof(int));
         if (!rc && tape)
             rc = sf_dev_reserve(c, (void**)&c->d_vfac, &c->cap_vfac, 3 * (size_t)c->batch_q_cells * sizeof(float));
         FwdLaunch L1, L2;

@@ -62,7 +62,7 @@ struct sf_ctx {
     std::string err;
 
     float* d_S = nullptr;       // padded slowness
-    int* d_flags = nullptr;     // [0] work counter, [1] error flag, [2..] adjoint counters
+    int* d_flags = nullptr;     // [1] error flag, [2] the slowness has a value outside in_fast_range
     float* d_model = nullptr;
     size_t cap_model = 0;
     uint16_t* d_cij_all = nullptr;  // six padded code fields
@@ -139,6 +139,7 @@ struct sf_ctx {
     // anisotropic adjoint: per-shot dSq/d{S, C11, C13} factors and the
     // stiffness gradients of the last adjoint (sf_batch_stiffness_gradient)
     float* d_vfac = nullptr; size_t cap_vfac = 0;
+    int* d_srange = nullptr; size_t cap_srange = 0;  // per shot: qP slowness outside in_fast_range
     float* d_gcij = nullptr; size_t cap_gcij = 0;
     bool gcij_valid = false;
     std::vector<int> h_kint;
@@ -172,6 +173,8 @@ int sf_dev_reserve_zero(sf_ctx* c, void** p, size_t* cap, size_t bytes);
 // Next handoff-tag epoch (never 0; wraps within 22 bits).
 unsigned sf_next_epoch(sf_ctx* c);
 int sf_check_flags(sf_ctx* c, cudaStream_t st);
+// Device check of the context's slowness after it changed.
+int sf_check_slowness(sf_ctx* c, cudaStream_t st);
 int sf_fwd_setup(sf_ctx* c);
 int sf_verify_divisors(sf_ctx* c);
 size_t sf_fwd_smem_bytes(int warps, bool comp, bool tape);

@@ -37,7 +37,10 @@ struct FwdParams {
     float* Tlpool;        // compensated: lo parts of the traveltimes, same layout as Tpool
     long long t_per_gang; // > 0: each gang reuses Tpool + gang * t_per_gang
     int* err;
-    unsigned long long* hand;  // tagged strip handoff pairs: per gang [4 sweeps][nstrips][maxcols] (x2 compensated)
+    // per gang (hand_words): tagged strip handoff pairs [4 sweeps][nstrips]
+    // [hand_pitch] (x2 compensated), then progress words [4 sweeps][nstrips]
+    unsigned long long* hand;
+    const int* srange;    // nonzero: the slowness has a value outside in_fast_range (per shot with Sshots)
     unsigned* bar;        // per gang barrier counter
     unsigned epoch;       // launch number (tags: epoch << 10 | shot-solve number)
     unsigned long long wait_ns;  // time limit of the bounded waits
@@ -78,9 +81,8 @@ __device__ __forceinline__ size_t tape_strip_base(long long tape_off, int sweep,
     return (size_t)tape_off + ((size_t)sweep * nstrips + k) * (size_t)(ncols + 31) * 32;
 }
 
-// Where a gang's warps sit: warp w of CTA g of the gang is slot w*G + g.
-// Strip k belongs to slot k mod slots in every sweep, so consecutive strips
-// run on different CTAs and SMs and a warp only rereads rows it wrote.
+// Where a gang's warps sit: warp w of CTA g of the gang is slot w*G + g, so
+// consecutive slots, which run consecutive strips, are on different CTAs and SMs.
 struct GangPos {
     int gang, g, warp, slot, slots;
 };
@@ -96,20 +98,42 @@ __device__ __forceinline__ GangPos gang_pos(int G)
     return q;
 }
 
-// The four sweeps of one solve of the current shot; every warp of the gang
-// runs the strips of its slot. No barrier between sweeps: consecutive sweeps
-// run the rows in opposite directions, a warp rereads only rows it wrote
-// itself, and the handoff chain orders everything else. Square cells (dx and
-// dz equal) run the strip loops' square-cell form. COMP: compensated
-// arithmetic, lo parts in Tl, two handoff pairs per column.
+// The strip of sweep SW that a.k names, in the loop form the shot needs.
+template <int SW, bool TAPE, bool REF, bool INTERIOR, bool COMP>
+__device__ __forceinline__ void sweep_strip(const StripArgs& a, bool exact)
+{
+    constexpr int SZ = (SW & 1) ? -1 : 1, SX = (SW < 2) ? 1 : -1;
+    if (exact)
+        run_strip<SZ, SX, SW == 0, TAPE, REF, false, false, COMP, true>(a);
+    else if (a.kc.dx == a.kc.dz)
+        run_strip<SZ, SX, SW == 0, TAPE, REF, INTERIOR, true, COMP, false>(a);
+    else
+        run_strip<SZ, SX, SW == 0, TAPE, REF, INTERIOR, false, COMP, false>(a);
+}
+
+// The four sweeps of one solve of the current shot. Sweeps 0 (down) and 1
+// (up) march to the right, 2 and 3 to the left. The strips of each such pair
+// are one list of tasks in dependency order (sweep 0's strips top to bottom,
+// then sweep 1's bottom to top), dealt to the gang's warps in turn: sweep 1's
+// bottom strip starts as soon as a warp is free and sweep 0's bottom strip
+// has written its first columns, instead of after the whole sweep. With a
+// warp per task a pair of sweeps takes ncols + 2 nstrips lags steps instead
+// of 2 (ncols + nstrips lags). Every task waits only on earlier ones (the
+// strip before it in its sweep; its own rows in the sweep before), and each
+// warp runs its tasks in order, so the schedule cannot deadlock. No barrier
+// between sweeps. Square cells (dx and dz equal) run the strip loops'
+// square-cell form. COMP: compensated arithmetic, lo parts in Tl, two handoff
+// pairs per column.
 template <bool TAPE, bool REF, bool INTERIOR, bool COMP>
 __device__ void solve_window(const FwdParams& p, const ShotDev& sh, const GangPos& gp, const float* Sw,
-                             int ldS, float* T, float* Tl, unsigned tag, CtaShared* cs, unsigned char* rings)
+                             int ldS, float* T, float* Tl, unsigned tag, bool exact, CtaShared* cs, unsigned char* rings)
 {
     const int nzz = p.nzz, ncols = sh.ncols;
     const int nstrips = (nzz + 31) >> 5;
     constexpr size_t HS = COMP ? 2 : 1;
-    unsigned long long* hb = p.hand + (size_t)gp.gang * 4 * nstrips * p.maxcols * HS;
+    const size_t row = (size_t)hand_pitch(p.maxcols) * HS;
+    unsigned long long* hb = p.hand + (size_t)gp.gang * hand_words(nstrips, p.maxcols, HS);
+    unsigned long long* prog = hb + 4 * (size_t)nstrips * row;
     StripArgs a;
     a.S = Sw;
     a.ldS = ldS;
@@ -117,12 +141,11 @@ __device__ void solve_window(const FwdParams& p, const ShotDev& sh, const GangPo
     a.Tl = Tl;
     a.nzz = nzz;
     a.ncols = ncols;
-    a.nstrips = nstrips;
     a.sIdz = sh.sIdz;
     a.sIdx = sh.sIdx - sh.c0;
     a.kc = p.kc;
     a.init = cs->init;
-    a.ring = rings + (size_t)gp.warp * ring_bytes<COMP>(FwdBlock<TAPE>::RING);
+    a.ring = rings + (size_t)gp.warp * ring_bytes<TAPE, COMP>();
     a.sh = cs;
     a.err = p.err;
     a.tcode = nullptr;
@@ -131,38 +154,29 @@ __device__ void solve_window(const FwdParams& p, const ShotDev& sh, const GangPo
     a.tag = tag;
     a.tag_in = p.stall_handoff ? 1u : tag;  // epoch 0 is never used, zeroed pairs carry tag 0
 #pragma unroll 1
-    for (int sw = 0; sw < 4; sw++) {
-        const bool szpos = !(sw == 1 || sw == 3);
+    for (int task = gp.slot; task < 4 * nstrips; task += gp.slots) {
+        const int sw = task / nstrips, pidx = task - sw * nstrips;
+        a.k = (sw & 1) ? nstrips - 1 - pidx : pidx;
         a.skip_i = sh.skip_i[sw];
         a.skip_j = sh.skip_j[sw];
-        unsigned long long* hs = hb + (size_t)sw * nstrips * p.maxcols * HS;
-        const int first = szpos ? gp.slot : ((nstrips - 1 - gp.slot) % gp.slots + gp.slots) % gp.slots;
-#pragma unroll 1
-        for (int pidx = first; pidx < nstrips; pidx += gp.slots) {
-            a.k = szpos ? pidx : nstrips - 1 - pidx;
-            a.h_in = (pidx > 0) ? hs + (size_t)pidx * p.maxcols * HS : nullptr;
-            a.h_out = (pidx < nstrips - 1) ? hs + (size_t)(pidx + 1) * p.maxcols * HS : nullptr;
-            if (TAPE) {
-                size_t base = tape_strip_base(sh.tape_off, sw, a.k, nstrips, ncols);
-                a.tcode = p.tcode + base;
-                a.tc1 = p.tc1 + base;
-                a.tc2 = p.tc2 + base;
-            }
-            if (p.kc.dx == p.kc.dz) {
-                switch (sw) {
-                case 0: run_strip<1, 1, true, TAPE, REF, INTERIOR, true, COMP>(a); break;
-                case 1: run_strip<-1, 1, false, TAPE, REF, INTERIOR, true, COMP>(a); break;
-                case 2: run_strip<1, -1, false, TAPE, REF, INTERIOR, true, COMP>(a); break;
-                default: run_strip<-1, -1, false, TAPE, REF, INTERIOR, true, COMP>(a); break;
-                }
-            } else {
-                switch (sw) {
-                case 0: run_strip<1, 1, true, TAPE, REF, INTERIOR, false, COMP>(a); break;
-                case 1: run_strip<-1, 1, false, TAPE, REF, INTERIOR, false, COMP>(a); break;
-                case 2: run_strip<1, -1, false, TAPE, REF, INTERIOR, false, COMP>(a); break;
-                default: run_strip<-1, -1, false, TAPE, REF, INTERIOR, false, COMP>(a); break;
-                }
-            }
+        unsigned long long* hs = hb + ((size_t)sw * nstrips + pidx) * row;
+        a.h_in = (pidx > 0) ? hs : nullptr;
+        a.h_out = (pidx < nstrips - 1) ? hs + row : nullptr;
+        a.prog_in = (sw > 0) ? prog + (size_t)(sw - 1) * nstrips + a.k : nullptr;
+        a.follow = sw & 1;
+        a.prog_out = (sw < 3) ? prog + (size_t)sw * nstrips + a.k : nullptr;
+        a.publish = !(sw & 1);
+        if (TAPE) {
+            size_t base = tape_strip_base(sh.tape_off, sw, a.k, nstrips, ncols);
+            a.tcode = p.tcode + base;
+            a.tc1 = p.tc1 + base;
+            a.tc2 = p.tc2 + base;
+        }
+        switch (sw) {
+        case 0: sweep_strip<0, TAPE, REF, INTERIOR, COMP>(a, exact); break;
+        case 1: sweep_strip<1, TAPE, REF, INTERIOR, COMP>(a, exact); break;
+        case 2: sweep_strip<2, TAPE, REF, INTERIOR, COMP>(a, exact); break;
+        default: sweep_strip<3, TAPE, REF, INTERIOR, COMP>(a, exact); break;
         }
     }
 }
@@ -205,7 +219,8 @@ __global__ void __launch_bounds__((COMP ? kMaxWarpsComp : ((TAPE && INTERIOR) ? 
         const unsigned tag = (p.epoch << 10) | (unsigned)(it & 1023);
         init_block<REF>(p, sh, Sw, cs->init);
         __syncthreads();
-        solve_window<TAPE, REF, INTERIOR, COMP>(p, sh, gp, Sw, nzz, T, Tl, tag, cs, rings);
+        const bool exact = p.kc.mflags != kFastFlags || p.srange[p.Sshots ? b : 0] != 0;
+        solve_window<TAPE, REF, INTERIOR, COMP>(p, sh, gp, Sw, nzz, T, Tl, tag, exact, cs, rings);
         // receivers (modeling.cu:161-194), spread over the gang once the field is final
         if (p.nrec > 0 && p.picks) {
             gang_barrier(bar, (++nbar) * p.G, cs, p.err);
@@ -244,6 +259,7 @@ struct QpParams {
     const uint16_t* cij[6];
     float mm[12];
     float* Sq;            // per-shot qP slowness windows at q_off
+    int* srange;          // per shot: set when its qP slowness has a value outside in_fast_range
     float* vfac;          // FACT: dSq/dS, dSq/dC11, dSq/dC13 per window cell (3 x vfac_total)
     long long vfac_total;
 };
@@ -290,6 +306,7 @@ __global__ void __launch_bounds__(128) k_qp(QpParams p)
                 if (FACT) qp_factors(dzr, dxr, s, p.kc.dx, p.kc.dz, c11, c13, c15, c33, c35, c55, fS, f11, f13);
             }
             Sq[idx] = out;
+            if (!in_fast_range(out, p.kc.dx, p.kc.dz)) p.srange[b] = 1;
             if (FACT) {
                 float* f = p.vfac + sh.q_off + idx;
                 f[0] = fS;

@@ -20,11 +20,14 @@ using namespace sf;
 
 namespace {
 
-// Scratch capacity: the tagged strip-handoff pairs of the four sweeps for
-// grids with ceil(nzz/32) * nxx <= kNoAllocCells (4 x 8 bytes each: 8 MiB),
-// plus a 256-byte header with the launch's error flag, barrier counter,
-// epoch and shot descriptor.
+// Scratch capacity: the tagged strip-handoff pairs of the four sweeps and
+// their strips' progress words for grids with ceil(nzz/32) * nxx <=
+// kNoAllocCells (4 x 8 bytes per strip and column, with up to three more
+// columns and a word per strip: nxx is at least 8, so half as much again
+// covers them), plus a 256-byte header with the launch's error flag, barrier
+// counter, epoch and shot descriptor.
 constexpr size_t kNoAllocCells = 262144;
+constexpr size_t kNoAllocWords = 4 * (kNoAllocCells + kNoAllocCells / 2);
 constexpr size_t kNoAllocHeader = 256;
 
 struct NoAllocHeader {
@@ -34,12 +37,13 @@ struct NoAllocHeader {
     int div_bad;       // k_verify_div: bit w set when divisor w failed (must start at 0)
     float divs[4];     // the four constant divisors (dx, dz, hyp, D) being verified
     float rdivs[4];    // their reciprocals, written by k_verify_div
+    int srange;        // set when S has a value outside in_fast_range (must start at 0)
     ShotDev shot;      // the one shot of the call
 };
 static_assert(sizeof(NoAllocHeader) <= 256, "header too large");
 
 // Shared by every call on a device; keeps the last call's contents.
-static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocHeader + 4 * kNoAllocCells * sizeof(unsigned long long)];
+static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocHeader + kNoAllocWords * sizeof(unsigned long long)];
 
 constexpr int kMaxDevices = 64;
 std::mutex g_setup_mutex;
@@ -163,7 +167,7 @@ extern "C" int sf_time_propagation_noalloc(const float* S, int nx, int nz, float
         k.rdz = rd[1];
         k.rhyp = rd[2];
         k.rD = rd[3];
-        k.mflags = (~bad) & 0xf;
+        k.mflags = ((~bad) & 0x3f) | (range_ok(dx, dz) ? 0x40 : 0);
         std::lock_guard<std::mutex> lock(g_setup_mutex);
         g_vdx[dev] = dx;
         g_vdz[dev] = dz;
@@ -171,7 +175,12 @@ extern "C" int sf_time_propagation_noalloc(const float* S, int nx, int nz, float
         g_mflags[dev] = k.mflags;
         g_verified[dev] = true;
     }
+    const size_t npad = (size_t)nxx * nzz;
+    k_check_range<<<(unsigned)std::min<size_t>((npad + 255) / 256, (size_t)g_sms[dev] * 8), 256, 0, st>>>(S, npad, dx, dz,
+                                                                                                       &dh->srange);
+    if (cudaGetLastError() != cudaSuccess) return SF_ERR_CUDA;
     FwdParams p{};
+    p.srange = &dh->srange;
     p.S = S;
     p.nzz = nzz;
     p.nxx = nxx;

@@ -9,22 +9,31 @@
 // upwind value. Consecutive strips (usually on other SMs) are chained through
 // global memory without fences: the last lane of strip p writes each value of
 // its row together with a tag (launch epoch and shot number) as one 64-bit
-// store; lane 0 of strip p+1 prefetches the pair through the same cp.async
-// pipeline as its own columns and checks the tag. A stale pair (the producer
-// has not got there yet) sends lane 0 into a bounded spin on the pair itself,
-// after which it waits until the producer is some columns further on, so
-// later prefetches find their data. Producers never wait on consumers, so
-// every wait points to a lower strip and the schedule cannot deadlock however
-// strips are spread over warps and CTAs.
+// store; strip p+1 prefetches the pairs (through L2 only, so that a line of
+// which the producer had written a part is never found again in L1) and
+// checks the tags. A stale pair (the producer has not got there yet) sends
+// lane 0 into a bounded spin on the pair itself, after which it waits until
+// the producer is some columns further on, so later prefetches find their
+// data. Producers never wait on consumers, so every wait points to an earlier
+// strip and the schedule cannot deadlock however strips are spread over warps
+// and CTAs.
+//
+// The two sweeps of a march direction overlap: the upward sweep's first strip
+// starts once the downward sweep's last strip is under way (solve_window). A
+// strip's traveltimes then pass from one warp to another, so the earlier
+// sweep's strip publishes how many columns it has written back (a fence and
+// a tagged counter, every 32 columns) and the later one stays behind it.
 //
 // Column chunks are staged into a per-warp shared-memory ring by cp.async,
 // a few march columns ahead (32 consecutive rows = one coalesced 128-byte
 // request per field), and lane l reads its own row of column s-l from the
-// ring. With slot pitches of 32 (T) and 36 (S, with the halo row and the
-// handoff pair) floats both the coalesced fill and the skewed read are
-// bank-conflict free. Finished columns go back to global memory through the
-// same ring, coalesced. The march runs in blocks of a few steps: one wait for
-// the staged columns per block, the block's ring reads, its node updates
+// ring. A ring slot holds one column: slowness rows rb-1..rb+31 at 0..32,
+// traveltimes at 36..67 and, in the compensated arithmetic, their lo parts at
+// 68..99. With slot pitches of 68 and 100 floats both the coalesced fill and
+// the skewed read are bank-conflict free, and one address serves all fields
+// of a node. Finished columns go back to global memory through the same
+// ring, coalesced. The march runs in blocks of a few steps: one wait for the
+// staged columns per block, the block's ring reads, its node updates
 // (the only serial chain), then its stores.
 //
 // Any order of node updates that respects the sweep's dependency DAG gives the
@@ -38,27 +47,30 @@
 namespace sf {
 
 constexpr int kU = 4;       // march steps per block of the reverse sweeps' strip loop
-constexpr int kRing = 48;   // column slots per warp ring of the reverse sweeps and the plain forward
+constexpr int kRing = 48;   // column slots per warp ring of the reverse sweeps
 
-// Block size, staging lead (march columns, a multiple of the block) and ring
-// length of a forward strip loop: 4, 8 and 48 slots for the plain solve; 2,
-// 4 and 40 for the taped one, which keeps a tape record per step of the
-// block in registers (measured 19% faster than 4 and 8 there). After a stall
-// a consumer lets its producer get `lead` columns ahead (lead + block
-// measured 1% slower). The ring holds the 32 marches the lanes work on, the
-// lead and two blocks, so a block's prefetches never refill a slot that the
-// block before it still read: RING >= 31 + LOOK + 2 U.
-template <bool TAPE>
+// Block size U, staging leads (march columns, multiples of the block) of the
+// columns (LOOK) and of the upwind strip's pairs (PLOOK), and ring length of
+// a forward strip loop. After a stall a consumer lets its producer get AHEAD
+// columns ahead. The ring holds the 32 marches the lanes work on, the lead
+// and two blocks, so a block's prefetches never refill a slot that the block
+// before it still read: RING >= 31 + LOOK + 2 U.
+template <bool TAPE, bool COMP>
 struct FwdBlock {
     static constexpr int U = TAPE ? 2 : 4;
     static constexpr int LOOK = TAPE ? 4 : 8;
-    static constexpr int AHEAD = LOOK;
+    static constexpr int PLOOK = 4;
+    static constexpr int AHEAD = PLOOK + U;
     static constexpr int RING = TAPE ? 40 : 48;
-    static_assert(LOOK % U == 0 && RING % U == 0 && RING >= 31 + LOOK + 2 * U, "ring too small");
+    static constexpr int SLOT = COMP ? 100 : 68;  // floats per slot
+    static constexpr int PAIRS = 16;              // columns of the pair ring
+    static_assert(LOOK % U == 0 && PLOOK % U == 0 && PLOOK <= LOOK && RING % U == 0 && RING >= 31 + LOOK + 2 * U,
+                  "ring too small");
+    static_assert(PAIRS % U == 0 && PAIRS >= PLOOK + U && U % 2 == 0, "pair ring too small");
+    static_assert((RING * SLOT) % 32 == 0, "a wrapped skewed read would conflict");
 };
-constexpr int kSP = 36;     // S slot pitch: rows rb-1 .. rb+31 at 0..32, handoff pair at 34..35
-constexpr int kSPc = 40;    // compensated: S slot pitch, handoff pairs {hi,tag},{lo,tag} at 36..39
-constexpr int kTP = 32;     // T slot pitch
+constexpr int kT0 = 36, kL0 = 68;  // traveltimes and their lo parts in a slot
+constexpr int kPublish = 32;       // columns between two publications of a strip's progress
 constexpr int kMaxWarps = 16;
 // compensated kernels keep a second traveltime ring (the lo parts): at most
 // 8 warps per CTA fit in shared memory
@@ -70,14 +82,23 @@ constexpr int kMaxWarpsTapedInterior = 8;
 constexpr long long kSpinLimit = 1ll << 30;          // iterations
 constexpr unsigned long long kSpinNs = 2000000000ull;  // and at most ~2 s (default; sf_set_wait_limit)
 
-// A warp's forward ring of R column slots: S (slot pitch kSP; compensated
-// kSPc, with the two handoff pairs of the hi and the lo parts), T, and in the
-// compensated arithmetic L (the lo parts of the traveltimes), one after the
-// other. Every size is a multiple of 16 bytes.
-template <bool COMP>
-constexpr size_t ring_bytes(int R)
+// A warp's forward ring: RING column slots, then the pair ring (a tagged
+// pair per column, two in the compensated arithmetic). Multiples of 16 bytes.
+template <bool TAPE, bool COMP>
+constexpr size_t ring_bytes()
 {
-    return sizeof(float) * (size_t)R * ((COMP ? kSPc : kSP) + (COMP ? 2 : 1) * kTP);
+    using B = FwdBlock<TAPE, COMP>;
+    return sizeof(float) * (size_t)B::RING * B::SLOT + 8 * (size_t)B::PAIRS * (COMP ? 2 : 1);
+}
+
+// Columns a row of handoff pairs is padded to: whole 16-byte pairs of pairs
+// past the last column.
+__host__ __device__ constexpr int hand_pitch(int maxcols) { return (maxcols + 3) & ~1; }
+// 64-bit words of one gang's handoff region: the pairs of four sweeps (hs
+// per column), then one progress word per sweep and strip.
+__host__ __device__ constexpr size_t hand_words(int nstrips, int maxcols, int hs)
+{
+    return 4 * (size_t)nstrips * ((size_t)hand_pitch(maxcols) * hs) + ((4 * (size_t)nstrips + 1) & ~(size_t)1);
 }
 
 // Per-CTA shared state (static part), followed by the CTA's warp rings in
@@ -94,15 +115,15 @@ __device__ __forceinline__ void cp_async4(void* smem, const void* gmem)
     unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(sa), "l"(gmem) : "memory");
 }
-__device__ __forceinline__ void cp_async8(void* smem, const void* gmem)
-{
-    unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sa), "l"(gmem) : "memory");
-}
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem)
 {
     unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
     asm volatile("cp.async.ca.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void cp_async16_cg(void* smem, const void* gmem)
+{
+    unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gmem) : "memory");
 }
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N>
@@ -145,17 +166,23 @@ struct StripArgs {
     float* Tl;        // compensated: their lo parts, same layout
     int nzz, ncols;
     int k;            // strip index: rows [32k, 32k+32)
-    int nstrips;
     int sIdz, sIdx;   // source node (window coordinates)
     int skip_i, skip_j;
     Consts kc;
     const float* init;  // 9 values in shared memory
-    unsigned char* ring;  // this warp's ring (ring_bytes<COMP>(FwdBlock<TAPE>::RING) bytes at least)
+    unsigned char* ring;  // this warp's ring (ring_bytes<TAPE, COMP>())
     CtaShared* sh;
     const unsigned long long* h_in;  // {value, tag} of the upwind strip's row by march column (nullptr: first strip)
     unsigned long long* h_out;       // pairs this strip feeds to the next one (nullptr: last strip)
     unsigned tag;                    // tag of this shot's pairs
     unsigned tag_in;                 // tag a consumer waits for (= tag; 1, which no launch writes, to test the timeout path)
+    // columns written back by the previous sweep of this strip (nullptr in
+    // the first sweep): all of them before the march starts, or (follow) a
+    // few more than the march has reached
+    const unsigned long long* prog_in;
+    bool follow;
+    unsigned long long* prog_out;    // this strip's own count (nullptr: nobody reads it)
+    bool publish;                    // every kPublish columns, not only at the end
     // tape (TAPE only): base of this sweep/strip, entries [step*32 + lane]
     uint8_t* tcode;
     float* tc1;
@@ -190,6 +217,46 @@ __device__ __forceinline__ float wait_pair(const unsigned long long* p, unsigned
     return val_of(e);
 }
 
+// Bounded wait of the whole warp until the progress word at p carries `tag`
+// and at least `need` columns (acquire, by lane 0); returns the columns seen.
+__device__ __forceinline__ int wait_progress(const unsigned long long* p, unsigned tag, int need, CtaShared* sh, int* err)
+{
+    int cols = need;
+    if ((threadIdx.x & 31) == 0) {
+        unsigned long long e;
+        unsigned long long t0 = 0;
+        long long n = 0;
+        while (true) {
+            asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(e) : "l"(p) : "memory");
+            if (tag_of(e) == tag && (int)(unsigned)e >= need) {
+                cols = (int)(unsigned)e;
+                break;
+            }
+            if (ld_volatile(&sh->abort_flag) || *(volatile int*)err) break;
+            if (n == 0) t0 = global_ns();
+            __nanosleep(32);
+            if (++n > kSpinLimit || ((n & 255) == 0 && global_ns() - t0 > sh->wait_ns)) {
+                st_volatile(&sh->abort_flag, 1);
+                atomicExch(err, 2);
+                break;
+            }
+        }
+    }
+    return __shfl_sync(0xffffffffu, cols, 0);
+}
+
+// Publishes that this warp's strip has written `cols` columns back: every
+// lane's stores, ordered by the warp barrier and lane 0's fence, before the word.
+__device__ __forceinline__ void publish_progress(unsigned long long* p, unsigned tag, int cols)
+{
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0) {
+        __threadfence();
+        asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(((unsigned long long)tag << 32) | (unsigned)cols)
+                     : "memory");
+    }
+}
+
 // Bounded wait until the counter at p reaches `target` (acquire); returns
 // the value seen. On timeout it raises the CTA's abort flag and the launch's
 // error flag and returns `target`, and every later wait of the CTA (or of any
@@ -213,92 +280,133 @@ __device__ __forceinline__ unsigned wait_counter(const unsigned* p, unsigned tar
     return v;
 }
 
-// INTERIOR: blocks whose marches all lie inside the window run a body without
-// bounds tests (fewer instructions per step, more code); otherwise every block
-// runs the general body. SQ: square cells (node_update). All forms give the
-// same bits. COMP: compensated arithmetic (node_update_comp): every
+// INTERIOR: blocks whose marches all lie inside the window (and touch neither
+// the source's 3x3 block nor a skipped cell) run a body without those tests
+// (fewer instructions per step, more code); otherwise every block runs the
+// general body. SQ: square cells (node_update). EXACT: IEEE division and
+// roots on any operand (a slowness outside in_fast_range). All forms give
+// the same bits. COMP: compensated arithmetic (node_update_comp): every
 // traveltime the loop carries, stages, hands on and writes back is a pair
 // (hi, lo); the second handoff pair of a column carries lo.
-template <int SZ, int SX, bool SW0, bool TAPE, bool REF, bool INTERIOR, bool SQ, bool COMP = false>
+template <int SZ, int SX, bool SW0, bool TAPE, bool REF, bool INTERIOR, bool SQ, bool COMP, bool EXACT>
 __device__ __forceinline__ void run_strip(const StripArgs& a)
 {
-    constexpr int kU = FwdBlock<TAPE>::U, kLook = FwdBlock<TAPE>::LOOK, kAhead = FwdBlock<TAPE>::AHEAD;
-    constexpr int kRing = FwdBlock<TAPE>::RING;
+    using B = FwdBlock<TAPE, COMP>;
+    constexpr int U = B::U, LOOK = B::LOOK, PLOOK = B::PLOOK, RING = B::RING, P = B::SLOT;
+    constexpr int HS = COMP ? 2 : 1;         // handoff pairs per column
     const int lane = threadIdx.x & 31;
     const int nzz = a.nzz, ncols = a.ncols;
     const int rb = 32 * a.k;
     const int r = (SZ > 0) ? rb + lane : rb + 31 - lane;
     const bool vrow = r < nzz;
     const bool irow = (r >= 1) && (r <= nzz - 2);
-    const int tix = r - rb;    // T slot index of row r; S slot index of row r-1
-    const int six = tix + 1;   // S slot index of row r
+    const bool row1 = r == 1;
+    const int tix = r - rb;    // the row's place among the strip's rows
     const int dr1 = (SZ > 0) ? 0 : 1;
     const int dc2 = (SX > 0) ? 0 : 1;
     const int dr2a = (r - 1 >= 1) ? 0 : 1;
 
-    constexpr int SP = COMP ? kSPc : kSP;    // S slot pitch
-    constexpr int PQ = COMP ? 36 : 34;       // first handoff pair in an S slot
-    float* Sring = reinterpret_cast<float*>(a.ring);
-    float* Tring = Sring + kRing * SP;
-    float* Lring = COMP ? Tring + kRing * kTP : nullptr;
-    constexpr int HS = COMP ? 2 : 1;         // handoff pairs per column
+    float* ring = reinterpret_cast<float*>(a.ring);
+    float* pring = ring + RING * P;          // handoff pairs of march q at (q mod PAIRS) * 2 HS
 
     // global rows this lane stages
     const int ls_row = rb - 1 + lane;
     const bool ls_ok = (ls_row >= 0) && (ls_row < nzz);
-    const bool lx_ok = (lane == 0) && (rb + 31 < nzz);
+    const bool lx_ok = (lane < U) && (rb + 31 < nzz);  // lanes 0..U-1: the halo row of the block's columns
     const bool lt_ok = (rb + lane) < nzz;
-    const float* Sg = a.S;
-    float* Tg = a.T;
     const int ldS = a.ldS;
 
     CtaShared* sh = a.sh;
-    const bool consumer = (lane == 0) && (a.h_in != nullptr);
+    const bool consumer = a.h_in != nullptr;
+    const bool lane0 = lane == 0;
+    const bool feeds = (lane == 31) && (a.h_out != nullptr);
     // the strip holds rows of the source's 3x3 block (first sweep only)
     const bool src_rows = SW0 && (a.sIdz + 1 >= rb) && (a.sIdz - 1 <= rb + 31);
     auto col_of = [&](int m) { return (SX > 0) ? m : ncols - 1 - m; };
-    // running source addresses of march column q (q advances by one per call)
+    // blocks whose first step lies in [g0, g0 + gn] need the general body for
+    // the source block (first sweep) or a skipped cell
+    int g0 = 0, gn = -1;
+    if (src_rows) {
+        const int ms = (SX > 0) ? a.sIdx : ncols - 1 - a.sIdx;
+        g0 = ms - 1;
+        gn = 2;
+    }
+    if (a.skip_i >= rb && a.skip_i <= rb + 31) {
+        const int ms = (SX > 0) ? a.skip_j : ncols - 1 - a.skip_j;
+        const int lo = (gn < 0) ? ms : min(g0, ms), hi = (gn < 0) ? ms : max(g0 + gn, ms);
+        g0 = lo;
+        gn = hi - lo;
+    }
+    // from marches to a block's first step (none: a range no step reaches)
+    g0 = (gn < 0) ? -(1 << 30) : g0 - (U - 1);
+    gn = (gn < 0) ? 0 : gn + U - 1 + 31;
+
+    // running source addresses of the next march columns to stage
     const long long dcol = (SX > 0) ? 1 : -1;
-    const float* pS = Sg + (size_t)ls_row + (long long)col_of(0) * (long long)ldS;
-    const float* pX = Sg + (size_t)(rb + 31) + (long long)col_of(0) * (long long)ldS;
-    const float* pT = Tg + (size_t)(rb + lane) + (long long)col_of(0) * (long long)nzz;
-    const float* pTl = COMP ? a.Tl + (size_t)(rb + lane) + (long long)col_of(0) * (long long)nzz : nullptr;
     const long long dS = dcol * (long long)ldS, dT = dcol * (long long)nzz;
+    const float* pS = a.S + (long long)ls_row + (long long)col_of(0) * (long long)ldS;
+    const float* pX = a.S + (long long)(rb + 31) + (long long)col_of(0) * (long long)ldS + lane * dS;
+    const float* pT = a.T + (long long)(rb + lane) + (long long)col_of(0) * (long long)nzz;
+    const float* pTl = COMP ? a.Tl + (long long)(rb + lane) + (long long)col_of(0) * (long long)nzz : nullptr;
+    // columns q .. q+U-1 into slots slot .. slot+U-1 (U divides RING: no wrap)
     // FAST: every march the call touches lies inside the window (no bounds tests)
-    auto prefetch = [&](int q, int slot, auto fast_tag) {
+    auto stage_cols = [&](int q, int slot, auto fast_tag) {
         constexpr bool FAST = decltype(fast_tag)::value;
-        if (FAST || q < ncols) {
-            if (ls_ok) cp_async4(&Sring[slot * SP + lane], pS);
-            if (lx_ok) cp_async4(&Sring[slot * SP + 32], pX);
-            if (!SW0 && lt_ok) {
-                cp_async4(&Tring[slot * kTP + lane], pT);
-                if (COMP) cp_async4(&Lring[slot * kTP + lane], pTl);
+        float* d = ring + slot * P + lane;
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            if (FAST || q + u < ncols) {
+                if (ls_ok) cp_async4(d + u * P, pS);
+                if (!SW0 && lt_ok) {
+                    cp_async4(d + u * P + kT0, pT);
+                    if (COMP) cp_async4(d + u * P + kL0, pTl);
+                }
             }
-            // upwind-row pair(s) of march q
-            if (consumer) {
-                if (COMP) cp_async16(&Sring[slot * SP + PQ], a.h_in + 2 * q);
-                else cp_async8(&Sring[slot * SP + PQ], a.h_in + q);
+            pS += dS;
+            if (!SW0) {
+                pT += dT;
+                if (COMP) pTl += dT;
             }
         }
-        cp_commit();
-        pS += dS;
-        pX += dS;
-        pT += dT;
-        if (COMP) pTl += dT;
+        if (lx_ok && (FAST || q + lane < ncols)) cp_async4(ring + (slot + lane) * P + 32, pX);
+        pX += U * dS;
+    };
+    // the upwind row's pairs of marches q .. q+U-1
+    auto stage_pairs = [&](int q, auto fast_tag) {
+        constexpr bool FAST = decltype(fast_tag)::value;
+        constexpr int N = COMP ? U : U / 2;  // 16-byte copies
+        const int c = COMP ? q + lane : q + 2 * lane;
+        if (consumer && lane < N && (FAST || c < ncols))
+            cp_async16_cg(pring + (c % B::PAIRS) * (2 * HS), a.h_in + (size_t)HS * c);
     };
 
-    // let the previous strip get kAhead columns ahead before the first
-    // prefetches of its values
-    if (consumer) wait_pair(a.h_in + HS * min(kAhead, ncols - 1), a.tag_in, sh, a.err);
-    __syncwarp();
+    // columns of the previous sweep known to be written back
+    int avail = SW0 ? 0x7fffffff : 0;
+    auto ensure = [&](int q) {  // marches below q may be staged
+        if (!SW0 && q > avail) {
+            avail = wait_progress(a.prog_in, a.tag, a.follow ? min(q, ncols) : ncols, sh, a.err);
+            if (avail >= ncols) avail = 0x7fffffff;
+        }
+    };
 
-    // prologue: march columns 0 .. kLook-1
+    // let the previous strip get AHEAD columns ahead before the first
+    // prefetches of its values
+    if (consumer && lane0) wait_pair(a.h_in + HS * min(B::AHEAD, ncols - 1), a.tag_in, sh, a.err);
+    __syncwarp();
+    ensure(LOOK);
+
+    // prologue: march columns 0 .. LOOK-1, pairs 0 .. PLOOK-1
 #pragma unroll 1
-    for (int q = 0; q < kLook; q++) prefetch(q, q, std::false_type{});
+    for (int q = 0; q < LOOK; q += U) {
+        stage_cols(q, q, std::false_type{});
+        if (q < PLOOK) stage_pairs(q, std::false_type{});
+        cp_commit();
+    }
 
     // running destinations: write-back of march column s-31 (row r), tape entry s*32+lane
-    float* pW = Tg + (size_t)r + (long long)col_of(0) * (long long)nzz;
-    float* pWl = COMP ? a.Tl + (size_t)r + (long long)col_of(0) * (long long)nzz : nullptr;
+    float* pW = a.T + (long long)r + (long long)col_of(0) * (long long)nzz;
+    float* pWl = COMP ? a.Tl + (long long)r + (long long)col_of(0) * (long long)nzz : nullptr;
+    unsigned long long* pH = a.h_out - 31 * HS;
     uint8_t* pcode = TAPE ? a.tcode + lane : nullptr;
     float* pc1 = TAPE ? a.tc1 + lane : nullptr;
     float* pc2 = TAPE ? a.tc2 + lane : nullptr;
@@ -308,81 +416,104 @@ __device__ __forceinline__ void run_strip(const StripArgs& a)
     float cU = 0.0f, cI = 0.0f;                           // carried S of rows r-1, r
     const int nsteps = ncols + 31;
     int b0 = 0;                                           // ring slot of march s0
+    // ring offset of the lane's march s0 - lane (its row's first slowness)
+    int ro = ((RING - lane) % RING) * P + tix;
 
-    // Blocks of kU steps: one wait for the staged columns per block, then the
-    // block's ring reads, its kU node updates, and its stores. Within a block
+    // Blocks of U steps: one wait for the staged columns per block, then the
+    // block's ring reads, its U node updates, and its stores. Within a block
     // the node updates are the only serial chain; the loads before and the
     // stores after it are independent of it.
     auto block = [&](int s0, auto fast_tag) {
         constexpr bool FAST = decltype(fast_tag)::value;
+        ensure(s0 + LOOK + U);
         {
-            int pf0 = b0 + kLook;
-            if (pf0 >= kRing) pf0 -= kRing;
-#pragma unroll
-            for (int u = 0; u < kU; u++) prefetch(s0 + kLook + u, pf0 + u, fast_tag);
+            int pf0 = b0 + LOOK;
+            if (pf0 >= RING) pf0 -= RING;
+            stage_cols(s0 + LOOK, pf0, fast_tag);
+            stage_pairs(s0 + PLOOK, fast_tag);
+            cp_commit();
         }
-        // march columns <= s0+kU are staged (SX < 0 reads one column ahead)
-        cp_wait<kLook - 1>();
+        // staged: columns up to s0+U (SX < 0 reads one column ahead), pairs up to s0+U-1
+        cp_wait<(LOOK / U - 1 < PLOOK / U) ? LOOK / U - 1 : PLOOK / U>();
         __syncwarp();
 
-        int ml = b0 - lane;                               // slot of march s0 - lane
-        if (ml < 0) ml += kRing;
-        int msl[kU];
-        float nU[kU], nI[kU], told[kU], toldl[kU];
-        unsigned long long pr[kU], prl[kU];
+        int off[U];
+        float nU[U], nI[U], told[U], toldl[U];
 #pragma unroll
-        for (int u = 0; u < kU; u++) {
-            int ms = ml + u;
-            if (ms >= kRing) ms -= kRing;
-            msl[u] = ms;
+        for (int u = 0; u < U; u++) {
+            off[u] = ro;
+            ro += P;
+            if (ro >= RING * P + tix) ro -= RING * P;
             // S of the new column: march m (SX>0) or m+1 (SX<0)
-            const int ns = (SX > 0) ? ms : (ms + 1 == kRing ? 0 : ms + 1);
-            nU[u] = Sring[ns * SP + tix];
-            nI[u] = Sring[ns * SP + six];
-            told[u] = SW0 ? kBig : Tring[ms * kTP + tix];
-            toldl[u] = (COMP && !SW0) ? Lring[ms * kTP + tix] : 0.0f;
-            pr[u] = consumer ? *reinterpret_cast<const unsigned long long*>(&Sring[ms * SP + PQ]) : 0ull;
-            prl[u] = (COMP && consumer) ? *reinterpret_cast<const unsigned long long*>(&Sring[ms * SP + PQ + 2]) : 0ull;
+            const int ns = (SX > 0) ? off[u] : ro;
+            nU[u] = ring[ns];
+            nI[u] = ring[ns + 1];
+            told[u] = SW0 ? kBig : ring[off[u] + kT0];
+            toldl[u] = (COMP && !SW0) ? ring[off[u] + kL0] : 0.0f;
         }
-        if (consumer) {
-            // a pair the previous strip had not written when it was prefetched:
-            // wait for it, then fall kAhead columns behind so later prefetches hit
+        // the upwind strip's values of the block (every lane reads them, lane 0 uses them)
+        float hv[U], hvl[U];
+        {
+            const float* q = pring + (s0 % B::PAIRS) * (2 * HS);
+            unsigned stale = 0;
+            if (COMP) {
 #pragma unroll
-            for (int u = 0; u < kU; u++) {
-                const int s = s0 + u;
-                if ((FAST || s < ncols) && (tag_of(pr[u]) != a.tag_in || (COMP && tag_of(prl[u]) != a.tag_in))) {
-                    pr[u] = pack_tag(wait_pair(a.h_in + HS * s, a.tag_in, sh, a.err), a.tag_in);
-                    if (COMP) prl[u] = pack_tag(wait_pair(a.h_in + HS * s + 1, a.tag_in, sh, a.err), a.tag_in);
-                    wait_pair(a.h_in + HS * min(s + kAhead, ncols - 1), a.tag_in, sh, a.err);
+                for (int u = 0; u < U; u++) {
+                    const uint4 e = *reinterpret_cast<const uint4*>(q + 4 * u);
+                    hv[u] = __uint_as_float(e.x);
+                    hvl[u] = __uint_as_float(e.z);
+                    if (FAST || s0 + u < ncols) stale |= (e.y ^ a.tag_in) | (e.w ^ a.tag_in);
                 }
+            } else {
+#pragma unroll
+                for (int u = 0; u < U; u += 2) {
+                    const uint4 e = *reinterpret_cast<const uint4*>(q + 2 * u);
+                    hv[u] = __uint_as_float(e.x);
+                    hv[u + 1] = __uint_as_float(e.z);
+                    hvl[u] = hvl[u + 1] = 0.0f;
+                    if (FAST || s0 + u < ncols) stale |= e.y ^ a.tag_in;
+                    if (FAST || s0 + u + 1 < ncols) stale |= e.w ^ a.tag_in;
+                }
+            }
+            if (consumer && stale != 0) {
+                // a pair the previous strip had not written when it was prefetched:
+                // wait for it, then fall AHEAD columns behind so later prefetches hit
+                if (lane0) {
+#pragma unroll
+                    for (int u = 0; u < U; u++) {
+                        const int s = s0 + u;
+                        if (FAST || s < ncols) {
+                            hv[u] = wait_pair(a.h_in + HS * s, a.tag_in, sh, a.err);
+                            if (COMP) hvl[u] = wait_pair(a.h_in + HS * s + 1, a.tag_in, sh, a.err);
+                        }
+                    }
+                    wait_pair(a.h_in + HS * min(s0 + U - 1 + B::AHEAD, ncols - 1), a.tag_in, sh, a.err);
+                }
+                __syncwarp();
             }
         }
 
-        float tnw[kU], tnwl[kU];
-        bool actv[kU];
-        Rec rec[kU];
-        // the block's kU node updates; EXACT divides with IEEE division
-        auto updates = [&](auto exact_tag) -> bool {
-        constexpr bool EXACT = decltype(exact_tag)::value;
-        bool bad = false;
+        float tnw[U], tnwl[U], sr[U];
+        Rec rec[U];
+        int any_far = 0;
 #pragma unroll
-        for (int u = 0; u < kU; u++) {
+        for (int u = 0; u < U; u++) {
             const int s = s0 + u;
             const int m = s - lane;
-            const bool act = FAST ? vrow : (vrow && (m >= 0) && (m < ncols));
             const int j = col_of(m);
+            const bool act = FAST || (vrow && (m >= 0) && (m < ncols));
             // upwind value from the lane above (or the previous strip)
             float tv = __shfl_up_sync(0xffffffffu, tn, 1);
             float tvl = COMP ? __shfl_up_sync(0xffffffffu, tnl, 1) : 0.0f;
-            if (consumer && (FAST || s < ncols)) {
-                tv = val_of(pr[u]);
-                if (COMP) tvl = val_of(prl[u]);
+            if (lane0) {
+                tv = hv[u];
+                if (COMP) tvl = hvl[u];
             }
             const float te = tn, tev = tvp;
             const float tel = tnl, tevl = tvpl;
 
             float to = told[u], tol = toldl[u];
-            if (SW0 && src_rows) {
+            if (!FAST && src_rows) {
                 const int da = r - a.sIdz + 1, db = j - a.sIdx + 1;
                 if (da >= 0 && da < 3 && db >= 0 && db < 3) {
                     to = a.init[da + 3 * db];
@@ -392,108 +523,111 @@ __device__ __forceinline__ void run_strip(const StripArgs& a)
             float U_j, I_j, U_jm, I_jm;
             if (SX > 0) { U_j = nU[u]; I_j = nI[u]; U_jm = cU; I_jm = cI; }
             else        { U_j = cU; I_j = cI; U_jm = nU[u]; I_jm = nI[u]; }
-
-            float tnew = to, tnewl = tol;
-            rec[u].code = 0; rec[u].c1 = 0.0f; rec[u].c2 = 0.0f;
-            const bool inner = act && irow && (FAST || ((j >= 1) && (j <= ncols - 2))) &&
-                               !(r == a.skip_i && j == a.skip_j);
+            const bool inner = FAST ? irow
+                                    : act && irow && (j >= 1) && (j <= ncols - 2) && !(r == a.skip_i && j == a.skip_j);
             // rows: i1 (SZ>0: r-1, else r); columns: j-1 (clamped to 1), j
             const float Si1_j = (SZ > 0) ? U_j : I_j;
             const float Si1_jm = (SZ > 0) ? U_jm : I_jm;
-            const float s1a = (j == 1) ? Si1_j : Si1_jm;   // S[i1][max(j-1,1)]
-            const float s1b = Si1_j;                       // S[i1][j]
-            const float Sa_j1 = (SX > 0) ? ((r == 1) ? I_jm : U_jm) : ((r == 1) ? I_j : U_j);
-            const float s2a = Sa_j1;                       // S[max(i-1,1)][j1]
-            const float s2b = (SX > 0) ? I_jm : I_j;       // S[i][j1]
-            const float sref = (SX > 0) ? Si1_jm : Si1_j;  // S[i1][j1]
-            const int dc1a = (j - 1 >= 1) ? 0 : 1;
-            bool bad_u = false;
-            if (inner) {
-                if constexpr (COMP)
-                    node_update_comp<TAPE, EXACT, SQ>(to, tol, tv, tvl, te, tel, tev, tevl, s1a, s1b, s2a, s2b, sref,
-                                                      a.kc, dr1, dc1a, dc2, dr2a, tnew, tnewl, rec[u], bad_u);
-                else
-                    tnew = node_update<TAPE, REF, EXACT, SQ>(to, tv, te, tev, s1a, s1b, s2a, s2b, sref, a.kc,
-                                                             dr1, dc1a, dc2, dr2a, rec[u], bad_u);
+            const float s1a = (!FAST && j == 1) ? Si1_j : Si1_jm;   // S[i1][max(j-1,1)]
+            const float s1b = Si1_j;                                // S[i1][j]
+            const float s2b = (SX > 0) ? I_jm : I_j;                // S[i][j1]
+            const float s2a = row1 ? s2b : ((SX > 0) ? U_jm : U_j); // S[max(i-1,1)][j1]
+            const float sref = (SX > 0) ? Si1_jm : Si1_j;           // S[i1][j1]
+            const int dc1a = (FAST || j - 1 >= 1) ? 0 : 1;
+            float tnew, tnewl = 0.0f;
+            if constexpr (COMP)
+                node_update_comp<TAPE, EXACT, SQ>(to, tol, tv, tvl, te, tel, tev, tevl, s1a, s1b, s2a, s2b, sref,
+                                                  a.kc, dr1, dc1a, dc2, dr2a, tnew, tnewl, rec[u]);
+            else
+                tnew = node_update<TAPE, REF, EXACT, SQ>(to, tv, te, tev, s1a, s1b, s2a, s2b, sref, a.kc,
+                                                         dr1, dc1a, dc2, dr2a, rec[u]);
+            tnw[u] = inner ? tnew : to;
+            tnwl[u] = COMP ? (inner ? tnewl : tol) : 0.0f;
+            if (TAPE) {
+                if (!inner) rec[u].code = 0;
+                sr[u] = sref;
+                any_far |= rec[u].code & 4;                         // 4, 5
+                any_far |= ((rec[u].code & 3) == 3);                // 3
             }
-            bad |= bad_u;
-            tnw[u] = tnew;
-            tnwl[u] = tnewl;
-            actv[u] = act;
             // carry state
             if (act) {
-                tn = tnew;
-                tnl = tnewl;
+                tn = tnw[u];
+                tnl = tnwl[u];
             }
             tvp = tv;
             tvpl = tvl;
             cU = nU[u];
             cI = nI[u];
         }
-        return bad;
-        };
-        {
-            const float tn0 = tn, tvp0 = tvp, cU0 = cU, cI0 = cI, tnl0 = tnl, tvpl0 = tvpl;
-            // a quotient outside the range the fast division was verified on
-            // (one vote per block): the block again with IEEE division
-            if (__any_sync(0xffffffffu, updates(std::false_type{}))) {
-                tn = tn0;
-                tvp = tvp0;
-                tnl = tnl0;
-                tvpl = tvpl0;
-                cU = cU0;
-                cI = cI0;
-                updates(std::true_type{});
-            }
-        }
 
+        if constexpr (TAPE) {
+            float c1[U], c2[U];
+            if (__any_sync(0xffffffffu, any_far)) {
+                bool ok = true;
 #pragma unroll
-        for (int u = 0; u < kU; u++) {
-            const int s = s0 + u;
-            if (actv[u]) {
-                Tring[msl[u] * kTP + tix] = tnw[u];
-                if (COMP) Lring[msl[u] * kTP + tix] = tnwl[u];
+                for (int u = 0; u < U; u++) ok &= node_record<EXACT, SQ>(rec[u], sr[u], a.kc, c1[u], c2[u]);
+                if (!EXACT && !ok) {
+#pragma unroll
+                    for (int u = 0; u < U; u++) node_record<true, SQ>(rec[u], sr[u], a.kc, c1[u], c2[u]);
+                }
+            } else {
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    c1[u] = 0.0f;
+                    c2[u] = (rec[u].code == 0) ? 0.0f : ((rec[u].code & 1) ? a.kc.dz : a.kc.dx);
+                }
             }
-            if (TAPE && (FAST || s < nsteps)) {
-                pcode[32 * u] = actv[u] ? rec[u].code : (uint8_t)0;
-                pc1[32 * u] = rec[u].c1;
-                pc2[32 * u] = rec[u].c2;
+#pragma unroll
+            for (int u = 0; u < U; u++)
+                if (FAST || s0 + u < nsteps) {
+                    pcode[32 * u] = (uint8_t)rec[u].code;
+                    pc1[32 * u] = c1[u];
+                    pc2[32 * u] = c2[u];
+                }
+            pcode += 32 * U;
+            pc1 += 32 * U;
+            pc2 += 32 * U;
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int m = s0 + u - lane;
+            const bool act = FAST || (vrow && (m >= 0) && (m < ncols));
+            if (act) {
+                ring[off[u] + kT0] = tnw[u];
+                if (COMP) ring[off[u] + kL0] = tnwl[u];
             }
             // feed the next strip: lane 31 just finished march s-31
-            if (lane == 31 && a.h_out != nullptr && actv[u]) {
-                st_u64(a.h_out + HS * (s - 31), pack_tag(tnw[u], a.tag));
-                if (COMP) st_u64(a.h_out + HS * (s - 31) + 1, pack_tag(tnwl[u], a.tag));
+            if (feeds && act) {
+                st_u64(pH + HS * u, pack_tag(tnw[u], a.tag));
+                if (COMP) st_u64(pH + HS * u + 1, pack_tag(tnwl[u], a.tag));
             }
         }
-        if (TAPE) {
-            pcode += 32 * kU;
-            pc1 += 32 * kU;
-            pc2 += 32 * kU;
-        }
+        pH += HS * U;
         // write back the columns every lane has finished (march s-31)
-        int wb = b0 + (kRing - 31);
-        if (wb >= kRing) wb -= kRing;
+        int wb = b0 + (RING - 31);
+        if (wb >= RING) wb -= RING;
 #pragma unroll
-        for (int u = 0; u < kU; u++) {
+        for (int u = 0; u < U; u++) {
             const int s = s0 + u;
             if (FAST || (s >= 31 && s < nsteps)) {
                 int ws = wb + u;
-                if (ws >= kRing) ws -= kRing;
+                if (ws >= RING) ws -= RING;
                 if (vrow) {
-                    *pW = Tring[ws * kTP + tix];
-                    if (COMP) *pWl = Lring[ws * kTP + tix];
+                    *pW = ring[ws * P + kT0 + tix];
+                    if (COMP) *pWl = ring[ws * P + kL0 + tix];
                 }
                 pW += dT;
                 if (COMP) pWl += dT;
             }
         }
-        b0 += kU;
-        if (b0 >= kRing) b0 -= kRing;
+        b0 += U;
+        if (b0 >= RING) b0 -= RING;
+        if (a.publish && (s0 + U) % kPublish == 0 && s0 + U > 31) publish_progress(a.prog_out, a.tag, min(s0 + U - 31, ncols));
     };
 #pragma unroll 1
-    for (int s0 = 0; s0 < nsteps; s0 += kU) {
+    for (int s0 = 0; s0 < nsteps; s0 += U) {
         if constexpr (INTERIOR) {
-            if (s0 >= 32 && s0 + kLook + kU <= ncols - 1)
+            if (s0 >= 33 && s0 + LOOK + U <= ncols - 1 && (unsigned)(s0 - g0) > (unsigned)gn)
                 block(s0, std::true_type{});
             else
                 block(s0, std::false_type{});
@@ -501,6 +635,7 @@ __device__ __forceinline__ void run_strip(const StripArgs& a)
             block(s0, std::false_type{});
         }
     }
+    if (a.prog_out) publish_progress(a.prog_out, a.tag, ncols);
     cp_wait<0>();
     __syncwarp();
 }

@@ -174,6 +174,8 @@ extern "C" int sf_update_slowness(sf_ctx* c, const float* grad, int grad_mem, fl
     }
     k_add_interior<<<grid, 256, 0, st>>>(c->d_S, c->nx, c->nz, c->nb, c->nzz, d_dS);
     CK(cudaGetLastError());
+    rc = sf_check_slowness(c, st);
+    if (rc) return rc;
     if (dS) CK(cudaMemcpyAsync(dS, d_dS, np * sizeof(float),
                                dS_mem == SF_MEM_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));  // the slowness is read by calls on any stream

@@ -185,7 +185,7 @@ int sf_adj_configure(sf_ctx* c, cudaStream_t st, AdjLaunch* A)
     if (rc) return rc;
     rc = sf_dev_reserve(c, (void**)&c->d_lam, &c->cap_lam, (size_t)NG * c->nzz * c->batch_maxcols * sizeof(float));
     if (!rc) rc = sf_dev_reserve_zero(c, (void**)&c->d_hand2, &c->cap_hand2,
-                                      (size_t)NG * 4 * nstrips * c->batch_maxcols * 2 * sizeof(unsigned long long));
+                                      (size_t)NG * hand_words(nstrips, c->batch_maxcols, 2) * sizeof(unsigned long long));
     if (!rc) rc = sf_dev_reserve(c, (void**)&c->d_lam_init, &c->cap_lam_init, (size_t)ns * 9 * sizeof(float));
     const size_t nctr = (size_t)NG;
     if (!rc) rc = sf_dev_reserve(c, (void**)&c->d_ctr2, &c->cap_ctr2, nctr * sizeof(unsigned));
@@ -259,7 +259,7 @@ int sf_adj_configure(sf_ctx* c, cudaStream_t st, AdjLaunch* A)
     A->block = dim3(c->warps * 32);
     A->smem = smem;
     A->nctr = nctr;
-    A->hand_bytes = (size_t)NG * 4 * nstrips * c->batch_maxcols * 2 * sizeof(unsigned long long);
+    A->hand_bytes = (size_t)NG * hand_words(nstrips, c->batch_maxcols, 2) * sizeof(unsigned long long);
     A->ggrid = dim3((unsigned)(nstrips * ((c->nxx + kGT - 1) / kGT)));
     A->gblock = dim3(256);
     // The gather inside the reverse-sweep launch (isotropic batches, 2 or 4

@@ -18,7 +18,14 @@
 // summed by their sender), the lane's own previous pe is kept in a register.
 // The tape was written in the forward strip's skewed step order, which makes
 // the reverse read of one step 32 consecutive entries (lane l of the reverse
-// march is lane 31-l of the forward one).
+// march is lane 31-l of the forward one), and of a block of four steps one
+// contiguous run. The reverse sweeps overlap in pairs as the forward's do.
+//
+// A step is a handful of multiply-adds on a short chain (one shfl, four
+// dependent operations), so its cost is its instruction stream: the block's
+// tape rows come in by three 16-byte copies per lane, the pushes are mu times
+// three coefficients selected from the code without branches, and the pair
+// for the next strip is one 16-byte store.
 //
 // The node terms v overwrite the tape's c2; the gradient gather (gather_tile)
 // sums them per slowness cell, either in its own launch (k_gather) or inside
@@ -31,22 +38,29 @@
 namespace sf {
 
 constexpr int kGT = 32;    // gather tile columns (the column blocks of the gradient gather)
-constexpr int kLP = 36;    // lambda slot pitch: 32 rows, then the {pv,tag},{pev,tag} handoff pairs
-// The reverse sweeps stage 4 columns ahead (one block): their tape rows come
-// from DRAM, but a shorter lead keeps consecutive strips closer together,
-// which measured faster than 8 or 12.
-constexpr int kLookA = 4;
-constexpr int kAheadA = kLookA + kU;  // a consumer's fall-back distance after a stall
-constexpr int kTR = 12;    // tape ring slots (a multiple of kU, > kLookA + kU)
-constexpr int kTPitch = 72;  // c1[32], c2[32], code bytes (8 words)
-// the prefetch slots b0 + kLookA + u and tb0 + kLookA + u are wrapped once:
-// blocks must tile the lead and both rings
-static_assert(kLookA % kU == 0 && kRing % kU == 0 && kTR % kU == 0, "ring slots of a block would wrap twice");
-static_assert(kTR >= kLookA + kU && kRing >= 32 + kLookA + kU, "ring too small for the lead");
+// Strip loop of the reverse sweeps: steps per block, staging leads of the
+// columns with their tape rows and of the upwind strip's pairs, ring lengths
+// (columns; blocks of tape rows; pairs). A block's prefetches never refill a
+// slot that this block or the one before it reads.
+constexpr int kU = 4;
+constexpr int kLookA = 12;
+constexpr int kPairLookA = 8;
+constexpr int kAheadA = kPairLookA + kU;  // a consumer's fall-back distance after a stall
+constexpr int kRingA = 52;
+constexpr int kTapeBlocks = kLookA / kU + 2;
+constexpr int kPairsA = 16;
+static_assert(kLookA % kU == 0 && kPairLookA % kU == 0 && kPairLookA <= kLookA && kRingA % kU == 0 &&
+              kRingA >= 31 + kLookA + 2 * kU && kPairsA >= kPairLookA + kU && kPairsA % kU == 0, "adjoint rings too small");
+static_assert(kU == 4, "a block's tape rows are one 16-byte copy per lane");
 
-struct AdjRing {
-    float L[kRing * kLP];
-    float TP[kTR * kTPitch];
+struct AdjTape {
+    float c1[kU * 32], c2[kU * 32];
+    uint8_t code[kU * 32];
+};
+struct __align__(16) AdjRing {
+    float L[kRingA * 32];             // lambda, one column of the strip's rows per slot
+    AdjTape tape[kTapeBlocks];        // forward step order: row U-1-u is the block's step u
+    uint4 pair[kPairsA];              // {pv, tag, pev, tag} of march q at q mod kPairsA
 };
 
 struct AdjStripArgs {
@@ -60,6 +74,11 @@ struct AdjStripArgs {
     const unsigned long long* h_in;  // {pv,tag},{pev,tag} of the upwind strip's row (nullptr: first strip)
     unsigned long long* h_out;       // pairs this strip feeds to the next one (nullptr: last strip)
     unsigned tag;
+    // columns of the strip finished by the reverse sweep before this one, and by this one (see StripArgs)
+    const unsigned long long* prog_in;
+    bool follow;
+    unsigned long long* prog_out;
+    bool publish;
     int* err;
     // last reverse sweep inside a fused launch: count each column block of
     // kGT padded columns once all lanes have finished its columns
@@ -80,186 +99,192 @@ __device__ __forceinline__ void adj_strip(const AdjStripArgs& a)
     const bool vrow = r < nzz;
     const int tix = r - rb;
     const int flane = 31 - lane;  // this row's lane in the forward strip
-    float* Lr = a.ring->L;
-    float* TPr = a.ring->TP;
-    float* lamg = a.lam;
+    AdjRing& R = *a.ring;
     const bool lt_ok = (rb + lane) < nzz;
     CtaShared* sh = a.sh;
-    const bool consumer = (lane == 0) && (a.h_in != nullptr);
+    const bool consumer = a.h_in != nullptr;
+    const bool lane0 = lane == 0;
+    const bool feeds = (lane == 31) && (a.h_out != nullptr);
     const int nsteps = ncols + 31;
     auto col_of = [&](int m) { return (SX < 0) ? m : ncols - 1 - m; };
-    // march q reads lambda column col_of(q), the pairs of march q and forward
-    // tape step ncols+30-q; the pointers below stand at the block's first
-    // march and move once per block, the steps inside a block are offsets
     const long long dL = (SX < 0) ? (long long)nzz : -(long long)nzz;
-    const float* pL = lamg + (size_t)(rb + lane) + (long long)col_of(0) * (long long)nzz;
-    const unsigned long long* pH = a.h_in;
-    const size_t fs0 = (size_t)(ncols + 30) * 32;
-    const float* pT1 = a.tc1 + fs0 + lane;
-    const float* pT2 = a.tc2 + fs0 + lane;
-    const uint8_t* pTc = a.tcode + fs0 + 4 * lane;
+    const float* pL = a.lam + (long long)(rb + lane) + (long long)col_of(0) * (long long)nzz;
+    // the lane's 16 bytes of a block's tape rows (rows of steps q+U-1 .. q, forward step order)
+    const long long fs0 = (long long)(ncols + 31 - kU) * 32;
+    const float* pT1 = a.tc1 + fs0 + 4 * lane;
+    const float* pT2 = a.tc2 + fs0 + 4 * lane;
+    const uint8_t* pTc = a.tcode + fs0 + 16 * lane;
+    // marches q .. q+U-1: columns into slots from `slot`, tape rows into block slot tb
     // FAST: every march of the call is inside the window (no bounds tests)
-    auto prefetch = [&](int q, int u, int lslot, int tslot, auto fast_tag) {
+    auto stage = [&](int q, int slot, int tb, auto fast_tag) {
         constexpr bool FAST = decltype(fast_tag)::value;
-        if (FAST || q < ncols) {
-            if (lt_ok) cp_async4(&Lr[lslot * kLP + lane], pL + u * dL);
-            if (consumer) cp_async16(&Lr[lslot * kLP + 32], pH + 2 * u);
+        float* d = &R.L[slot * 32 + lane];
+#pragma unroll
+        for (int u = 0; u < kU; u++) {
+            if ((FAST || q + u < ncols) && lt_ok) cp_async4(d + 32 * u, pL);
+            pL += dL;
         }
-        if (FAST || q < nsteps) {
-            cp_async4(&TPr[tslot * kTPitch + lane], pT1 - 32 * u);
-            cp_async4(&TPr[tslot * kTPitch + 32 + lane], pT2 - 32 * u);
-            if (lane < 8) cp_async4(&TPr[tslot * kTPitch + 64 + lane], pTc - 32 * u);
+        AdjTape& t = R.tape[tb];
+        if (FAST || q + kU - 1 - (lane >> 3) < nsteps) {
+            cp_async16_cg(&t.c1[4 * lane], pT1);
+            cp_async16_cg(&t.c2[4 * lane], pT2);
         }
-        cp_commit();
+        if (lane < 8 && (FAST || q + kU - 1 - (lane >> 1) < nsteps)) cp_async16_cg(&t.code[16 * lane], pTc);
+        pT1 -= 32 * kU;
+        pT2 -= 32 * kU;
+        pTc -= 32 * kU;
     };
-    auto advance = [&](int n) {
-        pL += n * dL;
-        pH += 2 * n;
-        pT1 -= 32 * n;
-        pT2 -= 32 * n;
-        pTc -= 32 * n;
+    auto stage_pairs = [&](int q, auto fast_tag) {
+        constexpr bool FAST = decltype(fast_tag)::value;
+        if (consumer && lane < kU && (FAST || q + lane < ncols))
+            cp_async16_cg(&R.pair[(q + lane) % kPairsA], a.h_in + 2 * (size_t)(q + lane));
     };
-
-    // let the previous strip get kAheadA columns ahead before the first prefetches
-    if (consumer) wait_pair(a.h_in + 2 * (size_t)min(kAheadA, ncols - 1) + 1, a.tag, sh, a.err);
-    __syncwarp();
+    int avail = a.prog_in ? 0 : 0x7fffffff;
+    auto ensure = [&](int q) {  // marches below q may be staged
+        if (q > avail) {
+            avail = wait_progress(a.prog_in, a.tag, a.follow ? min(q, ncols) : ncols, sh, a.err);
+            if (avail >= ncols) avail = 0x7fffffff;
+        }
+    };
+    // rows past the grid read zeros (their pushes stay zero)
+    if (!vrow)
+        for (int q = 0; q < kRingA; q++) R.L[q * 32 + tix] = 0.0f;
+    ensure(kLookA);
 #pragma unroll 1
-    for (int q = 0; q < kLookA; q++) {
-        prefetch(q, 0, q, q % kTR, std::false_type{});
-        advance(1);
+    for (int q = 0; q < kLookA; q += kU) {
+        stage(q, q, q / kU, std::false_type{});
+        // let the previous strip get kAheadA columns ahead before the first pairs
+        if (q == 0 && consumer && lane0) wait_pair(a.h_in + 2 * (size_t)min(kAheadA, ncols - 1) + 1, a.tag, sh, a.err);
+        __syncwarp();
+        if (q < kPairLookA) stage_pairs(q, std::false_type{});
+        cp_commit();
     }
 
-    // running destinations: the term v of forward tape step ncols+30-s, and
-    // the write-back of march column s-31 (row r)
-    float* pV = a.tc2 + fs0 + flane;
-    float* pW = lamg + (size_t)r + (long long)col_of(0) * (long long)nzz;
+    // running destinations: the term v of forward tape step ncols+30-s, the
+    // write-back of march column s-31 (row r), the pair of march s-31
+    float* pV = a.tc2 + (long long)(ncols + 30) * 32 + flane;
+    float* pW = a.lam + (long long)r + (long long)col_of(0) * (long long)nzz;
+    unsigned long long* pH = a.h_out - 2 * 31;
 
     float my_x = 0.0f, my_pe = 0.0f, my_pev = 0.0f, pev_hold = 0.0f;
-    int b0 = 0, tb0 = 0;  // ring slots of march s0 (lambda, tape)
+    int b0 = 0, tb0 = 0;  // ring slots of march s0 (lambda) and of the block's tape rows
+    int ro = ((kRingA - lane) % kRingA) * 32 + tix;
 
     // Blocks of kU steps, as in the forward: one wait per block, the block's
     // ring reads, its kU linear updates (the only serial chain), its stores.
     auto block = [&](int s0, auto fast_tag) {
         constexpr bool FAST = decltype(fast_tag)::value;
+        ensure(s0 + kLookA + kU);
         {
             int pf0 = b0 + kLookA;
-            if (pf0 >= kRing) pf0 -= kRing;
-            int tf0 = tb0 + kLookA;
-            if (tf0 >= kTR) tf0 -= kTR;
-#pragma unroll
-            for (int u = 0; u < kU; u++) prefetch(s0 + kLookA + u, u, pf0 + u, tf0 + u, fast_tag);
-            advance(kU);
+            if (pf0 >= kRingA) pf0 -= kRingA;
+            int tf0 = tb0 + kLookA / kU;
+            if (tf0 >= kTapeBlocks) tf0 -= kTapeBlocks;
+            stage(s0 + kLookA, pf0, tf0, fast_tag);
+            stage_pairs(s0 + kPairLookA, fast_tag);
+            cp_commit();
         }
-        cp_wait<kLookA>();
+        cp_wait<(kLookA < kPairLookA ? kLookA : kPairLookA) / kU>();
         __syncwarp();
 
-        int ml = b0 - lane;  // slot of march s0 - lane
-        if (ml < 0) ml += kRing;
-        int msl[kU], code[kU];
-        float lam_in[kU], c1[kU], c2[kU];
-        unsigned long long e0[kU], e1[kU];
+        const AdjTape& t = R.tape[tb0];
+        int off[kU], br[kU];
+        float lam_in[kU], c2[kU], av[kU], ae[kU], aev[kU], hx[kU];
 #pragma unroll
         for (int u = 0; u < kU; u++) {
-            int ms = ml + u;
-            if (ms >= kRing) ms -= kRing;
-            msl[u] = ms;
-            lam_in[u] = Lr[ms * kLP + tix];
-            const int ts = tb0 + u;
-            c1[u] = TPr[ts * kTPitch + flane];
-            c2[u] = TPr[ts * kTPitch + 32 + flane];
-            code[u] = reinterpret_cast<const uint8_t*>(&TPr[ts * kTPitch + 64])[flane];
-            if (consumer) {
-                const unsigned long long* e = reinterpret_cast<const unsigned long long*>(&Lr[ms * kLP + 32]);
-                e0[u] = e[0];
-                e1[u] = e[1];
-            } else {
-                e0[u] = e1[u] = 0ull;
-            }
+            off[u] = ro;
+            ro += 32;
+            if (ro >= kRingA * 32 + tix) ro -= kRingA * 32;
+            lam_in[u] = R.L[off[u]];
+            const int e = (kU - 1 - u) * 32 + flane;
+            const float c = t.c1[e], cm = fsub(1.0f, c);
+            c2[u] = t.c2[e];
+            br[u] = t.code[e] & 7;
+            // dT/d{tv, te, tev} of the candidate: (1,0,0), (0,1,0), (c,-c,1), (0,1-c,c), (1-c,0,c)
+            av[u] = (br[u] == 1) ? 1.0f : (br[u] == 3) ? c : (br[u] >= 5) ? cm : 0.0f;
+            ae[u] = (br[u] == 2) ? 1.0f : (br[u] == 3) ? -c : (br[u] == 4) ? cm : 0.0f;
+            aev[u] = (br[u] == 3) ? 1.0f : (br[u] >= 4) ? c : 0.0f;
         }
-        if (consumer) {
-            // pairs the previous strip had not written when they were prefetched:
-            // wait for them, then fall kAheadA columns behind so later prefetches hit
+        {
+            // the upwind row of lane 0: the previous strip's pairs, or nothing
+            // (every lane reads them, lane 0 uses them)
+            uint4 e[kU];
+            unsigned stale = 0;
 #pragma unroll
             for (int u = 0; u < kU; u++) {
-                const int s = s0 + u;
-                if ((FAST || s < ncols) && (tag_of(e0[u]) != a.tag || tag_of(e1[u]) != a.tag)) {
-                    e0[u] = pack_tag(wait_pair(a.h_in + 2 * (size_t)s, a.tag, sh, a.err), a.tag);
-                    e1[u] = pack_tag(wait_pair(a.h_in + 2 * (size_t)s + 1, a.tag, sh, a.err), a.tag);
-                    wait_pair(a.h_in + 2 * (size_t)min(s + kAheadA, ncols - 1) + 1, a.tag, sh, a.err);
+                e[u] = R.pair[(s0 + u) % kPairsA];
+                if (FAST || s0 + u < ncols) stale |= (e[u].y ^ a.tag) | (e[u].w ^ a.tag);
+            }
+            if (consumer && stale != 0) {
+                // pairs the previous strip had not written when they were prefetched:
+                // wait for them, then fall kAheadA columns behind so later prefetches hit
+                if (lane0) {
+#pragma unroll
+                    for (int u = 0; u < kU; u++)
+                        if (FAST || s0 + u < ncols) {
+                            e[u].x = __float_as_uint(wait_pair(a.h_in + 2 * (size_t)(s0 + u), a.tag, sh, a.err));
+                            e[u].z = __float_as_uint(wait_pair(a.h_in + 2 * (size_t)(s0 + u) + 1, a.tag, sh, a.err));
+                        }
+                    wait_pair(a.h_in + 2 * (size_t)min(s0 + kU - 1 + kAheadA, ncols - 1) + 1, a.tag, sh, a.err);
                 }
+                __syncwarp();
+            }
+#pragma unroll
+            for (int u = 0; u < kU; u++) {
+                const bool have = consumer && (FAST || s0 + u < ncols);
+                hx[u] = fadd(have ? __uint_as_float(e[u].x) : 0.0f, pev_hold);
+                pev_hold = have ? __uint_as_float(e[u].z) : 0.0f;
             }
         }
 
         float lo[kU], vv[kU], opv[kU], opev[kU];
-        bool actv[kU];
 #pragma unroll
         for (int u = 0; u < kU; u++) {
-            const int s = s0 + u;
-            const int m = s - lane;
-            const bool act = FAST ? vrow : (vrow && (m >= 0) && (m < ncols));
+            const int m = s0 + u - lane;
             // pv of the upwind row's node in this column plus pev of its node in
             // the previous column, summed by the lane above
-            float x_in = __shfl_up_sync(0xffffffffu, my_x, 1);
-            if (lane == 0) {  // upwind row of the strip: the previous strip, or outside the grid
-                const bool have = consumer && (FAST || s < ncols);
-                x_in = fadd(have ? val_of(e0[u]) : 0.0f, pev_hold);
-                pev_hold = have ? val_of(e1[u]) : 0.0f;
-            }
-            const float mu = fadd(fadd(lam_in[u], x_in), my_pe);
-            float npv = 0.0f, npe = 0.0f, npev = 0.0f, l = mu, v = 0.0f;
-            const int br = code[u] & 7;
-            if (act && br != 0) {
-                l = 0.0f;
-                v = fmul(mu, c2[u]);
-                const float cc = c1[u];
-                switch (br) {
-                case 1: npv = mu; break;
-                case 2: npe = mu; break;
-                case 3: npv = fmul(mu, cc); npe = fmul(mu, -cc); npev = mu; break;
-                case 4: npe = fmul(mu, fsub(1.0f, cc)); npev = fmul(mu, cc); break;
-                default: npv = fmul(mu, fsub(1.0f, cc)); npev = fmul(mu, cc); break;
-                }
-            }
-            lo[u] = l;
-            vv[u] = v;
-            opv[u] = npv;
-            opev[u] = npev;
-            actv[u] = act;
-            my_x = fadd(npv, my_pev);  // this node's pv + the previous node's pev
-            my_pe = npe;
-            my_pev = npev;
+            const float x_up = __shfl_up_sync(0xffffffffu, my_x, 1);
+            float mu = fadd(fadd(lam_in[u], lane0 ? hx[u] : x_up), my_pe);
+            if (!FAST && !(vrow && (m >= 0) && (m < ncols))) mu = 0.0f;
+            lo[u] = br[u] ? 0.0f : mu;
+            vv[u] = fmul(mu, c2[u]);
+            opv[u] = fmul(mu, av[u]);
+            opev[u] = fmul(mu, aev[u]);
+            my_x = fadd(opv[u], my_pev);  // this node's pv + the previous node's pev
+            my_pe = fmul(mu, ae[u]);
+            my_pev = opev[u];
         }
 
 #pragma unroll
         for (int u = 0; u < kU; u++) {
-            const int s = s0 + u;
-            if (actv[u]) {
-                Lr[msl[u] * kLP + tix] = lo[u];
+            const int m = s0 + u - lane;
+            if (FAST ? vrow : (vrow && (m >= 0) && (m < ncols))) {
+                R.L[off[u]] = lo[u];
                 pV[-32 * u] = vv[u];
-                if (lane == 31 && a.h_out != nullptr) {
-                    const int m = s - 31;
-                    st_u64(a.h_out + 2 * (size_t)m, pack_tag(opv[u], a.tag));
-                    st_u64(a.h_out + 2 * (size_t)m + 1, pack_tag(opev[u], a.tag));
-                }
+                if (feeds)
+                    asm volatile("st.global.v4.u32 [%0], {%1, %2, %3, %2};" ::"l"(pH + 2 * u), "r"(__float_as_uint(opv[u])),
+                                 "r"(a.tag), "r"(__float_as_uint(opev[u])) : "memory");
             }
         }
         pV -= 32 * kU;
-        int wb = b0 + (kRing - 31);  // slot of march s0 - 31
-        if (wb >= kRing) wb -= kRing;
+        pH += 2 * kU;
+        int wb = b0 + (kRingA - 31);  // slot of march s0 - 31
+        if (wb >= kRingA) wb -= kRingA;
 #pragma unroll
         for (int u = 0; u < kU; u++) {
             const int s = s0 + u;
             if (FAST || (s >= 31 && s < nsteps)) {
                 int ws = wb + u;
-                if (ws >= kRing) ws -= kRing;
-                if (vrow) *pW = Lr[ws * kLP + tix];
+                if (ws >= kRingA) ws -= kRingA;
+                if (vrow) *pW = R.L[ws * 32 + tix];
                 pW += dL;
             }
         }
         b0 += kU;
-        if (b0 >= kRing) b0 -= kRing;
-        tb0 += kU;
-        if (tb0 >= kTR) tb0 -= kTR;
+        if (b0 >= kRingA) b0 -= kRingA;
+        if (++tb0 >= kTapeBlocks) tb0 = 0;
+        if (a.publish && (s0 + kU) % kPublish == 0 && s0 + kU > 31)
+            publish_progress(a.prog_out, a.tag, min(s0 + kU - 31, ncols));
     };
     // column blocks in the order the march finishes them: the counted sweep
     // is the reverse of sweep 0 (SX > 0), which marches down the columns, so
@@ -290,6 +315,7 @@ __device__ __forceinline__ void adj_strip(const AdjStripArgs& a)
         }
         if (a.ready) count_done(s0 + kU - 1);
     }
+    if (a.prog_out) publish_progress(a.prog_out, a.tag, ncols);
     cp_wait<0>();
     __syncwarp();
 }
@@ -309,7 +335,9 @@ __device__ void adjoint_body(const AdjParams& p, const FuseParams* f)
     const GangPos gp = gang_pos(p.G);
     const int nzz = p.nzz, nstrips = p.nstrips;
     float* lam = p.lam + (size_t)gp.gang * p.lam_per_gang;
-    unsigned long long* hb = p.hand + (size_t)gp.gang * 4 * nstrips * 2 * p.maxcols;
+    const size_t row = 2 * (size_t)hand_pitch(p.maxcols);
+    unsigned long long* hb = p.hand + (size_t)gp.gang * hand_words(nstrips, p.maxcols, 2);
+    unsigned long long* prog = hb + 4 * (size_t)nstrips * row;
     unsigned* bar = p.bar + gp.gang;
     unsigned nbar = 0;
     if (tid == 0) {
@@ -351,8 +379,9 @@ __device__ void adjoint_body(const AdjParams& p, const FuseParams* f)
             }
         }
         gang_barrier(bar, (++nbar) * p.G, cs, p.err);
-        // reverse sweeps 3, 2, 1, 0 (consecutive ones run the rows in opposite
-        // directions: no barrier between them, as in the forward)
+        // reverse sweeps 3, 2, 1, 0 as one list of strip tasks dealt to the
+        // warps in turn (see solve_window): 3 and 2 march to the right, 1 and 0
+        // to the left; 3 and 1 take the strips top to bottom, 2 and 0 upwards
         AdjStripArgs a;
         a.lam = lam;
         a.nzz = nzz;
@@ -361,30 +390,28 @@ __device__ void adjoint_body(const AdjParams& p, const FuseParams* f)
         a.sh = cs;
         a.err = p.err;
         a.tag = tag;
+        a.c0 = sh.c0;
 #pragma unroll 1
-        for (int sw = 3; sw >= 0; sw--) {
-            const bool fz_pos = !(sw == 1 || sw == 3);  // forward SZ > 0: reverse march goes up
-            unsigned long long* hs = hb + (size_t)sw * nstrips * 2 * p.maxcols;
-            // strips have a fixed owner (strip k -> slot k mod slots) in every sweep;
-            // processing index pidx runs along the reverse march
-            const int first = fz_pos ? ((nstrips - 1 - gp.slot) % gp.slots + gp.slots) % gp.slots : gp.slot;
-#pragma unroll 1
-            for (int pidx = first; pidx < nstrips; pidx += gp.slots) {
-                a.k = fz_pos ? nstrips - 1 - pidx : pidx;
-                a.h_in = (pidx > 0) ? hs + 2 * (size_t)pidx * p.maxcols : nullptr;
-                a.h_out = (pidx < nstrips - 1) ? hs + 2 * (size_t)(pidx + 1) * p.maxcols : nullptr;
-                const size_t tb = tape_strip_base(sh.tape_off, sw, a.k, nstrips, ncols);
-                a.tcode = p.tcode + tb;
-                a.tc1 = p.tc1 + tb;
-                a.tc2 = p.tc2 + tb;
-                a.ready = (f && sw == 0) ? f->ready + (size_t)a.k * f->nblk : nullptr;
-                a.c0 = sh.c0;
-                switch (sw) {
-                case 0: adj_strip<1, 1, INTERIOR>(a); break;
-                case 1: adj_strip<-1, 1, INTERIOR>(a); break;
-                case 2: adj_strip<1, -1, INTERIOR>(a); break;
-                default: adj_strip<-1, -1, INTERIOR>(a); break;
-                }
+        for (int task = gp.slot; task < 4 * nstrips; task += gp.slots) {
+            const int rs = task / nstrips, pidx = task - rs * nstrips, sw = 3 - rs;
+            a.k = (rs & 1) ? nstrips - 1 - pidx : pidx;
+            unsigned long long* hs = hb + ((size_t)rs * nstrips + pidx) * row;
+            a.h_in = (pidx > 0) ? hs : nullptr;
+            a.h_out = (pidx < nstrips - 1) ? hs + row : nullptr;
+            a.prog_in = (rs > 0) ? prog + (size_t)(rs - 1) * nstrips + a.k : nullptr;
+            a.follow = rs & 1;
+            a.prog_out = (rs < 3) ? prog + (size_t)rs * nstrips + a.k : nullptr;
+            a.publish = !(rs & 1);
+            const size_t tb = tape_strip_base(sh.tape_off, sw, a.k, nstrips, ncols);
+            a.tcode = p.tcode + tb;
+            a.tc1 = p.tc1 + tb;
+            a.tc2 = p.tc2 + tb;
+            a.ready = (f && sw == 0) ? f->ready + (size_t)a.k * f->nblk : nullptr;
+            switch (sw) {
+            case 0: adj_strip<1, 1, INTERIOR>(a); break;
+            case 1: adj_strip<-1, 1, INTERIOR>(a); break;
+            case 2: adj_strip<1, -1, INTERIOR>(a); break;
+            default: adj_strip<-1, -1, INTERIOR>(a); break;
             }
         }
         gang_barrier(bar, (++nbar) * p.G, cs, p.err);

@@ -13,7 +13,7 @@ struct AdjParams {
     int G, NG, maxcols;     // gangs as in the forward
     float* lam;             // per-gang window adjoint, lam + gang * lam_per_gang
     long long lam_per_gang;
-    unsigned long long* hand;  // per gang [4][nstrips][2 * maxcols] tagged (pv, pev) pairs
+    unsigned long long* hand;  // per gang (hand_words, two pairs per column): tagged (pv, pev) pairs, then progress words
     unsigned* bar;          // per gang barrier counter
     unsigned epoch;         // launch number (tags)
     unsigned long long wait_ns;  // time limit of the bounded waits

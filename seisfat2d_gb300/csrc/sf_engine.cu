@@ -408,25 +408,15 @@ const void* sf_kqp_kernel(bool ref, bool comp, bool fact)
     return fact ? (const void*)k_qp<false, false, true> : (const void*)k_qp<false, false, false>;
 }
 
-// The interior-block body saves instructions per step but adds code. It
-// measured faster for 100 equal windows of 1707 x 357 with every shot at once
-// and one warp per strip (forward 3.93 -> 3.58 ms, reverse sweeps 6.66 ->
-// 5.46 ms), and slower for 1000 windows of 2-8 km with four strips per warp
-// (forward 46 -> 55 ms, reverse 46 -> 67 ms) and for 200 equal windows with
-// two strips per warp (9.39 -> 9.67 ms). SF_LOOP_AUTO takes it only when all
-// three conditions of the first case hold.
-bool sf_interior_loops(sf_ctx* c, const void* kernel, size_t smem, int G)
+// The interior-block body drops the bounds tests of the blocks whose marches
+// all lie inside the window; a narrow window has few of them and runs both
+// bodies. SF_LOOP_AUTO takes it when every window of the batch is at least
+// kInteriorCols wide.
+constexpr int kInteriorCols = 128;
+bool sf_interior_loops(const sf_ctx* c)
 {
-    if (c->strip_loop == SF_LOOP_GENERAL) return false;
-    if (c->strip_loop == SF_LOOP_INTERIOR) return true;
-    const int ns = (int)c->hshots.size();
-    if (ns == 0) return false;
-    if (c->hshots.front().ncols != c->hshots.back().ncols) return false;  // sorted widest first
-    if ((long long)G * c->warps < (c->nzz + 31) / 32) return false;       // a warp per strip
-    int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, c->warps * 32, smem) != cudaSuccess)
-        return false;
-    return (long long)ns * G <= (long long)per_sm * c->sms;
+    if (c->strip_loop != SF_LOOP_AUTO) return c->strip_loop == SF_LOOP_INTERIOR;
+    return !c->hshots.empty() && c->hshots.back().ncols >= kInteriorCols;  // sorted widest first
 }
 
 int sf_fwd_setup(sf_ctx* c)
@@ -676,27 +666,13 @@ int sf_fwd_configure(sf_ctx* c, int nrec, bool per_shot_T, bool tape, int gang_w
         return sf_fail(c, SF_ERR_ARG, "the compensated arithmetic runs at most 8 warps per CTA (sf_set_launch)");
     const bool ref = c->arith == SF_ARITH_REFERENCE;
     const size_t smem = sf_fwd_smem_bytes(c->warps, comp, tape);
-    const void* kern = sf_kshots_kernel(tape, ref, false, comp);
+    // the interior-block kernels of taped batches are built for at most
+    // kMaxWarpsTapedInterior warps per CTA
+    c->batch_interior = !(tape && c->warps > kMaxWarpsTapedInterior) && sf_interior_loops(c);
+    const void* kern = sf_kshots_kernel(tape, ref, c->batch_interior, comp);
     int G, NG;
     int rc = sf_gang_shape(c, kern, smem, nshots, nstrips, gang_warps, &G, &NG);
     if (rc) return rc;
-    // the interior-block kernels of taped batches are built for at most
-    // kMaxWarpsTapedInterior warps per CTA; the gang shape must come from the
-    // kernel that runs (every CTA of a gang resident at once)
-    c->batch_interior = !(tape && c->warps > kMaxWarpsTapedInterior) && sf_interior_loops(c, kern, smem, G);
-    if (c->batch_interior) {
-        const void* ik = sf_kshots_kernel(tape, ref, true, comp);
-        int Gi, NGi;
-        rc = sf_gang_shape(c, ik, smem, nshots, nstrips, gang_warps, &Gi, &NGi);
-        if (rc) return rc;
-        if (c->strip_loop == SF_LOOP_INTERIOR || sf_interior_loops(c, ik, smem, Gi)) {
-            kern = ik;
-            G = Gi;
-            NG = NGi;
-        } else {
-            c->batch_interior = false;
-        }
-    }
     if ((long long)(nshots + NG - 1) / NG > 1023)
         return sf_fail(c, SF_ERR_ARG, "too many shots per gang for one launch; split the batch");
     c->last_G = G;

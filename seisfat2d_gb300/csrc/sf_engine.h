@@ -181,8 +181,8 @@ size_t sf_fwd_smem_bytes(int warps, bool comp, bool tape);
 // k_shots instantiation (one object file each, sf_shots_inst.cu)
 const void* sf_kshots_kernel(bool tape, bool ref, bool interior, bool comp);
 const void* sf_kqp_kernel(bool ref, bool comp, bool fact);
-// whether the batch of hshots, G CTAs per shot, runs the interior-block body
-bool sf_interior_loops(sf_ctx* c, const void* kernel, size_t smem, int G);
+// whether the batch of hshots runs the interior-block body
+bool sf_interior_loops(const sf_ctx* c);
 void sf_skip_cells(int ncols, int nzz, int si[4], int sj[4]);
 int sf_prepare_shots(sf_ctx* c, const sf_shot* shots, int nshots, bool tape);
 int sf_launch_shots(sf_ctx* c, int ani, int nrec, float* d_picks, bool keep_tables, bool tape, int gang_warps,

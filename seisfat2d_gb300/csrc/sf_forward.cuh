@@ -188,9 +188,9 @@ __device__ void solve_window(const FwdParams& p, const ShotDev& sh, const GangPo
 // COMP: compensated arithmetic (node_update_comp; the 3x3 initial values are
 // the FP64 ones rounded once).
 template <bool TAPE, bool REF, bool INTERIOR, bool COMP = false>
-// (kMaxWarps * 32, 1): with the block size alone as the bound ptxas caps the
-// kernel at 64 registers and spills the strip loop's state to local memory.
-__global__ void __launch_bounds__((COMP ? kMaxWarpsComp : ((TAPE && INTERIOR) ? kMaxWarpsTapedInterior : kMaxWarps)) * 32, 1)
+// Register bounds: 168 keep three warps per scheduler (and 8 per CTA); the
+// plain FP32 kernels run CTAs of up to 16 warps, hence 128.
+__global__ void __maxnreg__((COMP || (TAPE && INTERIOR)) ? 168 : 128)
     k_shots(FwdParams p)
 {
     static_assert(!(COMP && REF), "the compensated arithmetic has no reference-build variant");

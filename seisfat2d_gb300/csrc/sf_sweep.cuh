@@ -46,9 +46,6 @@
 
 namespace sf {
 
-constexpr int kU = 4;       // march steps per block of the reverse sweeps' strip loop
-constexpr int kRing = 48;   // column slots per warp ring of the reverse sweeps
-
 // Block size U, staging leads (march columns, multiples of the block) of the
 // columns (LOOK) and of the upwind strip's pairs (PLOOK), and ring length of
 // a forward strip loop. After a stall a consumer lets its producer get AHEAD
@@ -389,16 +386,14 @@ __device__ __forceinline__ void run_strip(const StripArgs& a)
         }
     };
 
-    // let the previous strip get AHEAD columns ahead before the first
-    // prefetches of its values
-    if (consumer && lane0) wait_pair(a.h_in + HS * min(B::AHEAD, ncols - 1), a.tag_in, sh, a.err);
-    __syncwarp();
+    // prologue: march columns 0 .. LOOK-1, pairs 0 .. PLOOK-1; the previous
+    // strip gets AHEAD columns ahead before the first prefetches of its values
     ensure(LOOK);
-
-    // prologue: march columns 0 .. LOOK-1, pairs 0 .. PLOOK-1
 #pragma unroll 1
     for (int q = 0; q < LOOK; q += U) {
         stage_cols(q, q, std::false_type{});
+        if (q == 0 && consumer && lane0) wait_pair(a.h_in + HS * min(B::AHEAD, ncols - 1), a.tag_in, sh, a.err);
+        __syncwarp();
         if (q < PLOOK) stage_pairs(q, std::false_type{});
         cp_commit();
     }

@@ -187,7 +187,7 @@ int sf_adj_configure(sf_ctx* c, cudaStream_t st, AdjLaunch* A)
     if (!rc) rc = sf_dev_reserve_zero(c, (void**)&c->d_hand2, &c->cap_hand2,
                                       (size_t)NG * hand_words(nstrips, c->batch_maxcols, 2) * sizeof(unsigned long long));
     if (!rc) rc = sf_dev_reserve(c, (void**)&c->d_lam_init, &c->cap_lam_init, (size_t)ns * 9 * sizeof(float));
-    const size_t nctr = (size_t)NG;
+    const size_t nctr = gang_counters(NG);
     if (!rc) rc = sf_dev_reserve(c, (void**)&c->d_ctr2, &c->cap_ctr2, nctr * sizeof(unsigned));
     if (rc) return rc;
     rc = prepare_gather(c, st);

@@ -347,7 +347,7 @@ __device__ void adjoint_body(const AdjParams& p, const FuseParams* f)
     __syncthreads();
     int it = 0;
 #pragma unroll 1
-    for (int b = gp.gang; b < p.nshots; b += p.NG, it++) {
+    for (int b = gp.gang; b < p.nshots; it++) {
         const ShotDev sh = p.shots[b];
         const int ncols = sh.ncols;
         const unsigned tag = (p.epoch << 10) | (unsigned)(it & 1023);
@@ -425,7 +425,7 @@ __device__ void adjoint_body(const AdjParams& p, const FuseParams* f)
             __syncthreads();
             if (tid == 0) st_release_gpu(f->shot_done + sh.orig, f->done_tag);
         }
-        gang_barrier(bar, (++nbar) * p.G, cs, p.err);
+        b = next_shot(p.bar, p.NG, p.G, gp.gang, gp.g, it, nbar, cs, p.err);
     }
 }
 

@@ -14,7 +14,7 @@ struct AdjParams {
     float* lam;             // per-gang window adjoint, lam + gang * lam_per_gang
     long long lam_per_gang;
     unsigned long long* hand;  // per gang (hand_words, two pairs per column): tagged (pv, pev) pairs, then progress words
-    unsigned* bar;          // per gang barrier counter
+    unsigned* bar;          // gang_counters(NG), zeroed
     unsigned epoch;         // launch number (tags)
     unsigned long long wait_ns;  // time limit of the bounded waits
     uint8_t* tcode;

@@ -1,6 +1,5 @@
 // Whole-shot forward kernel: a gang of CTAs solves one shot window at a time
-// (init, 4 sweeps, receiver picks) and takes the shots k, k+NG, ... of its
-// gang. The same kernel with one shot and one CTA is the per-shot drop-in
+// (init, 4 sweeps, receiver picks) and takes the next shot of the queue. The same kernel with one shot and one CTA is the per-shot drop-in
 // solver. An anisotropic batch (eikonal_ani.cu:33-45) is three launches: the
 // solve of every shot on S, the qP pass over every shot's window (k_qp, a
 // map over cells), and the solve of every shot on its own qP slowness.
@@ -31,7 +30,7 @@ struct FwdParams {
     const ShotDev* shots;
     int nshots;
     int G;                // CTAs per gang (one gang solves one shot at a time)
-    int NG;               // gangs; gang k solves shots k, k+NG, ...
+    int NG;               // gangs; gang k solves shot k first, then takes shots from a queue
     int maxcols;          // widest window of the batch
     float* Tpool;
     float* Tlpool;        // compensated: lo parts of the traveltimes, same layout as Tpool
@@ -41,7 +40,7 @@ struct FwdParams {
     // [hand_pitch] (x2 compensated), then progress words [4 sweeps][nstrips]
     unsigned long long* hand;
     const int* srange;    // nonzero: the slowness has a value outside in_fast_range (per shot with Sshots)
-    unsigned* bar;        // per gang barrier counter
+    unsigned* bar;        // gang_counters(NG), zeroed
     unsigned epoch;       // launch number (tags: epoch << 10 | shot-solve number)
     unsigned long long wait_ns;  // time limit of the bounded waits
     int stall_handoff;    // test of the timeout path: consumers wait for a tag no producer writes
@@ -181,8 +180,8 @@ __device__ void solve_window(const FwdParams& p, const ShotDev& sh, const GangPo
     }
 }
 
-// Persistent gangs of G CTAs: gang k solves shots k, k+NG, ... (shots are
-// sorted widest window first). The grid never exceeds what the device can
+// Persistent gangs of G CTAs: gang k solves shot k, then the next of the queue
+// (shots are sorted widest window first). The grid never exceeds what the device can
 // hold at once, so every gang's CTAs are resident together. INTERIOR: the
 // strip loops' bounds-test-free body for interior blocks (see run_strip).
 // COMP: compensated arithmetic (node_update_comp; the 3x3 initial values are
@@ -209,7 +208,7 @@ __global__ void __maxnreg__((COMP || (TAPE && INTERIOR)) ? 168 : 128)
     __syncthreads();
     int it = 0;
 #pragma unroll 1
-    for (int b = gp.gang; b < p.nshots; b += p.NG, it++) {
+    for (int b = gp.gang; b < p.nshots; it++) {
         const ShotDev sh = p.shots[b];
         float* T = (p.t_per_gang > 0) ? p.Tpool + (size_t)gp.gang * p.t_per_gang : p.Tpool + sh.t_off;
         float* Tl = !COMP ? nullptr
@@ -233,8 +232,7 @@ __global__ void __maxnreg__((COMP || (TAPE && INTERIOR)) ? 168 : 128)
                 p.picks[(size_t)sh.orig * p.nrec + r] = v;
             }
         }
-        // the gang's buffers are reused by its next shot
-        gang_barrier(bar, (++nbar) * p.G, cs, p.err);
+        b = next_shot(p.bar, p.NG, p.G, gp.gang, gp.g, it, nbar, cs, p.err);
     }
 }
 

@@ -32,7 +32,7 @@ constexpr size_t kNoAllocHeader = 256;
 
 struct NoAllocHeader {
     int err;           // in-kernel wait timeout flag (must start at 0)
-    unsigned bar;      // gang barrier counter (must start at 0)
+    unsigned bar[4];   // counters of the launch's one gang (must start at 0)
     unsigned epoch;    // handoff tag epoch of the last call (host copy below)
     int div_bad;       // k_verify_div: bit w set when divisor w failed (must start at 0)
     float divs[4];     // the four constant divisors (dx, dz, hyp, D) being verified
@@ -41,6 +41,7 @@ struct NoAllocHeader {
     ShotDev shot;      // the one shot of the call
 };
 static_assert(sizeof(NoAllocHeader) <= 256, "header too large");
+static_assert(gang_counters(1) <= 4, "too few counters");
 
 // Shared by every call on a device; keeps the last call's contents.
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocHeader + kNoAllocWords * sizeof(unsigned long long)];
@@ -195,7 +196,7 @@ extern "C" int sf_time_propagation_noalloc(const float* S, int nx, int nz, float
     p.t_per_gang = 0;
     p.err = &dh->err;
     p.hand = reinterpret_cast<unsigned long long*>(base + kNoAllocHeader);
-    p.bar = &dh->bar;
+    p.bar = dh->bar;
     p.epoch = epoch;
     const int warps = 8;
     void* args[] = {&p};

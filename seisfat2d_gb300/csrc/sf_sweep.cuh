@@ -102,7 +102,7 @@ __host__ __device__ constexpr size_t hand_words(int nstrips, int maxcols, int hs
 // dynamic shared memory.
 struct CtaShared {
     int abort_flag;
-    int item;
+    int item;              // the gang's next shot
     unsigned long long wait_ns;  // time limit of every bounded wait of the CTA
     float init[9];
 };
@@ -647,6 +647,33 @@ __device__ __forceinline__ void gang_barrier(unsigned* ctr, unsigned target, Cta
         __threadfence();
     }
     __syncthreads();
+}
+
+// Counters of a persistent launch of NG gangs: a barrier counter per gang,
+// the queue (shots taken past the gangs' first ones), two next-shot words per gang.
+__host__ __device__ constexpr size_t gang_counters(int NG) { return 3 * (size_t)NG + 1; }
+constexpr int kMaxSolves = 1023;  // shots one gang takes in a launch (the tags' 10-bit shot-solve number)
+
+// Ends the gang's shot number `it` (its buffers are free for the next) and
+// returns the next one from the queue, for every thread of the gang. Shots
+// are sorted widest first, so taking them as gangs fall free balances uneven
+// windows: 1000 windows of 400 to 1600 columns on 456 gangs took 52.9 ms
+// (forward) and 26.0 ms (reverse) dealt in turn, where the gangs' sums range
+// from 0.7 to 1.4 of their mean.
+__device__ __forceinline__ int next_shot(unsigned* ctr, int NG, int G, int gang, int g, int it, unsigned& nbar,
+                                         CtaShared* sh, int* err)
+{
+    // two words in turn: a CTA may still read the last one
+    unsigned* slot = ctr + NG + 1 + 2 * (size_t)gang + (it & 1);
+    if (g == 0 && threadIdx.x == 0)
+        *(volatile unsigned*)slot = (it + 1 < kMaxSolves) ? (unsigned)NG + atomicAdd(ctr + NG, 1u) : 0x7fffffffu;
+    gang_barrier(ctr + gang, (++nbar) * G, sh, err);
+    if (threadIdx.x == 0) {
+        const bool stop = ld_volatile(&sh->abort_flag) || *(volatile int*)err;  // a wait gave up: results are void
+        sh->item = stop ? 0x7fffffff : (int)*(volatile unsigned*)slot;
+    }
+    __syncthreads();
+    return sh->item;
 }
 
 }  // namespace sf

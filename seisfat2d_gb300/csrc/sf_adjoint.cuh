@@ -66,6 +66,7 @@ struct __align__(16) AdjRing {
 struct AdjStripArgs {
     float* lam;        // window adjoint field (column stride nzz), in place
     int nzz, ncols, k;
+    bool down, right;  // directions of the reverse march
     const uint8_t* tcode;  // tape of this (sweep, strip): entries [fstep*32 + flane]
     const float* tc1;
     float* tc2;            // overwritten with v = mu * c2
@@ -86,16 +87,15 @@ struct AdjStripArgs {
     int c0;            // the window's first padded column
 };
 
-// SZ, SX: signs of the forward sweep being reversed. INTERIOR: blocks whose
-// marches all lie inside the window run a body without bounds tests.
-template <int SZ, int SX, bool INTERIOR>
+// INTERIOR: blocks whose marches all lie inside the window run a body without
+// bounds tests. One body serves the four sweeps (see run_strip).
+template <bool INTERIOR>
 __device__ __forceinline__ void adj_strip(const AdjStripArgs& a)
 {
     const int lane = threadIdx.x & 31;
     const int nzz = a.nzz, ncols = a.ncols;
     const int rb = 32 * a.k;
-    // reverse march: rows along -SZ, columns along -SX
-    const int r = (SZ < 0) ? rb + lane : rb + 31 - lane;
+    const int r = a.down ? rb + lane : rb + 31 - lane;
     const bool vrow = r < nzz;
     const int tix = r - rb;
     const int flane = 31 - lane;  // this row's lane in the forward strip
@@ -106,8 +106,8 @@ __device__ __forceinline__ void adj_strip(const AdjStripArgs& a)
     const bool lane0 = lane == 0;
     const bool feeds = (lane == 31) && (a.h_out != nullptr);
     const int nsteps = ncols + 31;
-    auto col_of = [&](int m) { return (SX < 0) ? m : ncols - 1 - m; };
-    const long long dL = (SX < 0) ? (long long)nzz : -(long long)nzz;
+    auto col_of = [&](int m) { return a.right ? m : ncols - 1 - m; };
+    const long long dL = a.right ? (long long)nzz : -(long long)nzz;
     const float* pL = a.lam + (long long)(rb + lane) + (long long)col_of(0) * (long long)nzz;
     // the lane's 16 bytes of a block's tape rows (rows of steps q+U-1 .. q, forward step order)
     const long long fs0 = (long long)(ncols + 31 - kU) * 32;
@@ -287,13 +287,13 @@ __device__ __forceinline__ void adj_strip(const AdjStripArgs& a)
             publish_progress(a.prog_out, a.tag, min(s0 + kU - 31, ncols));
     };
     // column blocks in the order the march finishes them: the counted sweep
-    // is the reverse of sweep 0 (SX > 0), which marches down the columns, so
+    // is the reverse of sweep 0, which marches down the columns, so
     // block b is done once lane 31 has passed its first window column (the
     // tile's extra node column, the next block's first, came earlier)
     const int blo = a.c0 / kGT, bhi = (a.c0 + ncols - 1) / kGT;
     int next_b = bhi;
     auto count_done = [&](int s_end) {
-        while (SX > 0 && next_b >= blo) {
+        while (next_b >= blo) {
             const int wcol = max(next_b * kGT, a.c0) - a.c0;
             const int m = ncols - 1 - wcol;  // march of that column
             if (m + 31 > s_end) break;
@@ -395,6 +395,8 @@ __device__ void adjoint_body(const AdjParams& p, const FuseParams* f)
         for (int task = gp.slot; task < 4 * nstrips; task += gp.slots) {
             const int rs = task / nstrips, pidx = task - rs * nstrips, sw = 3 - rs;
             a.k = (rs & 1) ? nstrips - 1 - pidx : pidx;
+            a.down = !(rs & 1);
+            a.right = rs < 2;
             unsigned long long* hs = hb + ((size_t)rs * nstrips + pidx) * row;
             a.h_in = (pidx > 0) ? hs : nullptr;
             a.h_out = (pidx < nstrips - 1) ? hs + row : nullptr;
@@ -407,12 +409,7 @@ __device__ void adjoint_body(const AdjParams& p, const FuseParams* f)
             a.tc1 = p.tc1 + tb;
             a.tc2 = p.tc2 + tb;
             a.ready = (f && sw == 0) ? f->ready + (size_t)a.k * f->nblk : nullptr;
-            switch (sw) {
-            case 0: adj_strip<1, 1, INTERIOR>(a); break;
-            case 1: adj_strip<-1, 1, INTERIOR>(a); break;
-            case 2: adj_strip<1, -1, INTERIOR>(a); break;
-            default: adj_strip<-1, -1, INTERIOR>(a); break;
-            }
+            adj_strip<INTERIOR>(a);
         }
         gang_barrier(bar, (++nbar) * p.G, cs, p.err);
         if (gp.g == 0 && tid < 9) {

@@ -97,17 +97,16 @@ __device__ __forceinline__ GangPos gang_pos(int G)
     return q;
 }
 
-// The strip of sweep SW that a.k names, in the loop form the shot needs.
-template <int SW, bool TAPE, bool REF, bool INTERIOR, bool COMP>
-__device__ __forceinline__ void sweep_strip(const StripArgs& a, bool exact)
+// One strip of a sweep in the loop form the shot needs.
+template <bool RIGHT, bool TAPE, bool REF, bool INTERIOR, bool COMP>
+__device__ __forceinline__ void strip(const StripArgs& a, bool exact)
 {
-    constexpr int SZ = (SW & 1) ? -1 : 1, SX = (SW < 2) ? 1 : -1;
     if (exact)
-        run_strip<SZ, SX, SW == 0, TAPE, REF, false, false, COMP, true>(a);
+        run_strip<RIGHT, TAPE, REF, false, false, COMP, true>(a);
     else if (a.kc.dx == a.kc.dz)
-        run_strip<SZ, SX, SW == 0, TAPE, REF, INTERIOR, true, COMP, false>(a);
+        run_strip<RIGHT, TAPE, REF, INTERIOR, true, COMP, false>(a);
     else
-        run_strip<SZ, SX, SW == 0, TAPE, REF, INTERIOR, false, COMP, false>(a);
+        run_strip<RIGHT, TAPE, REF, INTERIOR, false, COMP, false>(a);
 }
 
 // The four sweeps of one solve of the current shot. Sweeps 0 (down) and 1
@@ -156,6 +155,8 @@ __device__ void solve_window(const FwdParams& p, const ShotDev& sh, const GangPo
     for (int task = gp.slot; task < 4 * nstrips; task += gp.slots) {
         const int sw = task / nstrips, pidx = task - sw * nstrips;
         a.k = (sw & 1) ? nstrips - 1 - pidx : pidx;
+        a.down = !(sw & 1);
+        a.sw0 = sw == 0;
         a.skip_i = sh.skip_i[sw];
         a.skip_j = sh.skip_j[sw];
         unsigned long long* hs = hb + ((size_t)sw * nstrips + pidx) * row;
@@ -171,12 +172,10 @@ __device__ void solve_window(const FwdParams& p, const ShotDev& sh, const GangPo
             a.tc1 = p.tc1 + base;
             a.tc2 = p.tc2 + base;
         }
-        switch (sw) {
-        case 0: sweep_strip<0, TAPE, REF, INTERIOR, COMP>(a, exact); break;
-        case 1: sweep_strip<1, TAPE, REF, INTERIOR, COMP>(a, exact); break;
-        case 2: sweep_strip<2, TAPE, REF, INTERIOR, COMP>(a, exact); break;
-        default: sweep_strip<3, TAPE, REF, INTERIOR, COMP>(a, exact); break;
-        }
+        if (sw < 2)
+            strip<true, TAPE, REF, INTERIOR, COMP>(a, exact);
+        else
+            strip<false, TAPE, REF, INTERIOR, COMP>(a, exact);
     }
 }
 

@@ -163,6 +163,8 @@ struct StripArgs {
     float* Tl;        // compensated: their lo parts, same layout
     int nzz, ncols;
     int k;            // strip index: rows [32k, 32k+32)
+    bool down;        // rows downward (sweeps 0 and 2)
+    bool sw0;         // first sweep: every node starts at kBig but the source's 3x3 block
     int sIdz, sIdx;   // source node (window coordinates)
     int skip_i, skip_j;
     Consts kc;
@@ -285,7 +287,15 @@ __device__ __forceinline__ unsigned wait_counter(const unsigned* p, unsigned tar
 // the same bits. COMP: compensated arithmetic (node_update_comp): every
 // traveltime the loop carries, stages, hands on and writes back is a pair
 // (hi, lo); the second handoff pair of a column carries lo.
-template <int SZ, int SX, bool SW0, bool TAPE, bool REF, bool INTERIOR, bool SQ, bool COMP, bool EXACT>
+//
+// RIGHT: the march's direction. The row direction and the first sweep's start
+// values are runtime values, so the two sweeps that run at the same time share
+// their code: with a copy per sweep, loops of up to 14 KB were in flight on
+// an SM and instruction fetch was 16% of the stalls. The node's cells need no
+// more for it than a select: of the two slowness columns a lane holds, the
+// carried one is the cell column on the upwind side (j1) in either direction,
+// and the new one the other. Marches to the left read one column ahead.
+template <bool RIGHT, bool TAPE, bool REF, bool INTERIOR, bool SQ, bool COMP, bool EXACT>
 __device__ __forceinline__ void run_strip(const StripArgs& a)
 {
     using B = FwdBlock<TAPE, COMP>;
@@ -294,14 +304,15 @@ __device__ __forceinline__ void run_strip(const StripArgs& a)
     const int lane = threadIdx.x & 31;
     const int nzz = a.nzz, ncols = a.ncols;
     const int rb = 32 * a.k;
-    const int r = (SZ > 0) ? rb + lane : rb + 31 - lane;
+    constexpr bool right = RIGHT;
+    const bool down = a.down, sw0 = RIGHT && a.sw0;
+    const int r = down ? rb + lane : rb + 31 - lane;
     const bool vrow = r < nzz;
     const bool irow = (r >= 1) && (r <= nzz - 2);
     const bool row1 = r == 1;
     const int tix = r - rb;    // the row's place among the strip's rows
-    const int dr1 = (SZ > 0) ? 0 : 1;
-    const int dc2 = (SX > 0) ? 0 : 1;
-    const int dr2a = (r - 1 >= 1) ? 0 : 1;
+    const int cz = down ? 0 : 8, cx = right ? 0 : 16;  // tape bits of the cell (i1, j1)
+    const int dr2a = (r - 1 >= 1) ? 0 : 8;
 
     float* ring = reinterpret_cast<float*>(a.ring);
     float* pring = ring + RING * P;          // handoff pairs of march q at (q mod PAIRS) * 2 HS
@@ -318,18 +329,18 @@ __device__ __forceinline__ void run_strip(const StripArgs& a)
     const bool lane0 = lane == 0;
     const bool feeds = (lane == 31) && (a.h_out != nullptr);
     // the strip holds rows of the source's 3x3 block (first sweep only)
-    const bool src_rows = SW0 && (a.sIdz + 1 >= rb) && (a.sIdz - 1 <= rb + 31);
-    auto col_of = [&](int m) { return (SX > 0) ? m : ncols - 1 - m; };
+    const bool src_rows = sw0 && (a.sIdz + 1 >= rb) && (a.sIdz - 1 <= rb + 31);
+    auto col_of = [&](int m) { return right ? m : ncols - 1 - m; };
     // blocks whose first step lies in [g0, g0 + gn] need the general body for
     // the source block (first sweep) or a skipped cell
     int g0 = 0, gn = -1;
     if (src_rows) {
-        const int ms = (SX > 0) ? a.sIdx : ncols - 1 - a.sIdx;
+        const int ms = col_of(a.sIdx);  // its own inverse
         g0 = ms - 1;
         gn = 2;
     }
     if (a.skip_i >= rb && a.skip_i <= rb + 31) {
-        const int ms = (SX > 0) ? a.skip_j : ncols - 1 - a.skip_j;
+        const int ms = col_of(a.skip_j);
         const int lo = (gn < 0) ? ms : min(g0, ms), hi = (gn < 0) ? ms : max(g0 + gn, ms);
         g0 = lo;
         gn = hi - lo;
@@ -339,7 +350,7 @@ __device__ __forceinline__ void run_strip(const StripArgs& a)
     gn = (gn < 0) ? 0 : gn + U - 1 + 31;
 
     // running source addresses of the next march columns to stage
-    const long long dcol = (SX > 0) ? 1 : -1;
+    const long long dcol = right ? 1 : -1;
     const long long dS = dcol * (long long)ldS, dT = dcol * (long long)nzz;
     const float* pS = a.S + (long long)ls_row + (long long)col_of(0) * (long long)ldS;
     const float* pX = a.S + (long long)(rb + 31) + (long long)col_of(0) * (long long)ldS + lane * dS;
@@ -354,16 +365,14 @@ __device__ __forceinline__ void run_strip(const StripArgs& a)
         for (int u = 0; u < U; u++) {
             if (FAST || q + u < ncols) {
                 if (ls_ok) cp_async4(d + u * P, pS);
-                if (!SW0 && lt_ok) {
+                if (!sw0 && lt_ok) {
                     cp_async4(d + u * P + kT0, pT);
                     if (COMP) cp_async4(d + u * P + kL0, pTl);
                 }
             }
             pS += dS;
-            if (!SW0) {
-                pT += dT;
-                if (COMP) pTl += dT;
-            }
+            pT += dT;
+            if (COMP) pTl += dT;
         }
         if (lx_ok && (FAST || q + lane < ncols)) cp_async4(ring + (slot + lane) * P + 32, pX);
         pX += U * dS;
@@ -378,9 +387,9 @@ __device__ __forceinline__ void run_strip(const StripArgs& a)
     };
 
     // columns of the previous sweep known to be written back
-    int avail = SW0 ? 0x7fffffff : 0;
+    int avail = sw0 ? 0x7fffffff : 0;
     auto ensure = [&](int q) {  // marches below q may be staged
-        if (!SW0 && q > avail) {
+        if (q > avail) {
             avail = wait_progress(a.prog_in, a.tag, a.follow ? min(q, ncols) : ncols, sh, a.err);
             if (avail >= ncols) avail = 0x7fffffff;
         }
@@ -408,7 +417,7 @@ __device__ __forceinline__ void run_strip(const StripArgs& a)
 
     float tn = 0.0f, tvp = 0.0f;                          // own last result, last upwind value
     float tnl = 0.0f, tvpl = 0.0f;                        // their lo parts (compensated)
-    float cU = 0.0f, cI = 0.0f;                           // carried S of rows r-1, r
+    float cU = 0.0f, cI = 0.0f, cN = 0.0f;                // carried S of rows r-1, r and i1 (the one of the two on the upwind side)
     const int nsteps = ncols + 31;
     int b0 = 0;                                           // ring slot of march s0
     // ring offset of the lane's march s0 - lane (its row's first slowness)
@@ -428,7 +437,7 @@ __device__ __forceinline__ void run_strip(const StripArgs& a)
             stage_pairs(s0 + PLOOK, fast_tag);
             cp_commit();
         }
-        // staged: columns up to s0+U (SX < 0 reads one column ahead), pairs up to s0+U-1
+        // staged: columns up to s0+U (a leftward march reads one column ahead), pairs up to s0+U-1
         cp_wait<(LOOK / U - 1 < PLOOK / U) ? LOOK / U - 1 : PLOOK / U>();
         __syncwarp();
 
@@ -439,12 +448,14 @@ __device__ __forceinline__ void run_strip(const StripArgs& a)
             off[u] = ro;
             ro += P;
             if (ro >= RING * P + tix) ro -= RING * P;
-            // S of the new column: march m (SX>0) or m+1 (SX<0)
-            const int ns = (SX > 0) ? off[u] : ro;
+            // S of the new column: march m (rightward) or m+1
+            const int ns = right ? off[u] : ro;
             nU[u] = ring[ns];
             nI[u] = ring[ns + 1];
-            told[u] = SW0 ? kBig : ring[off[u] + kT0];
-            toldl[u] = (COMP && !SW0) ? ring[off[u] + kL0] : 0.0f;
+            told[u] = ring[off[u] + kT0];
+            toldl[u] = COMP ? ring[off[u] + kL0] : 0.0f;
+            if (sw0) told[u] = kBig;
+            if (COMP && sw0) toldl[u] = 0.0f;
         }
         // the upwind strip's values of the block (every lane reads them, lane 0 uses them)
         float hv[U], hvl[U];
@@ -505,7 +516,7 @@ __device__ __forceinline__ void run_strip(const StripArgs& a)
                 if (COMP) tvl = hvl[u];
             }
             const float te = tn, tev = tvp;
-            const float tel = tnl, tevl = tvpl;
+            [[maybe_unused]] const float tel = tnl, tevl = tvpl;
 
             float to = told[u], tol = toldl[u];
             if (!FAST && src_rows) {
@@ -515,32 +526,32 @@ __device__ __forceinline__ void run_strip(const StripArgs& a)
                     tol = 0.0f;
                 }
             }
-            float U_j, I_j, U_jm, I_jm;
-            if (SX > 0) { U_j = nU[u]; I_j = nI[u]; U_jm = cU; I_jm = cI; }
-            else        { U_j = cU; I_j = cI; U_jm = nU[u]; I_jm = nI[u]; }
             const bool inner = FAST ? irow
                                     : act && irow && (j >= 1) && (j <= ncols - 2) && !(r == a.skip_i && j == a.skip_j);
-            // rows: i1 (SZ>0: r-1, else r); columns: j-1 (clamped to 1), j
-            const float Si1_j = (SZ > 0) ? U_j : I_j;
-            const float Si1_jm = (SZ > 0) ? U_jm : I_jm;
-            const float s1a = (!FAST && j == 1) ? Si1_j : Si1_jm;   // S[i1][max(j-1,1)]
-            const float s1b = Si1_j;                                // S[i1][j]
-            const float s2b = (SX > 0) ? I_jm : I_j;                // S[i][j1]
-            const float s2a = row1 ? s2b : ((SX > 0) ? U_jm : U_j); // S[max(i-1,1)][j1]
-            const float sref = (SX > 0) ? Si1_jm : Si1_j;           // S[i1][j1]
-            const int dc1a = (FAST || j - 1 >= 1) ? 0 : 1;
+            // row i1 (downward r-1, else r), columns j-1 (clamped to 1) and j; the
+            // order matters to the tape only
+            const float nN = down ? nU[u] : nI[u];
+            float s1a = cN, s1b = nN;
+            if (TAPE || !FAST) {
+                s1a = right ? cN : nN;
+                s1b = right ? nN : cN;
+                if (!FAST && j == 1) s1a = s1b;
+            }
+            // column j1: rows max(i-1,1) and i
+            const float s2a = row1 ? cI : cU;
+            const int dc1a = (FAST || j - 1 >= 1) ? 0 : 16;
             float tnew, tnewl = 0.0f;
             if constexpr (COMP)
-                node_update_comp<TAPE, EXACT, SQ>(to, tol, tv, tvl, te, tel, tev, tevl, s1a, s1b, s2a, s2b, sref,
-                                                  a.kc, dr1, dc1a, dc2, dr2a, tnew, tnewl, rec[u]);
+                node_update_comp<TAPE, EXACT, SQ>(to, tol, tv, tvl, te, tel, tev, tevl, s1a, s1b, s2a, cI, cN,
+                                                  a.kc, cz, cx, dc1a, dr2a, tnew, tnewl, rec[u]);
             else
-                tnew = node_update<TAPE, REF, EXACT, SQ>(to, tv, te, tev, s1a, s1b, s2a, s2b, sref, a.kc,
-                                                         dr1, dc1a, dc2, dr2a, rec[u]);
+                tnew = node_update<TAPE, REF, EXACT, SQ>(to, tv, te, tev, s1a, s1b, s2a, cI, cN, a.kc,
+                                                         cz, cx, dc1a, dr2a, rec[u]);
             tnw[u] = inner ? tnew : to;
             tnwl[u] = COMP ? (inner ? tnewl : tol) : 0.0f;
             if (TAPE) {
                 if (!inner) rec[u].code = 0;
-                sr[u] = sref;
+                sr[u] = cN;
                 any_far |= rec[u].code & 4;                         // 4, 5
                 any_far |= ((rec[u].code & 3) == 3);                // 3
             }
@@ -553,6 +564,7 @@ __device__ __forceinline__ void run_strip(const StripArgs& a)
             tvpl = tvl;
             cU = nU[u];
             cI = nI[u];
+            cN = nN;
         }
 
         if constexpr (TAPE) {

@@ -263,8 +263,9 @@ int sf_adj_configure(sf_ctx* c, cudaStream_t st, AdjLaunch* A)
     A->ggrid = dim3((unsigned)(nstrips * ((c->nxx + kGT - 1) / kGT)));
     A->gblock = dim3(256);
     // The gather inside the reverse-sweep launch (isotropic batches, 2 or 4
-    // warps per CTA) when the device holds every reverse-sweep CTA and at
-    // least one gather CTA at once.
+    // warps per CTA) when the device holds every reverse-sweep CTA and two
+    // gather CTAs per SM at once (600 windows that left room for 8 gather CTAs
+    // took 834 ms in one launch, 26 ms in two).
     A->fused = false;
     if (c->fuse_gather && !c->batch_ani && (c->warps == 2 || c->warps == 4)) {
         const bool in = c->batch_interior;
@@ -276,7 +277,7 @@ int sf_adj_configure(sf_ctx* c, cudaStream_t st, AdjLaunch* A)
         const long long cap = (long long)per_sm * c->sms, nadj = (long long)NG * G;
         const int nblk = (c->nxx + kGT - 1) / kGT, ntiles = nstrips * nblk;
         const long long nga = std::min<long long>(cap - nadj, ntiles);
-        if (nga >= 1) {
+        if (nga >= std::min<long long>(2LL * c->sms, ntiles)) {
             const size_t nz = (size_t)ntiles + 1 + (size_t)ns;  // ready counters, tile counter, shot flags
             rc = sf_dev_reserve(c, (void**)&c->d_fuse, &c->cap_fuse, nz * sizeof(unsigned));
             if (rc) return rc;

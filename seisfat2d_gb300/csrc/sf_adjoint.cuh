@@ -161,7 +161,7 @@ __device__ __forceinline__ void adj_strip(const AdjStripArgs& a)
     }
 
     // running destinations: the term v of forward tape step ncols+30-s, the
-    // write-back of march column s-31 (row r), the pair of march s-31
+    // write-back of the next finished column (row r), the pair of march s-31
     float* pV = a.tc2 + (long long)(ncols + 30) * 32 + flane;
     float* pW = a.lam + (long long)r + (long long)col_of(0) * (long long)nzz;
     unsigned long long* pH = a.h_out - 2 * 31;
@@ -174,17 +174,7 @@ __device__ __forceinline__ void adj_strip(const AdjStripArgs& a)
     // ring reads, its kU linear updates (the only serial chain), its stores.
     auto block = [&](int s0, auto fast_tag) {
         constexpr bool FAST = decltype(fast_tag)::value;
-        ensure(s0 + kLookA + kU);
-        {
-            int pf0 = b0 + kLookA;
-            if (pf0 >= kRingA) pf0 -= kRingA;
-            int tf0 = tb0 + kLookA / kU;
-            if (tf0 >= kTapeBlocks) tf0 -= kTapeBlocks;
-            stage(s0 + kLookA, pf0, tf0, fast_tag);
-            stage_pairs(s0 + kPairLookA, fast_tag);
-            cp_commit();
-        }
-        cp_wait<(kLookA < kPairLookA ? kLookA : kPairLookA) / kU>();
+        cp_wait<(kLookA < kPairLookA ? kLookA : kPairLookA) / kU - 1>();
         __syncwarp();
 
         const AdjTape& t = R.tape[tb0];
@@ -204,6 +194,21 @@ __device__ __forceinline__ void adj_strip(const AdjStripArgs& a)
             av[u] = (br[u] == 1) ? 1.0f : (br[u] == 3) ? c : (br[u] >= 5) ? cm : 0.0f;
             ae[u] = (br[u] == 2) ? 1.0f : (br[u] == 3) ? -c : (br[u] == 4) ? cm : 0.0f;
             aev[u] = (br[u] == 3) ? 1.0f : (br[u] >= 4) ? c : 0.0f;
+        }
+        // write back the columns every lane had finished before this block (marches s0-kU-31 ..)
+        {
+            int wb = b0 + (kRingA - 31 - kU);
+            if (wb >= kRingA) wb -= kRingA;
+#pragma unroll
+            for (int u = 0; u < kU; u++) {
+                const int m = s0 + u - kU - 31;
+                if (FAST || (m >= 0 && m < ncols)) {
+                    int ws = wb + u;
+                    if (ws >= kRingA) ws -= kRingA;
+                    if (vrow) *pW = R.L[ws * 32 + tix];
+                    pW += dL;
+                }
+            }
         }
         {
             // the upwind row of lane 0: the previous strip's pairs, or nothing
@@ -237,6 +242,18 @@ __device__ __forceinline__ void adj_strip(const AdjStripArgs& a)
             }
         }
 
+        // next columns, tape rows and pairs (the ring reads above are in flight meanwhile)
+        ensure(s0 + kLookA + kU);
+        {
+            int pf0 = b0 + kLookA;
+            if (pf0 >= kRingA) pf0 -= kRingA;
+            int tf0 = tb0 + kLookA / kU;
+            if (tf0 >= kTapeBlocks) tf0 -= kTapeBlocks;
+            stage(s0 + kLookA, pf0, tf0, fast_tag);
+            stage_pairs(s0 + kPairLookA, fast_tag);
+            cp_commit();
+        }
+
         float lo[kU], vv[kU], opv[kU], opev[kU];
 #pragma unroll
         for (int u = 0; u < kU; u++) {
@@ -268,23 +285,10 @@ __device__ __forceinline__ void adj_strip(const AdjStripArgs& a)
         }
         pV -= 32 * kU;
         pH += 2 * kU;
-        int wb = b0 + (kRingA - 31);  // slot of march s0 - 31
-        if (wb >= kRingA) wb -= kRingA;
-#pragma unroll
-        for (int u = 0; u < kU; u++) {
-            const int s = s0 + u;
-            if (FAST || (s >= 31 && s < nsteps)) {
-                int ws = wb + u;
-                if (ws >= kRingA) ws -= kRingA;
-                if (vrow) *pW = R.L[ws * 32 + tix];
-                pW += dL;
-            }
-        }
         b0 += kU;
         if (b0 >= kRingA) b0 -= kRingA;
         if (++tb0 >= kTapeBlocks) tb0 = 0;
-        if (a.publish && (s0 + kU) % kPublish == 0 && s0 + kU > 31)
-            publish_progress(a.prog_out, a.tag, min(s0 + kU - 31, ncols));
+        if (a.publish && s0 % kPublish == 0 && s0 > 31) publish_progress(a.prog_out, a.tag, min(s0 - 31, ncols));
     };
     // column blocks in the order the march finishes them: the counted sweep
     // is the reverse of sweep 0, which marches down the columns, so
@@ -303,10 +307,11 @@ __device__ __forceinline__ void adj_strip(const AdjStripArgs& a)
             next_b--;
         }
     };
+    // one block past the last step writes the last columns back
 #pragma unroll 1
-    for (int s0 = 0; s0 < nsteps; s0 += kU) {
+    for (int s0 = 0; s0 < nsteps + kU; s0 += kU) {
         if constexpr (INTERIOR) {
-            if (s0 >= 31 && s0 + kLookA + kU <= ncols)
+            if (s0 >= 31 + kU && s0 + kLookA + kU <= ncols)
                 block(s0, std::true_type{});
             else
                 block(s0, std::false_type{});

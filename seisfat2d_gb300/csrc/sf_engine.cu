@@ -157,11 +157,9 @@ __global__ void k_picks(const float* __restrict__ T, int nzz, int ncols, int c0,
 
 }  // namespace
 
-size_t sf_fwd_smem_bytes(int warps, bool comp, bool tape)
+size_t sf_fwd_smem_bytes(int warps, bool comp)
 {
-    const size_t ring = tape ? (comp ? ring_bytes<true, true>() : ring_bytes<true, false>())
-                             : (comp ? ring_bytes<false, true>() : ring_bytes<false, false>());
-    return ((sizeof(CtaShared) + 15) & ~size_t(15)) + (size_t)warps * ring;
+    return ((sizeof(CtaShared) + 15) & ~size_t(15)) + (size_t)warps * (comp ? ring_bytes<true>() : ring_bytes<false>());
 }
 
 // ------------------------------------------------------------------ context
@@ -430,7 +428,7 @@ int sf_fwd_setup(sf_ctx* c)
 {
     for (int k = 0; k < 16; k++) {
         const bool tape = k & 8, comp = k & 1;
-        const size_t mx = sf_fwd_smem_bytes(comp ? kMaxWarpsComp : kMaxWarps, comp, tape);
+        const size_t mx = sf_fwd_smem_bytes(comp ? kMaxWarpsComp : kMaxWarps, comp);
         const void* f = sf_kshots_kernel(tape, k & 4, k & 2, comp);
         if (f) CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mx));
     }
@@ -672,7 +670,7 @@ int sf_fwd_configure(sf_ctx* c, int nrec, bool per_shot_T, bool tape, int gang_w
     if (comp && c->warps > kMaxWarpsComp)
         return sf_fail(c, SF_ERR_ARG, "the compensated arithmetic runs at most 8 warps per CTA (sf_set_launch)");
     const bool ref = c->arith == SF_ARITH_REFERENCE;
-    const size_t smem = sf_fwd_smem_bytes(c->warps, comp, tape);
+    const size_t smem = sf_fwd_smem_bytes(c->warps, comp);
     // the interior-block kernels of taped batches are built for at most
     // kMaxWarpsTapedInterior warps per CTA
     c->batch_interior = !(tape && c->warps > kMaxWarpsTapedInterior) && sf_interior_loops(c);

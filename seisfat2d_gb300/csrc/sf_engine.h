@@ -177,7 +177,7 @@ int sf_check_flags(sf_ctx* c, cudaStream_t st);
 int sf_check_slowness(sf_ctx* c, cudaStream_t st);
 int sf_fwd_setup(sf_ctx* c);
 int sf_verify_divisors(sf_ctx* c);
-size_t sf_fwd_smem_bytes(int warps, bool comp, bool tape);
+size_t sf_fwd_smem_bytes(int warps, bool comp);
 // k_shots instantiation (one object file each, sf_shots_inst.cu)
 const void* sf_kshots_kernel(bool tape, bool ref, bool interior, bool comp);
 const void* sf_kqp_kernel(bool ref, bool comp, bool fact);

@@ -143,7 +143,7 @@ __device__ void solve_window(const FwdParams& p, const ShotDev& sh, const GangPo
     a.sIdx = sh.sIdx - sh.c0;
     a.kc = p.kc;
     a.init = cs->init;
-    a.ring = rings + (size_t)gp.warp * ring_bytes<TAPE, COMP>();
+    a.ring = rings + (size_t)gp.warp * ring_bytes<COMP>();
     a.sh = cs;
     a.err = p.err;
     a.tcode = nullptr;

@@ -28,8 +28,8 @@
 // a few march columns ahead (32 consecutive rows = one coalesced 128-byte
 // request per field), and lane l reads its own row of column s-l from the
 // ring. A ring slot holds one column: slowness rows rb-1..rb+31 at 0..32,
-// traveltimes at 36..67 and, in the compensated arithmetic, their lo parts at
-// 68..99. With slot pitches of 68 and 100 floats both the coalesced fill and
+// traveltimes at 33..64 and, in the compensated arithmetic, their lo parts at
+// 65..96. With slot pitches of 66 and 98 floats both the coalesced fill and
 // the skewed read are bank-conflict free, and one address serves all fields
 // of a node. Finished columns go back to global memory through the same
 // ring, coalesced. The march runs in blocks of a few steps: one wait for the
@@ -48,25 +48,29 @@ namespace sf {
 
 // Block size U, staging leads (march columns, multiples of the block) of the
 // columns (LOOK) and of the upwind strip's pairs (PLOOK), and ring length of
-// a forward strip loop. After a stall a consumer lets its producer get AHEAD
-// columns ahead. The ring holds the 32 marches the lanes work on, the lead
-// and two blocks, so a block's prefetches never refill a slot that the block
-// before it still read: RING >= 31 + LOOK + 2 U.
-template <bool TAPE, bool COMP>
+// the forward strip loop. After a stall a consumer lets its producer get AHEAD
+// columns ahead. The ring holds the 32 marches the lanes work on, the block
+// still to be written back, the lead and a block. Blocks of four steps with
+// eight columns staged ahead measured best: blocks of two (lead four) took
+// 15% longer for the plain solve and 14% for the taped one (100 shots of
+// 1707 x 357: 1.82 and 3.21 ms), a lead of four 25%, pairs eight ahead 3% (they
+// lengthen the lag between strips).
+template <bool COMP>
 struct FwdBlock {
-    static constexpr int U = TAPE ? 2 : 4;
-    static constexpr int LOOK = TAPE ? 4 : 8;
+    static constexpr int U = 4;
+    static constexpr int LOOK = 8;
     static constexpr int PLOOK = 4;
     static constexpr int AHEAD = PLOOK + U;
-    static constexpr int RING = TAPE ? 40 : 48;
-    static constexpr int SLOT = COMP ? 100 : 68;  // floats per slot
+    static constexpr int RING = 48;
+    static constexpr int SLOT = COMP ? 98 : 66;   // floats per slot
     static constexpr int PAIRS = 16;              // columns of the pair ring
     static_assert(LOOK % U == 0 && PLOOK % U == 0 && PLOOK <= LOOK && RING % U == 0 && RING >= 31 + LOOK + 2 * U,
                   "ring too small");
     static_assert(PAIRS % U == 0 && PAIRS >= PLOOK + U && U % 2 == 0, "pair ring too small");
-    static_assert((RING * SLOT) % 32 == 0, "a wrapped skewed read would conflict");
+    static_assert((RING * SLOT) % 32 == 0 && SLOT % 32 == 2, "the skewed reads would conflict");
+    static_assert((RING * SLOT) % 4 == 0, "the pair ring must be 16-byte aligned");
 };
-constexpr int kT0 = 36, kL0 = 68;  // traveltimes and their lo parts in a slot
+constexpr int kT0 = 33, kL0 = 65;  // traveltimes and their lo parts in a slot
 constexpr int kPublish = 32;       // columns between two publications of a strip's progress
 constexpr int kMaxWarps = 16;
 // compensated kernels keep a second traveltime ring (the lo parts): at most
@@ -77,14 +81,15 @@ constexpr int kMaxWarpsComp = 8;
 // faster on the headline batch; the other kernels measured slower that way)
 constexpr int kMaxWarpsTapedInterior = 8;
 constexpr long long kSpinLimit = 1ll << 30;          // iterations
+constexpr unsigned kPollNs = 100;                    // pause between two polls of a wait
 constexpr unsigned long long kSpinNs = 2000000000ull;  // and at most ~2 s (default; sf_set_wait_limit)
 
 // A warp's forward ring: RING column slots, then the pair ring (a tagged
 // pair per column, two in the compensated arithmetic). Multiples of 16 bytes.
-template <bool TAPE, bool COMP>
+template <bool COMP>
 constexpr size_t ring_bytes()
 {
-    using B = FwdBlock<TAPE, COMP>;
+    using B = FwdBlock<COMP>;
     return sizeof(float) * (size_t)B::RING * B::SLOT + 8 * (size_t)B::PAIRS * (COMP ? 2 : 1);
 }
 
@@ -169,7 +174,7 @@ struct StripArgs {
     int skip_i, skip_j;
     Consts kc;
     const float* init;  // 9 values in shared memory
-    unsigned char* ring;  // this warp's ring (ring_bytes<TAPE, COMP>())
+    unsigned char* ring;  // this warp's ring (ring_bytes<COMP>())
     CtaShared* sh;
     const unsigned long long* h_in;  // {value, tag} of the upwind strip's row by march column (nullptr: first strip)
     unsigned long long* h_out;       // pairs this strip feeds to the next one (nullptr: last strip)
@@ -196,49 +201,63 @@ __device__ __forceinline__ unsigned long long global_ns()
     return t;
 }
 
-// Bounded wait until the pair at p carries `tag`; returns its value. On
-// timeout it behaves like wait_counter.
+// One round of a bounded wait: sleeps, and now and then looks whether the
+// wait must end: the launch's error flag or the CTA's abort flag is up, or its
+// own limit has run out, which raises both. Every later wait of the CTA (or of
+// any CTA once the launch's flag is up) then ends at once, so the kernel always
+// finishes (its results are void and the host reports SF_ERR_TIMEOUT). The
+// flags are read every eighth round only: the polling of warps that wait for
+// their turn was a third of all instructions of the reverse sweeps.
+struct WaitRound {
+    unsigned long long t0 = 0;
+    long long n = 0;
+    __device__ __forceinline__ bool give_up(CtaShared* sh, int* err)
+    {
+        if ((n & 7) == 0) {
+            if (ld_volatile(&sh->abort_flag) || *(volatile int*)err) return true;
+            const unsigned long long now = global_ns();
+            if (n == 0) t0 = now;
+            if (n > kSpinLimit || now - t0 > sh->wait_ns) {
+                st_volatile(&sh->abort_flag, 1);
+                atomicExch(err, 2);
+                return true;
+            }
+        }
+        n++;
+        __nanosleep(kPollNs);
+        return false;
+    }
+};
+
+// Bounded wait until the pair at p carries `tag`; returns its value (0 when
+// it gives up).
 __device__ __forceinline__ float wait_pair(const unsigned long long* p, unsigned tag, CtaShared* sh, int* err)
 {
     unsigned long long e = ld_relaxed_u64(p);
-    if (tag_of(e) == tag) return val_of(e);
-    const unsigned long long t0 = global_ns();
-    long long n = 0;
-    while (tag_of(e = ld_relaxed_u64(p)) != tag) {
-        if (ld_volatile(&sh->abort_flag) || *(volatile int*)err) return 0.0f;
-        __nanosleep(32);
-        if (++n > kSpinLimit || ((n & 255) == 0 && global_ns() - t0 > sh->wait_ns)) {
-            st_volatile(&sh->abort_flag, 1);
-            atomicExch(err, 2);
-            return 0.0f;
-        }
+    WaitRound w;
+    while (tag_of(e) != tag) {
+        if (w.give_up(sh, err)) return 0.0f;
+        e = ld_relaxed_u64(p);
     }
     return val_of(e);
 }
 
 // Bounded wait of the whole warp until the progress word at p carries `tag`
-// and at least `need` columns (acquire, by lane 0); returns the columns seen.
+// and at least `need` columns (acquire, by lane 0); returns the columns seen
+// (`need` when it gives up).
 __device__ __forceinline__ int wait_progress(const unsigned long long* p, unsigned tag, int need, CtaShared* sh, int* err)
 {
     int cols = need;
     if ((threadIdx.x & 31) == 0) {
-        unsigned long long e;
-        unsigned long long t0 = 0;
-        long long n = 0;
+        WaitRound w;
         while (true) {
+            unsigned long long e;
             asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(e) : "l"(p) : "memory");
             if (tag_of(e) == tag && (int)(unsigned)e >= need) {
                 cols = (int)(unsigned)e;
                 break;
             }
-            if (ld_volatile(&sh->abort_flag) || *(volatile int*)err) break;
-            if (n == 0) t0 = global_ns();
-            __nanosleep(32);
-            if (++n > kSpinLimit || ((n & 255) == 0 && global_ns() - t0 > sh->wait_ns)) {
-                st_volatile(&sh->abort_flag, 1);
-                atomicExch(err, 2);
-                break;
-            }
+            if (w.give_up(sh, err)) break;
         }
     }
     return __shfl_sync(0xffffffffu, cols, 0);
@@ -256,27 +275,12 @@ __device__ __forceinline__ void publish_progress(unsigned long long* p, unsigned
     }
 }
 
-// Bounded wait until the counter at p reaches `target` (acquire); returns
-// the value seen. On timeout it raises the CTA's abort flag and the launch's
-// error flag and returns `target`, and every later wait of the CTA (or of any
-// CTA once the launch's flag is up) returns at once, so the kernel always
-// finishes (its results are then void and the host reports SF_ERR_TIMEOUT).
-__device__ __forceinline__ unsigned wait_counter(const unsigned* p, unsigned target, CtaShared* sh, int* err)
+// Bounded wait until the counter at p reaches `target` (acquire).
+__device__ __forceinline__ void wait_counter(const unsigned* p, unsigned target, CtaShared* sh, int* err)
 {
-    unsigned v = ld_acquire_gpu(p);
-    if (v >= target) return v;
-    const unsigned long long t0 = global_ns();
-    long long n = 0;
-    while ((v = ld_acquire_gpu(p)) < target) {
-        if (ld_volatile(&sh->abort_flag) || *(volatile int*)err) return target;
-        __nanosleep(64);
-        if (++n > kSpinLimit || ((n & 255) == 0 && global_ns() - t0 > sh->wait_ns)) {
-            st_volatile(&sh->abort_flag, 1);
-            atomicExch(err, 2);
-            return target;
-        }
-    }
-    return v;
+    WaitRound w;
+    while (ld_acquire_gpu(p) < target)
+        if (w.give_up(sh, err)) return;
 }
 
 // INTERIOR: blocks whose marches all lie inside the window (and touch neither
@@ -298,7 +302,7 @@ __device__ __forceinline__ unsigned wait_counter(const unsigned* p, unsigned tar
 template <bool RIGHT, bool TAPE, bool REF, bool INTERIOR, bool SQ, bool COMP, bool EXACT>
 __device__ __forceinline__ void run_strip(const StripArgs& a)
 {
-    using B = FwdBlock<TAPE, COMP>;
+    using B = FwdBlock<COMP>;
     constexpr int U = B::U, LOOK = B::LOOK, PLOOK = B::PLOOK, RING = B::RING, P = B::SLOT;
     constexpr int HS = COMP ? 2 : 1;         // handoff pairs per column
     const int lane = threadIdx.x & 31;
@@ -363,16 +367,25 @@ __device__ __forceinline__ void run_strip(const StripArgs& a)
         float* d = ring + slot * P + lane;
 #pragma unroll
         for (int u = 0; u < U; u++) {
-            if (FAST || q + u < ncols) {
-                if (ls_ok) cp_async4(d + u * P, pS);
-                if (!sw0 && lt_ok) {
+            if ((FAST || q + u < ncols) && ls_ok) cp_async4(d + u * P, pS);
+            pS += dS;
+        }
+        if (sw0) {
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                d[u * P + kT0] = kBig;
+                if (COMP) d[u * P + kL0] = 0.0f;
+            }
+        } else {
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                if ((FAST || q + u < ncols) && lt_ok) {
                     cp_async4(d + u * P + kT0, pT);
                     if (COMP) cp_async4(d + u * P + kL0, pTl);
                 }
+                pT += dT;
+                if (COMP) pTl += dT;
             }
-            pS += dS;
-            pT += dT;
-            if (COMP) pTl += dT;
         }
         if (lx_ok && (FAST || q + lane < ncols)) cp_async4(ring + (slot + lane) * P + 32, pX);
         pX += U * dS;
@@ -407,7 +420,7 @@ __device__ __forceinline__ void run_strip(const StripArgs& a)
         cp_commit();
     }
 
-    // running destinations: write-back of march column s-31 (row r), tape entry s*32+lane
+    // running destinations: write-back of the next finished column (row r), tape entry s*32+lane
     float* pW = a.T + (long long)r + (long long)col_of(0) * (long long)nzz;
     float* pWl = COMP ? a.Tl + (long long)r + (long long)col_of(0) * (long long)nzz : nullptr;
     unsigned long long* pH = a.h_out - 31 * HS;
@@ -429,16 +442,17 @@ __device__ __forceinline__ void run_strip(const StripArgs& a)
     // stores after it are independent of it.
     auto block = [&](int s0, auto fast_tag) {
         constexpr bool FAST = decltype(fast_tag)::value;
-        ensure(s0 + LOOK + U);
-        {
+        auto stage_next = [&]() {
+            ensure(s0 + LOOK + U);
             int pf0 = b0 + LOOK;
             if (pf0 >= RING) pf0 -= RING;
             stage_cols(s0 + LOOK, pf0, fast_tag);
             stage_pairs(s0 + PLOOK, fast_tag);
             cp_commit();
-        }
-        // staged: columns up to s0+U (a leftward march reads one column ahead), pairs up to s0+U-1
-        cp_wait<(LOOK / U - 1 < PLOOK / U) ? LOOK / U - 1 : PLOOK / U>();
+        };
+        // staged: columns up to s0+U-1 (a leftward march reads one more), pairs up to s0+U-1
+        constexpr int kCols = LOOK / U - (right ? 1 : 2), kPairs = PLOOK / U - 1;
+        cp_wait<(kCols < kPairs) ? kCols : kPairs>();
         __syncwarp();
 
         int off[U];
@@ -454,8 +468,26 @@ __device__ __forceinline__ void run_strip(const StripArgs& a)
             nI[u] = ring[ns + 1];
             told[u] = ring[off[u] + kT0];
             toldl[u] = COMP ? ring[off[u] + kL0] : 0.0f;
-            if (sw0) told[u] = kBig;
-            if (COMP && sw0) toldl[u] = 0.0f;
+        }
+        // write back the columns every lane had finished before this block (marches s0-U-31 ..)
+        {
+            int wb = b0 + (RING - 31 - U);
+            if (wb >= RING) wb -= RING;
+            const float* q = ring + kT0 + tix;
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const int m = s0 + u - U - 31;
+                if (FAST || (m >= 0 && m < ncols)) {
+                    int ws = wb + u;
+                    if (ws >= RING) ws -= RING;
+                    if (vrow) {
+                        *pW = q[ws * P];
+                        if (COMP) *pWl = q[ws * P + kL0 - kT0];
+                    }
+                    pW += dT;
+                    if (COMP) pWl += dT;
+                }
+            }
         }
         // the upwind strip's values of the block (every lane reads them, lane 0 uses them)
         float hv[U], hvl[U];
@@ -499,9 +531,11 @@ __device__ __forceinline__ void run_strip(const StripArgs& a)
             }
         }
 
+        stage_next();  // the ring reads above are in flight meanwhile
+
         float tnw[U], tnwl[U], sr[U];
         Rec rec[U];
-        int any_far = 0;
+        bool any_far = false;
 #pragma unroll
         for (int u = 0; u < U; u++) {
             const int s = s0 + u;
@@ -552,8 +586,7 @@ __device__ __forceinline__ void run_strip(const StripArgs& a)
             if (TAPE) {
                 if (!inner) rec[u].code = 0;
                 sr[u] = cN;
-                any_far |= rec[u].code & 4;                         // 4, 5
-                any_far |= ((rec[u].code & 3) == 3);                // 3
+                any_far |= rec[u].far & inner;
             }
             // carry state
             if (act) {
@@ -610,31 +643,15 @@ __device__ __forceinline__ void run_strip(const StripArgs& a)
             }
         }
         pH += HS * U;
-        // write back the columns every lane has finished (march s-31)
-        int wb = b0 + (RING - 31);
-        if (wb >= RING) wb -= RING;
-#pragma unroll
-        for (int u = 0; u < U; u++) {
-            const int s = s0 + u;
-            if (FAST || (s >= 31 && s < nsteps)) {
-                int ws = wb + u;
-                if (ws >= RING) ws -= RING;
-                if (vrow) {
-                    *pW = ring[ws * P + kT0 + tix];
-                    if (COMP) *pWl = ring[ws * P + kL0 + tix];
-                }
-                pW += dT;
-                if (COMP) pWl += dT;
-            }
-        }
         b0 += U;
         if (b0 >= RING) b0 -= RING;
-        if (a.publish && (s0 + U) % kPublish == 0 && s0 + U > 31) publish_progress(a.prog_out, a.tag, min(s0 + U - 31, ncols));
+        if (a.publish && s0 % kPublish == 0 && s0 > 31) publish_progress(a.prog_out, a.tag, min(s0 - 31, ncols));
     };
+    // one block past the last step writes the last columns back
 #pragma unroll 1
-    for (int s0 = 0; s0 < nsteps; s0 += U) {
+    for (int s0 = 0; s0 < nsteps + U; s0 += U) {
         if constexpr (INTERIOR) {
-            if (s0 >= 33 && s0 + LOOK + U <= ncols - 1 && (unsigned)(s0 - g0) > (unsigned)gn)
+            if (s0 >= 31 + U && s0 + LOOK + U <= ncols - 1 && (unsigned)(s0 - g0) > (unsigned)gn)
                 block(s0, std::true_type{});
             else
                 block(s0, std::false_type{});

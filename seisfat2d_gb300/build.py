@@ -27,13 +27,20 @@ KSHOTS = [(0, 0, 0, 0), (0, 0, 1, 0), (0, 1, 0, 0), (0, 1, 1, 0), (1, 0, 0, 0), 
           (0, 0, 0, 1), (0, 0, 1, 1), (1, 0, 0, 1), (1, 0, 1, 1)]
 
 
+def _kshots_job(v, vec, tag):
+    flags = zip(("TAPE", "REF", "INTERIOR", "COMP", "VEC"), v + (vec,))
+    defs = [f"-DSF_{k}={'true' if b else 'false'}" for k, b in flags]
+    return "sf_shots_inst.cu", defs + [f"-DSF_KSHOTS_NAME=sf_kshots_{tag}"], f"sf_shots_{tag}.o"
+
+
 def _jobs():
     """(source, extra nvcc flags, object name) of every translation unit."""
     jobs = [(u, [], u.replace(".cu", ".o")) for u in UNITS]
     for v in KSHOTS:
         tag = "".join(str(b) for b in v)
-        defs = [f"-DSF_{k}={'true' if b else 'false'}" for k, b in zip(("TAPE", "REF", "INTERIOR", "COMP"), v)]
-        jobs.append(("sf_shots_inst.cu", defs + [f"-DSF_KSHOTS_NAME=sf_kshots_{tag}"], f"sf_shots_{tag}.o"))
+        jobs.append(_kshots_job(v, True, tag))
+    # the allocation-free solve works on the caller's own column stride
+    jobs.append(_kshots_job((0, 1, 1, 0), False, "noalloc"))
     return jobs
 
 

@@ -183,7 +183,7 @@ int sf_adj_configure(sf_ctx* c, cudaStream_t st, AdjLaunch* A)
     const void* akern = c->batch_interior ? (const void*)k_adjoint<true> : (const void*)k_adjoint<false>;
     int rc = sf_gang_shape(c, akern, smem, ns, nstrips, c->gang_warps, &G, &NG);
     if (rc) return rc;
-    rc = sf_dev_reserve(c, (void**)&c->d_lam, &c->cap_lam, (size_t)NG * c->nzz * c->batch_maxcols * sizeof(float));
+    rc = sf_dev_reserve(c, (void**)&c->d_lam, &c->cap_lam, (size_t)NG * strip_pitch(c->nzz) * c->batch_maxcols * sizeof(float));
     if (!rc) rc = sf_dev_reserve_zero(c, (void**)&c->d_hand2, &c->cap_hand2,
                                       (size_t)NG * hand_words(nstrips, c->batch_maxcols, 2) * sizeof(unsigned long long));
     if (!rc) rc = sf_dev_reserve(c, (void**)&c->d_lam_init, &c->cap_lam_init, (size_t)ns * 9 * sizeof(float));
@@ -207,7 +207,7 @@ int sf_adj_configure(sf_ctx* c, cudaStream_t st, AdjLaunch* A)
     p.NG = NG;
     p.maxcols = c->batch_maxcols;
     p.lam = c->d_lam;
-    p.lam_per_gang = (long long)c->nzz * c->batch_maxcols;
+    p.lam_per_gang = (long long)strip_pitch(c->nzz) * c->batch_maxcols;
     p.hand = c->d_hand2;
     p.bar = c->d_ctr2;
     p.tcode = c->d_tcode;

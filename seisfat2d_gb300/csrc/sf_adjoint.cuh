@@ -64,7 +64,7 @@ struct __align__(16) AdjRing {
 };
 
 struct AdjStripArgs {
-    float* lam;        // window adjoint field (column stride nzz), in place
+    float* lam;        // window adjoint field (column stride strip_pitch(nzz)), in place
     int nzz, ncols, k;
     bool down, right;  // directions of the reverse march
     const uint8_t* tcode;  // tape of this (sweep, strip): entries [fstep*32 + flane]
@@ -100,15 +100,17 @@ __device__ __forceinline__ void adj_strip(const AdjStripArgs& a)
     const int tix = r - rb;
     const int flane = 31 - lane;  // this row's lane in the forward strip
     AdjRing& R = *a.ring;
-    const bool lt_ok = (rb + lane) < nzz;
     CtaShared* sh = a.sh;
     const bool consumer = a.h_in != nullptr;
     const bool lane0 = lane == 0;
     const bool feeds = (lane == 31) && (a.h_out != nullptr);
     const int nsteps = ncols + 31;
     auto col_of = [&](int m) { return a.right ? m : ncols - 1 - m; };
-    const long long dL = a.right ? (long long)nzz : -(long long)nzz;
-    const float* pL = a.lam + (long long)(rb + lane) + (long long)col_of(0) * (long long)nzz;
+    // lane 8 u + c copies 16 bytes, rows rb+4c .. rb+4c+3, of the block's column u
+    const int vu = lane >> 3, vc = 4 * (lane & 7);
+    const long long ld = strip_pitch(nzz), dL = a.right ? ld : -ld;
+    const long long first = (long long)col_of(0) * ld + vu * dL + rb + vc;
+    const float* pL = a.lam + first;
     // the lane's 16 bytes of a block's tape rows (rows of steps q+U-1 .. q, forward step order)
     const long long fs0 = (long long)(ncols + 31 - kU) * 32;
     const float* pT1 = a.tc1 + fs0 + 4 * lane;
@@ -118,12 +120,8 @@ __device__ __forceinline__ void adj_strip(const AdjStripArgs& a)
     // FAST: every march of the call is inside the window (no bounds tests)
     auto stage = [&](int q, int slot, int tb, auto fast_tag) {
         constexpr bool FAST = decltype(fast_tag)::value;
-        float* d = &R.L[slot * 32 + lane];
-#pragma unroll
-        for (int u = 0; u < kU; u++) {
-            if ((FAST || q + u < ncols) && lt_ok) cp_async4(d + 32 * u, pL);
-            pL += dL;
-        }
+        if (FAST || q + vu < ncols) cp_async16_cg(&R.L[(slot + vu) * 32 + vc], pL);
+        pL += kU * dL;
         AdjTape& t = R.tape[tb];
         if (FAST || q + kU - 1 - (lane >> 3) < nsteps) {
             cp_async16_cg(&t.c1[4 * lane], pT1);
@@ -146,9 +144,6 @@ __device__ __forceinline__ void adj_strip(const AdjStripArgs& a)
             if (avail >= ncols) avail = 0x7fffffff;
         }
     };
-    // rows past the grid read zeros (their pushes stay zero)
-    if (!vrow)
-        for (int q = 0; q < kRingA; q++) R.L[q * 32 + tix] = 0.0f;
     ensure(kLookA);
 #pragma unroll 1
     for (int q = 0; q < kLookA; q += kU) {
@@ -161,9 +156,9 @@ __device__ __forceinline__ void adj_strip(const AdjStripArgs& a)
     }
 
     // running destinations: the term v of forward tape step ncols+30-s, the
-    // write-back of the next finished column (row r), the pair of march s-31
+    // columns written back by a block (march s0-kU-31 for its first), the pair of march s-31
     float* pV = a.tc2 + (long long)(ncols + 30) * 32 + flane;
-    float* pW = a.lam + (long long)r + (long long)col_of(0) * (long long)nzz;
+    float* pW = a.lam + first - (31 + kU) * dL;
     unsigned long long* pH = a.h_out - 2 * 31;
 
     float my_x = 0.0f, my_pe = 0.0f, my_pev = 0.0f, pev_hold = 0.0f;
@@ -197,18 +192,12 @@ __device__ __forceinline__ void adj_strip(const AdjStripArgs& a)
         }
         // write back the columns every lane had finished before this block (marches s0-kU-31 ..)
         {
-            int wb = b0 + (kRingA - 31 - kU);
-            if (wb >= kRingA) wb -= kRingA;
-#pragma unroll
-            for (int u = 0; u < kU; u++) {
-                const int m = s0 + u - kU - 31;
-                if (FAST || (m >= 0 && m < ncols)) {
-                    int ws = wb + u;
-                    if (ws >= kRingA) ws -= kRingA;
-                    if (vrow) *pW = R.L[ws * 32 + tix];
-                    pW += dL;
-                }
-            }
+            int ws = b0 + (kRingA - 31 - kU) + vu;
+            if (ws >= kRingA) ws -= kRingA;
+            const int m = s0 + vu - kU - 31;
+            if (FAST || (m >= 0 && m < ncols))
+                *reinterpret_cast<float4*>(pW) = *reinterpret_cast<const float4*>(&R.L[ws * 32 + vc]);
+            pW += kU * dL;
         }
         {
             // the upwind row of lane 0: the previous strip's pairs, or nothing
@@ -338,7 +327,7 @@ __device__ void adjoint_body(const AdjParams& p, const FuseParams* f)
     AdjRing* rings = reinterpret_cast<AdjRing*>(smem_raw + ((sizeof(CtaShared) + 15) & ~size_t(15)));
     const int tid = threadIdx.x;
     const GangPos gp = gang_pos(p.G);
-    const int nzz = p.nzz, nstrips = p.nstrips;
+    const int nzz = p.nzz, nstrips = p.nstrips, ld = strip_pitch(nzz);
     float* lam = p.lam + (size_t)gp.gang * p.lam_per_gang;
     const size_t row = 2 * (size_t)hand_pitch(p.maxcols);
     unsigned long long* hb = p.hand + (size_t)gp.gang * hand_words(nstrips, p.maxcols, 2);
@@ -362,7 +351,7 @@ __device__ void adjoint_body(const AdjParams& p, const FuseParams* f)
         // receiver accumulation, hence the same bits).
         {
             const int gt = gp.g * blockDim.x + tid, gn = p.G * blockDim.x;
-            const size_t nw = (size_t)nzz * ncols;
+            const size_t nw = (size_t)ld * ncols;  // rows past the grid stay zero
 #pragma unroll 4
             for (size_t q = gt; q < nw; q += gn) lam[q] = 0.0f;
             gang_barrier(bar, (++nbar) * p.G, cs, p.err);
@@ -380,7 +369,7 @@ __device__ void adjoint_body(const AdjParams& p, const FuseParams* f)
                     acc = fadd(acc, fmul(g, p.seed_w[e]));
                     any = true;
                 }
-                if (any) lam[(size_t)p.seed_row[n] + (size_t)col * nzz] = acc;
+                if (any) lam[(size_t)p.seed_row[n] + (size_t)col * ld] = acc;
             }
         }
         gang_barrier(bar, (++nbar) * p.G, cs, p.err);
@@ -420,7 +409,7 @@ __device__ void adjoint_body(const AdjParams& p, const FuseParams* f)
         if (gp.g == 0 && tid < 9) {
             const int aa = tid % 3, bb = tid / 3;
             const int zi = sh.sIdz + aa - 1, xl = sh.sIdx - sh.c0 + bb - 1;
-            p.lam_init[(size_t)sh.orig * 9 + tid] = lam[(size_t)zi + (size_t)xl * nzz];
+            p.lam_init[(size_t)sh.orig * 9 + tid] = lam[(size_t)zi + (size_t)xl * ld];
         }
         if (f && gp.g == 0) {
             __threadfence();
@@ -672,7 +661,7 @@ __device__ bool gather_tile(const GatherParams& p, GatherSmem& sm, int k, int cb
                         g[q] = fadd(g[q], fmul(li, __double2float_rn(d)));
                     }
                     if (VTI) {
-                        const float* f = p.vfac + t.q_off + (size_t)a + (size_t)bl * p.nzz;
+                        const float* f = p.vfac + t.q_off + (size_t)a + (size_t)bl * strip_pitch(p.nzz);
                         total[q] += (double)g[q] * (double)f[0];
                         t11[q] += (double)g[q] * (double)f[p.vfac_total];
                         t13[q] += (double)g[q] * (double)f[2 * p.vfac_total];

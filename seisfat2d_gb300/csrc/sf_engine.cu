@@ -131,13 +131,28 @@ __global__ void k_verify_div(const float* divs, int n, float* rbs, int* bad)
     }
 }
 
-// Sets *flag when a slowness of the field lies outside in_fast_range.
-__global__ void k_check_range(const float* __restrict__ S, size_t n, float dx, float dz, int* flag)
+// Sets *flag when a slowness of the field (nzz x nxx) lies outside
+// in_fast_range; with Sp, also copies the field at column stride ld (rows
+// past the grid repeat the last).
+__global__ void k_check_range(const float* __restrict__ S, int nzz, int nxx, int ld, float dx, float dz, int* flag,
+                              float* __restrict__ Sp)
 {
     bool ok = true;
-    for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x)
-        ok &= in_fast_range(S[q], dx, dz);
+    const size_t n = (size_t)ld * nxx;
+    for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x) {
+        const size_t j = q / ld;
+        const float s = S[min((int)(q - j * ld), nzz - 1) + j * nzz];
+        ok &= in_fast_range(s, dx, dz);
+        if (Sp) Sp[q] = s;
+    }
     if (!ok) *flag = 1;
+}
+
+// A window of column stride ld as nzz x ncols values.
+__global__ void k_unpitch(const float* __restrict__ in, int nzz, int ncols, int ld, float* __restrict__ out)
+{
+    for (int j = blockIdx.x; j < ncols; j += gridDim.x)
+        for (int i = threadIdx.x; i < nzz; i += blockDim.x) out[i + (size_t)j * nzz] = in[i + (size_t)j * ld];
 }
 
 // compute_seismogram on a device field (modeling.cu:161-194).
@@ -201,6 +216,8 @@ extern "C" int sf_ctx_create(sf_ctx** out, int nx, int nz, float dx, float dz, i
     size_t cap = 0;
     if (st == SF_OK) st = sf_dev_reserve(c, (void**)&c->d_S, &cap, sizeof(float) * (size_t)c->nxx * c->nzz);
     cap = 0;
+    if (st == SF_OK) st = sf_dev_reserve(c, (void**)&c->d_Sp, &cap, sizeof(float) * (size_t)c->nxx * strip_pitch(c->nzz));
+    cap = 0;
     if (st == SF_OK) st = sf_dev_reserve(c, (void**)&c->d_flags, &cap, 256);
     if (st == SF_OK) st = sf_cuda_check(c, cudaMemset(c->d_flags, 0, 256), "cudaMemset");
     if (st == SF_OK) st = sf_fwd_setup(c);
@@ -218,7 +235,7 @@ extern "C" int sf_ctx_destroy(sf_ctx* c)
     cudaSetDevice(c->dev);
     sf_plan_release(c);
     sf_adjoint_release(c);
-    void* bufs[] = {c->d_S, c->d_flags, c->d_shots, c->d_T, c->d_rx, c->d_rz, c->d_picks, c->d_Sq,
+    void* bufs[] = {c->d_S, c->d_Sp, c->d_Tc, c->d_flags, c->d_shots, c->d_T, c->d_rx, c->d_rz, c->d_picks, c->d_Sq,
                     c->d_tcode, c->d_tc1, c->d_tc2, c->d_model, c->d_cij_all, c->d_hand, c->d_ctr,
                     c->d_skern, c->d_upd, c->d_wav, c->d_mig, c->d_kgeo, c->d_kint, c->d_kpart,
                     c->d_vfac, c->d_gcij, c->d_fuse, c->d_Tl, c->d_srange};
@@ -381,6 +398,7 @@ const void* sf_kshots_0001();
 const void* sf_kshots_0011();
 const void* sf_kshots_1001();
 const void* sf_kshots_1011();
+const void* sf_kshots_noalloc();  // 0110 on windows of the caller's column stride
 }  // namespace sf
 
 // The compensated arithmetic has no reference-build variant.
@@ -437,14 +455,15 @@ int sf_fwd_setup(sf_ctx* c)
 
 // ------------------------------------------------------------------ models
 
-// Checks the context's slowness for the fast form of the updates (d_flags[2],
-// read by the solves), on the legacy stream like the copies that set it.
+// The solver's copy of the context's slowness at its column stride, and the
+// check for the fast form of the updates (d_flags[2], read by the solves).
 int sf_check_slowness(sf_ctx* c, cudaStream_t st)
 {
-    const size_t n = (size_t)c->nxx * c->nzz;
+    const int ld = strip_pitch(c->nzz);
+    const size_t n = (size_t)c->nxx * ld;
     CK(cudaMemsetAsync(c->d_flags + 2, 0, sizeof(int), st));
-    k_check_range<<<(unsigned)std::min<size_t>((n + 255) / 256, (size_t)c->sms * 8), 256, 0, st>>>(c->d_S, n, c->dx, c->dz,
-                                                                                                 c->d_flags + 2);
+    k_check_range<<<(unsigned)std::min<size_t>((n + 255) / 256, (size_t)c->sms * 8), 256, 0, st>>>(
+        c->d_S, c->nzz, c->nxx, ld, c->dx, c->dz, c->d_flags + 2, c->d_Sp);
     CK(cudaGetLastError());
     return SF_OK;
 }
@@ -633,11 +652,11 @@ int sf_prepare_shots(sf_ctx* c, const sf_shot* shots, int nshots, bool tape)
         for (int q = 0; q < 4; q++) { d.skip_i[q] = it->second[q]; d.skip_j[q] = it->second[4 + q]; }
         d.orig = b;
         d.t_off = toff;  // per-shot traveltime windows (tables, anisotropic batches)
-        toff += (long long)c->nzz * d.ncols;
+        toff += (long long)strip_pitch(c->nzz) * d.ncols;
         d.tape_off = tape_off;
         if (tape) tape_off += 4LL * nstrips * (d.ncols + 31) * 32;
         d.q_off = q_off;
-        q_off += (long long)c->nzz * d.ncols;
+        q_off += (long long)strip_pitch(c->nzz) * d.ncols;
         maxcols = std::max(maxcols, d.ncols);
         c->hshots[b] = d;
     }
@@ -664,7 +683,7 @@ int sf_fwd_configure(sf_ctx* c, int nrec, bool per_shot_T, bool tape, int gang_w
                      FwdLaunch* L, const float* Sshots)
 {
     const int nshots = (int)c->hshots.size();
-    const size_t nzz = c->nzz;
+    const int ld = strip_pitch(c->nzz);
     const int nstrips = (c->nzz + 31) / 32;
     const bool comp = c->arith == SF_ARITH_COMPENSATED;
     if (comp && c->warps > kMaxWarpsComp)
@@ -685,7 +704,7 @@ int sf_fwd_configure(sf_ctx* c, int nrec, bool per_shot_T, bool tape, int gang_w
     rc = sf_dev_reserve(c, (void**)&c->d_shots, &c->cap_shots, nshots * sizeof(ShotDev));
     if (rc) return rc;
     CK(cudaMemcpyAsync(c->d_shots, c->hshots.data(), nshots * sizeof(ShotDev), cudaMemcpyHostToDevice, st));
-    const long long t_per_gang = per_shot_T ? 0 : (long long)nzz * c->batch_maxcols;
+    const long long t_per_gang = per_shot_T ? 0 : (long long)ld * c->batch_maxcols;
     const size_t tfloats = per_shot_T ? (size_t)c->batch_T_floats : (size_t)NG * t_per_gang;
     rc = sf_dev_reserve(c, (void**)&c->d_T, &c->cap_T, tfloats * sizeof(float));
     if (rc) return rc;
@@ -709,9 +728,10 @@ int sf_fwd_configure(sf_ctx* c, int nrec, bool per_shot_T, bool tape, int gang_w
     }
     FwdParams& p = L->p;
     std::memset(&p, 0, sizeof(p));
-    p.S = c->d_S;
+    p.S = c->d_Sp;
     p.Sshots = Sshots;
     p.nzz = c->nzz;
+    p.ld = ld;
     p.nxx = c->nxx;
     p.nb = c->nb;
     p.kc = c->kc;
@@ -792,6 +812,7 @@ int sf_qp_launch(sf_ctx* c, bool fact, cudaStream_t st)
     std::memset(&q, 0, sizeof(q));
     q.S = c->d_S;
     q.nzz = c->nzz;
+    q.ld = strip_pitch(c->nzz);
     q.nb = c->nb;
     q.kc = c->kc;
     q.shots = c->d_shots;
@@ -931,6 +952,24 @@ extern "C" int sf_batch_forward(sf_ctx* c, int ani, const sf_shot* shots, int ns
     return SF_OK;
 }
 
+// A traveltime window of the solver's column stride to the caller's nzz x ncols buffer.
+static int table_out(sf_ctx* c, const float* window, int ncols, float* T, int mem, cudaStream_t st)
+{
+    const size_t n = (size_t)c->nzz * ncols;
+    float* out = T;
+    if (mem != SF_MEM_DEVICE) {
+        int rc = sf_dev_reserve(c, (void**)&c->d_Tc, &c->cap_Tc, n * sizeof(float));
+        if (rc) return rc;
+        out = c->d_Tc;
+    }
+    k_unpitch<<<std::min(ncols, 65535), std::min(256, strip_pitch(c->nzz)), 0, st>>>(window, c->nzz, ncols,
+                                                                                     strip_pitch(c->nzz), out);
+    CK(cudaGetLastError());
+    if (mem == SF_MEM_DEVICE) return SF_OK;
+    CK(cudaMemcpyAsync(T, out, n * sizeof(float), cudaMemcpyDeviceToHost, st));
+    return sf_check_flags(c, st);
+}
+
 extern "C" int sf_batch_table(sf_ctx* c, int shot, float* T, int mem, void* stream)
 {
     if (!c || !T) return SF_ERR_ARG;
@@ -939,10 +978,7 @@ extern "C" int sf_batch_table(sf_ctx* c, int shot, float* T, int mem, void* stre
     CK(cudaSetDevice(c->dev));
     const ShotDev& d = c->hshots[c->tables_index[shot]];
     cudaStream_t st = (cudaStream_t)stream;
-    CK(cudaMemcpyAsync(T, c->d_T + d.t_off, sizeof(float) * (size_t)c->nzz * d.ncols,
-                       mem == SF_MEM_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, st));
-    if (mem == SF_MEM_HOST) return sf_check_flags(c, st);
-    return SF_OK;
+    return table_out(c, c->d_T + d.t_off, d.ncols, T, mem, st);
 }
 
 // The tape is kept per (sweep, strip) in the strip's skewed step order: entry
@@ -992,26 +1028,10 @@ extern "C" int sf_time_propagation(sf_ctx* c, int ani, float sx, float sz, float
     sf_shot s{sx, sz, 0, c->nxx};
     int rc = sf_prepare_shots(c, &s, 1, false);
     if (rc) return rc;
-    const size_t npad = (size_t)c->nxx * c->nzz;
-    // the whole-grid table is written straight into the caller's device buffer
-    float* keepT = c->d_T;
-    size_t keepcap = c->cap_T;
-    if (T_mem == SF_MEM_DEVICE) {
-        c->d_T = T;
-        c->cap_T = npad * sizeof(float);
-    }
     rc = sf_launch_shots(c, ani, 0, nullptr, true, false, c->gang_warps, st);
-    if (T_mem == SF_MEM_DEVICE) {
-        c->d_T = keepT;
-        c->cap_T = keepcap;
-        c->tables_valid = false;
-    }
     if (rc) return rc;
-    if (T_mem == SF_MEM_HOST) {
-        CK(cudaMemcpyAsync(T, c->d_T, npad * sizeof(float), cudaMemcpyDeviceToHost, st));
-        return sf_check_flags(c, st);
-    }
-    return SF_OK;
+    if (T_mem == SF_MEM_DEVICE) c->tables_valid = false;
+    return table_out(c, c->d_T, c->nxx, T, T_mem, st);
 }
 
 extern "C" int sf_compute_seismogram(sf_ctx* c, const float* T_dev, const float* rx, const float* rz,

@@ -62,6 +62,7 @@ struct sf_ctx {
     std::string err;
 
     float* d_S = nullptr;       // padded slowness
+    float* d_Sp = nullptr;      // the same at the solver's column stride (sf_check_slowness)
     int* d_flags = nullptr;     // [1] error flag, [2] the slowness has a value outside in_fast_range
     float* d_model = nullptr;
     size_t cap_model = 0;
@@ -84,6 +85,7 @@ struct sf_ctx {
 
     sf::ShotDev* d_shots = nullptr; size_t cap_shots = 0;
     float* d_T = nullptr; size_t cap_T = 0;
+    float* d_Tc = nullptr; size_t cap_Tc = 0;  // a table on its way to a host buffer
     float* d_Tl = nullptr; size_t cap_Tl = 0;  // lo parts of the traveltimes (compensated arithmetic)
     float* d_rx = nullptr; size_t cap_rx = 0;
     float* d_rz = nullptr; size_t cap_rz = 0;
@@ -173,7 +175,7 @@ int sf_dev_reserve_zero(sf_ctx* c, void** p, size_t* cap, size_t bytes);
 // Next handoff-tag epoch (never 0; wraps within 22 bits).
 unsigned sf_next_epoch(sf_ctx* c);
 int sf_check_flags(sf_ctx* c, cudaStream_t st);
-// Device check of the context's slowness after it changed.
+// The solver's copy and the range check of the context's slowness after it changed.
 int sf_check_slowness(sf_ctx* c, cudaStream_t st);
 int sf_fwd_setup(sf_ctx* c);
 int sf_verify_divisors(sf_ctx* c);

@@ -17,15 +17,16 @@ struct ShotDev {
     int skip_j[4];        // (window coordinates, -1 = none), per sweep
     int orig;             // index of the shot in the caller's order
     int pad_;
-    long long t_off;      // traveltime window offset (floats) when tables are kept
+    long long t_off;      // traveltime window offset (floats, column stride strip_pitch) when tables are kept
     long long tape_off;   // tape offset (entries)
-    long long q_off;      // window cells of the shots before it (qP slowness and derivative factors)
+    long long q_off;      // offset of its qP slowness window and derivative factors (floats, column stride strip_pitch)
 };
 
 struct FwdParams {
-    const float* S;       // padded slowness, column stride nzz
-    const float* Sshots;  // per-shot slowness windows at q_off (column stride nzz) instead of S, or nullptr
+    const float* S;       // padded slowness, column stride ld
+    const float* Sshots;  // per-shot slowness windows at q_off (same stride) instead of S, or nullptr
     int nzz, nxx, nb;
+    int ld;               // column stride of the slowness and traveltime windows: strip_pitch(nzz) (VEC), or nzz
     Consts kc;
     const ShotDev* shots;
     int nshots;
@@ -65,7 +66,7 @@ __device__ __forceinline__ void init_block(const FwdParams& p, const ShotDev& sh
     if (tid < 9) {
         const int a = tid % 3, bb = tid / 3;
         const int zi = sh.sIdz + a - 1, xl = sh.sIdx - sh.c0 + bb - 1;
-        const float s = Sw[zi + (size_t)xl * p.nzz];
+        const float s = Sw[zi + (size_t)xl * p.ld];
         if (REF)
             out[tid] = src_value_f32(s, zi, xl + sh.c0, p.nb, p.kc.dx, p.kc.dz, sh.sx, sh.sz);
         else
@@ -98,15 +99,15 @@ __device__ __forceinline__ GangPos gang_pos(int G)
 }
 
 // One strip of a sweep in the loop form the shot needs.
-template <bool RIGHT, bool TAPE, bool REF, bool INTERIOR, bool COMP>
+template <bool RIGHT, bool TAPE, bool REF, bool INTERIOR, bool COMP, bool VEC>
 __device__ __forceinline__ void strip(const StripArgs& a, bool exact)
 {
     if (exact)
-        run_strip<RIGHT, TAPE, REF, false, false, COMP, true>(a);
+        run_strip<RIGHT, TAPE, REF, false, false, COMP, true, VEC>(a);
     else if (a.kc.dx == a.kc.dz)
-        run_strip<RIGHT, TAPE, REF, INTERIOR, true, COMP, false>(a);
+        run_strip<RIGHT, TAPE, REF, INTERIOR, true, COMP, false, VEC>(a);
     else
-        run_strip<RIGHT, TAPE, REF, INTERIOR, false, COMP, false>(a);
+        run_strip<RIGHT, TAPE, REF, INTERIOR, false, COMP, false, VEC>(a);
 }
 
 // The four sweeps of one solve of the current shot. Sweeps 0 (down) and 1
@@ -122,9 +123,8 @@ __device__ __forceinline__ void strip(const StripArgs& a, bool exact)
 // between sweeps. Square cells (dx and dz equal) run the strip loops'
 // square-cell form. COMP: compensated arithmetic, lo parts in Tl, two handoff
 // pairs per column.
-template <bool TAPE, bool REF, bool INTERIOR, bool COMP>
-__device__ void solve_window(const FwdParams& p, const ShotDev& sh, const GangPos& gp, const float* Sw,
-                             int ldS, float* T, float* Tl, unsigned tag, bool exact, CtaShared* cs, unsigned char* rings)
+template <bool TAPE, bool REF, bool INTERIOR, bool COMP, bool VEC>
+__device__ void solve_window(const FwdParams& p, const ShotDev& sh, const GangPos& gp, const float* Sw, float* T, float* Tl, unsigned tag, bool exact, CtaShared* cs, unsigned char* rings)
 {
     const int nzz = p.nzz, ncols = sh.ncols;
     const int nstrips = (nzz + 31) >> 5;
@@ -134,7 +134,7 @@ __device__ void solve_window(const FwdParams& p, const ShotDev& sh, const GangPo
     unsigned long long* prog = hb + 4 * (size_t)nstrips * row;
     StripArgs a;
     a.S = Sw;
-    a.ldS = ldS;
+    a.ld = p.ld;
     a.T = T;
     a.Tl = Tl;
     a.nzz = nzz;
@@ -173,9 +173,9 @@ __device__ void solve_window(const FwdParams& p, const ShotDev& sh, const GangPo
             a.tc2 = p.tc2 + base;
         }
         if (sw < 2)
-            strip<true, TAPE, REF, INTERIOR, COMP>(a, exact);
+            strip<true, TAPE, REF, INTERIOR, COMP, VEC>(a, exact);
         else
-            strip<false, TAPE, REF, INTERIOR, COMP>(a, exact);
+            strip<false, TAPE, REF, INTERIOR, COMP, VEC>(a, exact);
     }
 }
 
@@ -185,7 +185,7 @@ __device__ void solve_window(const FwdParams& p, const ShotDev& sh, const GangPo
 // strip loops' bounds-test-free body for interior blocks (see run_strip).
 // COMP: compensated arithmetic (node_update_comp; the 3x3 initial values are
 // the FP64 ones rounded once).
-template <bool TAPE, bool REF, bool INTERIOR, bool COMP = false>
+template <bool TAPE, bool REF, bool INTERIOR, bool COMP = false, bool VEC = true>
 // Register bounds: 168 keep three warps per scheduler (and 8 per CTA); the
 // plain FP32 kernels run CTAs of up to 16 warps, hence 128.
 __global__ void __maxnreg__((COMP || (TAPE && INTERIOR)) ? 168 : 128)
@@ -213,12 +213,12 @@ __global__ void __maxnreg__((COMP || (TAPE && INTERIOR)) ? 168 : 128)
         float* Tl = !COMP ? nullptr
                           : (p.t_per_gang > 0) ? p.Tlpool + (size_t)gp.gang * p.t_per_gang : p.Tlpool + sh.t_off;
         // the shot's slowness window: columns c0.. of S, or its own qP slowness
-        const float* Sw = p.Sshots ? p.Sshots + sh.q_off : p.S + (size_t)sh.c0 * nzz;
+        const float* Sw = p.Sshots ? p.Sshots + sh.q_off : p.S + (size_t)sh.c0 * p.ld;
         const unsigned tag = (p.epoch << 10) | (unsigned)(it & 1023);
         init_block<REF>(p, sh, Sw, cs->init);
         __syncthreads();
         const bool exact = p.kc.mflags != kFastFlags || p.srange[p.Sshots ? b : 0] != 0;
-        solve_window<TAPE, REF, INTERIOR, COMP>(p, sh, gp, Sw, nzz, T, Tl, tag, exact, cs, rings);
+        solve_window<TAPE, REF, INTERIOR, COMP, VEC>(p, sh, gp, Sw, T, Tl, tag, exact, cs, rings);
         // receivers (modeling.cu:161-194), spread over the gang once the field is final
         if (p.nrec > 0 && p.picks) {
             gang_barrier(bar, (++nbar) * p.G, cs, p.err);
@@ -227,7 +227,7 @@ __global__ void __maxnreg__((COMP || (TAPE && INTERIOR)) ? 168 : 128)
                 float xd, zd;
                 float v = __int_as_float(0x7fc00000);
                 if (pick_geom(p.rx[r], p.rz[r], p.kc.dx, p.kc.dz, p.nb, nzz, sh.ncols, sh.c0, i, j, xd, zd))
-                    v = pick_value(T, nzz, i, j, xd, zd);
+                    v = pick_value(T, p.ld, i, j, xd, zd);
                 p.picks[(size_t)sh.orig * p.nrec + r] = v;
             }
         }
@@ -246,8 +246,9 @@ __global__ void __maxnreg__((COMP || (TAPE && INTERIOR)) ? 168 : 128)
 // rows (coalesced, z fastest; four rows per thread unrolled measured 1.5%
 // faster on the VTI batch than 256 threads one row at a time).
 struct QpParams {
-    const float* S;       // padded slowness, column stride nzz
+    const float* S;       // padded slowness, column stride nzz (as the codes)
     int nzz, nb;
+    int ld;               // column stride of the shots' windows
     Consts kc;
     const ShotDev* shots;
     int nshots;
@@ -264,7 +265,7 @@ struct QpParams {
 template <bool REF, bool COMP, bool FACT>
 __global__ void __launch_bounds__(128) k_qp(QpParams p)
 {
-    const int nzz = p.nzz, nb = p.nb;
+    const int nzz = p.nzz, nb = p.nb, ld = p.ld;
 #pragma unroll 1
     for (int b = blockIdx.y; b < p.nshots; b += gridDim.y) {
         const ShotDev sh = p.shots[b];
@@ -276,7 +277,7 @@ __global__ void __launch_bounds__(128) k_qp(QpParams p)
         for (int j = blockIdx.x; j < ncols; j += gridDim.x)
 #pragma unroll 4
         for (int i = threadIdx.x; i < nzz; i += blockDim.x) {
-            const size_t idx = (size_t)i + (size_t)j * nzz;
+            const size_t idx = (size_t)i + (size_t)j * ld;
             const size_t g = (size_t)i + (size_t)(sh.c0 + j) * nzz;
             const float s = p.S[g];
             float out = s;
@@ -294,10 +295,10 @@ __global__ void __launch_bounds__(128) k_qp(QpParams p)
                 if (COMP) {
                     const float* Lc = Tl + idx;
                     dzr = ff_diff(Tc[1], Lc[1], Tc[-1], Lc[-1]);
-                    dxr = ff_diff(Tc[nzz], Lc[nzz], Tc[-(long)nzz], Lc[-(long)nzz]);
+                    dxr = ff_diff(Tc[ld], Lc[ld], Tc[-(long)ld], Lc[-(long)ld]);
                 } else {
                     dzr = fsub(Tc[1], Tc[-1]);
-                    dxr = fsub(Tc[nzz], Tc[-(long)nzz]);
+                    dxr = fsub(Tc[ld], Tc[-(long)ld]);
                 }
                 out = qp_slowness<REF>(dzr, dxr, s, p.kc.dx, p.kc.dz, c11, c13, c15, c33, c35, c55);
                 if (FACT) qp_factors(dzr, dxr, s, p.kc.dx, p.kc.dz, c11, c13, c15, c33, c35, c55, fS, f11, f13);

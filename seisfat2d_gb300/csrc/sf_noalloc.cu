@@ -67,7 +67,7 @@ int noalloc_setup(int dev, unsigned char** addr)
     if (!g_scratch_addr[dev]) {
         void* p = nullptr;
         if (cudaGetSymbolAddress(&p, g_noalloc_scratch) != cudaSuccess || !p) return SF_ERR_CUDA;
-        if (cudaFuncSetAttribute(sf_kshots_kernel(false, true, true, false), cudaFuncAttributeMaxDynamicSharedMemorySize,
+        if (cudaFuncSetAttribute(sf_kshots_noalloc(), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)sf_fwd_smem_bytes(kMaxWarps, false)) != cudaSuccess)
             return SF_ERR_CUDA;
         // the tagged pairs must not start with a valid-looking tag
@@ -177,13 +177,14 @@ extern "C" int sf_time_propagation_noalloc(const float* S, int nx, int nz, float
         g_verified[dev] = true;
     }
     const size_t npad = (size_t)nxx * nzz;
-    k_check_range<<<(unsigned)std::min<size_t>((npad + 255) / 256, (size_t)g_sms[dev] * 8), 256, 0, st>>>(S, npad, dx, dz,
-                                                                                                       &dh->srange);
+    k_check_range<<<(unsigned)std::min<size_t>((npad + 255) / 256, (size_t)g_sms[dev] * 8), 256, 0, st>>>(
+        S, nzz, nxx, nzz, dx, dz, &dh->srange, nullptr);
     if (cudaGetLastError() != cudaSuccess) return SF_ERR_CUDA;
     FwdParams p{};
     p.srange = &dh->srange;
     p.S = S;
     p.nzz = nzz;
+    p.ld = nzz;  // the caller's buffers, which this call cannot copy
     p.nxx = nxx;
     p.nb = nb;
     p.kc = k;
@@ -200,7 +201,7 @@ extern "C" int sf_time_propagation_noalloc(const float* S, int nx, int nz, float
     p.epoch = epoch;
     const int warps = 8;
     void* args[] = {&p};
-    if (cudaLaunchKernel(sf_kshots_kernel(false, true, true, false), dim3(1), dim3(warps * 32), args,
+    if (cudaLaunchKernel(sf_kshots_noalloc(), dim3(1), dim3(warps * 32), args,
                          sf_fwd_smem_bytes(warps, false), st) != cudaSuccess)
         return SF_ERR_CUDA;
     int err = 0;

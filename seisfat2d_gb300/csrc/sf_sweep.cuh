@@ -24,15 +24,19 @@
 // sweep's strip publishes how many columns it has written back (a fence and
 // a tagged counter, every 32 columns) and the later one stays behind it.
 //
-// Column chunks are staged into a per-warp shared-memory ring by cp.async,
-// a few march columns ahead (32 consecutive rows = one coalesced 128-byte
-// request per field), and lane l reads its own row of column s-l from the
-// ring. A ring slot holds one column: slowness rows rb-1..rb+31 at 0..32,
-// traveltimes at 33..64 and, in the compensated arithmetic, their lo parts at
-// 65..96. With slot pitches of 66 and 98 floats both the coalesced fill and
-// the skewed read are bank-conflict free, and one address serves all fields
-// of a node. Finished columns go back to global memory through the same
-// ring, coalesced. The march runs in blocks of a few steps: one wait for the
+// Columns are staged into a per-warp shared-memory ring by cp.async, a few
+// march columns ahead, and lane l reads its own row of column s-l from the
+// ring. A ring slot holds one column: slowness rows rb-1..rb+31 at 3..35,
+// traveltimes at 36..67 and, in the compensated arithmetic, their lo parts at
+// 68..99; one address serves all fields of a node, and with odd differences
+// of pitch and row stride the skewed reads are (but for the lanes past the
+// ring's end) bank-conflict free. The solver's own slowness and traveltime
+// windows have a column stride of whole strips (VEC), so a strip's column is
+// one aligned 128-byte line and the four columns of a block are one 16-byte
+// copy per lane and field; finished columns go back the same way, one
+// 16-byte load and store per lane. (Columns at the caller's stride, every one
+// at another alignment, took a 4-byte copy per lane and column, two lines per
+// column and L1 to merge them.) The march runs in blocks of a few steps: one wait for the
 // staged columns per block, the block's ring reads, its node updates
 // (the only serial chain), then its stores.
 //
@@ -61,16 +65,15 @@ struct FwdBlock {
     static constexpr int LOOK = 8;
     static constexpr int PLOOK = 4;
     static constexpr int AHEAD = PLOOK + U;
-    static constexpr int RING = 48;
-    static constexpr int SLOT = COMP ? 98 : 66;   // floats per slot
-    static constexpr int PAIRS = 16;              // columns of the pair ring
-    static_assert(LOOK % U == 0 && PLOOK % U == 0 && PLOOK <= LOOK && RING % U == 0 && RING >= 31 + LOOK + 2 * U,
-                  "ring too small");
+    static constexpr int RING = 47;
+    static constexpr int SLOT = COMP ? 100 : 68;  // floats per slot
+    static constexpr int PAIRS = 8;               // columns of the pair ring
+    static_assert(LOOK % U == 0 && PLOOK % U == 0 && PLOOK <= LOOK && RING >= 31 + LOOK + 2 * U, "ring too small");
     static_assert(PAIRS % U == 0 && PAIRS >= PLOOK + U && U % 2 == 0, "pair ring too small");
-    static_assert((RING * SLOT) % 32 == 0 && SLOT % 32 == 2, "the skewed reads would conflict");
-    static_assert((RING * SLOT) % 4 == 0, "the pair ring must be 16-byte aligned");
+    static_assert(SLOT % 4 == 0, "16-byte copies");
+    static_assert(U == 4, "a block's columns are one 16-byte copy per lane");
 };
-constexpr int kT0 = 33, kL0 = 65;  // traveltimes and their lo parts in a slot
+constexpr int kS0 = 3, kT0 = 36, kL0 = 68;  // slowness rows rb-1.., traveltimes, their lo parts in a slot
 constexpr int kPublish = 32;       // columns between two publications of a strip's progress
 constexpr int kMaxWarps = 16;
 // compensated kernels keep a second traveltime ring (the lo parts): at most
@@ -92,6 +95,9 @@ constexpr size_t ring_bytes()
     using B = FwdBlock<COMP>;
     return sizeof(float) * (size_t)B::RING * B::SLOT + 8 * (size_t)B::PAIRS * (COMP ? 2 : 1);
 }
+
+// Column stride of the solver's own windows: whole strips.
+__host__ __device__ constexpr int strip_pitch(int nzz) { return (nzz + 31) & ~31; }
 
 // Columns a row of handoff pairs is padded to: whole 16-byte pairs of pairs
 // past the last column.
@@ -162,9 +168,9 @@ __device__ __forceinline__ float val_of(unsigned long long e) { return __uint_as
 
 // Everything one warp needs for one strip of one sweep.
 struct StripArgs {
-    const float* S;   // slowness of the window, column stride ldS
-    int ldS;
-    float* T;         // traveltimes of the window, column stride nzz
+    const float* S;   // slowness of the window
+    float* T;         // traveltimes of the window
+    int ld;           // column stride of both: strip_pitch(nzz) (VEC), or nzz
     float* Tl;        // compensated: their lo parts, same layout
     int nzz, ncols;
     int k;            // strip index: rows [32k, 32k+32)
@@ -299,7 +305,8 @@ __device__ __forceinline__ void wait_counter(const unsigned* p, unsigned target,
 // more for it than a select: of the two slowness columns a lane holds, the
 // carried one is the cell column on the upwind side (j1) in either direction,
 // and the new one the other. Marches to the left read one column ahead.
-template <bool RIGHT, bool TAPE, bool REF, bool INTERIOR, bool SQ, bool COMP, bool EXACT>
+// VEC: the windows' column stride is strip_pitch(nzz).
+template <bool RIGHT, bool TAPE, bool REF, bool INTERIOR, bool SQ, bool COMP, bool EXACT, bool VEC>
 __device__ __forceinline__ void run_strip(const StripArgs& a)
 {
     using B = FwdBlock<COMP>;
@@ -320,13 +327,6 @@ __device__ __forceinline__ void run_strip(const StripArgs& a)
 
     float* ring = reinterpret_cast<float*>(a.ring);
     float* pring = ring + RING * P;          // handoff pairs of march q at (q mod PAIRS) * 2 HS
-
-    // global rows this lane stages
-    const int ls_row = rb - 1 + lane;
-    const bool ls_ok = (ls_row >= 0) && (ls_row < nzz);
-    const bool lx_ok = (lane < U) && (rb + 31 < nzz);  // lanes 0..U-1: the halo row of the block's columns
-    const bool lt_ok = (rb + lane) < nzz;
-    const int ldS = a.ldS;
 
     CtaShared* sh = a.sh;
     const bool consumer = a.h_in != nullptr;
@@ -353,42 +353,61 @@ __device__ __forceinline__ void run_strip(const StripArgs& a)
     g0 = (gn < 0) ? -(1 << 30) : g0 - (U - 1);
     gn = (gn < 0) ? 0 : gn + U - 1 + 31;
 
-    // running source addresses of the next march columns to stage
-    const long long dcol = right ? 1 : -1;
-    const long long dS = dcol * (long long)ldS, dT = dcol * (long long)nzz;
-    const float* pS = a.S + (long long)ls_row + (long long)col_of(0) * (long long)ldS;
-    const float* pX = a.S + (long long)(rb + 31) + (long long)col_of(0) * (long long)ldS + lane * dS;
-    const float* pT = a.T + (long long)(rb + lane) + (long long)col_of(0) * (long long)nzz;
-    const float* pTl = COMP ? a.Tl + (long long)(rb + lane) + (long long)col_of(0) * (long long)nzz : nullptr;
-    // columns q .. q+U-1 into slots slot .. slot+U-1 (U divides RING: no wrap)
+    // running source addresses of the next march columns to stage. VEC: lane
+    // 8 u + c copies 16 bytes, rows rb+4c .. rb+4c+3, of the block's column u;
+    // lanes 0..U-1 the row above of column `lane`. Else lane l copies row
+    // rb-1+l (traveltimes rb+l) of every column, lanes 0..U-1 also row rb+31.
+    const int vu = lane >> 3, vc = 4 * (lane & 7);
+    const long long dT = (right ? 1 : -1) * (long long)a.ld;
+    const long long c00 = (long long)col_of(0) * (long long)a.ld;
+    const int ls_row = rb - 1 + lane;
+    const bool ls_ok = VEC || ((ls_row >= 0) && (ls_row < nzz));
+    const bool lt_ok = VEC || (rb + lane) < nzz;
+    const bool lx_ok = (lane < U) && (VEC ? a.k > 0 : rb + 31 < nzz);
+    const long long first = VEC ? c00 + vu * dT + rb + vc : c00 + rb + lane;
+    const float* pS = a.S + (VEC ? first : first - 1);
+    const float* pX = a.S + (c00 + lane * dT + (VEC ? rb - 1 : rb + 31));
+    const float* pT = a.T + first;
+    const float* pTl = COMP ? a.Tl + first : nullptr;
+    // columns q .. q+U-1 into the slots from `slot`
     // FAST: every march the call touches lies inside the window (no bounds tests)
     auto stage_cols = [&](int q, int slot, auto fast_tag) {
         constexpr bool FAST = decltype(fast_tag)::value;
-        float* d = ring + slot * P + lane;
-#pragma unroll
-        for (int u = 0; u < U; u++) {
-            if ((FAST || q + u < ncols) && ls_ok) cp_async4(d + u * P, pS);
-            pS += dS;
-        }
-        if (sw0) {
-#pragma unroll
-            for (int u = 0; u < U; u++) {
-                d[u * P + kT0] = kBig;
-                if (COMP) d[u * P + kL0] = 0.0f;
+        auto wrap = [](int sl) { return sl >= RING ? sl - RING : sl; };
+        if constexpr (VEC) {
+            float* d = ring + wrap(slot + vu) * P + vc;
+            const bool in = FAST || q + vu < ncols;
+            if (in) cp_async16_cg(d + kS0 + 1, pS);
+            if (sw0) {
+                *reinterpret_cast<float4*>(d + kT0) = make_float4(kBig, kBig, kBig, kBig);
+                if (COMP) *reinterpret_cast<float4*>(d + kL0) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            } else if (in) {
+                cp_async16_cg(d + kT0, pT);
+                if (COMP) cp_async16_cg(d + kL0, pTl);
             }
+            pS += U * dT;
+            pT += U * dT;
+            if (COMP) pTl += U * dT;
         } else {
 #pragma unroll
             for (int u = 0; u < U; u++) {
-                if ((FAST || q + u < ncols) && lt_ok) {
-                    cp_async4(d + u * P + kT0, pT);
-                    if (COMP) cp_async4(d + u * P + kL0, pTl);
+                float* d = ring + wrap(slot + u) * P + lane;
+                const bool in = FAST || q + u < ncols;
+                if (in && ls_ok) cp_async4(d + kS0, pS);
+                if (sw0) {
+                    d[kT0] = kBig;
+                    if (COMP) d[kL0] = 0.0f;
+                } else if (in && lt_ok) {
+                    cp_async4(d + kT0, pT);
+                    if (COMP) cp_async4(d + kL0, pTl);
                 }
+                pS += dT;
                 pT += dT;
                 if (COMP) pTl += dT;
             }
         }
-        if (lx_ok && (FAST || q + lane < ncols)) cp_async4(ring + (slot + lane) * P + 32, pX);
-        pX += U * dS;
+        if (lx_ok && (FAST || q + lane < ncols)) cp_async4(ring + wrap(slot + lane) * P + (VEC ? kS0 : kS0 + 32), pX);
+        pX += U * dT;
     };
     // the upwind row's pairs of marches q .. q+U-1
     auto stage_pairs = [&](int q, auto fast_tag) {
@@ -420,9 +439,11 @@ __device__ __forceinline__ void run_strip(const StripArgs& a)
         cp_commit();
     }
 
-    // running destinations: write-back of the next finished column (row r), tape entry s*32+lane
-    float* pW = a.T + (long long)r + (long long)col_of(0) * (long long)nzz;
-    float* pWl = COMP ? a.Tl + (long long)r + (long long)col_of(0) * (long long)nzz : nullptr;
+    // running destinations: the columns written back by a block (march s0-U-31
+    // for its first), the next pair, the tape entry s*32+lane
+    const long long wfirst = VEC ? first - (31 + U) * dT : c00 + r - (31 + U) * dT;
+    float* pW = a.T + wfirst;
+    float* pWl = COMP ? a.Tl + wfirst : nullptr;
     unsigned long long* pH = a.h_out - 31 * HS;
     uint8_t* pcode = TAPE ? a.tcode + lane : nullptr;
     float* pc1 = TAPE ? a.tc1 + lane : nullptr;
@@ -433,7 +454,7 @@ __device__ __forceinline__ void run_strip(const StripArgs& a)
     float cU = 0.0f, cI = 0.0f, cN = 0.0f;                // carried S of rows r-1, r and i1 (the one of the two on the upwind side)
     const int nsteps = ncols + 31;
     int b0 = 0;                                           // ring slot of march s0
-    // ring offset of the lane's march s0 - lane (its row's first slowness)
+    // ring offset of the lane's march s0 - lane and row
     int ro = ((RING - lane) % RING) * P + tix;
 
     // Blocks of U steps: one wait for the staged columns per block, then the
@@ -464,8 +485,8 @@ __device__ __forceinline__ void run_strip(const StripArgs& a)
             if (ro >= RING * P + tix) ro -= RING * P;
             // S of the new column: march m (rightward) or m+1
             const int ns = right ? off[u] : ro;
-            nU[u] = ring[ns];
-            nI[u] = ring[ns + 1];
+            nU[u] = ring[ns + kS0];
+            nI[u] = ring[ns + kS0 + 1];
             told[u] = ring[off[u] + kT0];
             toldl[u] = COMP ? ring[off[u] + kL0] : 0.0f;
         }
@@ -473,21 +494,30 @@ __device__ __forceinline__ void run_strip(const StripArgs& a)
         {
             int wb = b0 + (RING - 31 - U);
             if (wb >= RING) wb -= RING;
-            const float* q = ring + kT0 + tix;
-#pragma unroll
-            for (int u = 0; u < U; u++) {
-                const int m = s0 + u - U - 31;
+            if constexpr (VEC) {
+                int ws = wb + vu;
+                if (ws >= RING) ws -= RING;
+                const int m = s0 + vu - U - 31;
                 if (FAST || (m >= 0 && m < ncols)) {
+                    const float* q = ring + ws * P + vc;
+                    *reinterpret_cast<float4*>(pW) = *reinterpret_cast<const float4*>(q + kT0);
+                    if (COMP) *reinterpret_cast<float4*>(pWl) = *reinterpret_cast<const float4*>(q + kL0);
+                }
+            } else {
+                const float* q = ring + kT0 + tix;
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    const int m = s0 + u - U - 31;
                     int ws = wb + u;
                     if (ws >= RING) ws -= RING;
-                    if (vrow) {
-                        *pW = q[ws * P];
-                        if (COMP) *pWl = q[ws * P + kL0 - kT0];
+                    if (vrow && (FAST || (m >= 0 && m < ncols))) {
+                        pW[u * dT] = q[ws * P];
+                        if (COMP) pWl[u * dT] = q[ws * P + kL0 - kT0];
                     }
-                    pW += dT;
-                    if (COMP) pWl += dT;
                 }
             }
+            pW += U * dT;
+            if (COMP) pWl += U * dT;
         }
         // the upwind strip's values of the block (every lane reads them, lane 0 uses them)
         float hv[U], hvl[U];

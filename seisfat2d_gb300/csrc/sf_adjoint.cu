@@ -19,8 +19,8 @@ using namespace sf;
 
 void sf_adjoint_release(sf_ctx* c)
 {
-    void* bufs[] = {c->d_lam, c->d_vrec, c->d_gshot, c->d_pg, c->d_misfit, c->d_colptr,
-                    c->d_lam_init, c->d_hand2, c->d_ctr2, c->d_seed_i, c->d_seed_w, c->d_gshots};
+    void* bufs[] = {c->d_lam, c->d_gshot, c->d_pg, c->d_misfit, c->d_colptr,
+                    c->d_lam_init, c->d_hand2, c->d_ctr2, c->d_seed_i, c->d_seed_w, c->d_gshots, c->d_vflag};
     for (void* b : bufs)
         if (b) cudaFree(b);
 }
@@ -188,6 +188,8 @@ int sf_adj_configure(sf_ctx* c, cudaStream_t st, AdjLaunch* A)
                                       (size_t)NG * hand_words(nstrips, c->batch_maxcols, 2) * sizeof(unsigned long long));
     if (!rc) rc = sf_dev_reserve(c, (void**)&c->d_lam_init, &c->cap_lam_init, (size_t)ns * 9 * sizeof(float));
     const size_t nctr = gang_counters(NG);
+    const size_t nflag = ((size_t)c->batch_tape_entries >> 10) + 1;
+    if (!rc) rc = sf_dev_reserve(c, (void**)&c->d_vflag, &c->cap_vflag, nflag);
     if (!rc) rc = sf_dev_reserve(c, (void**)&c->d_ctr2, &c->cap_ctr2, nctr * sizeof(unsigned));
     if (rc) return rc;
     rc = prepare_gather(c, st);
@@ -213,6 +215,7 @@ int sf_adj_configure(sf_ctx* c, cudaStream_t st, AdjLaunch* A)
     p.tcode = c->d_tcode;
     p.tc1 = c->d_tc1;
     p.tc2 = c->d_tc2;
+    p.vflag = c->d_vflag;
     p.rx = c->d_rx;
     p.rz = c->d_rz;
     p.nrec = c->batch_nrec;
@@ -242,6 +245,7 @@ int sf_adj_configure(sf_ctx* c, cudaStream_t st, AdjLaunch* A)
     g.blk_shots = c->d_gshots;
     g.tcode = c->d_tcode;
     g.vrec = c->d_tc2;
+    g.vflag = c->d_vflag;
     g.lam_init = c->d_lam_init;
     g.wait_ns = c->wait_ns;
     if (c->batch_ani) {
@@ -259,6 +263,7 @@ int sf_adj_configure(sf_ctx* c, cudaStream_t st, AdjLaunch* A)
     A->block = dim3(c->warps * 32);
     A->smem = smem;
     A->nctr = nctr;
+    A->nflag = nflag;
     A->hand_bytes = (size_t)NG * hand_words(nstrips, c->batch_maxcols, 2) * sizeof(unsigned long long);
     A->ggrid = dim3((unsigned)(nstrips * ((c->nxx + kGT - 1) / kGT)));
     A->gblock = dim3(256);
@@ -306,6 +311,7 @@ int sf_adj_enqueue(sf_ctx* c, AdjLaunch& A, const float* d_pg, float* d_grad, un
     A.p.epoch = epoch;
     A.g.grad = d_grad;
     CK(cudaMemsetAsync(A.p.bar, 0, A.nctr * sizeof(unsigned), st));
+    CK(cudaMemsetAsync(A.p.vflag, 0, A.nflag, st));
     if (c->hand_stale_a) {  // the epoch wrapped (sf_next_epoch)
         CK(cudaMemsetAsync(c->d_hand2, 0, c->cap_hand2, st));
         c->hand_stale_a = false;

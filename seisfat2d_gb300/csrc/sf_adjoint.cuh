@@ -70,6 +70,8 @@ struct AdjStripArgs {
     const uint8_t* tcode;  // tape of this (sweep, strip): entries [fstep*32 + flane]
     const float* tc1;
     float* tc2;            // overwritten with v = mu * c2
+    uint8_t* vflag;        // one per 1024 tape entries of the batch: set when a term is not zero
+    size_t tape_base;      // the strip's first tape entry
     AdjRing* ring;
     CtaShared* sh;
     const unsigned long long* h_in;  // {pv,tag},{pev,tag} of the upwind strip's row (nullptr: first strip)
@@ -272,6 +274,14 @@ __device__ __forceinline__ void adj_strip(const AdjStripArgs& a)
                                  "r"(a.tag), "r"(__float_as_uint(opev[u])) : "memory");
             }
         }
+        // mark the block's tape entries if a term is not zero (read by the gather)
+        bool nz = false;
+#pragma unroll
+        for (int u = 0; u < kU; u++) nz |= vv[u] != 0.0f;
+        if (__any_sync(0xffffffffu, nz) && lane < 2) {
+            const int fs = ncols + 30 - s0 - (lane ? kU - 1 : 0);
+            a.vflag[(a.tape_base + (size_t)max(fs, 0) * 32) >> 10] = 1;
+        }
         pV -= 32 * kU;
         pH += 2 * kU;
         b0 += kU;
@@ -385,6 +395,7 @@ __device__ void adjoint_body(const AdjParams& p, const FuseParams* f)
         a.err = p.err;
         a.tag = tag;
         a.c0 = sh.c0;
+        a.vflag = p.vflag;
 #pragma unroll 1
         for (int task = gp.slot; task < 4 * nstrips; task += gp.slots) {
             const int rs = task / nstrips, pidx = task - rs * nstrips, sw = 3 - rs;
@@ -402,6 +413,7 @@ __device__ void adjoint_body(const AdjParams& p, const FuseParams* f)
             a.tcode = p.tcode + tb;
             a.tc1 = p.tc1 + tb;
             a.tc2 = p.tc2 + tb;
+            a.tape_base = tb;
             a.ready = (f && sw == 0) ? f->ready + (size_t)a.k * f->nblk : nullptr;
             adj_strip<INTERIOR>(a);
         }
@@ -438,7 +450,9 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1) k_adjoint(AdjParams p)
 // These runs stream through kGStages shared-memory stages (cp.async) while
 // the threads sum their cells' terms in the order above. The shots covering
 // the tile's columns come from a per-column-block list built on the host,
-// staged in shared memory kGChunk at a time.
+// staged in shared memory kGChunk at a time. Runs without a nonzero term (the
+// rays of a shot pass through a part of its window only) are left out: the
+// reverse sweeps mark every 1024 tape entries that hold one (vflag).
 constexpr int kGSteps = kGT + 32;   // tape steps a tile's strip spans per sweep
 constexpr int kGStages = 3;
 constexpr int kGChunk = 128;
@@ -453,45 +467,59 @@ struct __align__(16) GatherStage {
 struct GatherSmem {
     GatherStage stg[kGStages];
     GatherShot shots[kGChunk];
+    uint16_t list[4 * kGChunk];      // runs to sum: shot of the chunk * 4 + sweep
+    int wcount[kMaxWarps];
 };
 
-// One stage's node terms for the thread's NQ = 32 / W cells (columns W
-// apart) when the tile lies inside the shot's window and is not the last
-// strip: the same terms and order as the general loop of gather_tile (cells q,
-// corners (0,0),(0,1),(1,0),(1,1)), with the node slots one base plus offsets
-// fixed by the sweep's directions.
-template <int W, bool SZPOS, bool SXPOS>
-__device__ __forceinline__ void gather_interior(const GatherStage& S, float* g, int a, int rb, int bl0, int ncols,
-                                                int fmlo, bool last_row)
+// One run's node terms for the thread's NQ cells: row a = rb + lane, NQ
+// consecutive columns from window column bl0. A node column is read once (its
+// rows a and a+1) and serves the cells on both its sides: corner (dr, dc) of
+// cell (a, b) is node (a + 1 - dr, b + 1 - dc). A kept node's code has bit 5
+// set and matches no corner. EDGE: node columns outside the window have no terms.
+template <int NQ, bool EDGE>
+__device__ __forceinline__ void gather_run(const GatherStage& S, float* g, int bl0, int ncols, int fmlo, bool szpos,
+                                           bool sxpos, bool next_strip)
 {
-    constexpr int NQ = 32 / W;
-    const unsigned char* cbytes = reinterpret_cast<const unsigned char*>(S.code);
-    // node (ni, nj) = (a + 1 - dr, bl + 1 - dc) of cell (a, bl), bl = bl0 + W q
-    const int fl0 = SZPOS ? a + 1 - rb : rb + 31 - (a + 1);
-    const int fm0 = SXPOS ? bl0 + 1 : ncols - 1 - (bl0 + 1);
-    const int base = (fm0 + fl0 - fmlo) * 32 + fl0;
-    constexpr int DR = SZPOS ? -33 : 33;            // ni - 1: fl -/+ 1
-    constexpr int DC = SXPOS ? -32 : 32;            // nj - 1: fm -/+ 1
-    constexpr int DQ = SXPOS ? 32 * W : -32 * W;    // nj + W: fm +/- W
+    const int lane = threadIdx.x & 31;
+    const bool last = lane == 31;   // its node row a+1 is the next strip's first
+    const int dir = sxpos ? 1 : -1;
+    const int fm0 = (sxpos ? bl0 : ncols - 1 - bl0) - fmlo;
+    const int fl0 = szpos ? lane : 31 - lane, fl1 = szpos ? lane + 1 : 30 - lane;
+    const uint8_t* cb = reinterpret_cast<const uint8_t*>(S.code);
+    const uint8_t* cb2 = reinterpret_cast<const uint8_t*>(S.code2);
+    const float* pv0 = S.v + ((fm0 + fl0) * 32 + fl0);
+    const uint8_t* pc0 = cb + ((fm0 + fl0) * 32 + fl0);
+    const float* pv1 = last ? S.v2 + fm0 : S.v + ((fm0 + fl1) * 32 + fl1);
+    const uint8_t* pc1 = last ? cb2 + (4 * fm0 + (szpos ? 0 : 3)) : cb + ((fm0 + fl1) * 32 + fl1);
+    const int s0 = 32 * dir, sv1 = last ? dir : s0, sc1 = last ? 4 * dir : s0;
+    const bool has1 = !last || next_strip;
+    float v0p = 0.0f, v1p = 0.0f;
+    int c0p = 0x20, c1p = 0x20;
 #pragma unroll
-    for (int q = 0; q < NQ; q++)
-#pragma unroll
-        for (int dr = 0; dr < 2; dr++)
-#pragma unroll
-            for (int dc = 0; dc < 2; dc++) {
-                int cd;
-                float v;
-                if (dr == 0 && last_row) {  // node row a + 1: the next strip's first row
-                    const int q2 = (SXPOS ? bl0 + W * q + 1 - dc : ncols - 1 - (bl0 + W * q + 1 - dc)) - fmlo;
-                    cd = (S.code2[q2] >> (SZPOS ? 0 : 24)) & 0xff;
-                    v = S.v2[q2];
-                } else {
-                    const int idx = base + q * DQ + dr * DR + dc * DC;
-                    cd = cbytes[idx];
-                    v = S.v[idx];
-                }
-                if ((cd & 7) && (cd & 0x18) == ((dr << 3) | (dc << 4))) g[q] = fadd(g[q], v);
+    for (int q = 0; q <= NQ; q++) {
+        const bool in = !EDGE || (bl0 + q >= 0 && bl0 + q < ncols);
+        float v0 = 0.0f, v1 = 0.0f;
+        int c0 = 0x20, c1 = 0x20;
+        if (in) {
+            v0 = pv0[q * s0];
+            c0 = pc0[q * s0] & 0x38;
+            if (has1) {
+                v1 = pv1[q * sv1];
+                c1 = pc1[q * sc1] & 0x38;
             }
+        }
+        if (q > 0) {
+            float& x = g[q - 1];
+            if (c1 == 0x00) x = fadd(x, v1);
+            if (c1p == 0x10) x = fadd(x, v1p);
+            if (c0 == 0x08) x = fadd(x, v0);
+            if (c0p == 0x18) x = fadd(x, v0p);
+        }
+        v0p = v0;
+        v1p = v1;
+        c0p = c0;
+        c1p = c1;
+    }
 }
 
 // Bounded wait of one thread until *p >= target (acquire); false after the
@@ -514,7 +542,7 @@ __device__ __forceinline__ bool wait_count(const unsigned* p, unsigned target, i
 }
 
 // g(a, b) of one tile (strip k, column block cb) by 32 W threads: thread
-// (warp w, lane l) owns cells (32 k + l, 32 cb + w + W q), q < 32 / W.
+// (warp w, lane l) owns the 32 / W cells (32 k + l, 32 cb + w 32/W ..).
 // VTI: the batch was anisotropic; each shot's summed terms (its gradient with
 // respect to its own qP slowness) are multiplied by the shot's derivative
 // factors of the qP slowness before the FP64 sum over shots, giving dJ/dS,
@@ -526,40 +554,57 @@ template <int W, bool VTI, bool FUSED>
 __device__ bool gather_tile(const GatherParams& p, GatherSmem& sm, int k, int cb)
 {
     constexpr int NQ = 32 / W;
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int c = cb * kGT;
     const int rb = 32 * k;
     const bool next_strip = k + 1 < p.nstrips;
-    const int a = rb + (tid & 31);   // the thread's cells: row a, columns c + (tid>>5) + W q
-    const int cq = tid >> 5;
+    const int a = rb + lane, cw = c + warp * NQ;  // the thread's cells: row a, columns cw ..
 
-    // node-column range of stage (shot entry e, sweep sw) in march order
+    // node-column range of run (shot t, sweep sw) in march order
     auto fm_range = [&](const GatherShot& t, int sw, int& fmlo, int& fmhi) {
         const int jlo = max(c - t.c0, 0);
         const int jhi = min(c + kGT - t.c0, t.ncols - 1);   // covered cells' columns and one more
         fmlo = (sw < 2) ? jlo : t.ncols - 1 - jhi;
         fmhi = (sw < 2) ? jhi : t.ncols - 1 - jlo;
     };
-    auto issue = [&](const GatherShot& t, int sw, GatherStage& S) {
+    // the tile holds cells of the shot's 3x3 initialisation
+    auto has_source = [&](const GatherShot& t) {
+        return t.sIdz + 1 >= rb && t.sIdz - 1 < rb + 32 && t.sIdx + 1 >= c && t.sIdx - 1 < c + kGT;
+    };
+    auto marked = [&](size_t lo, size_t hi) {  // a nonzero term among tape entries lo .. hi
+        unsigned any = 0;
+        for (size_t q = lo >> 10; q <= hi >> 10; q++) any |= __ldcg(p.vflag + q);
+        return any != 0;
+    };
+    auto wanted = [&](const GatherShot& t, int sw) {
+        if (sw == 3 && has_source(t)) return true;
+        int fmlo, fmhi;
+        fm_range(t, sw, fmlo, fmhi);
+        const size_t base = tape_strip_base(t.tape_off, sw, k, p.nstrips, t.ncols);
+        if (marked(base + (size_t)fmlo * 32, base + (size_t)(fmhi + 31) * 32 + 31)) return true;
+        const int fl2 = (sw == 1 || sw == 3) ? 31 : 0;
+        const size_t base2 = base + (size_t)(t.ncols + 31) * 32;
+        return next_strip && marked(base2 + (size_t)(fmlo + fl2) * 32, base2 + (size_t)(fmhi + fl2) * 32 + 31);
+    };
+    auto issue = [&](int x, GatherStage& S) {
+        const GatherShot& t = sm.shots[x >> 2];
+        const int sw = x & 3;
         int fmlo, fmhi;
         fm_range(t, sw, fmlo, fmhi);
         const int nst = t.ncols + 31;
         const size_t base = tape_strip_base(t.tape_off, sw, k, p.nstrips, t.ncols);
-        for (int q = tid; q < kGSteps * 8; q += blockDim.x) {
+        for (int q = tid; q < kGSteps * 8; q += 32 * W) {
             const int st = fmlo + (q >> 3);
-            if (st < nst) {
-                if (FUSED) cp_async16_cg(&S.v[q * 4], p.vrec + base + (size_t)st * 32 + (q & 7) * 4);
-                else cp_async16(&S.v[q * 4], p.vrec + base + (size_t)st * 32 + (q & 7) * 4);
-            }
+            if (st < nst) cp_async16_cg(&S.v[q * 4], p.vrec + base + (size_t)st * 32 + (q & 7) * 4);
         }
-        for (int q = tid; q < kGSteps * 2; q += blockDim.x) {
+        for (int q = tid; q < kGSteps * 2; q += 32 * W) {
             const int st = fmlo + (q >> 1);
-            if (st < nst) cp_async16(&S.code[q * 4], p.tcode + base + (size_t)st * 32 + (q & 1) * 16);
+            if (st < nst) cp_async16_cg(&S.code[q * 4], p.tcode + base + (size_t)st * 32 + (q & 1) * 16);
         }
         if (next_strip) {
-            const size_t base2 = tape_strip_base(t.tape_off, sw, k + 1, p.nstrips, t.ncols);
+            const size_t base2 = base + (size_t)nst * 32;
             const int fl2 = (sw == 1 || sw == 3) ? 31 : 0;
-            for (int q = tid; q <= fmhi - fmlo; q += blockDim.x) {
+            for (int q = tid; q <= fmhi - fmlo; q += 32 * W) {
                 const size_t e = base2 + (size_t)(fmlo + q + fl2) * 32 + fl2;
                 if (FUSED) {
                     S.v2[q] = __ldcg(p.vrec + e);
@@ -581,102 +626,94 @@ __device__ bool gather_tile(const GatherParams& p, GatherSmem& sm, int k, int cb
         if (VTI) t11[q] = t13[q] = 0.0;
     }
     bool ok = true;
+    // a shot's sum is complete: its initialisation term, then the sum over shots
+    auto close_shot = [&](const GatherShot& t) {
+        const bool src = has_source(t);
+#pragma unroll
+        for (int q = 0; q < NQ; q++) {
+            const int bc = cw + q, bl = bc - t.c0;
+            if (src) {
+                const int da = a - t.sIdz + 1, db = bc - t.sIdx + 1;
+                if (da >= 0 && da < 3 && db >= 0 && db < 3) {
+                    const double d = src_dist(a, bc, p.nb, p.dx, p.dz, t.sx, t.sz);
+                    const float* li = p.lam_init + (size_t)t.orig * 9 + da + 3 * db;
+                    g[q] = fadd(g[q], fmul(FUSED ? __ldcg(li) : *li, __double2float_rn(d)));
+                }
+            }
+            if (g[q] != 0.0f && a < p.nzz && bc < p.nxx && bl >= 0 && bl < t.ncols) {
+                if (VTI) {
+                    const float* f = p.vfac + t.q_off + (size_t)a + (size_t)bl * strip_pitch(p.nzz);
+                    total[q] += (double)g[q] * (double)f[0];
+                    t11[q] += (double)g[q] * (double)f[p.vfac_total];
+                    t13[q] += (double)g[q] * (double)f[2 * p.vfac_total];
+                } else {
+                    total[q] += (double)g[q];
+                }
+            }
+            g[q] = 0.0f;
+        }
+    };
     const int e_end = p.blk_ptr[cb + 1];
 #pragma unroll 1
     for (int e0 = p.blk_ptr[cb]; e0 < e_end; e0 += kGChunk) {
         const int n = min(kGChunk, e_end - e0);
         __syncthreads();  // the previous chunk's list and stages are no longer read
-        for (int q = tid; q < n; q += blockDim.x) sm.shots[q] = p.blk_shots[e0 + q];
+        for (int q = tid; q < n; q += 32 * W) sm.shots[q] = p.blk_shots[e0 + q];
         __syncthreads();
-        const int nst = 4 * n;  // stages (entry, sweep) of the chunk
-        for (int i = 0; i < kGStages - 1 && i < nst; i++) issue(sm.shots[i >> 2], i & 3, sm.stg[i]);
+        // the chunk's runs with terms, in order
+        int nrun = 0;
 #pragma unroll 1
-        for (int i = 0; i < nst; i++) {
-            const int ahead = min(kGStages - 1, nst - 1 - i);  // stages issued after stage i
-            if (i + kGStages - 1 < nst) {
+        for (int x0 = 0; x0 < 4 * n; x0 += 32 * W) {
+            const int x = x0 + tid;
+            const bool keep = x < 4 * n && wanted(sm.shots[x >> 2], x & 3);
+            const unsigned m = __ballot_sync(0xffffffffu, keep);
+            if (lane == 0) sm.wcount[warp] = __popc(m);
+            __syncthreads();
+            int before = nrun;
+#pragma unroll
+            for (int w = 0; w < W; w++) {
+                before += (w < warp) ? sm.wcount[w] : 0;
+                nrun += sm.wcount[w];
+            }
+            if (keep) sm.list[before + __popc(m & ((1u << lane) - 1))] = (uint16_t)x;
+            __syncthreads();
+        }
+        for (int i = 0; i < kGStages - 1 && i < nrun; i++) issue(sm.list[i], sm.stg[i]);
+#pragma unroll 1
+        for (int i = 0; i < nrun; i++) {
+            const int ahead = min(kGStages - 1, nrun - 1 - i);  // stages issued after stage i
+            if (i + kGStages - 1 < nrun) {
                 const int j = i + kGStages - 1;
-                issue(sm.shots[j >> 2], j & 3, sm.stg[j % kGStages]);
+                issue(sm.list[j], sm.stg[j % kGStages]);
                 cp_wait<kGStages - 1>();
             } else if (ahead == 1) {
                 cp_wait<1>();
             } else {
                 cp_wait<0>();
             }
-            const GatherShot& t = sm.shots[i >> 2];
-            const int sw = i & 3;
+            const int x = sm.list[i];
+            const GatherShot& t = sm.shots[x >> 2];
+            const int sw = x & 3;
             if (FUSED && sw == 3 && tid == 0) {
                 // the shot's initialisation term is written when its reverse sweeps end
-                const bool src = t.sIdz + 1 >= rb && t.sIdz - 1 < rb + 32 && t.sIdx + 1 >= c && t.sIdx - 1 < c + kGT;
-                if (src && !wait_count(p.shot_done + t.orig, p.done_tag, p.err, p.wait_ns)) ok = false;
+                if (has_source(t) && !wait_count(p.shot_done + t.orig, p.done_tag, p.err, p.wait_ns)) ok = false;
             }
             __syncthreads();
-            const bool szpos = !(sw == 1 || sw == 3), sxpos = sw < 2;
             int fmlo, fmhi;
             fm_range(t, sw, fmlo, fmhi);
-            const GatherStage& S = sm.stg[i % kGStages];
-            const unsigned char* cbytes = reinterpret_cast<const unsigned char*>(S.code);
-            // the tile's cells and their nodes all inside the window, rows below the last strip
-            const bool interior = (c >= t.c0) && (c + kGT - t.c0 <= t.ncols - 1) && (rb + 33 <= p.nzz);
-            if (interior) {
-                const int bl0 = c + cq - t.c0;
-                const bool last_row = a == rb + 31;
-                switch (sw) {
-                case 0: gather_interior<W, true, true>(S, g, a, rb, bl0, t.ncols, fmlo, last_row); break;
-                case 1: gather_interior<W, false, true>(S, g, a, rb, bl0, t.ncols, fmlo, last_row); break;
-                case 2: gather_interior<W, true, false>(S, g, a, rb, bl0, t.ncols, fmlo, last_row); break;
-                default: gather_interior<W, false, false>(S, g, a, rb, bl0, t.ncols, fmlo, last_row); break;
-                }
-            }
-#pragma unroll
-            for (int q = 0; q < NQ; q++) {
-                const int bc = c + cq + W * q;
-                const int bl = bc - t.c0;
-                if (a >= p.nzz || bc >= p.nxx || bl < 0 || bl >= t.ncols) continue;
-                if (!interior)
-                for (int dr = 0; dr < 2; dr++)
-                    for (int dc = 0; dc < 2; dc++) {
-                        const int ni = a + 1 - dr, nj = bl + 1 - dc;
-                        if (ni >= p.nzz || nj >= t.ncols) continue;
-                        const int fm = sxpos ? nj : t.ncols - 1 - nj;
-                        int cd;
-                        float v;
-                        if (ni < rb + 32) {
-                            const int fl = szpos ? ni - rb : rb + 31 - ni;
-                            const int idx = (fm + fl - fmlo) * 32 + fl;
-                            cd = cbytes[idx];
-                            v = S.v[idx];
-                        } else {
-                            const int q2 = fm - fmlo;
-                            cd = (S.code2[q2] >> (szpos ? 0 : 24)) & 0xff;
-                            v = S.v2[q2];
-                        }
-                        if ((cd & 7) && ((cd >> 3) & 1) == dr && ((cd >> 4) & 1) == dc) g[q] = fadd(g[q], v);
-                    }
-                if (sw == 3) {
-                    const int da = a - t.sIdz + 1, db = bc - t.sIdx + 1;
-                    if (da >= 0 && da < 3 && db >= 0 && db < 3) {
-                        const double d = src_dist(a, bc, p.nb, p.dx, p.dz, t.sx, t.sz);
-                        const float li = FUSED ? __ldcg(p.lam_init + (size_t)t.orig * 9 + da + 3 * db)
-                                               : p.lam_init[(size_t)t.orig * 9 + da + 3 * db];
-                        g[q] = fadd(g[q], fmul(li, __double2float_rn(d)));
-                    }
-                    if (VTI) {
-                        const float* f = p.vfac + t.q_off + (size_t)a + (size_t)bl * strip_pitch(p.nzz);
-                        total[q] += (double)g[q] * (double)f[0];
-                        t11[q] += (double)g[q] * (double)f[p.vfac_total];
-                        t13[q] += (double)g[q] * (double)f[2 * p.vfac_total];
-                    } else {
-                        total[q] += (double)g[q];
-                    }
-                    g[q] = 0.0f;
-                }
-            }
+            const bool szpos = !(sw & 1), sxpos = sw < 2;
+            const int bl0 = cw - t.c0;
+            if (c >= t.c0 && c + kGT - t.c0 <= t.ncols - 1)
+                gather_run<NQ, false>(sm.stg[i % kGStages], g, bl0, t.ncols, fmlo, szpos, sxpos, next_strip);
+            else
+                gather_run<NQ, true>(sm.stg[i % kGStages], g, bl0, t.ncols, fmlo, szpos, sxpos, next_strip);
+            if (i + 1 == nrun || (sm.list[i + 1] >> 2) != (x >> 2)) close_shot(t);
             __syncthreads();  // stage i's buffer is refilled by stage i + kGStages
         }
     }
 #pragma unroll
     for (int q = 0; q < NQ; q++) {
-        const int bc = c + cq + W * q;
+        const int bc = cw + q;
         if (a < p.nzz && bc < p.nxx) {
             p.grad[(size_t)a + (size_t)bc * p.nzz] = __double2float_rn(total[q]);
             if (VTI) {

@@ -20,6 +20,7 @@ struct AdjParams {
     uint8_t* tcode;
     float* tc1;
     float* tc2;
+    uint8_t* vflag;         // one per 1024 tape entries, zeroed: set when a node term is not zero
     const float* pick_grad; // nshots x nrec, caller order (NaN = no pick)
     const float* rx;
     const float* rz;
@@ -57,6 +58,7 @@ struct GatherParams {
     float dx, dz;
     const uint8_t* tcode;
     const float* vrec;       // v terms (tape c2 after the reverse sweeps)
+    const uint8_t* vflag;    // which 1024 tape entries hold a nonzero term (AdjParams)
     const float* lam_init;   // nshots x 9 (caller order)
     float* grad;             // nzz x nxx
     // anisotropic batches: each shot's gradient with respect to its qP

@@ -1009,7 +1009,7 @@ extern "C" int sf_batch_tape_codes(sf_ctx* c, int shot, uint8_t* codes, int mem,
                     const int r = zdown ? 32 * k + lane : 32 * k + 31 - lane, m = step - lane;
                     if (r >= nzz || m < 0 || m >= ncols) continue;
                     const int j = xright ? m : ncols - 1 - m;
-                    out[((size_t)sw * ncols + j) * nzz + r] = blk[(size_t)step * 32 + lane];
+                    out[((size_t)sw * ncols + j) * nzz + r] = blk[(size_t)step * 32 + lane] & 0x1f;  // kKept is 0 here
                 }
         }
     }

@@ -30,6 +30,7 @@ struct AdjLaunch {
     dim3 grid, block, ggrid, gblock;
     size_t smem = 0;
     size_t nctr = 0;
+    size_t nflag = 0;             // bytes of the marks of nonzero terms, zeroed before the launch
     size_t hand_bytes = 0;
     // reverse sweeps and gather in one launch (k_adjoint_gather)
     bool fused = false;
@@ -102,7 +103,7 @@ struct sf_ctx {
 
     // adjoint state
     float* d_lam = nullptr; size_t cap_lam = 0;
-    float* d_vrec = nullptr; size_t cap_vrec = 0;
+    uint8_t* d_vflag = nullptr; size_t cap_vflag = 0;  // marks of nonzero node terms
     float* d_gshot = nullptr; size_t cap_gshot = 0;
     float* d_pg = nullptr; size_t cap_pg = 0;
     double* d_misfit = nullptr; size_t cap_misfit = 0;

@@ -614,7 +614,7 @@ __device__ __forceinline__ void run_strip(const StripArgs& a)
             tnw[u] = inner ? tnew : to;
             tnwl[u] = COMP ? (inner ? tnewl : tol) : 0.0f;
             if (TAPE) {
-                if (!inner) rec[u].code = 0;
+                if (!inner) rec[u].code = kKept;
                 sr[u] = cN;
                 any_far |= rec[u].far & inner;
             }
@@ -644,7 +644,7 @@ __device__ __forceinline__ void run_strip(const StripArgs& a)
 #pragma unroll
                 for (int u = 0; u < U; u++) {
                     c1[u] = 0.0f;
-                    c2[u] = (rec[u].code == 0) ? 0.0f : ((rec[u].code & 1) ? a.kc.dz : a.kc.dx);
+                    c2[u] = (rec[u].code == kKept) ? 0.0f : ((rec[u].code & 1) ? a.kc.dz : a.kc.dx);
                 }
             }
 #pragma unroll

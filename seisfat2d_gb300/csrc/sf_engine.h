@@ -136,6 +136,7 @@ struct sf_ctx {
     double* d_wav = nullptr; size_t cap_wav = 0;
     float* d_mig = nullptr; size_t cap_mig = 0;
     float* d_kgeo = nullptr; size_t cap_kgeo = 0;
+    void* d_kterm = nullptr; size_t cap_kterm = 0;  // terms of the call's traveltime tables
     int* d_kint = nullptr; size_t cap_kint = 0;
     float* d_kpart = nullptr; size_t cap_kpart = 0;  // forward operator chunk partials
 

@@ -30,6 +30,7 @@ using namespace sf;
 namespace {
 
 constexpr float kEps = 1e-6f;  // EPS of migration.cuh:7
+constexpr size_t kTermBytes = (size_t)4 << 30;  // workspace of the tables' terms (TermTable): blocks of cells or tables that fit
 
 // The reference adds each term with a global float atomicAdd, which flushes
 // subnormal operands and results to zero; the gather adds the same way.
@@ -40,93 +41,169 @@ __device__ __forceinline__ float add_ftz(float a, float b)
     return r;
 }
 
+// The part of a cell's weight that depends on one table only, as the
+// reference's four Kirchhoff kernels compute it (migration.cu:418-466,
+// :505-553, :592-640, :685-733) for the source's and the receiver's table of
+// every trace: the time, the gradient norm, the Hessian's determinant, the
+// angle to the vertical, the direction's cosine to it (signed), the spreading
+// term, and the gradient.
+struct CellTerms {
+    float T, norm, detH, theta;
+    float u, R, dx1, dz1;
+};
+
+// The terms of a call's tables at a block of model cells (rows iz0 .. iz0+nr-1
+// of columns jx0 .., z fastest) are computed once (k_table_terms) into two
+// float4 per table and cell: a trace then costs a cell the products of two
+// tables' terms instead of both tables' stencils, roots, divisions and arc
+// cosines.
+struct TermTable {
+    float4* a;         // T, norm, detH, theta; table t, cell q of the block at t * n + q
+    float4* b;         // u, R, dx1, dz1
+    size_t n;          // cells of the block
+    int iz0, nr, jx0;
+};
+
+__device__ __forceinline__ CellTerms load_terms(const TermTable& q, size_t t, size_t cell)
+{
+    const float4 a = __ldg(q.a + t * q.n + cell), b = __ldg(q.b + t * q.n + cell);
+    return CellTerms{a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+}
+
+// Centred first and second differences of one table at padded node (i, j),
+// gradient norm, unit direction (migration.cu:418-450). blockIdx.y strides over
+// the tables (the sources' first), blockIdx.x over the cells.
+__global__ void k_table_terms(const float* __restrict__ S, const float* __restrict__ Ts, const float* __restrict__ Tr,
+                              int nsrc, int ntab, int nxx, int nzz, int nb, float dx, float dz, TermTable out)
+{
+    const size_t matsize = (size_t)nzz * nxx;
+    for (int t = blockIdx.y; t < ntab; t += gridDim.y) {
+        const float* T = (t < nsrc) ? Ts + matsize * t : Tr + matsize * (t - nsrc);
+        for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < out.n; q += (size_t)gridDim.x * blockDim.x) {
+            const int i = out.iz0 + (int)(q % out.nr) + nb, j = out.jx0 + (int)(q / out.nr) + nb;
+            const float* c0 = T + i + (size_t)j * nzz;
+            const float c = c0[0];
+            const float zp = c0[1], zm = c0[-1];
+            const float xp = c0[nzz], xm = c0[-nzz];
+            float d_dz = 0.5f * (zp - zm) / dz;
+            float d_dx = 0.5f * (xp - xm) / dx;
+            float d2_dz2 = (zp - 2.0f * c + zm) / (dz * dz);
+            float d2_dx2 = (xp - 2.0f * c + xm) / (dx * dx);
+            float d2_dxdz = (c0[nzz + 1] - c0[nzz - 1] - c0[1 - nzz] + c0[-1 - nzz]) / (4.0f * dx * dz);
+            // the multiply-adds the reference build fuses, written out
+            const float norm = __fadd_rn(__fsqrt_rn(__fmaf_rn(d_dz, d_dz, __fmul_rn(d_dx, d_dx))), kEps);
+            const float det = __fmaf_rn(d2_dx2, d2_dz2, -__fmul_rn(d2_dxdz, d2_dxdz));
+            const float u = -(d_dz / norm);  // the direction's product with (0, -1)
+            const float theta = acosf(min(1.0f, max(-1.0f, u)));
+            const float R = max(c / S[i + (size_t)j * nzz], kEps);
+            const size_t o = (size_t)t * out.n + q;
+            out.a[o] = make_float4(c, norm, fabsf(det) + kEps, theta);
+            out.b[o] = make_float4(u, R, d_dx, d_dz);
+        }
+    }
+}
+
+// The exponent of a trace's taper at a cell: x - cmp over the aperture width
+// tan(aperture) z + EPS, `width`.
+__device__ __forceinline__ float taper_exponent(float x, float cmp, float width)
+{
+    const float q = __fdiv_rn(__fsub_rn(x, cmp), width);
+    return __fmul_rn(__fmul_rn(-0.5f, q), q);
+}
+
+// The cosine of the angle between two tables' gradients, with the multiply-add
+// the reference build fuses.
+__device__ __forceinline__ float gradient_cosine(const CellTerms& s, const CellTerms& r)
+{
+    return __fdiv_rn(__fmaf_rn(s.dz1, r.dz1, __fmul_rn(s.dx1, r.dx1)), __fmul_rn(s.norm, r.norm));
+}
+
+// A cell's weight for a trace from both tables' terms.
+__device__ __forceinline__ float kirchhoff_weight(const CellTerms& s, const CellTerms& r, float Sc, float texp)
+{
+    const float Jterm = sqrtf(s.detH * r.detH) * Sc / (s.norm * r.norm);
+    const float cos_s = fabsf(s.u), cos_r = fabsf(r.u);
+    const float obliquity = sqrt(max(0.0f, cos_s) * max(0.0f, cos_r));
+    const float G = 1.0f / sqrt(s.R * r.R);
+    const float theta = 0.5f * (s.theta + r.theta);
+    const float R = 1.0f + 0.2f * cosf(theta);
+    const float scale_const = 1.0f / (2.0f * M_PI);
+    const float taper = expf(texp);
+    return scale_const * Jterm * obliquity * G * R * taper;
+}
+
+// Whether a term is certainly zero: expf underflows to 0 below this exponent
+// (0.5 times the smallest subnormal is exp(-103.98)), and every other factor
+// is finite, so that the product is 0. Cells outside a trace's aperture, most
+// of a shallow row, leave the weight out.
+__device__ __forceinline__ bool outside_aperture(float texp, const CellTerms& s, const CellTerms& r, float Sc, float v)
+{
+    // any infinite or NaN factor makes the sum of magnitudes infinite or NaN
+    const float sum = fabsf(s.detH) + fabsf(r.detH) + fabsf(s.norm) + fabsf(r.norm) + fabsf(s.R) + fabsf(r.R) +
+                      fabsf(s.u) + fabsf(r.u) + fabsf(Sc) + fabsf(v);
+    return texp < -106.0f && sum < 1e18f;
+}
+
+// RN(RN64(180 a / pi)), the angle in degrees as the reference's double
+// expression rounds it, without the GPU's slow FP64 pipe: x / pi as x times a
+// two-term reciprocal (relative error below 2^-45). Where the second term,
+// moved by 2^-18 of itself either way, rounds differently, the quotient lies
+// too near a rounding boundary and the double expression decides.
+__device__ __forceinline__ float degrees_of(float a)
+{
+    const float x = 180.0f * a;
+    const float hi = 0.318309873f;                    // RN(1/pi)
+    const float lo = (float)(1.0 / M_PI - (double)0.318309873f);
+    const float h = __fmul_rn(x, hi);
+    const float e = __fmaf_rn(x, lo, __fmaf_rn(x, hi, -h));
+    const float d = __fmul_rn(e, 3.8146973e-6f);      // 2^-18
+    const float r1 = __fadd_rn(h, __fadd_rn(e, d)), r2 = __fadd_rn(h, __fsub_rn(e, d));
+    if (r1 == r2) return r1;
+    return (float)((double)x / M_PI);
+}
+
 struct KirchParams {
     const float* S;     // padded slowness
-    const float* Ts;    // nsrc padded tables
-    const float* Tr;    // nrec padded tables
+    TermTable tab;      // nsrc source tables, then nrec receiver tables
     const float* xs;    // nsrc
     const float* xr;    // nrec
     const float* data;  // nsrc x nrec x nt correlated traces
     float* image;       // nz x nx
-    int nsrc, nrec, nt, nxx, nzz, nb;
+    int nsrc, nrec, nt, nzz, nb;
     float dt, dx, dz, aperture, max_offset;
 };
 
-// The geometric terms of one table at padded node (i, j): centred first and
-// second differences, gradient norm, unit direction (migration.cu:418-450).
-struct TableTerms {
-    float dx1, dz1, norm, detH;
-};
-
-__device__ __forceinline__ TableTerms table_terms(const float* T, int i, int j, int nzz, float dx, float dz)
+// One thread per image cell of the block (whole columns) walks every trace in
+// trace order.
+__global__ void __launch_bounds__(128) k_kirchhoff_image(KirchParams p)
 {
-    TableTerms t;
-    const float c = T[i + j * nzz];
-    const float zp = T[(i + 1) + j * nzz], zm = T[(i - 1) + j * nzz];
-    const float xp = T[i + (j + 1) * nzz], xm = T[i + (j - 1) * nzz];
-    float d_dz = 0.5f * (zp - zm) / dz;
-    float d_dx = 0.5f * (xp - xm) / dx;
-    float d2_dz2 = (zp - 2.0f * c + zm) / (dz * dz);
-    float d2_dx2 = (xp - 2.0f * c + xm) / (dx * dx);
-    float d2_dxdz = (T[(i + 1) + (j + 1) * nzz] - T[(i - 1) + (j + 1) * nzz] -
-                     T[(i + 1) + (j - 1) * nzz] + T[(i - 1) + (j - 1) * nzz]) / (4.0f * dx * dz);
-    t.dz1 = d_dz;
-    t.dx1 = d_dx;
-    t.norm = sqrtf(d_dx * d_dx + d_dz * d_dz) + kEps;
-    float a = d2_dx2, b = d2_dxdz, cc = d2_dz2;
-    float det = a * cc - b * b;
-    t.detH = fabsf(det) + kEps;
-    return t;
-}
-
-__global__ void k_kirchhoff_image(KirchParams p)
-{
-    const int nz = p.nzz - 2 * p.nb, nx = p.nxx - 2 * p.nb;
-    const size_t ncell = (size_t)nz * nx;
-    for (size_t m = blockIdx.x * (size_t)blockDim.x + threadIdx.x; m < ncell; m += (size_t)gridDim.x * blockDim.x) {
-        const int i = (int)(m % nz) + p.nb, j = (int)(m / nz) + p.nb;
-        const size_t index = (size_t)i + (size_t)j * p.nzz;
-        const size_t matsize = (size_t)p.nzz * p.nxx;
+    const int nz = p.nzz - 2 * p.nb;
+    for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < p.tab.n; q += (size_t)gridDim.x * blockDim.x) {
+        const int i = (int)(q % nz) + p.nb, j = p.tab.jx0 + (int)(q / nz) + p.nb;
         const float z = __int2float_rd(i - p.nb) * p.dz;
         const float x = __int2float_rd(j - p.nb) * p.dx;
-        const float Sc = p.S[index];
-        const float scale_const = 1.0f / (2.0f * M_PI);
-        const float sigma = tanf(p.aperture * M_PI / 180.0f) * z;
+        const float Sc = p.S[(size_t)i + (size_t)j * p.nzz];
+        const float width = __fmaf_rn(tanf(p.aperture * M_PI / 180.0f), z, kEps);  // fused in the reference's image kernel
         float acc = 0.0f;
         for (int s = 0; s < p.nsrc; s++) {
-            const float* Ts = p.Ts + matsize * s;
-            const TableTerms ts = table_terms(Ts, i, j, p.nzz, p.dx, p.dz);
-            const float Tsc = Ts[index];
-            const float ux_s = ts.dx1 / ts.norm, uz_s = ts.dz1 / ts.norm;
-            const float nx_norm = 0.0f, nz_norm = -1.0f;
-            const float cos_s = fabs(ux_s * nx_norm + uz_s * nz_norm);
-            const float R_s = max(Tsc / Sc, kEps);
-            const float theta_s = acosf(min(1.0f, max(-1.0f, ux_s * nx_norm + uz_s * nz_norm)));
+            const CellTerms ts = load_terms(p.tab, s, q);
             const float xs = p.xs[s];
+#pragma unroll 2
             for (int r = 0; r < p.nrec; r++) {
                 const float offset = fabsf((xs - p.xr[r]));
                 if (!(offset < p.max_offset)) continue;
-                const float cmp = 0.5f * (xs + p.xr[r]);
-                const float* Tr = p.Tr + matsize * r;
-                const float T = Tsc + Tr[index];
+                const CellTerms tr = load_terms(p.tab, (size_t)p.nsrc + r, q);
+                const float T = ts.T + tr.T;
                 const int tId = __float2int_rd(T / p.dt);
                 if (tId >= p.nt) continue;
-                const TableTerms tr = table_terms(Tr, i, j, p.nzz, p.dx, p.dz);
-                const float Jterm = sqrtf(ts.detH * tr.detH) * Sc / (ts.norm * tr.norm);
-                const float ux_r = tr.dx1 / tr.norm, uz_r = tr.dz1 / tr.norm;
-                const float cos_r = fabs(ux_r * nx_norm + uz_r * nz_norm);
-                const float obliquity = sqrt(max(0.0f, cos_s) * max(0.0f, cos_r));
-                const float R_r = max(Tr[index] / Sc, kEps);
-                const float G = 1.0f / sqrt(R_s * R_r);
-                const float theta_r = acosf(min(1.0f, max(-1.0f, ux_r * nx_norm + uz_r * nz_norm)));
-                const float theta = 0.5f * (theta_s + theta_r);
-                const float R = 1.0f + 0.2f * cosf(theta);
-                const float taper = expf(-0.5f * ((x - cmp) / (sigma + kEps)) * ((x - cmp) / (sigma + kEps)));
-                const float weights = scale_const * Jterm * obliquity * G * R * taper;
-                acc = add_ftz(acc, __fmul_rn(weights, p.data[((size_t)s * p.nrec + r) * p.nt + tId]));
+                const float cmp = 0.5f * (xs + p.xr[r]);
+                const float v = p.data[((size_t)s * p.nrec + r) * p.nt + tId];
+                const float texp = taper_exponent(x, cmp, width);
+                if (outside_aperture(texp, ts, tr, Sc, v)) continue;
+                acc = add_ftz(acc, __fmul_rn(kirchhoff_weight(ts, tr, Sc, texp), v));
             }
         }
-        p.image[m] = acc;
+        p.image[(size_t)p.tab.jx0 * nz + q] = acc;
     }
 }
 
@@ -158,8 +235,7 @@ constexpr int kMaxAngles = 256;
 
 struct AngleParams {
     const float* S;
-    const float* Ts;
-    const float* Tr;
+    TermTable tab;          // rows of every column; nsrc source tables, then nrec receiver tables
     const float* xs;
     const float* xr;
     const float* data;      // nsrc x nrec x nt correlated traces
@@ -179,87 +255,44 @@ struct AngleParams {
 __global__ void k_kirchhoff_angles(AngleParams p)
 {
     const int nz = p.nzz - 2 * p.nb;
-    const size_t nthr = (size_t)nz * p.ncmp;
+    const size_t nthr = (size_t)p.tab.nr * p.ncmp;
     float acc[kMaxAngles];
     for (size_t w = blockIdx.x * (size_t)blockDim.x + threadIdx.x; w < nthr; w += (size_t)gridDim.x * blockDim.x) {
-        const int iz = (int)(w % nz), b = (int)(w / nz);
-        const int i = iz + p.nb;
+        const int ir = (int)(w % p.tab.nr), b = (int)(w / p.tab.nr);
+        const int iz = p.tab.iz0 + ir, i = iz + p.nb;
         for (int a = 0; a < p.nang; a++) acc[a] = 0.0f;
-        const size_t matsize = (size_t)p.nzz * p.nxx;
         const float z = __int2float_rd(i - p.nb) * p.dz;
-        const float scale_const = 1.0f / (2.0f * M_PI);
-        const float sigma = tanf(p.aperture * M_PI / 180.0f) * z;
+        const float width = __fadd_rn(__fmul_rn(tanf(p.aperture * M_PI / 180.0f), z), kEps);
         for (int e = p.cmp_ptr[b]; e < p.cmp_ptr[b + 1]; e++) {
             const int tr_id = p.cmp_tr[e];
             const int s = tr_id / p.nrec, r = tr_id % p.nrec;
             const float cmp = 0.5f * (p.xs[s] + p.xr[r]);
-            const float* Ts = p.Ts + matsize * s;
-            const float* Tr = p.Tr + matsize * r;
             const float* trace = p.data + (size_t)tr_id * p.nt;
+#pragma unroll 2
             for (int j = p.nb; j < p.nxx - p.nb; j++) {
-                const size_t index = (size_t)i + (size_t)j * p.nzz;
+                const size_t m = (size_t)ir + (size_t)(j - p.nb) * p.tab.nr;
+                const CellTerms ts = load_terms(p.tab, s, m), tr = load_terms(p.tab, (size_t)p.nsrc + r, m);
                 const float x = __int2float_rd(j - p.nb) * p.dx;
-                const float T = Ts[index] + Tr[index];
+                const float T = ts.T + tr.T;
                 const int tId = __float2int_rd(T / p.dt);
                 if (tId >= p.nt) continue;
-                const TableTerms ts = table_terms(Ts, i, j, p.nzz, p.dx, p.dz);
-                const TableTerms tr = table_terms(Tr, i, j, p.nzz, p.dx, p.dz);
-                const float Sc = p.S[index];
-                const float Jterm = sqrtf(ts.detH * tr.detH) * Sc / (ts.norm * tr.norm);
-                const float ux_s = ts.dx1 / ts.norm, uz_s = ts.dz1 / ts.norm;
-                const float ux_r = tr.dx1 / tr.norm, uz_r = tr.dz1 / tr.norm;
-                const float nx_norm = 0.0f, nz_norm = -1.0f;
-                const float cos_s = fabs(ux_s * nx_norm + uz_s * nz_norm);
-                const float cos_r = fabs(ux_r * nx_norm + uz_r * nz_norm);
-                const float obliquity = sqrt(max(0.0f, cos_s) * max(0.0f, cos_r));
-                const float R_s = max(Ts[index] / Sc, kEps);
-                const float R_r = max(Tr[index] / Sc, kEps);
-                const float G = 1.0f / sqrt(R_s * R_r);
-                const float theta_s = acosf(min(1.0f, max(-1.0f, ux_s * nx_norm + uz_s * nz_norm)));
-                const float theta_r = acosf(min(1.0f, max(-1.0f, ux_r * nx_norm + uz_r * nz_norm)));
-                const float theta = 0.5f * (theta_s + theta_r);
-                const float R = 1.0f + 0.2f * cosf(theta);
-                const float taper = expf(-0.5f * ((x - cmp) / (sigma + kEps)) * ((x - cmp) / (sigma + kEps)));
-                const float weights = scale_const * Jterm * obliquity * G * R * taper;
-                const float reflection_angle = 0.5f * acos((ts.dx1 * tr.dx1 + ts.dz1 * tr.dz1) / (ts.norm * tr.norm));
-                const float ang = 180.0f * reflection_angle / M_PI;
-                const int aId = __float2int_rd(ang / p.da);
-                if (aId >= 0 && aId < p.nang) acc[aId] = add_ftz(acc[aId], __fmul_rn(weights, trace[tId]));
+                const float Sc = p.S[(size_t)i + (size_t)j * p.nzz];
+                const float v = trace[tId];
+                const float texp = taper_exponent(x, cmp, width);
+                if (outside_aperture(texp, ts, tr, Sc, v)) continue;
+                const float weights = kirchhoff_weight(ts, tr, Sc, texp);
+                const float reflection_angle = 0.5f * acosf(gradient_cosine(ts, tr));
+                const int aId = __float2int_rd(degrees_of(reflection_angle) / p.da);
+                if (aId >= 0 && aId < p.nang) acc[aId] = add_ftz(acc[aId], __fmul_rn(weights, v));
             }
         }
         for (int a = 0; a < p.nang; a++) p.gathers[(size_t)iz + (size_t)a * nz + (size_t)b * p.nang * nz] = acc[a];
     }
 }
 
-// The trace-independent part of one cell's weight, as the reference's four
-// Kirchhoff kernels compute it (migration.cu:418-466, :505-553, :592-640,
-// :685-733), from both tables' terms at the cell; sigma = tan(aperture) z.
-__device__ __forceinline__ float kirchhoff_weight(const TableTerms& ts, const TableTerms& tr, float Tsc, float Trc,
-                                                  float Sc, float x, float cmp, float sigma)
-{
-    const float Jterm = sqrtf(ts.detH * tr.detH) * Sc / (ts.norm * tr.norm);
-    const float ux_s = ts.dx1 / ts.norm, uz_s = ts.dz1 / ts.norm;
-    const float ux_r = tr.dx1 / tr.norm, uz_r = tr.dz1 / tr.norm;
-    const float nx_norm = 0.0f, nz_norm = -1.0f;
-    const float cos_s = fabs(ux_s * nx_norm + uz_s * nz_norm);
-    const float cos_r = fabs(ux_r * nx_norm + uz_r * nz_norm);
-    const float obliquity = sqrt(max(0.0f, cos_s) * max(0.0f, cos_r));
-    const float R_s = max(Tsc / Sc, kEps);
-    const float R_r = max(Trc / Sc, kEps);
-    const float G = 1.0f / sqrt(R_s * R_r);
-    const float theta_s = acosf(min(1.0f, max(-1.0f, ux_s * nx_norm + uz_s * nz_norm)));
-    const float theta_r = acosf(min(1.0f, max(-1.0f, ux_r * nx_norm + uz_r * nz_norm)));
-    const float theta = 0.5f * (theta_s + theta_r);
-    const float R = 1.0f + 0.2f * cosf(theta);
-    const float scale_const = 1.0f / (2.0f * M_PI);
-    const float taper = expf(-0.5f * ((x - cmp) / (sigma + kEps)) * ((x - cmp) / (sigma + kEps)));
-    return scale_const * Jterm * obliquity * G * R * taper;
-}
-
 struct KirchFwdParams {
     const float* S;
-    const float* Ts;
-    const float* Tr;
+    TermTable tab;       // every cell; nsrc source tables from s0, then receiver tables from r0
     const float* xs;
     const float* xr;
     const float* model;  // image (nz x nx) or angle gathers (nz x nang x ncmp)
@@ -267,7 +300,7 @@ struct KirchFwdParams {
     const int* cmp;      // work trace e -> CMP bin (angle domain)
     float* part;         // ntrace x nchunk x nt partial traces (nchunk > 1)
     float* data;         // nsrc x nrec x nt
-    int nchunk, chunk, nrec, nt, nxx, nzz, nb, nang, warps;
+    int nchunk, chunk, s0, r0, nsrc, nrec, nt, nxx, nzz, nb, nang, warps;
     float dt, dx, dz, da, aperture;
 };
 
@@ -296,10 +329,8 @@ __global__ void k_kirchhoff_forward(KirchFwdParams p)
     const int tid = p.trace[e], s = tid / p.nrec, r = tid % p.nrec;
     const float cmp = 0.5f * (p.xs[s] + p.xr[r]);
     const int cmpId = ANGLE ? p.cmp[e] : 0;
-    const size_t matsize = (size_t)p.nzz * p.nxx;
-    const float* Ts = p.Ts + matsize * s;
-    const float* Tr = p.Tr + matsize * r;
     const int nz = p.nzz - 2 * p.nb;
+    const float tan_ap = tanf(p.aperture * M_PI / 180.0f);
     const long ncell = (long)nz * (p.nxx - 2 * p.nb);
     const long m0 = (long)ck * p.chunk, m1 = min(m0 + (long)p.chunk, ncell);
     for (long g = m0 + 32L * warp; g < m1; g += 32L * W) {
@@ -307,30 +338,34 @@ __global__ void k_kirchhoff_forward(KirchFwdParams p)
         int tq = -1;
         float v = 0.0f;
         if (m < m1) {
-            const int i = (int)(m % nz) + p.nb, j = (int)(m / nz) + p.nb;
-            const size_t index = (size_t)i + (size_t)j * p.nzz;
-            const float T = Ts[index] + Tr[index];
+            const CellTerms ts = load_terms(p.tab, s - p.s0, (size_t)m);
+            const CellTerms tr = load_terms(p.tab, (size_t)p.nsrc + (r - p.r0), (size_t)m);
+            const float T = ts.T + tr.T;
             const int tId = __float2int_rd(T / p.dt);
             if (tId >= 0 && tId < p.nt) {
+                const int i = (int)(m % nz) + p.nb, j = (int)(m / nz) + p.nb;
                 const float z = __int2float_rd(i - p.nb) * p.dz;
                 const float x = __int2float_rd(j - p.nb) * p.dx;
-                const float sigma = tanf(p.aperture * M_PI / 180.0f) * z;
-                const TableTerms ts = table_terms(Ts, i, j, p.nzz, p.dx, p.dz);
-                const TableTerms tr = table_terms(Tr, i, j, p.nzz, p.dx, p.dz);
-                const float weights = kirchhoff_weight(ts, tr, Ts[index], Tr[index], p.S[index], x, cmp, sigma);
+                const float Sc = p.S[(size_t)i + (size_t)j * p.nzz];
+                const float texp = taper_exponent(x, cmp, __fadd_rn(__fmul_rn(tan_ap, z), kEps));
                 if (ANGLE) {
                     const float reflection_angle =
-                        0.5f * acos((ts.dx1 * tr.dx1 + ts.dz1 * tr.dz1) / (ts.norm * tr.norm));
-                    const float ang = 180.0f * reflection_angle / M_PI;
-                    const int aId = __float2int_rd(ang / p.da);
+                        0.5f * acosf(gradient_cosine(ts, tr));
+                    const int aId = __float2int_rd(degrees_of(reflection_angle) / p.da);
                     if (aId >= 0 && aId < p.nang) {
                         const size_t mId = (size_t)(i - p.nb) + (size_t)aId * nz + (size_t)cmpId * p.nang * nz;
-                        v = __fmul_rn(weights, p.model[mId]);
-                        tq = tId;
+                        const float w = p.model[mId];
+                        if (!outside_aperture(texp, ts, tr, Sc, w)) {
+                            v = __fmul_rn(kirchhoff_weight(ts, tr, Sc, texp), w);
+                            tq = tId;
+                        }
                     }
                 } else {
-                    v = __fmul_rn(weights, p.model[m]);
-                    tq = tId;
+                    const float w = p.model[m];
+                    if (!outside_aperture(texp, ts, tr, Sc, w)) {
+                        v = __fmul_rn(kirchhoff_weight(ts, tr, Sc, texp), w);
+                        tq = tId;
+                    }
                 }
             }
         }
@@ -465,6 +500,27 @@ extern "C" int sf_forward_convolution(sf_ctx* c, const float* traces, float* out
     return wavelet_filter(c, traces, out, ntr, nt, dt, fmax, mem, stream, true);
 }
 
+// Terms of the tables at rows iz0 .. iz0+nr-1 of columns jx0 .. jx0+nc-1 into
+// the context's workspace.
+static int table_terms(sf_ctx* c, const float* Ts, const float* Tr, int nsrc, int nrec, int iz0, int nr, int jx0, int nc,
+                       TermTable* q, cudaStream_t st)
+{
+    const size_t ntab = (size_t)nsrc + nrec, n = (size_t)nr * nc;
+    int rc = sf_dev_reserve(c, (void**)&c->d_kterm, &c->cap_kterm, 2 * ntab * n * sizeof(float4));
+    if (rc) return rc;
+    q->a = reinterpret_cast<float4*>(c->d_kterm);
+    q->b = q->a + ntab * n;
+    q->n = n;
+    q->iz0 = iz0;
+    q->nr = nr;
+    q->jx0 = jx0;
+    const unsigned gx = (unsigned)std::min<size_t>((n + 127) / 128, 65535);
+    k_table_terms<<<dim3(gx, (unsigned)std::min<size_t>(ntab, 65535)), 128, 0, st>>>(
+        c->d_S, Ts, Tr, nsrc, (int)ntab, c->nxx, c->nzz, c->nb, c->dx, c->dz, *q);
+    CK(cudaGetLastError());
+    return SF_OK;
+}
+
 extern "C" int sf_kirchhoff_image(sf_ctx* c, const float* Ts, const float* Tr, int nsrc, int nrec, const float* xsrc,
                                   const float* xrec, const float* data, int data_mem, int nt, float dt,
                                   float aperture, float max_offset, float* image, int image_mem, void* stream)
@@ -490,8 +546,6 @@ extern "C" int sf_kirchhoff_image(sf_ctx* c, const float* Ts, const float* Tr, i
     if (image_mem == SF_MEM_HOST) di = c->d_mig + nd;
     KirchParams p;
     p.S = c->d_S;
-    p.Ts = Ts;
-    p.Tr = Tr;
     p.xs = c->d_kgeo;
     p.xr = c->d_kgeo + nsrc;
     p.data = dd;
@@ -499,7 +553,6 @@ extern "C" int sf_kirchhoff_image(sf_ctx* c, const float* Ts, const float* Tr, i
     p.nsrc = nsrc;
     p.nrec = nrec;
     p.nt = nt;
-    p.nxx = c->nxx;
     p.nzz = c->nzz;
     p.nb = c->nb;
     p.dt = dt;
@@ -507,8 +560,16 @@ extern "C" int sf_kirchhoff_image(sf_ctx* c, const float* Ts, const float* Tr, i
     p.dz = c->dz;
     p.aperture = aperture;
     p.max_offset = max_offset;
-    k_kirchhoff_image<<<(unsigned)std::min<size_t>((ni + 127) / 128, (size_t)c->sms * 32), 128, 0, st>>>(p);
-    CK(cudaGetLastError());
+    // blocks of whole columns whose terms fit the workspace
+    const size_t per_column = 2 * ((size_t)nsrc + nrec) * sizeof(float4) * c->nz;
+    const int cols = (int)std::min<size_t>(c->nx, std::max<size_t>(kTermBytes / per_column, 1));
+    for (int j0 = 0; j0 < c->nx; j0 += cols) {
+        const int nc = std::min(cols, c->nx - j0);
+        rc = table_terms(c, Ts, Tr, nsrc, nrec, 0, c->nz, j0, nc, &p.tab, st);
+        if (rc) return rc;
+        k_kirchhoff_image<<<(unsigned)std::min<size_t>((p.tab.n + 127) / 128, (size_t)c->sms * 32), 128, 0, st>>>(p);
+        CK(cudaGetLastError());
+    }
     if (image_mem == SF_MEM_HOST) {
         CK(cudaMemcpyAsync(image, di, ni * sizeof(float), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
@@ -597,8 +658,6 @@ extern "C" int sf_kirchhoff_angle_gathers(sf_ctx* c, const float* Ts, const floa
     if (gathers_mem == SF_MEM_HOST) dg = c->d_mig + nd;
     AngleParams p;
     p.S = c->d_S;
-    p.Ts = Ts;
-    p.Tr = Tr;
     p.xs = c->d_kgeo;
     p.xr = c->d_kgeo + nsrc;
     p.data = dd;
@@ -618,9 +677,16 @@ extern "C" int sf_kirchhoff_angle_gathers(sf_ctx* c, const float* Ts, const floa
     p.dz = c->dz;
     p.da = da;
     p.aperture = aperture;
-    const size_t nthr = (size_t)(c->nzz - 2 * c->nb) * ncmp;
-    k_kirchhoff_angles<<<(unsigned)std::min<size_t>((nthr + 127) / 128, (size_t)c->sms * 64), 128, 0, st>>>(p);
-    CK(cudaGetLastError());
+    // blocks of whole rows whose terms fit the workspace
+    const size_t per_row = 2 * ((size_t)nsrc + nrec) * sizeof(float4) * c->nx;
+    const int rows = (int)std::min<size_t>(c->nz, std::max<size_t>(kTermBytes / per_row, 1));
+    for (int i0 = 0; i0 < c->nz; i0 += rows) {
+        rc = table_terms(c, Ts, Tr, nsrc, nrec, i0, std::min(rows, c->nz - i0), 0, c->nx, &p.tab, st);
+        if (rc) return rc;
+        const size_t nthr = (size_t)p.tab.nr * ncmp;
+        k_kirchhoff_angles<<<(unsigned)std::min<size_t>((nthr + 127) / 128, (size_t)c->sms * 64), 128, 0, st>>>(p);
+        CK(cudaGetLastError());
+    }
     if (gathers_mem == SF_MEM_HOST) {
         CK(cudaMemcpyAsync(gathers, dg, ng * sizeof(float), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
@@ -646,17 +712,31 @@ static int kirchhoff_forward(sf_ctx* c, bool angle, const float* Ts, const float
 {
     CK(cudaSetDevice(c->dev));
     cudaStream_t st = (cudaStream_t)stream;
+    // the tables in groups whose terms fit the workspace (a trace needs its
+    // source's and its receiver's): one group unless the grid or the survey is
+    // large; each trace is summed in one launch whatever the groups
+    const size_t per_table = 2 * sizeof(float4) * (size_t)c->nx * c->nz;
+    const int fit = (int)std::max<size_t>(2, std::min<size_t>(kTermBytes / per_table, (size_t)nsrc + nrec));
+    const int gs = std::max(1, std::min(nsrc, fit - std::min(nrec, fit / 2))), gr = std::max(1, std::min(nrec, fit - gs));
+    struct Group { int s0, ns, r0, nr, first, n; };
+    std::vector<Group> groups;
     std::vector<int> ids, bins;
-    for (int s = 0; s < nsrc; s++)
-        for (int r = 0; r < nrec; r++) {
-            if (!(fabsf(xsrc[s] - xrec[r]) < max_offset)) continue;
-            if (angle) {
-                const float cmp = 0.5f * (xsrc[s] + xrec[r]);
-                const int b = (int)((cmp - mincmp) / dcmp);
-                if (b < 0 || b >= ncmp) continue;
-                bins.push_back(b);
-            }
-            ids.push_back(s * nrec + r);
+    for (int s0 = 0; s0 < nsrc; s0 += gs)
+        for (int r0 = 0; r0 < nrec; r0 += gr) {
+            Group g{s0, std::min(gs, nsrc - s0), r0, std::min(gr, nrec - r0), (int)ids.size(), 0};
+            for (int s = s0; s < s0 + g.ns; s++)
+                for (int r = r0; r < r0 + g.nr; r++) {
+                    if (!(fabsf(xsrc[s] - xrec[r]) < max_offset)) continue;
+                    if (angle) {
+                        const float cmp = 0.5f * (xsrc[s] + xrec[r]);
+                        const int b = (int)((cmp - mincmp) / dcmp);
+                        if (b < 0 || b >= ncmp) continue;
+                        bins.push_back(b);
+                    }
+                    ids.push_back(s * nrec + r);
+                }
+            g.n = (int)ids.size() - g.first;
+            if (g.n) groups.push_back(g);
         }
     const int ntrace = (int)ids.size();
     const size_t per_warp = (size_t)nt * sizeof(float) + 64 * sizeof(float);
@@ -690,20 +770,24 @@ static int kirchhoff_forward(sf_ctx* c, bool angle, const float* Ts, const float
     }
     if (data_mem == SF_MEM_HOST) dd = c->d_mig;
     CK(cudaMemsetAsync(dd, 0, nd * sizeof(float), st));
-    if (ntrace > 0) {
+    for (const Group& g : groups) {
         KirchFwdParams p;
+        const size_t matsize = (size_t)c->nxx * c->nzz;
+        rc = table_terms(c, Ts + matsize * g.s0, Tr + matsize * g.r0, g.ns, g.nr, 0, c->nz, 0, c->nx, &p.tab, st);
+        if (rc) return rc;
         p.S = c->d_S;
-        p.Ts = Ts;
-        p.Tr = Tr;
         p.xs = c->d_kgeo;
         p.xr = c->d_kgeo + nsrc;
         p.model = dm;
-        p.trace = c->d_kint;
-        p.cmp = c->d_kint + ntrace;
-        p.part = c->d_kpart;
+        p.trace = c->d_kint + g.first;
+        p.cmp = c->d_kint + ntrace + g.first;
+        p.part = c->d_kpart + (size_t)g.first * nchunk * nt;
         p.data = dd;
         p.nchunk = nchunk;
         p.chunk = chunk;
+        p.s0 = g.s0;
+        p.r0 = g.r0;
+        p.nsrc = g.ns;
         p.nrec = nrec;
         p.nt = nt;
         p.nxx = c->nxx;
@@ -717,16 +801,13 @@ static int kirchhoff_forward(sf_ctx* c, bool angle, const float* Ts, const float
         p.da = da;
         p.aperture = aperture;
         const size_t smem = (size_t)W * per_warp;
-        const unsigned grid = (unsigned)((long)ntrace * nchunk);
-        if (angle) {
-            CK(cudaFuncSetAttribute(k_kirchhoff_forward<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-            k_kirchhoff_forward<true><<<grid, 32 * W, smem, st>>>(p);
-        } else {
-            CK(cudaFuncSetAttribute(k_kirchhoff_forward<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)smem));
-            k_kirchhoff_forward<false><<<grid, 32 * W, smem, st>>>(p);
-        }
-        CK(cudaGetLastError());
+        const unsigned grid = (unsigned)((long)g.n * nchunk);
+        const void* kern = angle ? (const void*)k_kirchhoff_forward<true> : (const void*)k_kirchhoff_forward<false>;
+        CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        void* args[] = {&p};
+        CK(cudaLaunchKernel(kern, dim3(grid), dim3(32 * W), args, smem, st));
+    }
+    if (ntrace > 0) {
         if (nchunk > 1) {
             const size_t n = (size_t)ntrace * nt;
             k_sum_chunks<<<(unsigned)std::min<size_t>((n + 255) / 256, (size_t)c->sms * 16), 256, 0, st>>>(

@@ -95,19 +95,30 @@ __global__ void k_table_terms(const float* __restrict__ S, const float* __restri
             const float det = __fmaf_rn(d2_dx2, d2_dz2, -__fmul_rn(d2_dxdz, d2_dxdz));
             const float u = -(d_dz / norm);  // the direction's product with (0, -1)
             const float theta = acosf(min(1.0f, max(-1.0f, u)));
-            const float R = max(c / S[i + (size_t)j * nzz], kEps);
+            const float Sc = S[i + (size_t)j * nzz];
+            float R = max(c / Sc, kEps);
+            const float detH = fabsf(det) + kEps;
+            // every factor well inside FP32's range (their minima are EPS): the
+            // weight's roots and quotients may take the fast form. A negative R
+            // marks a cell where they may not.
+            const bool regular = norm < 1e6f && detH < 1e10f && R < 1e10f && fabsf(u) > 1e-12f && fabsf(u) < 2.0f &&
+                                 fabsf(c) < 1e10f && Sc > 1e-9f && Sc < 1e9f;
+            if (!regular) R = -R;
             const size_t o = (size_t)t * out.n + q;
-            out.a[o] = make_float4(c, norm, fabsf(det) + kEps, theta);
+            out.a[o] = make_float4(c, norm, detH, theta);
             out.b[o] = make_float4(u, R, d_dx, d_dz);
         }
     }
 }
 
 // The exponent of a trace's taper at a cell: x - cmp over the aperture width
-// tan(aperture) z + EPS, `width`.
-__device__ __forceinline__ float taper_exponent(float x, float cmp, float width)
+// tan(aperture) z + EPS (rwidth = RN(1/width); the fast quotient where both
+// are in range).
+__device__ __forceinline__ float taper_exponent(float x, float cmp, float width, float rwidth)
 {
-    const float q = __fdiv_rn(__fsub_rn(x, cmp), width);
+    const float d = __fsub_rn(x, cmp);
+    const bool fast = width >= 1e-7f && width < 1e12f && fabsf(d) < 1e12f;  // a quotient below FP32's range gives taper 1 anyhow
+    const float q = fast ? fdiv_k<false>(d, width, rwidth) : __fdiv_rn(d, width);
     return __fmul_rn(__fmul_rn(-0.5f, q), q);
 }
 
@@ -118,13 +129,19 @@ __device__ __forceinline__ float gradient_cosine(const CellTerms& s, const CellT
     return __fdiv_rn(__fmaf_rn(s.dz1, r.dz1, __fmul_rn(s.dx1, r.dx1)), __fmul_rn(s.norm, r.norm));
 }
 
-// A cell's weight for a trace from both tables' terms.
+// A cell's weight for a trace from both tables' terms. REGULAR: both cells are
+// (k_table_terms); roots and quotients are Markstein corrections (sf_device.cuh)
+// with IEEE's bits, without the branches of the general ones.
+template <bool REGULAR>
 __device__ __forceinline__ float kirchhoff_weight(const CellTerms& s, const CellTerms& r, float Sc, float texp)
 {
-    const float Jterm = sqrtf(s.detH * r.detH) * Sc / (s.norm * r.norm);
+    const float num = __fmul_rn(fsqrt_k<!REGULAR>(__fmul_rn(s.detH, r.detH)), Sc);
+    const float nn = __fmul_rn(s.norm, r.norm), RR = __fmul_rn(s.R, r.R);
+    const float Jterm = REGULAR ? fdiv_k<false>(num, nn, frcp_k(nn)) : __fdiv_rn(num, nn);
     const float cos_s = fabsf(s.u), cos_r = fabsf(r.u);
-    const float obliquity = sqrt(max(0.0f, cos_s) * max(0.0f, cos_r));
-    const float G = 1.0f / sqrt(s.R * r.R);
+    const float obliquity = fsqrt_k<!REGULAR>(__fmul_rn(max(0.0f, cos_s), max(0.0f, cos_r)));
+    const float rR = fsqrt_k<!REGULAR>(REGULAR ? RR : __fmul_rn(fabsf(s.R), fabsf(r.R)));
+    const float G = REGULAR ? frcp_k(rR) : __fdiv_rn(1.0f, rR);
     const float theta = 0.5f * (s.theta + r.theta);
     const float R = 1.0f + 0.2f * cosf(theta);
     const float scale_const = 1.0f / (2.0f * M_PI);
@@ -132,16 +149,24 @@ __device__ __forceinline__ float kirchhoff_weight(const CellTerms& s, const Cell
     return scale_const * Jterm * obliquity * G * R * taper;
 }
 
-// Whether a term is certainly zero: expf underflows to 0 below this exponent
-// (0.5 times the smallest subnormal is exp(-103.98)), and every other factor
-// is finite, so that the product is 0. Cells outside a trace's aperture, most
-// of a shallow row, leave the weight out.
-__device__ __forceinline__ bool outside_aperture(float texp, const CellTerms& s, const CellTerms& r, float Sc, float v)
+// weight * v, the term that a trace adds at a cell.
+__device__ __forceinline__ float kirchhoff_term(const CellTerms& s, const CellTerms& r, float Sc, float texp, float v)
 {
-    // any infinite or NaN factor makes the sum of magnitudes infinite or NaN
-    const float sum = fabsf(s.detH) + fabsf(r.detH) + fabsf(s.norm) + fabsf(r.norm) + fabsf(s.R) + fabsf(r.R) +
-                      fabsf(s.u) + fabsf(r.u) + fabsf(Sc) + fabsf(v);
-    return texp < -106.0f && sum < 1e18f;
+    if (fminf(s.R, r.R) > 0.0f) {
+        // expf underflows to 0 below this exponent (half the smallest subnormal is
+        // exp(-103.98)): outside the trace's aperture, most of a shallow row, a
+        // finite sample's term is 0
+        if (texp < -106.0f && fabsf(v) < 1e30f) return 0.0f;
+        return __fmul_rn(kirchhoff_weight<true>(s, r, Sc, texp), v);
+    }
+    return __fmul_rn(kirchhoff_weight<false>(s, r, Sc, texp), v);
+}
+
+// floor(T / dt): the sample of a time.
+__device__ __forceinline__ int sample_of(float T, float dt, float rdt)
+{
+    const float q = fdiv_k<false>(T, dt, rdt);
+    return __float2int_rd((T > 1e-20f && T < 1e20f) ? q : T / dt);
 }
 
 // RN(RN64(180 a / pi)), the angle in degrees as the reference's double
@@ -170,7 +195,7 @@ struct KirchParams {
     const float* data;  // nsrc x nrec x nt correlated traces
     float* image;       // nz x nx
     int nsrc, nrec, nt, nzz, nb;
-    float dt, dx, dz, aperture, max_offset;
+    float dt, rdt, dx, dz, aperture, max_offset;  // rdt: RN(1/dt)
 };
 
 // One thread per image cell of the block (whole columns) walks every trace in
@@ -184,6 +209,7 @@ __global__ void __launch_bounds__(128) k_kirchhoff_image(KirchParams p)
         const float x = __int2float_rd(j - p.nb) * p.dx;
         const float Sc = p.S[(size_t)i + (size_t)j * p.nzz];
         const float width = __fmaf_rn(tanf(p.aperture * M_PI / 180.0f), z, kEps);  // fused in the reference's image kernel
+        const float rwidth = __frcp_rn(width);
         float acc = 0.0f;
         for (int s = 0; s < p.nsrc; s++) {
             const CellTerms ts = load_terms(p.tab, s, q);
@@ -194,40 +220,74 @@ __global__ void __launch_bounds__(128) k_kirchhoff_image(KirchParams p)
                 if (!(offset < p.max_offset)) continue;
                 const CellTerms tr = load_terms(p.tab, (size_t)p.nsrc + r, q);
                 const float T = ts.T + tr.T;
-                const int tId = __float2int_rd(T / p.dt);
+                const int tId = sample_of(T, p.dt, p.rdt);
                 if (tId >= p.nt) continue;
                 const float cmp = 0.5f * (xs + p.xr[r]);
                 const float v = p.data[((size_t)s * p.nrec + r) * p.nt + tId];
-                const float texp = taper_exponent(x, cmp, width);
-                if (outside_aperture(texp, ts, tr, Sc, v)) continue;
-                acc = add_ftz(acc, __fmul_rn(kirchhoff_weight(ts, tr, Sc, texp), v));
+                acc = add_ftz(acc, kirchhoff_term(ts, tr, Sc, taper_exponent(x, cmp, width, rwidth), v));
             }
         }
         p.image[(size_t)p.tab.jx0 * nz + q] = acc;
     }
 }
 
-// Cross-correlation of each trace with the wavelet as the reference's FFT
-// product A conj(B) with FFTW's unnormalised inverse gives it: for output
-// sample t >= shift, nfft * sum_m trace[t - shift + m] * w[m] in FP64 (the
-// zero padding to nfft >= nt + nw - 1 makes the circular sum a linear one),
-// rounded once to FP32 (each FP64 operation rounded once, in the order of
-// the sum); samples before the shift are 0.
-__global__ void k_correlate(const float* __restrict__ in, float* __restrict__ out, int ntr, int nt,
-                            const double* __restrict__ w, int nw, int shift, double nfft)
+// Correlation and convolution of traces with the wavelet, both in FP64 with
+// the reference's order of the sum, rounded once to FP32: a block of threads
+// takes kFilterBlock output samples of one trace from its input samples in
+// shared memory as doubles. A product of two FP32 values is exact in FP64, so
+// one fused multiply-add gives the bits of the multiplication and addition
+// each rounded once. Two FP64 lanes per SM bound them: converting every tap's
+// sample anew and multiplying and adding apart took three FP64 instructions a
+// tap (2000 traces of 1000 samples, 58 taps: 0.67 ms), this takes one.
+constexpr int kFilterBlock = 256;
+constexpr int kFilterTaps = 1024;  // taps staged at a time
+
+// Correlation, as the reference's FFT product A conj(B) with FFTW's
+// unnormalised inverse gives it: for output sample t >= shift, nfft * sum_m
+// trace[t - shift + m] * w[m] (the zero padding to nfft >= nt + nw - 1 makes
+// the circular sum a linear one); samples before the shift are 0.
+// Convolution (FORWARD), the product A B (Migration::forward_convolution,
+// migration.cu:230-261): nfft * sum_m trace[t + shift - m] * w[m] over the
+// samples inside the trace, m ascending.
+template <bool FORWARD>
+__global__ void __launch_bounds__(kFilterBlock) k_filter(const float* __restrict__ in, float* __restrict__ out, int ntr,
+                                                         int nt, const double* __restrict__ w, int nw, int shift,
+                                                         double nfft)
 {
-    const size_t n = (size_t)ntr * nt;
-    for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x) {
-        const int t = (int)(q % nt);
-        const float* a = in + (q - t);
-        float v = 0.0f;
-        if (t >= shift) {
-            const int l = t - shift;
-            double acc = 0.0;
-            for (int m = 0; m < nw && l + m < nt; m++) acc = __dadd_rn(acc, __dmul_rn((double)a[l + m], w[m]));
-            v = __double2float_rn(__dmul_rn(acc, nfft));
+    __shared__ double sw[kFilterTaps], sa[kFilterTaps + kFilterBlock];
+    const int nblk = (nt + kFilterBlock - 1) / kFilterBlock;
+    const size_t njob = (size_t)ntr * nblk;
+    for (size_t job = blockIdx.x; job < njob; job += gridDim.x) {
+        const float* a = in + (job / nblk) * nt;
+        const int t0 = (int)(job % nblk) * kFilterBlock, t = t0 + threadIdx.x;
+        // the output's taps: input sample c - m (FORWARD) or c + m
+        const int c = FORWARD ? t + shift : t - shift;
+        const int m0 = FORWARD ? max(0, c - nt + 1) : 0;
+        const int m1 = (t >= nt || c < 0) ? 0 : min(nw, FORWARD ? c + 1 : nt - c);
+        double acc = 0.0;
+        for (int mc = 0; mc < nw; mc += kFilterTaps) {
+            const int mn = min(kFilterTaps, nw - mc);
+            // samples of these taps from sample lo
+            const int lo = FORWARD ? t0 + shift - (mc + mn - 1) : t0 - shift + mc;
+            __syncthreads();
+            for (int q = threadIdx.x; q < mn; q += kFilterBlock) sw[q] = w[mc + q];
+            for (int q = threadIdx.x; q < mn + kFilterBlock - 1; q += kFilterBlock) {
+                const int k = lo + q;
+                sa[q] = (k >= 0 && k < nt) ? (double)a[k] : 0.0;
+            }
+            __syncthreads();
+            const int first = max(m0, mc), last = min(m1, mc + mn);
+            if (FORWARD) {
+                const double* x = sa + (c - lo);
+#pragma unroll 4
+                for (int m = first; m < last; m++) acc = __fma_rn(x[-m], sw[m - mc], acc);
+            } else {
+                const double* x = sa + (c - lo);
+#pragma unroll 4
+                for (int m = first; m < last; m++) acc = __fma_rn(x[m], sw[m - mc], acc);
+            }
         }
-        out[q] = v;
+        if (t < nt) out[(job / nblk) * nt + t] = (m1 > 0 || FORWARD || c >= 0) ? __double2float_rn(__dmul_rn(acc, nfft)) : 0.0f;
     }
 }
 
@@ -243,7 +303,7 @@ struct AngleParams {
     const int* cmp_tr;      // trace s * nrec + r, trace order within a bin
     float* gathers;         // nz x nang x ncmp
     int nsrc, nrec, nt, nxx, nzz, nb, nang, ncmp;
-    float dt, dx, dz, da, aperture;
+    float dt, rdt, dx, dz, da, aperture;  // rdt: RN(1/dt)
 };
 
 // ADKDM's angle_domain_adjoint_kernel (migration.cu:572-663) as a gather: one
@@ -263,6 +323,7 @@ __global__ void k_kirchhoff_angles(AngleParams p)
         for (int a = 0; a < p.nang; a++) acc[a] = 0.0f;
         const float z = __int2float_rd(i - p.nb) * p.dz;
         const float width = __fadd_rn(__fmul_rn(tanf(p.aperture * M_PI / 180.0f), z), kEps);
+        const float rwidth = __frcp_rn(width);
         for (int e = p.cmp_ptr[b]; e < p.cmp_ptr[b + 1]; e++) {
             const int tr_id = p.cmp_tr[e];
             const int s = tr_id / p.nrec, r = tr_id % p.nrec;
@@ -274,16 +335,13 @@ __global__ void k_kirchhoff_angles(AngleParams p)
                 const CellTerms ts = load_terms(p.tab, s, m), tr = load_terms(p.tab, (size_t)p.nsrc + r, m);
                 const float x = __int2float_rd(j - p.nb) * p.dx;
                 const float T = ts.T + tr.T;
-                const int tId = __float2int_rd(T / p.dt);
+                const int tId = sample_of(T, p.dt, p.rdt);
                 if (tId >= p.nt) continue;
                 const float Sc = p.S[(size_t)i + (size_t)j * p.nzz];
-                const float v = trace[tId];
-                const float texp = taper_exponent(x, cmp, width);
-                if (outside_aperture(texp, ts, tr, Sc, v)) continue;
-                const float weights = kirchhoff_weight(ts, tr, Sc, texp);
+                const float term = kirchhoff_term(ts, tr, Sc, taper_exponent(x, cmp, width, rwidth), trace[tId]);
                 const float reflection_angle = 0.5f * acosf(gradient_cosine(ts, tr));
                 const int aId = __float2int_rd(degrees_of(reflection_angle) / p.da);
-                if (aId >= 0 && aId < p.nang) acc[aId] = add_ftz(acc[aId], __fmul_rn(weights, v));
+                if (aId >= 0 && aId < p.nang) acc[aId] = add_ftz(acc[aId], term);
             }
         }
         for (int a = 0; a < p.nang; a++) p.gathers[(size_t)iz + (size_t)a * nz + (size_t)b * p.nang * nz] = acc[a];
@@ -301,7 +359,7 @@ struct KirchFwdParams {
     float* part;         // ntrace x nchunk x nt partial traces (nchunk > 1)
     float* data;         // nsrc x nrec x nt
     int nchunk, chunk, s0, r0, nsrc, nrec, nt, nxx, nzz, nb, nang, warps;
-    float dt, dx, dz, da, aperture;
+    float dt, rdt, dx, dz, da, aperture;  // rdt: RN(1/dt)
 };
 
 // The forward (demigration) operator of the least-squares variants:
@@ -341,31 +399,25 @@ __global__ void k_kirchhoff_forward(KirchFwdParams p)
             const CellTerms ts = load_terms(p.tab, s - p.s0, (size_t)m);
             const CellTerms tr = load_terms(p.tab, (size_t)p.nsrc + (r - p.r0), (size_t)m);
             const float T = ts.T + tr.T;
-            const int tId = __float2int_rd(T / p.dt);
+            const int tId = sample_of(T, p.dt, p.rdt);
             if (tId >= 0 && tId < p.nt) {
                 const int i = (int)(m % nz) + p.nb, j = (int)(m / nz) + p.nb;
                 const float z = __int2float_rd(i - p.nb) * p.dz;
                 const float x = __int2float_rd(j - p.nb) * p.dx;
                 const float Sc = p.S[(size_t)i + (size_t)j * p.nzz];
-                const float texp = taper_exponent(x, cmp, __fadd_rn(__fmul_rn(tan_ap, z), kEps));
+                const float width = __fadd_rn(__fmul_rn(tan_ap, z), kEps);
+                const float texp = taper_exponent(x, cmp, width, frcp_k(width));
+                size_t mId = (size_t)m;
+                bool in = true;
                 if (ANGLE) {
-                    const float reflection_angle =
-                        0.5f * acosf(gradient_cosine(ts, tr));
+                    const float reflection_angle = 0.5f * acosf(gradient_cosine(ts, tr));
                     const int aId = __float2int_rd(degrees_of(reflection_angle) / p.da);
-                    if (aId >= 0 && aId < p.nang) {
-                        const size_t mId = (size_t)(i - p.nb) + (size_t)aId * nz + (size_t)cmpId * p.nang * nz;
-                        const float w = p.model[mId];
-                        if (!outside_aperture(texp, ts, tr, Sc, w)) {
-                            v = __fmul_rn(kirchhoff_weight(ts, tr, Sc, texp), w);
-                            tq = tId;
-                        }
-                    }
-                } else {
-                    const float w = p.model[m];
-                    if (!outside_aperture(texp, ts, tr, Sc, w)) {
-                        v = __fmul_rn(kirchhoff_weight(ts, tr, Sc, texp), w);
-                        tq = tId;
-                    }
+                    in = aId >= 0 && aId < p.nang;
+                    mId = (size_t)(i - p.nb) + (size_t)aId * nz + (size_t)cmpId * p.nang * nz;
+                }
+                if (in) {
+                    v = kirchhoff_term(ts, tr, Sc, texp, p.model[mId]);
+                    if (v != 0.0f) tq = tId;  // (NaN is kept)
                 }
             }
         }
@@ -400,25 +452,6 @@ __global__ void k_sum_chunks(const float* __restrict__ part, const int* __restri
         float a = pp[0];
         for (int c = 1; c < nchunk; c++) a = add_ftz(a, pp[(size_t)c * nt]);
         data[(size_t)trace[e] * nt + t] = a;
-    }
-}
-
-// Convolution of each trace with the wavelet as the reference's FFT product
-// A B with FFTW's unnormalised inverse gives it (Migration::
-// forward_convolution, migration.cu:230-261): for output sample t,
-// nfft * sum_m trace[t + shift - m] * w[m] over the samples inside the trace,
-// in FP64 (m ascending), rounded once to FP32.
-__global__ void k_convolve(const float* __restrict__ in, float* __restrict__ out, int ntr, int nt,
-                           const double* __restrict__ w, int nw, int shift, double nfft)
-{
-    const size_t n = (size_t)ntr * nt;
-    for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x) {
-        const int t = (int)(q % nt);
-        const float* a = in + (q - t);
-        const int c = t + shift;
-        double acc = 0.0;
-        for (int m = max(0, c - nt + 1); m < nw && m <= c; m++) acc = __dadd_rn(acc, __dmul_rn((double)a[c - m], w[m]));
-        out[q] = __double2float_rn(__dmul_rn(acc, nfft));
     }
 }
 
@@ -473,12 +506,13 @@ static int wavelet_filter(sf_ctx* c, const float* traces, float* out, int ntr, i
     }
     const size_t n = (size_t)ntr * nt;
     if (n) {
-        const unsigned grid = (unsigned)std::min<size_t>((n + 255) / 256, (size_t)c->sms * 16);
         const double nfft = (double)next_pow2(nt + nw - 1);
+        const size_t njob = (size_t)ntr * ((nt + kFilterBlock - 1) / kFilterBlock);
+        const unsigned grid = (unsigned)std::min<size_t>(njob, (size_t)c->sms * 16);
         if (forward)
-            k_convolve<<<grid, 256, 0, st>>>(din, dout, ntr, nt, c->d_wav, nw, nw / 2 + nw / 10, nfft);
+            k_filter<true><<<grid, kFilterBlock, 0, st>>>(din, dout, ntr, nt, c->d_wav, nw, nw / 2 + nw / 10, nfft);
         else
-            k_correlate<<<grid, 256, 0, st>>>(din, dout, ntr, nt, c->d_wav, nw, nw / 2 + nw / 10, nfft);
+            k_filter<false><<<grid, kFilterBlock, 0, st>>>(din, dout, ntr, nt, c->d_wav, nw, nw / 2 + nw / 10, nfft);
         CK(cudaGetLastError());
     }
     if (mem == SF_MEM_HOST) {
@@ -556,6 +590,7 @@ extern "C" int sf_kirchhoff_image(sf_ctx* c, const float* Ts, const float* Tr, i
     p.nzz = c->nzz;
     p.nb = c->nb;
     p.dt = dt;
+    p.rdt = 1.0f / dt;
     p.dx = c->dx;
     p.dz = c->dz;
     p.aperture = aperture;
@@ -673,6 +708,7 @@ extern "C" int sf_kirchhoff_angle_gathers(sf_ctx* c, const float* Ts, const floa
     p.nang = nang;
     p.ncmp = ncmp;
     p.dt = dt;
+    p.rdt = 1.0f / dt;
     p.dx = c->dx;
     p.dz = c->dz;
     p.da = da;
@@ -796,6 +832,7 @@ static int kirchhoff_forward(sf_ctx* c, bool angle, const float* Ts, const float
         p.nang = nang;
         p.warps = W;
         p.dt = dt;
+        p.rdt = 1.0f / dt;
         p.dx = c->dx;
         p.dz = c->dz;
         p.da = da;

@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include <cmath>
+#include <type_traits>
 #include <vector>
 
 #include "sf_engine.h"
@@ -25,25 +26,71 @@ namespace {
 // grid) in FP32, xk outer, zk inner, product then sum. Every model cell lies
 // at least mid = samples/2 cells inside the padded grid, so every model cell
 // is smoothed.
-__global__ void k_smooth(const float* __restrict__ in, int nx, int nz, int n, const float* __restrict__ K,
-                         float* __restrict__ out)
+//
+// A CTA smooths a tile of 32 x 32 cells: a lane owns a column, a warp four
+// rows of it, and a thread slides down its column of the input tile, where each
+// value and each tap (both read once from shared memory) serve four cells. The
+// kernel's columns come in groups of xc, so that the tile and the taps fit in
+// shared memory for any kernel size.
+constexpr int kTile = 32, kRows = 4;
+
+__global__ void __launch_bounds__(kTile / kRows * 32) k_smooth(const float* __restrict__ in, int nx, int nz, int n, int xc,
+                                                               const float* __restrict__ K, float* __restrict__ out)
 {
-    const size_t np = (size_t)nx * nz;
-    const int mid = n / 2;
-    for (size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x; idx < np;
-         idx += (size_t)gridDim.x * blockDim.x) {
-        const int i = (int)(idx % nz), j = (int)(idx / nz);
-        float acc = 0.0f;
-        for (int xk = 0; xk < n; xk++) {
-            const int mj = j - mid + xk;          // model column of the tap
-            for (int zk = 0; zk < n; zk++) {
-                const int mi = i - mid + zk;      // model row of the tap
-                const float v = (mi >= 0 && mi < nz && mj >= 0 && mj < nx) ? in[mi + (size_t)mj * nz] : 0.0f;
-                acc = __fadd_rn(acc, __fmul_rn(v, K[zk + xk * n]));
+    extern __shared__ float sm_smooth[];
+    const int mid = n / 2, rows = kTile + n - 1, pitch = rows | 1;
+    float* tile = sm_smooth;                                     // kTile + xc - 1 columns of `rows` rows
+    float* taps = sm_smooth + (size_t)(kTile + xc - 1) * pitch;  // xc x n
+    const int lane = threadIdx.x & 31, row0 = (threadIdx.x >> 5) * kRows;
+    const int ntz = (nz + kTile - 1) / kTile;
+    const int i0 = (blockIdx.x % ntz) * kTile, j0 = (blockIdx.x / ntz) * kTile;
+    float acc[kRows];
+#pragma unroll
+    for (int r = 0; r < kRows; r++) acc[r] = 0.0f;
+    for (int x0 = 0; x0 < n; x0 += xc) {
+        const int nxk = min(xc, n - x0);
+        __syncthreads();
+        for (int cj = threadIdx.x >> 5; cj < kTile + nxk - 1; cj += kTile / kRows) {
+            const int mj = j0 - mid + x0 + cj;
+            for (int ci = lane; ci < rows; ci += 32) {
+                const int mi = i0 - mid + ci;
+                tile[cj * pitch + ci] = (mi >= 0 && mi < nz && mj >= 0 && mj < nx) ? in[mi + (size_t)mj * nz] : 0.0f;
             }
         }
-        out[idx] = acc;
+        for (int q = threadIdx.x; q < nxk * n; q += blockDim.x) taps[q] = K[(size_t)x0 * n + q];
+        __syncthreads();
+        for (int xk = 0; xk < nxk; xk++) {
+            const float* col = tile + (lane + xk) * pitch + row0;
+            const float* k = taps + xk * n;
+            float kk[kRows];  // tap t at t mod kRows
+            // input row t serves cell r with tap t - r; the first and the last rows
+            // serve fewer cells
+            auto rows_from = [&](int tb, auto all) {
+#pragma unroll
+                for (int u = 0; u < kRows; u++) {
+                    const int t = tb + u;
+                    const float v = col[t];
+                    kk[u] = (all.value || t < n) ? k[t] : 0.0f;
+#pragma unroll
+                    for (int r = 0; r < kRows; r++)
+                        if (all.value || (t - r >= 0 && t - r < n))
+                            acc[r] = __fadd_rn(acc[r], __fmul_rn(v, kk[(u - r) & (kRows - 1)]));
+                }
+            };
+            int tb = 0;
+            rows_from(tb, std::false_type{});
+#pragma unroll 2
+            for (tb = kRows; tb + kRows <= n; tb += kRows) rows_from(tb, std::true_type{});
+            for (; tb < n + kRows - 1; tb += kRows) rows_from(tb, std::false_type{});
+        }
     }
+    const int j = j0 + lane;
+    if (j < nx)
+#pragma unroll
+        for (int r = 0; r < kRows; r++) {
+            const int i = i0 + row0 + r;
+            if (i < nz) out[i + (size_t)j * nz] = acc[r];
+        }
 }
 
 // dS = scale * grad over the model interior of the padded gradient.
@@ -102,9 +149,15 @@ static int smooth_on_device(sf_ctx* c, const float* d_in, float* d_out, float st
     if (rc) return rc;
     c->h_skern.swap(k);
     CK(cudaMemcpyAsync(c->d_skern, c->h_skern.data(), c->h_skern.size() * sizeof(float), cudaMemcpyHostToDevice, st));
-    const size_t np = (size_t)c->nx * c->nz;
-    k_smooth<<<(unsigned)std::min<size_t>((np + 255) / 256, (size_t)c->sms * 8), 256, 0, st>>>(
-        d_in, c->nx, c->nz, samples, c->d_skern, d_out);
+    // as many kernel columns at a time as fit in shared memory
+    int xc = std::min(samples, 16);
+    auto smem = [&](int x) {
+        return ((size_t)(kTile + x - 1) * ((kTile + samples - 1) | 1) + kRows + (size_t)x * samples) * sizeof(float);
+    };
+    while (xc > 1 && smem(xc) > (size_t)200 * 1024) xc /= 2;
+    CK(cudaFuncSetAttribute(k_smooth, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem(xc)));
+    const unsigned grid = (unsigned)((c->nz + kTile - 1) / kTile) * (unsigned)((c->nx + kTile - 1) / kTile);
+    k_smooth<<<grid, kTile / kRows * 32, smem(xc), st>>>(d_in, c->nx, c->nz, samples, xc, c->d_skern, d_out);
     CK(cudaGetLastError());
     return SF_OK;
 }

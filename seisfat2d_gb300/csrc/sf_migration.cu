@@ -53,21 +53,25 @@ struct CellTerms {
 };
 
 // The terms of a call's tables at a block of model cells (rows iz0 .. iz0+nr-1
-// of columns jx0 .., z fastest) are computed once (k_table_terms) into two
-// float4 per table and cell: a trace then costs a cell the products of two
+// of columns jx0 .., z fastest) are computed once (k_table_terms), 32 bytes per
+// table and cell: a trace then costs a cell the products of two
 // tables' terms instead of both tables' stencils, roots, divisions and arc
 // cosines.
 struct TermTable {
     float4* a;         // T, norm, detH, theta; table t, cell q of the block at t * n + q
-    float4* b;         // u, R, dx1, dz1
+    float2* b;         // u, R
+    float2* g;         // dx1, dz1 (the angle operators)
     size_t n;          // cells of the block
     int iz0, nr, jx0;
 };
 
+template <bool GRAD>
 __device__ __forceinline__ CellTerms load_terms(const TermTable& q, size_t t, size_t cell)
 {
-    const float4 a = __ldg(q.a + t * q.n + cell), b = __ldg(q.b + t * q.n + cell);
-    return CellTerms{a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    const size_t o = t * q.n + cell;
+    const float4 a = __ldg(q.a + o);
+    const float2 b = __ldg(q.b + o), g = GRAD ? __ldg(q.g + o) : make_float2(0.0f, 0.0f);
+    return CellTerms{a.x, a.y, a.z, a.w, b.x, b.y, g.x, g.y};
 }
 
 // Centred first and second differences of one table at padded node (i, j),
@@ -80,7 +84,8 @@ __global__ void k_table_terms(const float* __restrict__ S, const float* __restri
     for (int t = blockIdx.y; t < ntab; t += gridDim.y) {
         const float* T = (t < nsrc) ? Ts + matsize * t : Tr + matsize * (t - nsrc);
         for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < out.n; q += (size_t)gridDim.x * blockDim.x) {
-            const int i = out.iz0 + (int)(q % out.nr) + nb, j = out.jx0 + (int)(q / out.nr) + nb;
+            const unsigned col = (unsigned)q / (unsigned)out.nr;  // (a block's cells fit 32 bits)
+            const int i = out.iz0 + (int)((unsigned)q - col * out.nr) + nb, j = out.jx0 + (int)col + nb;
             const float* c0 = T + i + (size_t)j * nzz;
             const float c = c0[0];
             const float zp = c0[1], zm = c0[-1];
@@ -106,7 +111,8 @@ __global__ void k_table_terms(const float* __restrict__ S, const float* __restri
             if (!regular) R = -R;
             const size_t o = (size_t)t * out.n + q;
             out.a[o] = make_float4(c, norm, detH, theta);
-            out.b[o] = make_float4(u, R, d_dx, d_dz);
+            out.b[o] = make_float2(u, R);
+            out.g[o] = make_float2(d_dx, d_dz);
         }
     }
 }
@@ -126,7 +132,15 @@ __device__ __forceinline__ float taper_exponent(float x, float cmp, float width,
 // the reference build fuses.
 __device__ __forceinline__ float gradient_cosine(const CellTerms& s, const CellTerms& r)
 {
-    return __fdiv_rn(__fmaf_rn(s.dz1, r.dz1, __fmul_rn(s.dx1, r.dx1)), __fmul_rn(s.norm, r.norm));
+    const float dot = __fmaf_rn(s.dz1, r.dz1, __fmul_rn(s.dx1, r.dx1)), nn = __fmul_rn(s.norm, r.norm);
+    return (fminf(s.R, r.R) > 0.0f) ? fdiv_k<false>(dot, nn, frcp_k(nn)) : __fdiv_rn(dot, nn);  // regular cells
+}
+
+// floor(angle / da): the angle bin (rda = RN(1/da), 0 where the quotient
+// needs IEEE division).
+__device__ __forceinline__ int angle_bin(float deg, float da, float rda)
+{
+    return __float2int_rd(rda > 0.0f ? fdiv_k<false>(deg, da, rda) : __fdiv_rn(deg, da));
 }
 
 // A cell's weight for a trace from both tables' terms. REGULAR: both cells are
@@ -198,36 +212,68 @@ struct KirchParams {
     float dt, rdt, dx, dz, aperture, max_offset;  // rdt: RN(1/dt)
 };
 
-// One thread per image cell of the block (whole columns) walks every trace in
-// trace order.
-__global__ void __launch_bounds__(128) k_kirchhoff_image(KirchParams p)
+// The image cells of the block (whole columns), 32 per CTA. The image is the
+// sum of the traces' terms in trace order; a CTA's warps compute the terms of a
+// source's receivers side by side (a warp takes every kImageWarps-th receiver
+// for the 32 cells), and one of them adds them to the cells in receiver order
+// while the others go on to the next. So few cells are in flight that the
+// terms of their receivers stay in L1 and L2 from source to source: with a
+// thread per cell every source streamed all tables' terms from DRAM (0.58 GB
+// for 120 tables at 1001 x 201 cells; 2.3 ms against 1.1).
+constexpr int kImageWarps = 8;
+constexpr int kImageRec = 128;   // receivers whose terms are buffered
+
+__global__ void __launch_bounds__(32 * kImageWarps) k_kirchhoff_image(KirchParams p)
 {
+    __shared__ float term[2][kImageRec][32];
+    __shared__ float sum[32];
     const int nz = p.nzz - 2 * p.nb;
-    for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < p.tab.n; q += (size_t)gridDim.x * blockDim.x) {
-        const int i = (int)(q % nz) + p.nb, j = p.tab.jx0 + (int)(q / nz) + p.nb;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (size_t q0 = (size_t)blockIdx.x * 32; q0 < p.tab.n; q0 += (size_t)gridDim.x * 32) {
+        const size_t q = min(q0 + lane, p.tab.n - 1);  // lanes past the end repeat the last cell
+        const unsigned col = (unsigned)q / (unsigned)nz;
+        const int i = (int)((unsigned)q - col * nz) + p.nb, j = p.tab.jx0 + (int)col + p.nb;
         const float z = __int2float_rd(i - p.nb) * p.dz;
         const float x = __int2float_rd(j - p.nb) * p.dx;
         const float Sc = p.S[(size_t)i + (size_t)j * p.nzz];
         const float width = __fmaf_rn(tanf(p.aperture * M_PI / 180.0f), z, kEps);  // fused in the reference's image kernel
         const float rwidth = __frcp_rn(width);
-        float acc = 0.0f;
+        if (warp == 0) sum[lane] = 0.0f;
+        int buf = 0, turn = 0;
         for (int s = 0; s < p.nsrc; s++) {
-            const CellTerms ts = load_terms(p.tab, s, q);
+            const CellTerms ts = load_terms<false>(p.tab, s, q);
             const float xs = p.xs[s];
+            for (int r0 = 0; r0 < p.nrec; r0 += kImageRec) {
+                const int n = min(kImageRec, p.nrec - r0);
 #pragma unroll 2
-            for (int r = 0; r < p.nrec; r++) {
-                const float offset = fabsf((xs - p.xr[r]));
-                if (!(offset < p.max_offset)) continue;
-                const CellTerms tr = load_terms(p.tab, (size_t)p.nsrc + r, q);
-                const float T = ts.T + tr.T;
-                const int tId = sample_of(T, p.dt, p.rdt);
-                if (tId >= p.nt) continue;
-                const float cmp = 0.5f * (xs + p.xr[r]);
-                const float v = p.data[((size_t)s * p.nrec + r) * p.nt + tId];
-                acc = add_ftz(acc, kirchhoff_term(ts, tr, Sc, taper_exponent(x, cmp, width, rwidth), v));
+                for (int k = warp; k < n; k += kImageWarps) {
+                    const int r = r0 + k;
+                    const float xr = p.xr[r];
+                    float v = 0.0f;  // a trace left out adds nothing
+                    if (fabsf((xs - xr)) < p.max_offset) {
+                        const CellTerms tr = load_terms<false>(p.tab, (size_t)p.nsrc + r, q);
+                        const int tId = sample_of(ts.T + tr.T, p.dt, p.rdt);
+                        if (tId < p.nt)
+                            v = kirchhoff_term(ts, tr, Sc, taper_exponent(x, 0.5f * (xs + xr), width, rwidth),
+                                               p.data[((size_t)s * p.nrec + r) * p.nt + tId]);
+                    }
+                    term[buf][k][lane] = v;
+                }
+                // the terms are complete, and the warp that added the last ones is done
+                __syncthreads();
+                if (warp == turn) {
+                    float acc = sum[lane];
+#pragma unroll 8
+                    for (int k = 0; k < n; k++) acc = add_ftz(acc, term[buf][k][lane]);
+                    sum[lane] = acc;
+                }
+                buf ^= 1;
+                turn = (turn + 1) % kImageWarps;
             }
         }
-        p.image[(size_t)p.tab.jx0 * nz + q] = acc;
+        __syncthreads();
+        if (warp == 0 && q0 + lane < p.tab.n) p.image[(size_t)p.tab.jx0 * nz + q] = sum[lane];
+        __syncthreads();
     }
 }
 
@@ -303,7 +349,7 @@ struct AngleParams {
     const int* cmp_tr;      // trace s * nrec + r, trace order within a bin
     float* gathers;         // nz x nang x ncmp
     int nsrc, nrec, nt, nxx, nzz, nb, nang, ncmp;
-    float dt, rdt, dx, dz, da, aperture;  // rdt: RN(1/dt)
+    float dt, rdt, dx, dz, da, rda, aperture;  // rdt: RN(1/dt); rda: angle_bin's
 };
 
 // ADKDM's angle_domain_adjoint_kernel (migration.cu:572-663) as a gather: one
@@ -332,7 +378,7 @@ __global__ void k_kirchhoff_angles(AngleParams p)
 #pragma unroll 2
             for (int j = p.nb; j < p.nxx - p.nb; j++) {
                 const size_t m = (size_t)ir + (size_t)(j - p.nb) * p.tab.nr;
-                const CellTerms ts = load_terms(p.tab, s, m), tr = load_terms(p.tab, (size_t)p.nsrc + r, m);
+                const CellTerms ts = load_terms<true>(p.tab, s, m), tr = load_terms<true>(p.tab, (size_t)p.nsrc + r, m);
                 const float x = __int2float_rd(j - p.nb) * p.dx;
                 const float T = ts.T + tr.T;
                 const int tId = sample_of(T, p.dt, p.rdt);
@@ -340,7 +386,7 @@ __global__ void k_kirchhoff_angles(AngleParams p)
                 const float Sc = p.S[(size_t)i + (size_t)j * p.nzz];
                 const float term = kirchhoff_term(ts, tr, Sc, taper_exponent(x, cmp, width, rwidth), trace[tId]);
                 const float reflection_angle = 0.5f * acosf(gradient_cosine(ts, tr));
-                const int aId = __float2int_rd(degrees_of(reflection_angle) / p.da);
+                const int aId = angle_bin(degrees_of(reflection_angle), p.da, p.rda);
                 if (aId >= 0 && aId < p.nang) acc[aId] = add_ftz(acc[aId], term);
             }
         }
@@ -359,7 +405,7 @@ struct KirchFwdParams {
     float* part;         // ntrace x nchunk x nt partial traces (nchunk > 1)
     float* data;         // nsrc x nrec x nt
     int nchunk, chunk, s0, r0, nsrc, nrec, nt, nxx, nzz, nb, nang, warps;
-    float dt, rdt, dx, dz, da, aperture;  // rdt: RN(1/dt)
+    float dt, rdt, dx, dz, da, rda, aperture;  // rdt: RN(1/dt); rda: angle_bin's
 };
 
 // The forward (demigration) operator of the least-squares variants:
@@ -379,8 +425,7 @@ __global__ void k_kirchhoff_forward(KirchFwdParams p)
     extern __shared__ float smem[];
     const int W = p.warps, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     float* hist = smem + (size_t)warp * p.nt;
-    int* st_t = reinterpret_cast<int*>(smem + (size_t)W * p.nt) + warp * 32;
-    float* st_v = smem + (size_t)W * p.nt + W * 32 + warp * 32;
+    float* st_v = smem + (size_t)W * p.nt + warp * 32;
     for (int q = threadIdx.x; q < W * p.nt; q += blockDim.x) smem[q] = 0.0f;
     __syncthreads();
     const int e = blockIdx.x / p.nchunk, ck = blockIdx.x % p.nchunk;
@@ -391,29 +436,32 @@ __global__ void k_kirchhoff_forward(KirchFwdParams p)
     const float tan_ap = tanf(p.aperture * M_PI / 180.0f);
     const long ncell = (long)nz * (p.nxx - 2 * p.nb);
     const long m0 = (long)ck * p.chunk, m1 = min(m0 + (long)p.chunk, ncell);
+    // the lane's cell as (row, column), moved on by 32 W cells at a time
+    const int step_i = (32 * W) % nz, step_j = (32 * W) / nz;
+    const long first = m0 + 32L * warp + lane;
+    int iz = (int)(first % nz), jx = (int)(first / nz);
     for (long g = m0 + 32L * warp; g < m1; g += 32L * W) {
         const long m = g + lane;
         int tq = -1;
         float v = 0.0f;
         if (m < m1) {
-            const CellTerms ts = load_terms(p.tab, s - p.s0, (size_t)m);
-            const CellTerms tr = load_terms(p.tab, (size_t)p.nsrc + (r - p.r0), (size_t)m);
+            const CellTerms ts = load_terms<ANGLE>(p.tab, s - p.s0, (size_t)m);
+            const CellTerms tr = load_terms<ANGLE>(p.tab, (size_t)p.nsrc + (r - p.r0), (size_t)m);
             const float T = ts.T + tr.T;
             const int tId = sample_of(T, p.dt, p.rdt);
             if (tId >= 0 && tId < p.nt) {
-                const int i = (int)(m % nz) + p.nb, j = (int)(m / nz) + p.nb;
-                const float z = __int2float_rd(i - p.nb) * p.dz;
-                const float x = __int2float_rd(j - p.nb) * p.dx;
-                const float Sc = p.S[(size_t)i + (size_t)j * p.nzz];
+                const float z = __int2float_rd(iz) * p.dz;
+                const float x = __int2float_rd(jx) * p.dx;
+                const float Sc = p.S[(size_t)(iz + p.nb) + (size_t)(jx + p.nb) * p.nzz];
                 const float width = __fadd_rn(__fmul_rn(tan_ap, z), kEps);
                 const float texp = taper_exponent(x, cmp, width, frcp_k(width));
                 size_t mId = (size_t)m;
                 bool in = true;
                 if (ANGLE) {
                     const float reflection_angle = 0.5f * acosf(gradient_cosine(ts, tr));
-                    const int aId = __float2int_rd(degrees_of(reflection_angle) / p.da);
+                    const int aId = angle_bin(degrees_of(reflection_angle), p.da, p.rda);
                     in = aId >= 0 && aId < p.nang;
-                    mId = (size_t)(i - p.nb) + (size_t)aId * nz + (size_t)cmpId * p.nang * nz;
+                    mId = (size_t)iz + (size_t)aId * nz + (size_t)cmpId * p.nang * nz;
                 }
                 if (in) {
                     v = kirchhoff_term(ts, tr, Sc, texp, p.model[mId]);
@@ -421,7 +469,12 @@ __global__ void k_kirchhoff_forward(KirchFwdParams p)
                 }
             }
         }
-        st_t[lane] = tq;
+        iz += step_i;
+        jx += step_j;
+        if (iz >= nz) {
+            iz -= nz;
+            jx++;
+        }
         st_v[lane] = v;
         __syncwarp();
         const unsigned grp = __match_any_sync(0xffffffffu, tq);
@@ -543,7 +596,8 @@ static int table_terms(sf_ctx* c, const float* Ts, const float* Tr, int nsrc, in
     int rc = sf_dev_reserve(c, (void**)&c->d_kterm, &c->cap_kterm, 2 * ntab * n * sizeof(float4));
     if (rc) return rc;
     q->a = reinterpret_cast<float4*>(c->d_kterm);
-    q->b = q->a + ntab * n;
+    q->b = reinterpret_cast<float2*>(q->a + ntab * n);
+    q->g = q->b + ntab * n;
     q->n = n;
     q->iz0 = iz0;
     q->nr = nr;
@@ -602,7 +656,7 @@ extern "C" int sf_kirchhoff_image(sf_ctx* c, const float* Ts, const float* Tr, i
         const int nc = std::min(cols, c->nx - j0);
         rc = table_terms(c, Ts, Tr, nsrc, nrec, 0, c->nz, j0, nc, &p.tab, st);
         if (rc) return rc;
-        k_kirchhoff_image<<<(unsigned)std::min<size_t>((p.tab.n + 127) / 128, (size_t)c->sms * 32), 128, 0, st>>>(p);
+        k_kirchhoff_image<<<(unsigned)std::min<size_t>((p.tab.n + 31) / 32, (size_t)1 << 30), 32 * kImageWarps, 0, st>>>(p);
         CK(cudaGetLastError());
     }
     if (image_mem == SF_MEM_HOST) {
@@ -712,6 +766,7 @@ extern "C" int sf_kirchhoff_angle_gathers(sf_ctx* c, const float* Ts, const floa
     p.dx = c->dx;
     p.dz = c->dz;
     p.da = da;
+    p.rda = (da > 1e-6f && da < 1e6f) ? 1.0f / da : 0.0f;
     p.aperture = aperture;
     // blocks of whole rows whose terms fit the workspace
     const size_t per_row = 2 * ((size_t)nsrc + nrec) * sizeof(float4) * c->nx;
@@ -775,7 +830,7 @@ static int kirchhoff_forward(sf_ctx* c, bool angle, const float* Ts, const float
             if (g.n) groups.push_back(g);
         }
     const int ntrace = (int)ids.size();
-    const size_t per_warp = (size_t)nt * sizeof(float) + 64 * sizeof(float);
+    const size_t per_warp = (size_t)nt * sizeof(float) + 32 * sizeof(float);
     const int W = (int)std::min<size_t>(8, kFwdSmem / per_warp);
     if (W < 1) return sf_fail(c, SF_ERR_RANGE, "too many time samples for the forward operator");
     const int nz = c->nzz - 2 * c->nb;
@@ -836,6 +891,7 @@ static int kirchhoff_forward(sf_ctx* c, bool angle, const float* Ts, const float
         p.dx = c->dx;
         p.dz = c->dz;
         p.da = da;
+        p.rda = (da > 1e-6f && da < 1e6f) ? 1.0f / da : 0.0f;
         p.aperture = aperture;
         const size_t smem = (size_t)W * per_warp;
         const unsigned grid = (unsigned)((long)g.n * nchunk);

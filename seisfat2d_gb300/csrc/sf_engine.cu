@@ -828,9 +828,15 @@ int sf_qp_launch(sf_ctx* c, bool fact, cudaStream_t st)
     q.vfac = fact ? c->d_vfac : nullptr;
     q.vfac_total = c->batch_q_cells;
     const bool comp = c->arith == SF_ARITH_COMPENSATED, ref = c->arith == SF_ARITH_REFERENCE;
-    // x: the widest window's columns (grid-strided past 2048); y: the shots
-    const unsigned gx = (unsigned)std::min(c->batch_maxcols, 2048);
-    const unsigned gy = (unsigned)std::min(q.nshots, 65535);
+    // x: the model's columns (grid-strided past 2048); y: groups of shots,
+    // as many shots to a group as leave some 16 CTAs to every SM (their 64
+    // warps; 12 shots of 1701 x 501 cells in groups of 8 take 102 us, of 16
+    // 123 us, 4 shots in groups of 2 or 4 61-62 us)
+    q.ncolumns = c->nxx;
+    const long long want = 16LL * c->sms;
+    q.chunk = (int)std::max(1LL, std::min<long long>(kQpChunk, (long long)c->nxx * q.nshots / want));
+    const unsigned gx = (unsigned)std::min(c->nxx, 2048);
+    const unsigned gy = (unsigned)std::min((q.nshots + q.chunk - 1) / q.chunk, 65535);
     void* args[] = {&q};
     CK(cudaLaunchKernel(sf_kqp_kernel(ref, comp, fact), dim3(gx, gy), dim3(128), args, 0, st));
     return SF_OK;

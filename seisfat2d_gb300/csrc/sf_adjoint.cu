@@ -344,7 +344,7 @@ int sf_residual_enqueue(sf_ctx* c, const float* d_picks, const float* d_obs, flo
     const size_t npk = (size_t)c->batch_nshots * c->batch_nrec;
     int rc = sf_kt_begin(c, SF_KT_RESIDUAL, st);
     if (rc) return rc;
-    k_residual<<<1, 1024, 0, st>>>(d_picks, d_obs, npk, d_pg, d_misfit);
+    k_residual<<<kResCtas, kResThreads, 0, st>>>(d_picks, d_obs, npk, d_pg, d_misfit);
     CK(cudaGetLastError());
     return sf_kt_end(c, SF_KT_RESIDUAL, st);
 }

@@ -174,6 +174,7 @@ struct StripArgs {
     float* Tl;        // compensated: their lo parts, same layout
     int nzz, ncols;
     int k;            // strip index: rows [32k, 32k+32)
+    bool right;       // columns to the right (sweeps 0 and 1)
     bool down;        // rows downward (sweeps 0 and 2)
     bool sw0;         // first sweep: every node starts at kBig but the source's 3x3 block
     int sIdz, sIdx;   // source node (window coordinates)
@@ -298,7 +299,8 @@ __device__ __forceinline__ void wait_counter(const unsigned* p, unsigned target,
 // traveltime the loop carries, stages, hands on and writes back is a pair
 // (hi, lo); the second handoff pair of a column carries lo.
 //
-// RIGHT: the march's direction. The row direction and the first sweep's start
+// DIR: the march's direction, right (1), left (-1) or a runtime value (0, one
+// body for both; solve_window says when). The row direction and the first sweep's start
 // values are runtime values, so the two sweeps that run at the same time share
 // their code: with a copy per sweep, loops of up to 14 KB were in flight on
 // an SM and instruction fetch was 16% of the stalls. The node's cells need no
@@ -306,7 +308,7 @@ __device__ __forceinline__ void wait_counter(const unsigned* p, unsigned target,
 // carried one is the cell column on the upwind side (j1) in either direction,
 // and the new one the other. Marches to the left read one column ahead.
 // VEC: the windows' column stride is strip_pitch(nzz).
-template <bool RIGHT, bool TAPE, bool REF, bool INTERIOR, bool SQ, bool COMP, bool EXACT, bool VEC>
+template <int DIR, bool TAPE, bool REF, bool INTERIOR, bool SQ, bool COMP, bool EXACT, bool VEC>
 __device__ __forceinline__ void run_strip(const StripArgs& a)
 {
     using B = FwdBlock<COMP>;
@@ -315,8 +317,7 @@ __device__ __forceinline__ void run_strip(const StripArgs& a)
     const int lane = threadIdx.x & 31;
     const int nzz = a.nzz, ncols = a.ncols;
     const int rb = 32 * a.k;
-    constexpr bool right = RIGHT;
-    const bool down = a.down, sw0 = RIGHT && a.sw0;
+    const bool right = DIR > 0 || (DIR == 0 && a.right), down = a.down, sw0 = DIR >= 0 && a.sw0;
     const int r = down ? rb + lane : rb + 31 - lane;
     const bool vrow = r < nzz;
     const bool irow = (r >= 1) && (r <= nzz - 2);
@@ -472,7 +473,7 @@ __device__ __forceinline__ void run_strip(const StripArgs& a)
             cp_commit();
         };
         // staged: columns up to s0+U-1 (a leftward march reads one more), pairs up to s0+U-1
-        constexpr int kCols = LOOK / U - (right ? 1 : 2), kPairs = PLOOK / U - 1;
+        constexpr int kCols = LOOK / U - (DIR > 0 ? 1 : 2), kPairs = PLOOK / U - 1;
         cp_wait<(kCols < kPairs) ? kCols : kPairs>();
         __syncwarp();
 

@@ -32,6 +32,7 @@ struct FwdParams {
     int nshots;
     int G;                // CTAs per gang (one gang solves one shot at a time)
     int NG;               // gangs; gang k solves shot k first, then takes shots from a queue
+    bool drift;           // gangs may be at sweeps of both march directions at the same time
     int maxcols;          // widest window of the batch
     float* Tpool;
     float* Tlpool;        // compensated: lo parts of the traveltimes, same layout as Tpool
@@ -173,15 +174,7 @@ __device__ void solve_window(const FwdParams& p, const ShotDev& sh, const GangPo
             a.tc1 = p.tc1 + base;
             a.tc2 = p.tc2 + base;
         }
-        // Gangs that take shots from the queue drift apart, so marches in both
-        // directions are in flight on an SM, and the largest bodies (12 KB
-        // each: taped, compensated) then wait for instructions: one body for
-        // both directions takes 32.1 ms instead of 37.3 for 1000 windows of
-        // about 1000 x 1001 cells. With a gang per shot all gangs march the same
-        // way at the same time and a body per direction is the faster (60
-        // shots of 801 x 401: 2.84 ms, 2.95 with one). The smaller bodies of
-        // the other forms measured the same either way (within 1%).
-        if (TAPE && COMP && INTERIOR && p.nshots > p.NG)
+        if (TAPE && COMP && INTERIOR && p.drift)
             strip<(TAPE && COMP && INTERIOR) ? 0 : 1, TAPE, REF, INTERIOR, COMP, VEC>(a, exact);
         else if (sw < 2)
             strip<1, TAPE, REF, INTERIOR, COMP, VEC>(a, exact);

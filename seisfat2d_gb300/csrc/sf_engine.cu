@@ -206,6 +206,7 @@ extern "C" int sf_ctx_create(sf_ctx** out, int nx, int nz, float dx, float dz, i
     k.kA = k.dz2i - k.dx2i;
     k.kB = k.dx2i - k.dz2i;
     k.k2K = 2.0f * k.K;
+    set_scaled(k);
     int st = sf_cuda_check(c, cudaSetDevice(device), "cudaSetDevice");
     if (st == SF_OK) {
         cudaDeviceProp prop;

@@ -126,6 +126,7 @@ extern "C" int sf_time_propagation_noalloc(const float* S, int nx, int nz, float
     k.kA = k.dz2i - k.dx2i;
     k.kB = k.dx2i - k.dz2i;
     k.k2K = 2.0f * k.K;
+    set_scaled(k);
     NoAllocHeader hdr{};
     hdr.shot = sh;  // err, the barrier counter and the division check start at zero
     hdr.epoch = epoch;

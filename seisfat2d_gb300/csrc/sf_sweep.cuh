@@ -564,9 +564,7 @@ __device__ __forceinline__ void run_strip(const StripArgs& a)
 
         stage_next();  // the ring reads above are in flight meanwhile
 
-        float tnw[U], tnwl[U], sr[U];
-        Rec rec[U];
-        bool any_far = false;
+        float tnw[U], tnwl[U];
 #pragma unroll
         for (int u = 0; u < U; u++) {
             const int s = s0 + u;
@@ -606,18 +604,26 @@ __device__ __forceinline__ void run_strip(const StripArgs& a)
             const float s2a = row1 ? cI : cU;
             const int dc1a = (FAST || j - 1 >= 1) ? 0 : 16;
             float tnew, tnewl = 0.0f;
+            Rec rec;
             if constexpr (COMP)
                 node_update_comp<TAPE, EXACT, SQ>(to, tol, tv, tvl, te, tel, tev, tevl, s1a, s1b, s2a, cI, cN,
-                                                  a.kc, cz, cx, dc1a, dr2a, tnew, tnewl, rec[u]);
+                                                  a.kc, cz, cx, dc1a, dr2a, tnew, tnewl, rec);
             else
                 tnew = node_update<TAPE, REF, EXACT, SQ>(to, tv, te, tev, s1a, s1b, s2a, cI, cN, a.kc,
-                                                         cz, cx, dc1a, dr2a, rec[u]);
+                                                         cz, cx, dc1a, dr2a, rec);
             tnw[u] = inner ? tnew : to;
             tnwl[u] = COMP ? (inner ? tnewl : tol) : 0.0f;
             if (TAPE) {
-                if (!inner) rec[u].code = kKept;
-                sr[u] = cN;
-                any_far |= rec[u].far & inner;
+                rec.code = inner ? rec.code : kKept;
+                rec.upd &= inner;
+                rec.far &= inner;
+                float c1, c2;
+                node_record<COMP, EXACT, SQ>(rec, cN, a.kc, c1, c2);
+                if (FAST || s < nsteps) {
+                    pcode[32 * u] = (uint8_t)rec.code;
+                    pc1[32 * u] = c1;
+                    pc2[32 * u] = c2;
+                }
             }
             // carry state
             if (act) {
@@ -632,29 +638,6 @@ __device__ __forceinline__ void run_strip(const StripArgs& a)
         }
 
         if constexpr (TAPE) {
-            float c1[U], c2[U];
-            if (__any_sync(0xffffffffu, any_far)) {
-                bool ok = true;
-#pragma unroll
-                for (int u = 0; u < U; u++) ok &= node_record<EXACT, SQ>(rec[u], sr[u], a.kc, c1[u], c2[u]);
-                if (!EXACT && !ok) {
-#pragma unroll
-                    for (int u = 0; u < U; u++) node_record<true, SQ>(rec[u], sr[u], a.kc, c1[u], c2[u]);
-                }
-            } else {
-#pragma unroll
-                for (int u = 0; u < U; u++) {
-                    c1[u] = 0.0f;
-                    c2[u] = (rec[u].code == kKept) ? 0.0f : ((rec[u].code & 1) ? a.kc.dz : a.kc.dx);
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < U; u++)
-                if (FAST || s0 + u < nsteps) {
-                    pcode[32 * u] = (uint8_t)rec[u].code;
-                    pc1[32 * u] = c1[u];
-                    pc2[32 * u] = c2[u];
-                }
             pcode += 32 * U;
             pc1 += 32 * U;
             pc2 += 32 * U;

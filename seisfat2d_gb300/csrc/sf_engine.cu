@@ -740,14 +740,14 @@ int sf_fwd_configure(sf_ctx* c, int nrec, bool per_shot_T, bool tape, int gang_w
     p.nshots = nshots;
     p.G = G;
     p.NG = NG;
-    // The largest strip loop (12 KB per march direction: taped, compensated)
-    // waits for instructions while marches in both directions share an SM;
-    // one body for both then is the faster, 4% slower otherwise. Gangs march
-    // the same way at the same time when each solves one shot and the
-    // windows are of one size (60 shots of 801 x 401: 2.84 ms, 2.95 with one
-    // body), and hardly meet on an SM when there are few (windows of about
-    // 1000 x 1001 cells: 40 shots 3.27 ms, with one body 3.51; 152 shots 9.28
-    // and 7.17, 400 shots 23.9 and 17.5; 60 of about 400 x 401: 1.44, 1.45).
+    // The largest strip loop (taped, compensated) waits for instructions while
+    // marches in both directions share an SM; one body for both then is the
+    // faster, some 6% slower otherwise. Gangs march the same way at the same
+    // time when each solves one shot and the windows are of one size (100
+    // shots of 1701 x 351: 2.57 ms, 2.73 with one body), and hardly meet on an
+    // SM when there are few (windows of about 1000 x 1001 cells: 40 shots 2.91
+    // ms, with one body 3.18; 152 shots 8.20 and 6.70, 400 shots 21.0 and
+    // 17.1; 60 of about 430 x 351: 1.35 both).
     p.drift = (nshots > NG || c->hshots.back().ncols != c->batch_maxcols) && 2 * NG > c->sms;
     p.maxcols = c->batch_maxcols;
     p.Tpool = c->d_T;

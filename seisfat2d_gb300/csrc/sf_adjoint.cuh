@@ -188,11 +188,13 @@ __device__ __forceinline__ void adj_strip(const AdjStripArgs& a)
             const int e = (kU - 1 - u) * 32 + flane;
             const float c = t.c1[e], cm = fsub(1.0f, c);
             c2[u] = t.c2[e];
+            // dT/d{tv, te, tev} of the candidate: (1,0,0), (0,1,0), (c,-c,1), (0,1-c,c), (1-c,0,c);
+            // c is zero for the first two, so 1 goes with 5 and 2 with 4, and a kept node's is zero too
             br[u] = t.code[e] & 7;
-            // dT/d{tv, te, tev} of the candidate: (1,0,0), (0,1,0), (c,-c,1), (0,1-c,c), (1-c,0,c)
-            av[u] = (br[u] == 1) ? 1.0f : (br[u] == 3) ? c : (br[u] >= 5) ? cm : 0.0f;
-            ae[u] = (br[u] == 2) ? 1.0f : (br[u] == 3) ? -c : (br[u] == 4) ? cm : 0.0f;
-            aev[u] = (br[u] == 3) ? 1.0f : (br[u] >= 4) ? c : 0.0f;
+            const bool two = br[u] == 3, odd = br[u] & 1, any = br[u] != 0;
+            av[u] = two ? c : (odd ? cm : 0.0f);
+            ae[u] = two ? -c : (any & !odd ? cm : 0.0f);
+            aev[u] = two ? 1.0f : c;
         }
         // write back the columns every lane had finished before this block (marches s0-kU-31 ..)
         {

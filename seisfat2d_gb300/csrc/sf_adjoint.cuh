@@ -83,7 +83,7 @@ struct AdjStripArgs {
     const unsigned long long* prog_in;
     bool follow;
     unsigned long long* prog_out;
-    bool publish;
+    int publish;
     int* err;
     // last reverse sweep inside a fused launch: count each column block of
     // kGT padded columns once all lanes have finished its columns
@@ -291,7 +291,7 @@ __device__ __forceinline__ void adj_strip(const AdjStripArgs& a)
         b0 += kU;
         if (b0 >= kRingA) b0 -= kRingA;
         if (++tb0 >= kTapeBlocks) tb0 = 0;
-        if (a.publish && s0 % kPublish == 0 && s0 > 31) publish_progress(a.prog_out, a.tag, min(s0 - 31, ncols));
+        if (a.publish && (s0 & (a.publish - 1)) == 0 && s0 > 31) publish_progress(a.prog_out, a.tag, min(s0 - 31, ncols));
     };
     // column blocks in the order the march finishes them: the counted sweep
     // is the reverse of sweep 0, which marches down the columns, so
@@ -412,7 +412,7 @@ __device__ void adjoint_body(const AdjParams& p, const FuseParams* f)
             a.prog_in = (rs > 0) ? prog + (size_t)(rs - 1) * nstrips + a.k : nullptr;
             a.follow = rs & 1;
             a.prog_out = (rs < 3) ? prog + (size_t)rs * nstrips + a.k : nullptr;
-            a.publish = !(rs & 1);
+            a.publish = (rs & 1) ? 0 : publish_every(nstrips - 1 - pidx);
             const size_t tb = tape_strip_base(sh.tape_off, sw, a.k, nstrips, ncols);
             a.tcode = p.tcode + tb;
             a.tc1 = p.tc1 + tb;

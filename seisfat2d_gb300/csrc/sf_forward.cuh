@@ -167,7 +167,7 @@ __device__ void solve_window(const FwdParams& p, const ShotDev& sh, const GangPo
         a.prog_in = (sw > 0) ? prog + (size_t)(sw - 1) * nstrips + a.k : nullptr;
         a.follow = sw & 1;
         a.prog_out = (sw < 3) ? prog + (size_t)sw * nstrips + a.k : nullptr;
-        a.publish = !(sw & 1);
+        a.publish = (sw & 1) ? 0 : publish_every(nstrips - 1 - pidx);
         if (TAPE) {
             size_t base = tape_strip_base(sh.tape_off, sw, a.k, nstrips, ncols);
             a.tcode = p.tcode + base;

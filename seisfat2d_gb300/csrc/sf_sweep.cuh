@@ -22,7 +22,7 @@
 // starts once the downward sweep's last strip is under way (solve_window). A
 // strip's traveltimes then pass from one warp to another, so the earlier
 // sweep's strip publishes how many columns it has written back (a fence and
-// a tagged counter, every 32 columns) and the later one stays behind it.
+// a tagged counter, every 32 to 256 columns) and the later one stays behind it.
 //
 // Columns are staged into a per-warp shared-memory ring by cp.async, a few
 // march columns ahead, and lane l reads its own row of column s-l from the

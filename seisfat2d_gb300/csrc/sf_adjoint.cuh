@@ -120,11 +120,13 @@ __device__ __forceinline__ void adj_strip(const AdjStripArgs& a)
     const float* pT1 = a.tc1 + fs0 + 4 * lane;
     const float* pT2 = a.tc2 + fs0 + 4 * lane;
     const uint8_t* pTc = a.tcode + fs0 + 16 * lane;
-    // marches q .. q+U-1: columns into slots from `slot`, tape rows into block slot tb
+    // marches q .. q+U-1: columns into the next slots, tape rows into block slot tb
     // FAST: every march of the call is inside the window (no bounds tests)
-    auto stage = [&](int q, int slot, int tb, auto fast_tag) {
+    unsigned so = vu * 32, wo = (kRingA - 31 - kU + vu) * 32;  // ring offsets of the columns staged and written back
+    auto stage = [&](int q, int tb, auto fast_tag) {
         constexpr bool FAST = decltype(fast_tag)::value;
-        if (FAST || q + vu < ncols) cp_async16_cg(&R.L[(slot + vu) * 32 + vc], pL);
+        if (FAST || q + vu < ncols) cp_async16_cg(&R.L[so + vc], pL);
+        so = ring_next<kU * 32, kRingA * 32>(so);
         pL += kU * dL;
         AdjTape& t = R.tape[tb];
         if (FAST || q + kU - 1 - (lane >> 3) < nsteps) {
@@ -151,7 +153,7 @@ __device__ __forceinline__ void adj_strip(const AdjStripArgs& a)
     ensure(kLookA);
 #pragma unroll 1
     for (int q = 0; q < kLookA; q += kU) {
-        stage(q, q, q / kU, std::false_type{});
+        stage(q, q / kU, std::false_type{});
         // let the previous strip get kAheadA columns ahead before the first pairs
         if (q == 0 && consumer && lane0) wait_pair(a.h_in + 2 * (size_t)min(kAheadA, ncols - 1) + 1, a.tag, sh, a.err);
         __syncwarp();
@@ -166,8 +168,9 @@ __device__ __forceinline__ void adj_strip(const AdjStripArgs& a)
     unsigned long long* pH = a.h_out - 2 * 31;
 
     float my_x = 0.0f, my_pe = 0.0f, my_pev = 0.0f, pev_hold = 0.0f;
-    int b0 = 0, tb0 = 0;  // ring slots of march s0 (lambda) and of the block's tape rows
-    int ro = ((kRingA - lane) % kRingA) * 32 + tix;
+    int tb0 = 0;  // ring slot of the block's tape rows
+    unsigned ro = ((kRingA - lane) % kRingA) * 32;  // ring offset of the lane's march s0 - lane
+    float* const Lr = R.L + tix;
 
     // Blocks of kU steps, as in the forward: one wait per block, the block's
     // ring reads, its kU linear updates (the only serial chain), its stores.
@@ -177,14 +180,14 @@ __device__ __forceinline__ void adj_strip(const AdjStripArgs& a)
         __syncwarp();
 
         const AdjTape& t = R.tape[tb0];
-        int off[kU], br[kU];
+        unsigned off[kU];
+        int br[kU];
         float lam_in[kU], c2[kU], av[kU], ae[kU], aev[kU], hx[kU];
 #pragma unroll
         for (int u = 0; u < kU; u++) {
             off[u] = ro;
-            ro += 32;
-            if (ro >= kRingA * 32 + tix) ro -= kRingA * 32;
-            lam_in[u] = R.L[off[u]];
+            ro = ring_next<32, kRingA * 32>(ro);
+            lam_in[u] = Lr[off[u]];
             const int e = (kU - 1 - u) * 32 + flane;
             const float c = t.c1[e], cm = fsub(1.0f, c);
             c2[u] = t.c2[e];
@@ -198,11 +201,10 @@ __device__ __forceinline__ void adj_strip(const AdjStripArgs& a)
         }
         // write back the columns every lane had finished before this block (marches s0-kU-31 ..)
         {
-            int ws = b0 + (kRingA - 31 - kU) + vu;
-            if (ws >= kRingA) ws -= kRingA;
             const int m = s0 + vu - kU - 31;
             if (FAST || (m >= 0 && m < ncols))
-                *reinterpret_cast<float4*>(pW) = *reinterpret_cast<const float4*>(&R.L[ws * 32 + vc]);
+                *reinterpret_cast<float4*>(pW) = *reinterpret_cast<const float4*>(&R.L[wo + vc]);
+            wo = ring_next<kU * 32, kRingA * 32>(wo);
             pW += kU * dL;
         }
         {
@@ -240,11 +242,9 @@ __device__ __forceinline__ void adj_strip(const AdjStripArgs& a)
         // next columns, tape rows and pairs (the ring reads above are in flight meanwhile)
         ensure(s0 + kLookA + kU);
         {
-            int pf0 = b0 + kLookA;
-            if (pf0 >= kRingA) pf0 -= kRingA;
             int tf0 = tb0 + kLookA / kU;
             if (tf0 >= kTapeBlocks) tf0 -= kTapeBlocks;
-            stage(s0 + kLookA, pf0, tf0, fast_tag);
+            stage(s0 + kLookA, tf0, fast_tag);
             stage_pairs(s0 + kPairLookA, fast_tag);
             cp_commit();
         }
@@ -271,7 +271,7 @@ __device__ __forceinline__ void adj_strip(const AdjStripArgs& a)
         for (int u = 0; u < kU; u++) {
             const int m = s0 + u - lane;
             if (FAST ? vrow : (vrow && (m >= 0) && (m < ncols))) {
-                R.L[off[u]] = lo[u];
+                Lr[off[u]] = lo[u];
                 pV[-32 * u] = vv[u];
                 if (feeds)
                     asm volatile("st.global.v4.u32 [%0], {%1, %2, %3, %2};" ::"l"(pH + 2 * u), "r"(__float_as_uint(opv[u])),
@@ -288,8 +288,6 @@ __device__ __forceinline__ void adj_strip(const AdjStripArgs& a)
         }
         pV -= 32 * kU;
         pH += 2 * kU;
-        b0 += kU;
-        if (b0 >= kRingA) b0 -= kRingA;
         if (++tb0 >= kTapeBlocks) tb0 = 0;
         if (a.publish && (s0 & (a.publish - 1)) == 0 && s0 > 31) publish_progress(a.prog_out, a.tag, min(s0 - 31, ncols));
     };

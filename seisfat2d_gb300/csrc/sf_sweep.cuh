@@ -175,6 +175,14 @@ __device__ __forceinline__ unsigned tag_of(unsigned long long e) { return (unsig
 __device__ __forceinline__ float val_of(unsigned long long e) { return __uint_as_float((unsigned)e); }
 
 // Everything one warp needs for one strip of one sweep.
+// The ring offset STEP further on in a ring of END words (x < END, STEP <= END).
+template <int STEP, int END>
+__device__ __forceinline__ unsigned ring_next(unsigned x)
+{
+    x += STEP;
+    return min(x, x - END);  // x - END wraps past 2^31 while x < END
+}
+
 struct StripArgs {
     const float* S;   // slowness of the window
     float* T;         // traveltimes of the window
@@ -378,13 +386,16 @@ __device__ __forceinline__ void run_strip(const StripArgs& a)
     const float* pX = a.S + (c00 + lane * dT + (VEC ? rb - 1 : rb + 31));
     const float* pT = a.T + first;
     const float* pTl = COMP ? a.Tl + first : nullptr;
+    // ring offsets of the slots these go to, and of the columns written back
+    unsigned so = vu * P, xo = lane * P, wo = (RING - 31 - U + vu) * P;
     // columns q .. q+U-1 into the slots from `slot`
     // FAST: every march the call touches lies inside the window (no bounds tests)
     auto stage_cols = [&](int q, int slot, auto fast_tag) {
         constexpr bool FAST = decltype(fast_tag)::value;
         auto wrap = [](int sl) { return sl >= RING ? sl - RING : sl; };
         if constexpr (VEC) {
-            float* d = ring + wrap(slot + vu) * P + vc;
+            float* d = ring + so + vc;
+            so = ring_next<U * P, RING * P>(so);
             const bool in = FAST || q + vu < ncols;
             if (in) cp_async16_cg(d + kS0 + 1, pS);
             if (sw0) {
@@ -415,7 +426,8 @@ __device__ __forceinline__ void run_strip(const StripArgs& a)
                 if (COMP) pTl += dT;
             }
         }
-        if (lx_ok && (FAST || q + lane < ncols)) cp_async4(ring + wrap(slot + lane) * P + (VEC ? kS0 : kS0 + 32), pX);
+        if (lx_ok && (FAST || q + lane < ncols)) cp_async4(ring + xo + (VEC ? kS0 : kS0 + 32), pX);
+        xo = ring_next<U * P, RING * P>(xo);
         pX += U * dT;
     };
     // the upwind row's pairs of marches q .. q+U-1
@@ -463,8 +475,9 @@ __device__ __forceinline__ void run_strip(const StripArgs& a)
     float cU = 0.0f, cI = 0.0f, cN = 0.0f;                // carried S of rows r-1, r and i1 (the one of the two on the upwind side)
     const int nsteps = ncols + 31;
     int b0 = 0;                                           // ring slot of march s0
-    // ring offset of the lane's march s0 - lane and row
-    int ro = ((RING - lane) % RING) * P + tix;
+    // ring offset of the lane's march s0 - lane; the lane's row of a slot
+    unsigned ro = ((RING - lane) % RING) * P;
+    float* const ringr = ring + tix;
 
     // Blocks of U steps: one wait for the staged columns per block, then the
     // block's ring reads, its U node updates, and its stores. Within a block
@@ -485,34 +498,32 @@ __device__ __forceinline__ void run_strip(const StripArgs& a)
         cp_wait<(kCols < kPairs) ? kCols : kPairs>();
         __syncwarp();
 
-        int off[U];
+        unsigned off[U];
         float nU[U], nI[U], told[U], toldl[U];
 #pragma unroll
         for (int u = 0; u < U; u++) {
             off[u] = ro;
-            ro += P;
-            if (ro >= RING * P + tix) ro -= RING * P;
+            ro = ring_next<P, RING * P>(ro);
             // S of the new column: march m (rightward) or m+1
-            const int ns = right ? off[u] : ro;
-            nU[u] = ring[ns + kS0];
-            nI[u] = ring[ns + kS0 + 1];
-            told[u] = ring[off[u] + kT0];
-            toldl[u] = COMP ? ring[off[u] + kL0] : 0.0f;
+            const unsigned ns = right ? off[u] : ro;
+            nU[u] = ringr[ns + kS0];
+            nI[u] = ringr[ns + kS0 + 1];
+            told[u] = ringr[off[u] + kT0];
+            toldl[u] = COMP ? ringr[off[u] + kL0] : 0.0f;
         }
         // write back the columns every lane had finished before this block (marches s0-U-31 ..)
         {
-            int wb = b0 + (RING - 31 - U);
-            if (wb >= RING) wb -= RING;
             if constexpr (VEC) {
-                int ws = wb + vu;
-                if (ws >= RING) ws -= RING;
                 const int m = s0 + vu - U - 31;
+                const float* q = ring + wo + vc;
+                wo = ring_next<U * P, RING * P>(wo);
                 if (FAST || (m >= 0 && m < ncols)) {
-                    const float* q = ring + ws * P + vc;
                     *reinterpret_cast<float4*>(pW) = *reinterpret_cast<const float4*>(q + kT0);
                     if (COMP) *reinterpret_cast<float4*>(pWl) = *reinterpret_cast<const float4*>(q + kL0);
                 }
             } else {
+                int wb = b0 + (RING - 31 - U);
+                if (wb >= RING) wb -= RING;
                 const float* q = ring + kT0 + tix;
 #pragma unroll
                 for (int u = 0; u < U; u++) {
@@ -683,13 +694,16 @@ __device__ __forceinline__ void run_strip(const StripArgs& a)
             const int m = s0 + u - lane;
             const bool act = FAST || (vrow && (m >= 0) && (m < ncols));
             if (act) {
-                ring[off[u] + kT0] = tnw[u];
-                if (COMP) ring[off[u] + kL0] = tnwl[u];
+                ringr[off[u] + kT0] = tnw[u];
+                if (COMP) ringr[off[u] + kL0] = tnwl[u];
             }
             // feed the next strip: lane 31 just finished march s-31
             if (feeds && act) {
-                st_u64(pH + HS * u, pack_tag(tnw[u], a.tag));
-                if (COMP) st_u64(pH + HS * u + 1, pack_tag(tnwl[u], a.tag));
+                if constexpr (COMP)
+                    asm volatile("st.global.v4.u32 [%0], {%1, %2, %3, %2};" ::"l"(pH + HS * u),
+                                 "r"(__float_as_uint(tnw[u])), "r"(a.tag), "r"(__float_as_uint(tnwl[u])) : "memory");
+                else
+                    st_u64(pH + HS * u, pack_tag(tnw[u], a.tag));
             }
         }
         pH += HS * U;

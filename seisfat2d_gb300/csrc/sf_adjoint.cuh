@@ -138,10 +138,14 @@ __device__ __forceinline__ void adj_strip(const AdjStripArgs& a)
         pT2 -= 32 * kU;
         pTc -= 32 * kU;
     };
+    const bool pair_lane = consumer && lane < kU;
+    const unsigned long long* pP = a.h_in + 2 * lane;
+    unsigned po = lane % kPairsA;
     auto stage_pairs = [&](int q, auto fast_tag) {
         constexpr bool FAST = decltype(fast_tag)::value;
-        if (consumer && lane < kU && (FAST || q + lane < ncols))
-            cp_async16_cg(&R.pair[(q + lane) % kPairsA], a.h_in + 2 * (size_t)(q + lane));
+        if (pair_lane && (FAST || q + lane < ncols)) cp_async16_cg(&R.pair[po], pP);
+        pP += 2 * kU;
+        po = (po + kU) % kPairsA;
     };
     int avail = a.prog_in ? 0 : 0x7fffffff;
     auto ensure = [&](int q) {  // marches below q may be staged
@@ -168,7 +172,8 @@ __device__ __forceinline__ void adj_strip(const AdjStripArgs& a)
     unsigned long long* pH = a.h_out - 2 * 31;
 
     float my_x = 0.0f, my_pe = 0.0f, my_pev = 0.0f, pev_hold = 0.0f;
-    int tb0 = 0;  // ring slot of the block's tape rows
+    int tb0 = 0, tf0 = kLookA / kU;  // ring slots of the block's tape rows and of those staged next
+    int next_pub = a.publish ? a.publish : -1;  // the block that publishes the progress next
     unsigned ro = ((kRingA - lane) % kRingA) * 32;  // ring offset of the lane's march s0 - lane
     float* const Lr = R.L + tix;
 
@@ -242,9 +247,8 @@ __device__ __forceinline__ void adj_strip(const AdjStripArgs& a)
         // next columns, tape rows and pairs (the ring reads above are in flight meanwhile)
         ensure(s0 + kLookA + kU);
         {
-            int tf0 = tb0 + kLookA / kU;
-            if (tf0 >= kTapeBlocks) tf0 -= kTapeBlocks;
             stage(s0 + kLookA, tf0, fast_tag);
+            if (++tf0 >= kTapeBlocks) tf0 = 0;
             stage_pairs(s0 + kPairLookA, fast_tag);
             cp_commit();
         }
@@ -289,7 +293,10 @@ __device__ __forceinline__ void adj_strip(const AdjStripArgs& a)
         pV -= 32 * kU;
         pH += 2 * kU;
         if (++tb0 >= kTapeBlocks) tb0 = 0;
-        if (a.publish && (s0 & (a.publish - 1)) == 0 && s0 > 31) publish_progress(a.prog_out, a.tag, min(s0 - 31, ncols));
+        if (s0 == next_pub) {
+            publish_progress(a.prog_out, a.tag, min(s0 - 31, ncols));
+            next_pub += a.publish;
+        }
     };
     // column blocks in the order the march finishes them: the counted sweep
     // is the reverse of sweep 0, which marches down the columns, so
@@ -309,10 +316,11 @@ __device__ __forceinline__ void adj_strip(const AdjStripArgs& a)
         }
     };
     // one block past the last step writes the last columns back
+    [[maybe_unused]] const unsigned nfast = max(ncols + 1 - kLookA - kU - (31 + kU), 0);  // first steps of interior blocks: 31 + kU ..
 #pragma unroll 1
     for (int s0 = 0; s0 < nsteps + kU; s0 += kU) {
         if constexpr (INTERIOR) {
-            if (s0 >= 31 + kU && s0 + kLookA + kU <= ncols)
+            if ((unsigned)(s0 - (31 + kU)) < nfast)
                 block(s0, std::true_type{});
             else
                 block(s0, std::false_type{});

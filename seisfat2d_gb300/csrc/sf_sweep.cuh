@@ -430,13 +430,17 @@ __device__ __forceinline__ void run_strip(const StripArgs& a)
         xo = ring_next<U * P, RING * P>(xo);
         pX += U * dT;
     };
-    // the upwind row's pairs of marches q .. q+U-1
+    // the upwind row's pairs of marches q .. q+U-1; the ring holds two blocks
+    static_assert(B::PAIRS == 2 * U, "pair slots alternate");
+    constexpr int kPairWords = U * 2 * HS;
+    const bool pair_lane = consumer && lane < (COMP ? U : U / 2);  // 16-byte copies
+    const unsigned long long* pP = a.h_in + 2 * lane;
+    unsigned po = 4 * lane, pi = 0;  // ring offsets of the pairs staged and read
     auto stage_pairs = [&](int q, auto fast_tag) {
         constexpr bool FAST = decltype(fast_tag)::value;
-        constexpr int N = COMP ? U : U / 2;  // 16-byte copies
-        const int c = COMP ? q + lane : q + 2 * lane;
-        if (consumer && lane < N && (FAST || c < ncols))
-            cp_async16_cg(pring + (c % B::PAIRS) * (2 * HS), a.h_in + (size_t)HS * c);
+        if (pair_lane && (FAST || q + (COMP ? lane : 2 * lane) < ncols)) cp_async16_cg(pring + po, pP);
+        pP += U * HS;
+        po ^= kPairWords;
     };
 
     // columns of the previous sweep known to be written back
@@ -474,6 +478,7 @@ __device__ __forceinline__ void run_strip(const StripArgs& a)
     float tnl = 0.0f, tvpl = 0.0f;                        // their lo parts (compensated)
     float cU = 0.0f, cI = 0.0f, cN = 0.0f;                // carried S of rows r-1, r and i1 (the one of the two on the upwind side)
     const int nsteps = ncols + 31;
+    int next_pub = a.publish ? a.publish : -1;            // the block that publishes the progress next
     int b0 = 0;                                           // ring slot of march s0
     // ring offset of the lane's march s0 - lane; the lane's row of a slot
     unsigned ro = ((RING - lane) % RING) * P;
@@ -542,7 +547,8 @@ __device__ __forceinline__ void run_strip(const StripArgs& a)
         // the upwind strip's values of the block (every lane reads them, lane 0 uses them)
         float hv[U], hvl[U];
         {
-            const float* q = pring + (s0 % B::PAIRS) * (2 * HS);
+            const float* q = pring + pi;
+            pi ^= kPairWords;
             unsigned stale = 0;
             if (COMP) {
 #pragma unroll
@@ -709,13 +715,17 @@ __device__ __forceinline__ void run_strip(const StripArgs& a)
         pH += HS * U;
         b0 += U;
         if (b0 >= RING) b0 -= RING;
-        if (a.publish && (s0 & (a.publish - 1)) == 0 && s0 > 31) publish_progress(a.prog_out, a.tag, min(s0 - 31, ncols));
+        if (s0 == next_pub) {
+            publish_progress(a.prog_out, a.tag, min(s0 - 31, ncols));
+            next_pub += a.publish;
+        }
     };
     // one block past the last step writes the last columns back
+    [[maybe_unused]] const unsigned nfast = max(ncols - LOOK - U - (31 + U), 0);  // first steps of interior blocks: 31 + U ..
 #pragma unroll 1
     for (int s0 = 0; s0 < nsteps + U; s0 += U) {
         if constexpr (INTERIOR) {
-            if (s0 >= 31 + U && s0 + LOOK + U <= ncols - 1 && (unsigned)(s0 - g0) > (unsigned)gn)
+            if ((unsigned)(s0 - (31 + U)) < nfast && (unsigned)(s0 - g0) > (unsigned)gn)
                 block(s0, std::true_type{});
             else
                 block(s0, std::false_type{});

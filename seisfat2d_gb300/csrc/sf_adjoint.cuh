@@ -222,19 +222,27 @@ __device__ __forceinline__ void adj_strip(const AdjStripArgs& a)
                 e[u] = R.pair[(s0 + u) % kPairsA];
                 if (FAST || s0 + u < ncols) stale |= (e[u].y ^ a.tag) | (e[u].w ^ a.tag);
             }
-            if (consumer && stale != 0) {
-                // pairs the previous strip had not written when they were prefetched:
-                // wait for them, then fall kAheadA columns behind so later prefetches hit
-                if (lane0) {
+            // the rare cases of a block behind one branch
+            if ((consumer && stale != 0) || s0 + kLookA + kU > avail || s0 == next_pub) {
+                if (consumer && stale != 0) {
+                    // pairs the previous strip had not written when they were prefetched:
+                    // wait for them, then fall kAheadA columns behind so later prefetches hit
+                    if (lane0) {
 #pragma unroll
-                    for (int u = 0; u < kU; u++)
-                        if (FAST || s0 + u < ncols) {
-                            e[u].x = __float_as_uint(wait_pair(a.h_in + 2 * (size_t)(s0 + u), a.tag, sh, a.err));
-                            e[u].z = __float_as_uint(wait_pair(a.h_in + 2 * (size_t)(s0 + u) + 1, a.tag, sh, a.err));
-                        }
-                    wait_pair(a.h_in + 2 * (size_t)min(s0 + kU - 1 + kAheadA, ncols - 1) + 1, a.tag, sh, a.err);
+                        for (int u = 0; u < kU; u++)
+                            if (FAST || s0 + u < ncols) {
+                                e[u].x = __float_as_uint(wait_pair(a.h_in + 2 * (size_t)(s0 + u), a.tag, sh, a.err));
+                                e[u].z = __float_as_uint(wait_pair(a.h_in + 2 * (size_t)(s0 + u) + 1, a.tag, sh, a.err));
+                            }
+                        wait_pair(a.h_in + 2 * (size_t)min(s0 + kU - 1 + kAheadA, ncols - 1) + 1, a.tag, sh, a.err);
+                    }
+                    __syncwarp();
                 }
-                __syncwarp();
+                ensure(s0 + kLookA + kU);
+                if (s0 == next_pub) {
+                    publish_progress(a.prog_out, a.tag, min(s0 - 31, ncols));
+                    next_pub += a.publish;
+                }
             }
 #pragma unroll
             for (int u = 0; u < kU; u++) {
@@ -245,7 +253,6 @@ __device__ __forceinline__ void adj_strip(const AdjStripArgs& a)
         }
 
         // next columns, tape rows and pairs (the ring reads above are in flight meanwhile)
-        ensure(s0 + kLookA + kU);
         {
             stage(s0 + kLookA, tf0, fast_tag);
             if (++tf0 >= kTapeBlocks) tf0 = 0;
@@ -293,10 +300,6 @@ __device__ __forceinline__ void adj_strip(const AdjStripArgs& a)
         pV -= 32 * kU;
         pH += 2 * kU;
         if (++tb0 >= kTapeBlocks) tb0 = 0;
-        if (s0 == next_pub) {
-            publish_progress(a.prog_out, a.tag, min(s0 - 31, ncols));
-            next_pub += a.publish;
-        }
     };
     // column blocks in the order the march finishes them: the counted sweep
     // is the reverse of sweep 0, which marches down the columns, so

@@ -491,7 +491,6 @@ __device__ __forceinline__ void run_strip(const StripArgs& a)
     auto block = [&](int s0, auto fast_tag) {
         constexpr bool FAST = decltype(fast_tag)::value;
         auto stage_next = [&]() {
-            ensure(s0 + LOOK + U);
             int pf0 = b0 + LOOK;
             if (pf0 >= RING) pf0 -= RING;
             stage_cols(s0 + LOOK, pf0, fast_tag);
@@ -569,21 +568,29 @@ __device__ __forceinline__ void run_strip(const StripArgs& a)
                     if (FAST || s0 + u + 1 < ncols) stale |= e.w ^ a.tag_in;
                 }
             }
-            if (consumer && stale != 0) {
-                // a pair the previous strip had not written when it was prefetched:
-                // wait for it, then fall AHEAD columns behind so later prefetches hit
-                if (lane0) {
+            // the rare cases of a block behind one branch
+            if ((consumer && stale != 0) || s0 + LOOK + U > avail || s0 == next_pub) {
+                if (consumer && stale != 0) {
+                    // a pair the previous strip had not written when it was prefetched:
+                    // wait for it, then fall AHEAD columns behind so later prefetches hit
+                    if (lane0) {
 #pragma unroll
-                    for (int u = 0; u < U; u++) {
-                        const int s = s0 + u;
-                        if (FAST || s < ncols) {
-                            hv[u] = wait_pair(a.h_in + HS * s, a.tag_in, sh, a.err);
-                            if (COMP) hvl[u] = wait_pair(a.h_in + HS * s + 1, a.tag_in, sh, a.err);
+                        for (int u = 0; u < U; u++) {
+                            const int s = s0 + u;
+                            if (FAST || s < ncols) {
+                                hv[u] = wait_pair(a.h_in + HS * s, a.tag_in, sh, a.err);
+                                if (COMP) hvl[u] = wait_pair(a.h_in + HS * s + 1, a.tag_in, sh, a.err);
+                            }
                         }
+                        wait_pair(a.h_in + HS * min(s0 + U - 1 + B::AHEAD, ncols - 1), a.tag_in, sh, a.err);
                     }
-                    wait_pair(a.h_in + HS * min(s0 + U - 1 + B::AHEAD, ncols - 1), a.tag_in, sh, a.err);
+                    __syncwarp();
                 }
-                __syncwarp();
+                ensure(s0 + LOOK + U);
+                if (s0 == next_pub) {
+                    publish_progress(a.prog_out, a.tag, min(s0 - 31, ncols));
+                    next_pub += a.publish;
+                }
             }
         }
 
@@ -715,10 +722,6 @@ __device__ __forceinline__ void run_strip(const StripArgs& a)
         pH += HS * U;
         b0 += U;
         if (b0 >= RING) b0 -= RING;
-        if (s0 == next_pub) {
-            publish_progress(a.prog_out, a.tag, min(s0 - 31, ncols));
-            next_pub += a.publish;
-        }
     };
     // one block past the last step writes the last columns back
     [[maybe_unused]] const unsigned nfast = max(ncols - LOOK - U - (31 + U), 0);  // first steps of interior blocks: 31 + U ..

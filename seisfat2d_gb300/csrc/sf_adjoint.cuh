@@ -140,7 +140,8 @@ __device__ __forceinline__ void adj_strip(const AdjStripArgs& a)
     };
     const bool pair_lane = consumer && lane < kU;
     const unsigned long long* pP = a.h_in + 2 * lane;
-    unsigned po = lane % kPairsA;
+    unsigned po = lane % kPairsA, pi = 0;  // ring slots of the pairs staged and read
+    if (!consumer && lane < kPairsA) R.pair[lane] = make_uint4(0, 0, 0, 0);
     auto stage_pairs = [&](int q, auto fast_tag) {
         constexpr bool FAST = decltype(fast_tag)::value;
         if (pair_lane && (FAST || q + lane < ncols)) cp_async16_cg(&R.pair[po], pP);
@@ -219,9 +220,10 @@ __device__ __forceinline__ void adj_strip(const AdjStripArgs& a)
             unsigned stale = 0;
 #pragma unroll
             for (int u = 0; u < kU; u++) {
-                e[u] = R.pair[(s0 + u) % kPairsA];
+                e[u] = R.pair[pi + u];
                 if (FAST || s0 + u < ncols) stale |= (e[u].y ^ a.tag) | (e[u].w ^ a.tag);
             }
+            pi = (pi + kU) % kPairsA;
             // the rare cases of a block behind one branch
             if ((consumer && stale != 0) || s0 + kLookA + kU > avail || s0 == next_pub) {
                 if (consumer && stale != 0) {
@@ -246,9 +248,8 @@ __device__ __forceinline__ void adj_strip(const AdjStripArgs& a)
             }
 #pragma unroll
             for (int u = 0; u < kU; u++) {
-                const bool have = consumer && (FAST || s0 + u < ncols);
-                hx[u] = fadd(have ? __uint_as_float(e[u].x) : 0.0f, pev_hold);
-                pev_hold = have ? __uint_as_float(e[u].z) : 0.0f;
+                hx[u] = fadd(__uint_as_float(e[u].x), pev_hold);
+                pev_hold = __uint_as_float(e[u].z);
             }
         }
 

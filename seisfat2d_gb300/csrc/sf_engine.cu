@@ -334,6 +334,13 @@ extern "C" int sf_get_launch(const sf_ctx* c, int* warps, int* gang_warps)
 // warps each that fit, 3.76 with 12 (both two rounds of 24 tasks), 4.70 with
 // 10 (three); 24 warps each, where they fit, 1.96 against 2.11 with 12. 200
 // shots of 16 strips: 3.90 ms with the 12 warps each that fit, 4.04 with 8.
+// With more shots than that leaves room for, a shot still gets four warps (or
+// one per two strips) and the rest wait in the queue: fewer windows are then in
+// use at a time, and the last shots end together. Taped forward and reverse
+// sweeps of 1000 windows of about 1000 x 1001 cells 27.9 + 14.2 ms with four,
+// 31.0 + 18.1 with two, 53 + 18 with one; 1000 shots of 801 x 351 9.7 + 5.0,
+// 12.4 + 4.9, 11.7 + 6.4; 1500 shots of 401 x 101 (4 strips) 2.5 + 1.4 with
+// four, 2.2 + 1.6 with two, 2.3 + 1.5 with one.
 int sf_gang_shape(sf_ctx* c, const void* kernel, size_t smem, int nshots, int nstrips, int gang_warps, int* G,
                   int* NG)
 {
@@ -344,7 +351,8 @@ int sf_gang_shape(sf_ctx* c, const void* kernel, size_t smem, int nshots, int ns
     int slots = gang_warps;
     if (slots <= 0) {
         const long long cap_warps = cap_ctas * c->warps;
-        const long long most = std::max(1LL, std::min<long long>(2LL * nstrips, cap_warps / std::max(1, nshots)));
+        const long long least = std::min(4, (nstrips + 1) / 2);
+        const long long most = std::max(least, std::min<long long>(2LL * nstrips, cap_warps / std::max(1, nshots)));
         const int rounds = (int)((2 * nstrips + most - 1) / most);
         slots = (2 * nstrips) % rounds ? (int)most : 2 * nstrips / rounds;
     }
@@ -746,9 +754,9 @@ int sf_fwd_configure(sf_ctx* c, int nrec, bool per_shot_T, bool tape, int gang_w
     // time when each solves one shot and the windows are of one size (100
     // shots of 1701 x 351: 2.57 ms, 2.73 with one body), and hardly meet on an
     // SM when there are few (windows of about 1000 x 1001 cells: 40 shots 2.91
-    // ms, with one body 3.18; 152 shots 8.20 and 6.70, 400 shots 21.0 and
-    // 17.1; 60 of about 430 x 351: 1.35 both).
-    p.drift = (nshots > NG || c->hshots.back().ncols != c->batch_maxcols) && 2 * NG > c->sms;
+    // ms, with one body 3.18; 152 shots 8.20 and 6.70; from a queue, 400 shots
+    // 21.0 and 17.1; 60 of about 430 x 351: 1.35 both).
+    p.drift = nshots > NG || (c->hshots.back().ncols != c->batch_maxcols && 2 * NG > c->sms);
     p.maxcols = c->batch_maxcols;
     p.Tpool = c->d_T;
     p.Tlpool = comp ? c->d_Tl : nullptr;

@@ -267,12 +267,16 @@ int sf_adj_configure(sf_ctx* c, cudaStream_t st, AdjLaunch* A)
     A->hand_bytes = (size_t)NG * hand_words(nstrips, c->batch_maxcols, 2) * sizeof(unsigned long long);
     A->ggrid = dim3((unsigned)(nstrips * ((c->nxx + kGT - 1) / kGT)));
     A->gblock = dim3(256);
-    // The gather inside the reverse-sweep launch (isotropic batches, 2 or 4
-    // warps per CTA) when the device holds every reverse-sweep CTA and two
+    // The gather inside the reverse-sweep launch if asked for (isotropic
+    // batches, 2 or 4 warps per CTA): in its own launch it reads each node
+    // column once and skips what has no term, which left it too short to be
+    // worth hiding (10 shots of 1701 x 351: 0.89 ms in one launch, 0.75 + 0.05
+    // in two; 40 of 801 x 351 0.82, 0.60 + 0.11; 200 of 333 x 97 1.10, 0.28 +
+    // 0.52). Also only when the device holds every reverse-sweep CTA and two
     // gather CTAs per SM at once (600 windows that left room for 8 gather CTAs
     // took 834 ms in one launch, 26 ms in two).
     A->fused = false;
-    if (c->fuse_gather && !c->batch_ani && (c->warps == 2 || c->warps == 4)) {
+    if (c->fuse_gather > 0 && !c->batch_ani && (c->warps == 2 || c->warps == 4)) {
         const bool in = c->batch_interior;
         const void* fk = (c->warps == 2) ? (in ? (const void*)k_adjoint_gather<true, 2> : (const void*)k_adjoint_gather<false, 2>)
                                          : (in ? (const void*)k_adjoint_gather<true, 4> : (const void*)k_adjoint_gather<false, 4>);
@@ -452,7 +456,7 @@ extern "C" int sf_batch_stiffness_gradient(sf_ctx* c, float* grad_c11, float* gr
 extern "C" int sf_set_fused_gather(sf_ctx* c, int enable)
 {
     if (!c) return SF_ERR_ARG;
-    c->fuse_gather = enable != 0;
+    c->fuse_gather = enable != 0 ? 1 : 0;
     c->plan_dirty = true;
     return SF_OK;
 }

@@ -87,19 +87,6 @@ unsigned sf_next_epoch(sf_ctx* c)
 
 namespace {
 
-// expand_boundary (modeling.cu:204-232): clamp-to-edge copy of the model.
-__global__ void k_expand(const float* __restrict__ in, int nx, int nz, int nb, float* __restrict__ out)
-{
-    const int nzz = nz + 2 * nb, nxx = nx + 2 * nb;
-    const size_t n = (size_t)nzz * nxx;
-    for (size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x; idx < n;
-         idx += (size_t)gridDim.x * blockDim.x) {
-        int i = (int)(idx % nzz), j = (int)(idx / nzz);
-        int si = min(max(i - nb, 0), nz - 1), sj = min(max(j - nb, 0), nx - 1);
-        out[idx] = in[si + (size_t)sj * nz];
-    }
-}
-
 // Checks fdiv_k against __fdiv_rn for b = divs[w] over all dividends of [1, 2)
 // (both signs follow by symmetry); rbs[w] = RN(1/b), bad bit w set on any
 // difference. Then (w = n) frcp_k on [1, 2), bad bit 5, and (w = n+1, n+2)
@@ -132,20 +119,54 @@ __global__ void k_verify_div(const float* divs, int n, float* rbs, int* bad)
 }
 
 // Sets *flag when a slowness of the field (nzz x nxx) lies outside
-// in_fast_range; with Sp, also copies the field at column stride ld (rows
-// past the grid repeat the last).
-__global__ void k_check_range(const float* __restrict__ S, int nzz, int nxx, int ld, float dx, float dz, int* flag,
-                              float* __restrict__ Sp)
+// in_fast_range.
+__global__ void k_check_range(const float* __restrict__ S, int nzz, int nxx, float dx, float dz, int* flag)
 {
     bool ok = true;
-    const size_t n = (size_t)ld * nxx;
-    for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x) {
-        const size_t j = q / ld;
-        const float s = S[min((int)(q - j * ld), nzz - 1) + j * nzz];
-        ok &= in_fast_range(s, dx, dz);
-        if (Sp) Sp[q] = s;
-    }
+    const size_t n = (size_t)nzz * nxx;
+    for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x)
+        ok &= in_fast_range(S[q], dx, dz);
     if (!ok) *flag = 1;
+}
+
+// The context's padded slowness S from a model (expand_boundary,
+// modeling.cu:204-232: clamp to the edge), or with a step dS added on the
+// model's cells, or as it is; its copy Sp at the solver's column stride ld
+// (rows past the grid repeat the last); and flags[2], whether a value lies
+// outside in_fast_range. One launch: with a memset, an expansion or addition and
+// a check of their own, an update of a small model took 10 us (of 60) longer. The
+// CTAs join in flags[3] and count in flags[4]; the last one publishes and clears.
+__global__ void k_solver_slowness(float* __restrict__ S, int nx, int nz, int nb, int ld, float dx, float dz,
+                                  const float* __restrict__ model, const float* __restrict__ dS,
+                                  float* __restrict__ Sp, int* flags)
+{
+    const int nzz = nz + 2 * nb, nxx = nx + 2 * nb;
+    bool ok = true;
+    for (int j = blockIdx.x; j < nxx; j += gridDim.x)
+        for (int i = threadIdx.x; i < ld; i += blockDim.x) {
+            const int r = min(i, nzz - 1);
+            const size_t at = (size_t)r + (size_t)j * nzz;
+            float s;
+            if (model) {
+                s = model[min(max(r - nb, 0), nz - 1) + (size_t)min(max(j - nb, 0), nx - 1) * nz];
+            } else {
+                s = S[at];
+                if (dS && r >= nb && r < nzz - nb && j >= nb && j < nxx - nb)
+                    s = fadd(s, dS[(r - nb) + (size_t)(j - nb) * nz]);
+            }
+            if ((model || dS) && i < nzz) S[at] = s;
+            Sp[(size_t)i + (size_t)j * ld] = s;
+            ok &= in_fast_range(s, dx, dz);
+        }
+    const int bad = __syncthreads_or(!ok);
+    if (threadIdx.x == 0) {
+        if (bad) atomicOr(flags + 3, 1);
+        __threadfence();
+        if (atomicAdd(flags + 4, 1) == (int)gridDim.x - 1) {
+            flags[2] = atomicExch(flags + 3, 0);
+            flags[4] = 0;
+        }
+    }
 }
 
 // A window of column stride ld as nzz x ncols values.
@@ -464,15 +485,14 @@ int sf_fwd_setup(sf_ctx* c)
 
 // ------------------------------------------------------------------ models
 
-// The solver's copy of the context's slowness at its column stride, and the
-// check for the fast form of the updates (d_flags[2], read by the solves).
-int sf_check_slowness(sf_ctx* c, cudaStream_t st)
+// The context's slowness from a model on the device, by a step dS or as it is
+// (both null), with the solver's copy and the check for the fast form of the
+// updates (k_solver_slowness).
+int sf_solver_slowness(sf_ctx* c, const float* model, const float* dS, cudaStream_t st)
 {
     const int ld = strip_pitch(c->nzz);
-    const size_t n = (size_t)c->nxx * ld;
-    CK(cudaMemsetAsync(c->d_flags + 2, 0, sizeof(int), st));
-    k_check_range<<<(unsigned)std::min<size_t>((n + 255) / 256, (size_t)c->sms * 8), 256, 0, st>>>(
-        c->d_S, c->nzz, c->nxx, ld, c->dx, c->dz, c->d_flags + 2, c->d_Sp);
+    k_solver_slowness<<<std::min(c->nxx, 2 * c->sms), std::min(ld, 512), 0, st>>>(c->d_S, c->nx, c->nz, c->nb, ld, c->dx, c->dz,
+                                                                            model, dS, c->d_Sp, c->d_flags);
     CK(cudaGetLastError());
     return SF_OK;
 }
@@ -485,7 +505,7 @@ extern "C" int sf_set_slowness(sf_ctx* c, const float* s, int layout, int mem)
     if (layout == SF_LAYOUT_PADDED) {
         CK(cudaMemcpy(c->d_S, s, npad * sizeof(float),
                       mem == SF_MEM_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice));
-        int rc = sf_check_slowness(c, nullptr);
+        int rc = sf_solver_slowness(c, nullptr, nullptr, nullptr);
         // a host copy is finished when the call returns: so is its check
         if (!rc && mem != SF_MEM_DEVICE) CK(cudaStreamSynchronize(nullptr));
         return rc;
@@ -496,9 +516,7 @@ extern "C" int sf_set_slowness(sf_ctx* c, const float* s, int layout, int mem)
     if (st) return st;
     CK(cudaMemcpy(c->d_model, s, nm * sizeof(float),
                   mem == SF_MEM_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice));
-    k_expand<<<std::min<size_t>((npad + 255) / 256, 4096), 256>>>(c->d_model, c->nx, c->nz, c->nb, c->d_S);
-    CK(cudaGetLastError());
-    int rc = sf_check_slowness(c, nullptr);
+    int rc = sf_solver_slowness(c, c->d_model, nullptr, nullptr);
     if (rc) return rc;
     CK(cudaDeviceSynchronize());
     return SF_OK;

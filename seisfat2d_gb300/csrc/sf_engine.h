@@ -63,8 +63,8 @@ struct sf_ctx {
     std::string err;
 
     float* d_S = nullptr;       // padded slowness
-    float* d_Sp = nullptr;      // the same at the solver's column stride (sf_check_slowness)
-    int* d_flags = nullptr;     // [1] error flag, [2] the slowness has a value outside in_fast_range
+    float* d_Sp = nullptr;      // the same at the solver's column stride (sf_solver_slowness)
+    int* d_flags = nullptr;     // [1] error flag, [2] the slowness has a value outside in_fast_range ([3], [4]: its making)
     float* d_model = nullptr;
     size_t cap_model = 0;
     uint16_t* d_cij_all = nullptr;  // six padded code fields
@@ -178,7 +178,7 @@ int sf_dev_reserve_zero(sf_ctx* c, void** p, size_t* cap, size_t bytes);
 unsigned sf_next_epoch(sf_ctx* c);
 int sf_check_flags(sf_ctx* c, cudaStream_t st);
 // The solver's copy and the range check of the context's slowness after it changed.
-int sf_check_slowness(sf_ctx* c, cudaStream_t st);
+int sf_solver_slowness(sf_ctx* c, const float* model, const float* dS, cudaStream_t st);
 int sf_fwd_setup(sf_ctx* c);
 int sf_verify_divisors(sf_ctx* c);
 size_t sf_fwd_smem_bytes(int warps, bool comp);

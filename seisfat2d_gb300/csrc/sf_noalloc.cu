@@ -179,7 +179,7 @@ extern "C" int sf_time_propagation_noalloc(const float* S, int nx, int nz, float
     }
     const size_t npad = (size_t)nxx * nzz;
     k_check_range<<<(unsigned)std::min<size_t>((npad + 255) / 256, (size_t)g_sms[dev] * 8), 256, 0, st>>>(
-        S, nzz, nxx, nzz, dx, dz, &dh->srange, nullptr);
+        S, nzz, nxx, dx, dz, &dh->srange);
     if (cudaGetLastError() != cudaSuccess) return SF_ERR_CUDA;
     FwdParams p{};
     p.srange = &dh->srange;

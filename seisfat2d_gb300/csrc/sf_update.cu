@@ -32,8 +32,13 @@ namespace {
 // value and each tap (both read once from shared memory) serve four cells. The
 // kernel's columns come in groups of xc, so that the tile and the taps fit in
 // shared memory for any kernel size.
-constexpr int kTile = 32, kRows = 4;
+// On a grid with fewer tiles than SMs a thread has one cell instead: the rest of
+// the chip is idle, and the tile is done in a quarter of the steps (307 x 75
+// cells, 9 samples: 7.6 us, 9.0 with four; 1701 x 351, 11 samples, where a
+// thread's four cells share their reads: 19 us with four, 26 with one).
+constexpr int kTile = 32;
 
+template <int kRows>
 __global__ void __launch_bounds__(kTile / kRows * 32) k_smooth(const float* __restrict__ in, int nx, int nz, int n, int xc,
                                                                const float* __restrict__ K, float* __restrict__ out)
 {
@@ -105,19 +110,6 @@ __global__ void k_scale_interior(const float* __restrict__ g, int nx, int nz, in
     }
 }
 
-// S += dS on the model interior of the padded slowness (the pad ring keeps its
-// values, as in the reference).
-__global__ void k_add_interior(float* __restrict__ S, int nx, int nz, int nb, int nzz, const float* __restrict__ dS)
-{
-    const size_t np = (size_t)nx * nz;
-    for (size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x; idx < np;
-         idx += (size_t)gridDim.x * blockDim.x) {
-        const int i = (int)(idx % nz), j = (int)(idx / nz);
-        float* p = S + (i + nb) + (size_t)(j + nb) * nzz;
-        *p = __fadd_rn(*p, dS[idx]);
-    }
-}
-
 }  // namespace
 
 // The reference's normalised Gaussian: weight 1/(pi stdv) exp(-r^2/(2 stdv^2))
@@ -152,12 +144,15 @@ static int smooth_on_device(sf_ctx* c, const float* d_in, float* d_out, float st
     // as many kernel columns at a time as fit in shared memory
     int xc = std::min(samples, 16);
     auto smem = [&](int x) {
-        return ((size_t)(kTile + x - 1) * ((kTile + samples - 1) | 1) + kRows + (size_t)x * samples) * sizeof(float);
+        return ((size_t)(kTile + x - 1) * ((kTile + samples - 1) | 1) + 4 + (size_t)x * samples) * sizeof(float);
     };
     while (xc > 1 && smem(xc) > (size_t)200 * 1024) xc /= 2;
-    CK(cudaFuncSetAttribute(k_smooth, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem(xc)));
     const unsigned grid = (unsigned)((c->nz + kTile - 1) / kTile) * (unsigned)((c->nx + kTile - 1) / kTile);
-    k_smooth<<<grid, kTile / kRows * 32, smem(xc), st>>>(d_in, c->nx, c->nz, samples, xc, c->d_skern, d_out);
+    const int rows = (int)grid < c->sms ? 1 : 4;
+    const auto kern = rows == 1 ? k_smooth<1> : k_smooth<4>;
+    if (smem(xc) > size_t(48) * 1024)  // more than a kernel has without asking
+        CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem(xc)));
+    kern<<<grid, kTile / rows * 32, smem(xc), st>>>(d_in, c->nx, c->nz, samples, xc, c->d_skern, d_out);
     CK(cudaGetLastError());
     return SF_OK;
 }
@@ -225,9 +220,7 @@ extern "C" int sf_update_slowness(sf_ctx* c, const float* grad, int grad_mem, fl
         if (rc) return rc;
         d_dS = d_b;
     }
-    k_add_interior<<<grid, 256, 0, st>>>(c->d_S, c->nx, c->nz, c->nb, c->nzz, d_dS);
-    CK(cudaGetLastError());
-    rc = sf_check_slowness(c, st);
+    rc = sf_solver_slowness(c, nullptr, d_dS, st);
     if (rc) return rc;
     if (dS) CK(cudaMemcpyAsync(dS, d_dS, np * sizeof(float),
                                dS_mem == SF_MEM_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, st));

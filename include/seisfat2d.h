@@ -47,7 +47,7 @@ extern "C" {
 #define SF_ARITH_COMPENSATED 2 /* traveltimes carried as FP32 pairs hi + lo (see sf_set_arithmetic) */
 
 /* strip-loop forms (sf_set_strip_loop) */
-#define SF_LOOP_AUTO -1    /* interior-block body when all shots run at once, one window width, a warp per strip */
+#define SF_LOOP_AUTO -1    /* interior-block body for windows of 128 columns and more */
 #define SF_LOOP_GENERAL 0  /* one loop body with bounds tests in every block            */
 #define SF_LOOP_INTERIOR 1 /* blocks inside the window run a body without bounds tests   */
 
@@ -109,7 +109,8 @@ int sf_compute_seismogram(sf_ctx* ctx, const float* T_dev, const float* rx, cons
  * ani = 1: three launches (eikonal_ani.cu:33-45): the solve of every shot on
  * S, the qP pass over every shot's window, the solve of every shot on its
  * qP slowness. Every shot then keeps its traveltime window and its qP
- * slowness window on the device (nzz x ncols floats each, a second
+ * slowness window on the device (ncols columns of nzz floats, rounded up to
+ * whole strips of 32, each; a second
  * traveltime window in the compensated arithmetic, three factor windows
  * with SF_KEEP_TAPE), so device memory grows with the batch: split batches
  * whose windows exceed it (SF_ERR_CUDA when an allocation fails). */
@@ -200,7 +201,7 @@ int sf_get_arithmetic(const sf_ctx* ctx, int* mode);
  * sf_time_propagation in the default (reference) arithmetic, isotropic.
  * S: padded slowness on the current device (nzz x nxx, nzz = nz+6, nxx =
  * nx+6); T: output on the current device (nzz x nxx). Scratch lives in one
- * static device array of about 8 MiB that every GPU loading the library
+ * static device array of about 12 MiB that every GPU loading the library
  * holds until exit: grids with ceil(nzz/32) * nxx > 262144 are rejected with
  * SF_ERR_RANGE. The first call on a device sets that device up (looks up the
  * array's device address, sets the kernel's shared-memory limit). The first
@@ -213,19 +214,21 @@ int sf_get_arithmetic(const sf_ctx* ctx, int* mode);
 int sf_time_propagation_noalloc(const float* S, int nx, int nz, float dx, float dz, float sx, float sz,
                                 float* T, void* stream);
 
-/* Launch shape. A shot is solved by a gang of CTAs whose warps each run
- * every k-th 32-row strip. warps: warps per CTA (1..16; 0 keeps the current
- * value, default 1); gang_warps: warps per shot (0: chosen per batch so that
- * all shots of the batch are resident at once when possible). */
+/* Launch shape. A shot is solved by a gang of CTAs whose warps take the
+ * 32-row strips of its four sweeps in turn; two sweeps overlap, so up to two
+ * warps per strip find work. warps: warps per CTA (1..16; 0 keeps the current
+ * value, default 1); gang_warps: warps per shot (0: chosen per batch:
+ * two per strip when all shots are then resident at once, else an equal
+ * share of the device that divides the strips into full rounds, at least
+ * four; shots that find no gang wait in a queue). */
 int sf_set_launch(sf_ctx* ctx, int warps, int gang_warps);
 int sf_get_launch(const sf_ctx* ctx, int* warps, int* gang_warps);
 
 /* Form of the strip loops of the forward and reverse sweeps (no counterpart
  * in the reference). Both forms compute the same bits; the interior-block
  * form runs fewer instructions per step but is larger code, which measured
- * faster for a batch whose shots all run at once with one window width and
- * one warp per strip, slower for uneven windows or several strips per warp.
- * SF_LOOP_AUTO (default) chooses per batch (taped batches with more than 8
+ * faster where most of a march lies inside the window, that is for windows of
+ * 128 columns and more. SF_LOOP_AUTO (default) chooses per batch (taped batches with more than 8
  * warps per CTA always run the general form);
  * sf_plan_autotune times both. last_interior: whether the last batch's
  * forward used the interior-block form (the reverse sweeps follow it). */

@@ -113,6 +113,31 @@ def test_slowness_outside_fast_range(oracle, engine_lib, cuda, arith, ani, outli
                    nonzero=outlier or not ani)
 
 
+def test_tables_in_a_row(oracle, engine_lib, cuda):
+    """Table copies follow each other, the solve before them and other work on
+    their stream in order, eagerly and in a captured graph."""
+    m = smooth_model(203, 87, 10.0, seed=6)
+    S = oracle.expand_boundary(m)
+    shots = [(100.0 * k + 30.0, 0.0) for k in range(12)]
+    want = np.stack([oracle.solve_f32(S, 10.0, 10.0, *s) for s in shots])
+    e = engine(m)
+    none = np.zeros(0, np.float32)
+    T = cuda.zeros(want.shape, device="cuda")
+    for _ in range(3):
+        e.batch_forward(shots, none, none, keep_tables=True)
+        for k in range(12):
+            e.batch_table(k, e.nxx, out=T[k])
+            T[k].mul_(2.0)
+        assert np.array_equal(T.cpu().numpy(), 2 * want)
+    st, g = cuda.cuda.Stream(), cuda.cuda.CUDAGraph()
+    with cuda.cuda.graph(g, stream=st):
+        for k in range(12):
+            e.batch_table(k, e.nxx, out=T[k], stream=st)
+        T.mul_(4.0)
+    g.replay()
+    assert np.array_equal(T.cpu().numpy(), 4 * want)
+
+
 # the qP pass's groups of shots: one shot, a partly filled last group
 @pytest.mark.parametrize("nshots", [1, 41])
 def test_qp_groups(oracle, engine_lib, cuda, nshots):

@@ -286,8 +286,7 @@ __device__ __forceinline__ void adj_strip(const AdjStripArgs& a)
                 Lr[off[u]] = lo[u];
                 pV[-32 * u] = vv[u];
                 if (feeds)
-                    asm volatile("st.global.v4.u32 [%0], {%1, %2, %3, %2};" ::"l"(pH + 2 * u), "r"(__float_as_uint(opv[u])),
-                                 "r"(a.tag), "r"(__float_as_uint(opev[u])) : "memory");
+                    st_pairs(pH + 2 * u, opv[u], opev[u], a.tag);
             }
         }
         // mark the block's tape entries if a term is not zero (read by the gather)
@@ -755,8 +754,8 @@ __global__ void __launch_bounds__(256) k_gather(GatherParams p)
 // (r^2 is exact there, so one multiply-add per element, and the half waits
 // for the end) and the latency of each sum's chain, so the sums are spread
 // over the 8 CTAs of one cluster, which leave them in the first CTA's shared
-// memory; one CTA of 1024 threads took
-// 0.70 ms for 801000 picks, the cluster takes 0.18 ms.
+// memory; one CTA of 1024 threads took 0.70 ms for 801000 picks, the cluster
+// takes 0.18 ms.
 constexpr int kResCtas = 8, kResThreads = 1024 / kResCtas, kResUnroll = 8;
 __global__ void __cluster_dims__(kResCtas, 1, 1) __launch_bounds__(kResThreads)
     k_residual(const float* picks, const float* tobs, size_t n, float* res, double* misfit)

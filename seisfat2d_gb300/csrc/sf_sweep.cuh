@@ -9,9 +9,9 @@
 // upwind value. Consecutive strips (usually on other SMs) are chained through
 // global memory without fences: the last lane of strip p writes each value of
 // its row together with a tag (launch epoch and shot number) as one 64-bit
-// store; strip p+1 prefetches the pairs (through L2 only, so that a line of
-// which the producer had written a part is never found again in L1) and
-// checks the tags. A stale pair (the producer has not got there yet) sends
+// store (two pairs in one 16-byte store in the compensated arithmetic); strip
+// p+1 prefetches the pairs (through L2 only, so that a line of which the
+// producer had written a part is never found again in L1) and checks the tags. A stale pair (the producer has not got there yet) sends
 // lane 0 into a bounded spin on the pair itself, after which it waits until
 // the producer is some columns further on, so later prefetches find their
 // data. Producers never wait on consumers, so every wait points to an earlier
@@ -131,11 +131,6 @@ __device__ __forceinline__ void cp_async4(void* smem, const void* gmem)
     unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(sa), "l"(gmem) : "memory");
 }
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem)
-{
-    unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gmem) : "memory");
-}
 __device__ __forceinline__ void cp_async16_cg(void* smem, const void* gmem)
 {
     unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
@@ -166,6 +161,13 @@ __device__ __forceinline__ unsigned long long ld_relaxed_u64(const unsigned long
 __device__ __forceinline__ void st_u64(unsigned long long* p, unsigned long long v)
 {
     asm volatile("st.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+// Two pairs {v, tag}, {w, tag} in one 16-byte store, each one 64-bit element of it.
+__device__ __forceinline__ void st_pairs(unsigned long long* p, float v, float w, unsigned tag)
+{
+    asm volatile("{\n.reg .b64 a, b;\nmov.b64 a, {%1, %3};\nmov.b64 b, {%2, %3};\nst.global.v2.b64 [%0], {a, b};\n}\n" ::"l"(p),
+                 "r"(__float_as_uint(v)), "r"(__float_as_uint(w)), "r"(tag)
+                 : "memory");
 }
 __device__ __forceinline__ unsigned long long pack_tag(float v, unsigned tag)
 {
@@ -713,8 +715,7 @@ __device__ __forceinline__ void run_strip(const StripArgs& a)
             // feed the next strip: lane 31 just finished march s-31
             if (feeds && act) {
                 if constexpr (COMP)
-                    asm volatile("st.global.v4.u32 [%0], {%1, %2, %3, %2};" ::"l"(pH + HS * u),
-                                 "r"(__float_as_uint(tnw[u])), "r"(a.tag), "r"(__float_as_uint(tnwl[u])) : "memory");
+                    st_pairs(pH + HS * u, tnw[u], tnwl[u], a.tag);
                 else
                     st_u64(pH + HS * u, pack_tag(tnw[u], a.tag));
             }

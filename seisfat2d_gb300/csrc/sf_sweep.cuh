@@ -285,7 +285,9 @@ __device__ __forceinline__ int wait_progress(const unsigned long long* p, unsign
             if (w.give_up(sh, err)) break;
         }
     }
-    return __shfl_sync(0xffffffffu, cols, 0);
+    cols = __shfl_sync(0xffffffffu, cols, 0);
+    __syncwarp();  // orders the other lanes' copies after lane 0's acquire
+    return cols;
 }
 
 // Publishes that this warp's strip has written `cols` columns back: every
@@ -318,8 +320,8 @@ __device__ __forceinline__ void wait_counter(const unsigned* p, unsigned target,
 // (hi, lo); the second handoff pair of a column carries lo.
 //
 // DIR: the march's direction, right (1), left (-1) or a runtime value (0, one
-// body for both; solve_window says when). The row direction and the first sweep's start
-// values are runtime values, so the two sweeps that run at the same time share
+// body for both, where FwdParams::drift is set). The row direction and the
+// first sweep's start values are runtime values, so the two sweeps that run at the same time share
 // their code: with a copy per sweep, loops of up to 14 KB were in flight on
 // an SM and instruction fetch was 16% of the stalls. The node's cells need no
 // more for it than a select: of the two slowness columns a lane holds, the

@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include <cmath>
+#include <cstring>
 #include <type_traits>
 #include <vector>
 
@@ -38,9 +39,17 @@ namespace {
 // thread's four cells share their reads: 19 us with four, 26 with one).
 constexpr int kTile = 32;
 
-template <int kRows>
+// Kernels of up to 31 x 31 taps go along as an argument of the launch instead of
+// a copy before it (update of 307 x 75 cells, 9 samples: 64.7 -> 62.2 us).
+constexpr int kInlineTaps = 31 * 31;
+struct Taps {
+    float k[kInlineTaps];
+    __device__ float operator[](size_t q) const { return k[q]; }
+};
+
+template <int kRows, class K_t>
 __global__ void __launch_bounds__(kTile / kRows * 32) k_smooth(const float* __restrict__ in, int nx, int nz, int n, int xc,
-                                                               const float* __restrict__ K, float* __restrict__ out)
+                                                               const __grid_constant__ K_t K, float* __restrict__ out)
 {
     extern __shared__ float sm_smooth[];
     const int mid = n / 2, rows = kTile + n - 1, pitch = rows | 1;
@@ -137,10 +146,16 @@ static int smooth_on_device(sf_ctx* c, const float* d_in, float* d_out, float st
 {
     std::vector<float> k;
     sf_smooth_kernel(stdv, samples, k);
-    int rc = sf_dev_reserve(c, (void**)&c->d_skern, &c->cap_skern, k.size() * sizeof(float));
-    if (rc) return rc;
-    c->h_skern.swap(k);
-    CK(cudaMemcpyAsync(c->d_skern, c->h_skern.data(), c->h_skern.size() * sizeof(float), cudaMemcpyHostToDevice, st));
+    const bool along = k.size() <= (size_t)kInlineTaps;
+    Taps taps;
+    if (along) {
+        std::memcpy(taps.k, k.data(), k.size() * sizeof(float));
+    } else {
+        int rc = sf_dev_reserve(c, (void**)&c->d_skern, &c->cap_skern, k.size() * sizeof(float));
+        if (rc) return rc;
+        c->h_skern.swap(k);
+        CK(cudaMemcpyAsync(c->d_skern, c->h_skern.data(), c->h_skern.size() * sizeof(float), cudaMemcpyHostToDevice, st));
+    }
     // as many kernel columns at a time as fit in shared memory
     int xc = std::min(samples, 16);
     auto smem = [&](int x) {
@@ -149,10 +164,16 @@ static int smooth_on_device(sf_ctx* c, const float* d_in, float* d_out, float st
     while (xc > 1 && smem(xc) > (size_t)200 * 1024) xc /= 2;
     const unsigned grid = (unsigned)((c->nz + kTile - 1) / kTile) * (unsigned)((c->nx + kTile - 1) / kTile);
     const int rows = (int)grid < c->sms ? 1 : 4;
-    const auto kern = rows == 1 ? k_smooth<1> : k_smooth<4>;
-    if (smem(xc) > size_t(48) * 1024)  // more than a kernel has without asking
-        CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem(xc)));
-    kern<<<grid, kTile / rows * 32, smem(xc), st>>>(d_in, c->nx, c->nz, samples, xc, c->d_skern, d_out);
+    auto launch = [&](auto kern, const auto& K) {
+        if (smem(xc) > size_t(48) * 1024)  // more than a kernel has without asking
+            CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem(xc)));
+        kern<<<grid, kTile / rows * 32, smem(xc), st>>>(d_in, c->nx, c->nz, samples, xc, K, d_out);
+        return (int)SF_OK;
+    };
+    const float* dk = c->d_skern;
+    const int rc = along ? (rows == 1 ? launch(k_smooth<1, Taps>, taps) : launch(k_smooth<4, Taps>, taps))
+                         : (rows == 1 ? launch(k_smooth<1, const float*>, dk) : launch(k_smooth<4, const float*>, dk));
+    if (rc) return rc;
     CK(cudaGetLastError());
     return SF_OK;
 }

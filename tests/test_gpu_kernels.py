@@ -171,8 +171,10 @@ def test_residual_sums(engine_lib, cuda, nrec):
     assert J == 0.5 * part[0]
 
 
-# the smoothing's 32 x 32 tiles of four rows a thread, kernels up to wider than a tile
-@pytest.mark.parametrize("nx,nz,samples", [(4, 4, 3), (31, 33, 5), (32, 32, 1), (33, 63, 31), (65, 36, 71)])
+# the smoothing's 32 x 32 tiles, a cell or (from a tile per SM on) four cells a
+# thread, kernels up to wider than a tile, as an argument (31) or copied (33)
+@pytest.mark.parametrize("nx,nz,samples", [(4, 4, 3), (31, 33, 5), (32, 32, 1), (33, 63, 31), (65, 36, 71),
+                                           (700, 253, 31), (703, 250, 33)])
 def test_smoothing_tiles(oracle, engine_lib, cuda, nx, nz, samples):
     f = np.random.default_rng(nx).standard_normal((nx, nz)).astype(np.float32)
     e = engine(smooth_model(nx, nz, 10.0))

@@ -78,9 +78,11 @@ unsigned sf_next_epoch(sf_ctx* c)
 {
     // after a wrap an epoch's tags could meet pairs an earlier cycle left in
     // the handoff buffers: the next forward and adjoint launches clear them
-    if (c->epoch == (1u << 22) - 1) c->hand_stale_f = c->hand_stale_a = true;
-    c->epoch = (c->epoch % ((1u << 22) - 1)) + 1;
-    return c->epoch;
+    if (c->epoch == (1u << 22) - 1) {
+        c->hand_stale_f = c->hand_stale_a = true;
+        c->epoch = kGraphEpoch;
+    }
+    return ++c->epoch;
 }
 
 // ------------------------------------------------------------------ kernels

@@ -44,6 +44,11 @@ struct AdjLaunch {
 // Kernels timed by sf_kernel_times (events around each launch when enabled).
 enum { SF_KT_FORWARD = 0, SF_KT_RESIDUAL = 1, SF_KT_ADJOINT = 2, SF_KT_GATHER = 3, SF_KT_N = 4 };
 
+// Handoff-tag epoch of every captured launch. A graph replays the epoch of its
+// capture, which no later eager launch may then have: it clears no buffer and
+// would take the last replay's pairs and progress words for its own.
+constexpr unsigned kGraphEpoch = 1;
+
 struct sf_ctx {
     int dev = 0;
     int nx = 0, nz = 0, nb = 3, nxx = 0, nzz = 0;
@@ -94,7 +99,7 @@ struct sf_ctx {
     float* d_Sq = nullptr; size_t cap_Sq = 0;
     unsigned long long* d_hand = nullptr; size_t cap_hand = 0;
     unsigned* d_ctr = nullptr; size_t cap_ctr = 0;
-    unsigned epoch = 0;  // launches so far (handoff tags)
+    unsigned epoch = kGraphEpoch;  // of the last launch (handoff tags)
     bool hand_stale_f = false, hand_stale_a = false;  // the epoch wrapped: clear the handoff buffers
     int last_G = 1, last_NG = 1;
     uint8_t* d_tcode = nullptr; size_t cap_tcode = 0;
@@ -174,7 +179,7 @@ int sf_cuda_check(sf_ctx* c, cudaError_t e, const char* what);
 int sf_dev_reserve(sf_ctx* c, void** p, size_t* cap, size_t bytes);
 // Same, zero-filled whenever it (re)allocates.
 int sf_dev_reserve_zero(sf_ctx* c, void** p, size_t* cap, size_t bytes);
-// Next handoff-tag epoch (never 0; wraps within 22 bits).
+// Next handoff-tag epoch (never 0 or kGraphEpoch; wraps within 22 bits).
 unsigned sf_next_epoch(sf_ctx* c);
 int sf_check_flags(sf_ctx* c, cudaStream_t st);
 // The solver's copy and the range check of the context's slowness after it changed.

@@ -3,13 +3,14 @@
 // eagerly or be replayed from a CUDA graph; the launch-shape autotuner; and
 // per-kernel timing with CUDA events.
 //
-// A graph replays its kernels with the handoff-tag epoch of the capture, so a
-// consumer could take a pair left by the previous replay for one of this
-// replay's. A planned iteration therefore zeroes the handoff pairs of both
-// persistent kernels before launching them (32 B per gang, strip and column
-// for the forward, 64 B for the adjoint: 0.2 GB for 100 gangs on a 1707 x 357
-// grid, a few tens of microseconds), which makes it safe to replay from any
-// graph, the context's own or one the caller captured.
+// A graph replays its kernels with the handoff-tag epoch of the capture
+// (kGraphEpoch, which eager launches skip), so a consumer could take a pair
+// left by the previous replay for one of this replay's. A planned iteration
+// therefore zeroes the handoff pairs of both persistent kernels before
+// launching them (32 B per gang, strip and column for the forward, 64 B for
+// the adjoint: 0.2 GB for 100 gangs on a 1707 x 357 grid, a few tens of
+// microseconds), which makes it safe to replay from any graph, the context's
+// own or one the caller captured.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -150,15 +151,16 @@ extern "C" int sf_plan_iteration(sf_ctx* c, const float* t_obs, float* picks, do
     if (rc) return rc;
     CK(cudaSetDevice(c->dev));
     cudaStream_t st = (cudaStream_t)stream;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    CK(cudaStreamIsCapturing(st, &cs));
+    const bool capturing = cs != cudaStreamCaptureStatusNone;
     if (c->plan_dirty) {
-        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-        CK(cudaStreamIsCapturing(st, &cs));
-        if (cs != cudaStreamCaptureStatusNone)
+        if (capturing)
             return sf_fail(c, SF_ERR_STATE, "launch shape changed: run the plan once before capturing it");
         rc = plan_configure(c, st);
         if (rc) return rc;
     }
-    const unsigned ef = sf_next_epoch(c), ea = sf_next_epoch(c);
+    const unsigned ef = capturing ? kGraphEpoch : sf_next_epoch(c), ea = capturing ? kGraphEpoch : sf_next_epoch(c);
     rc = plan_enqueue(c, t_obs, picks, misfit, grad, ef, ea, st);
     if (rc) return rc;
     plan_done(c, t_obs, picks);
@@ -172,7 +174,7 @@ static int graph_capture(sf_ctx* c, const float* t_obs, float* picks, double* mi
     const bool timing = c->timing;
     c->timing = false;  // no event records inside the graph
     CK(cudaStreamBeginCapture(c->cap_stream, cudaStreamCaptureModeThreadLocal));
-    int rc = plan_enqueue(c, t_obs, picks, misfit, grad, 1, 1, c->cap_stream);
+    int rc = plan_enqueue(c, t_obs, picks, misfit, grad, kGraphEpoch, kGraphEpoch, c->cap_stream);
     cudaGraph_t g = nullptr;
     cudaError_t e = cudaStreamEndCapture(c->cap_stream, &g);
     c->timing = timing;

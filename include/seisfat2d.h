@@ -75,7 +75,10 @@ int sf_ctx_destroy(sf_ctx* ctx);
 int sf_ctx_dims(const sf_ctx* ctx, int* nxx, int* nzz, int* nb);
 
 /* Modeling::set_properties + expand_boundary (modeling.cu:47-60, :204-232)
- * and copy_slowness_to_device (:281-284). */
+ * and copy_slowness_to_device (:281-284). Runs on the legacy default stream.
+ * With a padded device field the call returns before its copy is done; calls
+ * that use the slowness, on any stream, and replays of graphs captured from
+ * them follow it. It does not wait for earlier calls on non-blocking streams. */
 int sf_set_slowness(sf_ctx* ctx, const float* s, int layout, int mem);
 /* padded slowness back (nzz x nxx) */
 int sf_get_slowness(sf_ctx* ctx, float* out, int mem);

@@ -248,6 +248,8 @@ extern "C" int sf_ctx_create(sf_ctx** out, int nx, int nz, float dx, float dz, i
     cap = 0;
     if (st == SF_OK) st = sf_dev_reserve(c, (void**)&c->d_flags, &cap, 256);
     if (st == SF_OK) st = sf_cuda_check(c, cudaMemset(c->d_flags, 0, 256), "cudaMemset");
+    if (st == SF_OK)
+        st = sf_cuda_check(c, cudaEventCreateWithFlags(&c->slowness_ev, cudaEventDisableTiming), "cudaEventCreateWithFlags");
     if (st == SF_OK) st = sf_fwd_setup(c);
     if (st != SF_OK) {
         sf_ctx_destroy(c);
@@ -269,6 +271,7 @@ extern "C" int sf_ctx_destroy(sf_ctx* c)
                     c->d_vfac, c->d_gcij, c->d_fuse, c->d_Tl, c->d_srange, c->d_kterm};
     for (void* b : bufs)
         if (b) cudaFree(b);
+    if (c->slowness_ev) cudaEventDestroy(c->slowness_ev);
     delete c;
     return SF_OK;
 }
@@ -507,6 +510,26 @@ int sf_solver_slowness(sf_ctx* c, const float* model, const float* dS, cudaStrea
     return SF_OK;
 }
 
+// Orders work on `st` that reads or updates the slowness after the last
+// sf_set_slowness, which returns before its work on the legacy stream is done
+// when its source is a padded device field. Blocking streams follow the legacy
+// stream by themselves. A captured launch waits at every replay, for the
+// sf_set_slowness called last by then.
+int sf_wait_slowness(sf_ctx* c, cudaStream_t st)
+{
+    if (!st || st == cudaStreamLegacy) return SF_OK;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    CK(cudaStreamIsCapturing(st, &cs));
+    if (cs != cudaStreamCaptureStatusNone) {
+        CK(cudaStreamWaitEvent(st, c->slowness_ev, cudaEventWaitExternal));
+        return SF_OK;
+    }
+    unsigned flags = 0;
+    CK(cudaStreamGetFlags(st, &flags));
+    if (flags & cudaStreamNonBlocking) CK(cudaStreamWaitEvent(st, c->slowness_ev, 0));
+    return SF_OK;
+}
+
 extern "C" int sf_set_slowness(sf_ctx* c, const float* s, int layout, int mem)
 {
     if (!c || !s) return SF_ERR_ARG;
@@ -516,9 +539,10 @@ extern "C" int sf_set_slowness(sf_ctx* c, const float* s, int layout, int mem)
         CK(cudaMemcpy(c->d_S, s, npad * sizeof(float),
                       mem == SF_MEM_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice));
         int rc = sf_solver_slowness(c, nullptr, nullptr, nullptr);
-        // a host copy is finished when the call returns: so is its check
-        if (!rc && mem != SF_MEM_DEVICE) CK(cudaStreamSynchronize(nullptr));
-        return rc;
+        if (rc) return rc;
+        if (mem == SF_MEM_DEVICE) CK(cudaEventRecord(c->slowness_ev, nullptr));  // see sf_wait_slowness
+        else CK(cudaStreamSynchronize(nullptr));  // a host copy is finished when the call returns: so is its check
+        return SF_OK;
     }
     if (layout != SF_LAYOUT_MODEL) return sf_fail(c, SF_ERR_ARG, "unknown layout");
     const size_t nm = (size_t)c->nx * c->nz;
@@ -893,7 +917,8 @@ int sf_launch_shots(sf_ctx* c, int ani, int nrec, float* d_picks, bool keep_tabl
 {
     const bool stall = c->stall_next;  // sf_test_stall_next_batch
     c->stall_next = false;
-    int rc;
+    int rc = sf_wait_slowness(c, st);
+    if (rc) return rc;
     if (!ani) {
         FwdLaunch L;
         rc = sf_fwd_configure(c, nrec, keep_tables, tape, gang_warps, st, &L, nullptr);

@@ -70,6 +70,7 @@ struct sf_ctx {
     float* d_S = nullptr;       // padded slowness
     float* d_Sp = nullptr;      // the same at the solver's column stride (sf_solver_slowness)
     int* d_flags = nullptr;     // [1] error flag, [2] the slowness has a value outside in_fast_range ([3], [4]: its making)
+    cudaEvent_t slowness_ev = nullptr;  // the end of the last sf_set_slowness that returned before it (sf_wait_slowness)
     float* d_model = nullptr;
     size_t cap_model = 0;
     uint16_t* d_cij_all = nullptr;  // six padded code fields
@@ -184,6 +185,8 @@ unsigned sf_next_epoch(sf_ctx* c);
 int sf_check_flags(sf_ctx* c, cudaStream_t st);
 // The solver's copy and the range check of the context's slowness after it changed.
 int sf_solver_slowness(sf_ctx* c, const float* model, const float* dS, cudaStream_t st);
+// Work on `st` follows the slowness that was set last.
+int sf_wait_slowness(sf_ctx* c, cudaStream_t st);
 int sf_fwd_setup(sf_ctx* c);
 int sf_verify_divisors(sf_ctx* c);
 size_t sf_fwd_smem_bytes(int warps, bool comp);

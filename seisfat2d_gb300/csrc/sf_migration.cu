@@ -593,7 +593,8 @@ static int table_terms(sf_ctx* c, const float* Ts, const float* Tr, int nsrc, in
                        TermTable* q, cudaStream_t st)
 {
     const size_t ntab = (size_t)nsrc + nrec, n = (size_t)nr * nc;
-    int rc = sf_dev_reserve(c, (void**)&c->d_kterm, &c->cap_kterm, 2 * ntab * n * sizeof(float4));
+    int rc = sf_wait_slowness(c, st);  // (the operators' kernels follow this one)
+    if (!rc) rc = sf_dev_reserve(c, (void**)&c->d_kterm, &c->cap_kterm, 2 * ntab * n * sizeof(float4));
     if (rc) return rc;
     q->a = reinterpret_cast<float4*>(c->d_kterm);
     q->b = reinterpret_cast<float2*>(q->a + ntab * n);

@@ -160,6 +160,8 @@ extern "C" int sf_plan_iteration(sf_ctx* c, const float* t_obs, float* picks, do
         rc = plan_configure(c, st);
         if (rc) return rc;
     }
+    rc = sf_wait_slowness(c, st);
+    if (rc) return rc;
     const unsigned ef = capturing ? kGraphEpoch : sf_next_epoch(c), ea = capturing ? kGraphEpoch : sf_next_epoch(c);
     rc = plan_enqueue(c, t_obs, picks, misfit, grad, ef, ea, st);
     if (rc) return rc;
@@ -208,6 +210,8 @@ extern "C" int sf_plan_graph_launch(sf_ctx* c, const float* t_obs, float* picks,
         rc = graph_capture(c, t_obs, picks, misfit, grad);
         if (rc) return rc;
     }
+    rc = sf_wait_slowness(c, st);
+    if (rc) return rc;
     CK(cudaGraphLaunch(c->graph_exec, st));
     plan_done(c, t_obs, picks);
     return SF_OK;
@@ -224,6 +228,8 @@ extern "C" int sf_plan_autotune(sf_ctx* c, const float* t_obs, float* picks, dou
     if (reps < 1) return sf_fail(c, SF_ERR_ARG, "reps must be >= 1");
     CK(cudaSetDevice(c->dev));
     cudaStream_t st = (cudaStream_t)stream;
+    rc = sf_wait_slowness(c, st);
+    if (rc) return rc;
     const int nstrips = (c->nzz + 31) / 32;
     std::vector<int> gangs = {0, nstrips};
     for (int d = 2; d <= 4; d++)

@@ -241,7 +241,8 @@ extern "C" int sf_update_slowness(sf_ctx* c, const float* grad, int grad_mem, fl
         if (rc) return rc;
         d_dS = d_b;
     }
-    rc = sf_solver_slowness(c, nullptr, d_dS, st);
+    rc = sf_wait_slowness(c, st);
+    if (!rc) rc = sf_solver_slowness(c, nullptr, d_dS, st);
     if (rc) return rc;
     if (dS) CK(cudaMemcpyAsync(dS, d_dS, np * sizeof(float),
                                dS_mem == SF_MEM_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, st));

@@ -1,5 +1,6 @@
 """Calls that share a context's buffers stay in order whatever their streams
-and however they were launched: eager calls after graph replays."""
+and however they were launched: eager calls after graph replays, streams that
+do not wait for the default one."""
 import numpy as np
 import pytest
 
@@ -52,3 +53,64 @@ def test_eager_calls_after_a_replay(engine_lib, cuda, arith, captured):
     e2 = engine(b, arith)
     e2.batch_forward(SHOTS, rx, rz, keep_tape=True)
     assert np.array_equal(g1, e2.misfit_gradient(np.zeros_like(want))[1])
+
+
+# a padded device slowness is set while its stream is busy (some 50 ms); the
+# calls after it, on a stream that does not wait for that one, use it all the
+# same. The second model has values outside the fast updates' range.
+@pytest.mark.parametrize("call", ["batch", "table", "plan", "graph", "captured", "autotune", "update", "image"])
+def test_slowness_reaches_other_streams(engine_lib, cuda, call):
+    a, b = models()
+    b[40:60, 30:50] *= 1e-6
+    rx, rz = surface_receivers(NX, 10.0, step=3)
+    e, ref = engine(a), engine(b)
+    pad = lambda m: cuda.from_numpy(np.pad(m, 3, mode="edge")).cuda()
+    S = {0: pad(a), 1: pad(b)}
+    st = cuda.cuda.Stream()
+    t_obs = cuda.zeros((len(SHOTS), len(rx)), device="cuda")
+    picks, grad = cuda.empty_like(t_obs), cuda.empty((e.nxx, e.nzz), device="cuda")
+    want = cuda.from_numpy(ref.batch_forward(SHOTS, rx, rz)).cuda()
+    T = cuda.empty((e.nxx, e.nzz), device="cuda")
+    if call in ("plan", "graph", "captured", "autotune"):
+        e.plan_batch(SHOTS, rx, rz)
+    if call == "captured":
+        g = cuda.cuda.CUDAGraph()
+        with cuda.cuda.graph(g, stream=st):
+            e.plan_iteration(picks, t_obs, grad, stream=st)
+    if call == "table":
+        want = cuda.from_numpy(ref.time_propagation(*SHOTS[0])).cuda()
+    if call == "update":
+        grad.copy_(cuda.linspace(0.0, 1.0, grad.numel(), device="cuda").view_as(grad))
+        ref.update_slowness(grad, 1e-5)
+        want = cuda.from_numpy(ref.get_slowness()).cuda()
+    if call == "image":
+        e.time_propagation(*SHOTS[0], out=T)
+        args = (T[None], T[None], np.array([120.0]), np.array([300.0]), cuda.ones((1, 1, 400), device="cuda"), 0.004, 40.0, 1e4)
+        want = ref.kirchhoff_image(*args, out=cuda.empty((NX, NZ), device="cuda"))
+    cuda.cuda.synchronize()
+    for _ in range(3):
+        e.set_slowness(S[0], padded=True)
+        cuda.cuda.synchronize()
+        cuda.cuda._sleep(100_000_000)
+        e.set_slowness(S[1], padded=True)
+        with cuda.cuda.stream(st):
+            if call == "batch":
+                got = e.batch_forward(SHOTS, rx, rz, out=picks, stream=st)
+            elif call == "table":
+                got = e.time_propagation(*SHOTS[0], out=T, stream=st)
+            elif call in ("plan", "graph"):
+                (e.plan_iteration if call == "plan" else e.plan_graph_launch)(picks, t_obs, grad, stream=st)
+                got = picks
+            elif call == "captured":
+                g.replay()
+                got = picks
+            elif call == "autotune":
+                e.plan_autotune(picks, t_obs, grad, reps=1, stream=st)
+                got = picks
+            elif call == "update":
+                e.update_slowness(grad, 1e-5, stream=st)
+                got = cuda.from_numpy(e.get_slowness()).cuda()
+            else:
+                got = e.kirchhoff_image(*args, out=cuda.empty((NX, NZ), device="cuda"), stream=st)
+            st.synchronize()
+        assert np.array_equal(got.cpu().numpy(), want.cpu().numpy(), equal_nan=True)

@@ -198,11 +198,11 @@ __device__ __forceinline__ void adj_strip(const AdjStripArgs& a)
             const float c = t.c1[e], cm = fsub(1.0f, c);
             c2[u] = t.c2[e];
             // dT/d{tv, te, tev} of the candidate: (1,0,0), (0,1,0), (c,-c,1), (0,1-c,c), (1-c,0,c);
-            // c is zero for the first two, so 1 goes with 5 and 2 with 4, and a kept node's is zero too
+            // c is zero for the first two, so 1 goes with 5 and 2 with 4; the zeros are selected below
             br[u] = t.code[e] & 7;
-            const bool two = br[u] == 3, odd = br[u] & 1, any = br[u] != 0;
-            av[u] = two ? c : (odd ? cm : 0.0f);
-            ae[u] = two ? -c : (any & !odd ? cm : 0.0f);
+            const bool two = br[u] == 3;
+            av[u] = two ? c : cm;
+            ae[u] = two ? -c : cm;
             aev[u] = two ? 1.0f : c;
         }
         // write back the columns every lane had finished before this block (marches s0-kU-31 ..)
@@ -272,10 +272,10 @@ __device__ __forceinline__ void adj_strip(const AdjStripArgs& a)
             if (!FAST && !(vrow && (m >= 0) && (m < ncols))) mu = 0.0f;
             lo[u] = br[u] ? 0.0f : mu;
             vv[u] = fmul(mu, c2[u]);
-            opv[u] = fmul(mu, av[u]);
-            opev[u] = fmul(mu, aev[u]);
+            opv[u] = (br[u] & 1) ? fmul(mu, av[u]) : 0.0f;
+            opev[u] = (br[u] >= 3) ? fmul(mu, aev[u]) : 0.0f;
             my_x = fadd(opv[u], my_pev);  // this node's pv + the previous node's pev
-            my_pe = fmul(mu, ae[u]);
+            my_pe = ((unsigned)(br[u] - 2) < 3u) ? fmul(mu, ae[u]) : 0.0f;
             my_pev = opev[u];
         }
 

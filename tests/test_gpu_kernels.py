@@ -261,3 +261,23 @@ def test_fast_root_reciprocal_and_quotient(tmp_path, cuda):
                     os.path.join(ROOT, "seisfat2d_gb300", "csrc"), "-o", str(exe), str(src)], check=True)
     out = subprocess.run([str(exe)], check=True, capture_output=True, text=True, timeout=60).stdout
     assert out.split() == ["0", "0", "0"]
+
+
+@pytest.mark.parametrize("big", [np.inf, 3e38])
+def test_infinite_pick_gradients(oracle, engine_lib, cuda, arith, big):
+    """An infinite pick gradient, and finite ones whose sums overflow, run
+    along their own rays: nodes push an exact zero to the neighbours they did
+    not take their value from."""
+    m = smooth_model(170, 70, 10.0, seed=7, noise=0.02)
+    rx, rz = receivers(170, 10.0)
+    rx, rz = rx[2:-2] + np.float32(3.7), rz[2:-2] + np.float32(12.3)  # off the nodes: all 16 weights differ from 0
+    shots = [(100.0, 0.0), (1500.0, 20.0), (800.0, 300.0, 20, 140)]
+    e = engine(m, arith=arith)
+    pk = e.batch_forward(shots, rx, rz, keep_tape=True)
+    pg = np.ones_like(pk)
+    pg[0, 4], pg[2, 9:11] = big, -big
+    g = e.batch_adjoint(pg)
+    want, _ = oracle.batch_gradient(oracle.expand_boundary(m), 10.0, 10.0, shots, rx, rz, pg)
+    bad = ~np.isfinite(want)
+    assert 0 < bad.sum() < 0.5 * bad.size
+    assert np.array_equal(g, want, equal_nan=True)

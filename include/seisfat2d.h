@@ -18,6 +18,7 @@
 #ifndef SEISFAT2D_H
 #define SEISFAT2D_H
 
+#include <stddef.h>
 #include <stdint.h>
 
 #ifdef __cplusplus
@@ -178,6 +179,9 @@ int sf_set_wait_limit(sf_ctx* ctx, double seconds);
  * each wait runs into the limit. Nothing else changes; later launches are
  * unaffected. */
 int sf_test_stall_next_batch(sf_ctx* ctx);
+/* Test of the Kirchhoff operators on a full device: an allocation of their
+ * workspace of more than `bytes` fails (0: none does). */
+int sf_test_workspace_limit(sf_ctx* ctx, size_t bytes);
 
 /* FP32 arithmetic of the solves. SF_ARITH_REFERENCE reproduces the
  * reference build of inner_sweep/time_init (modeling.cu:293-357 compiled by
@@ -336,7 +340,13 @@ int sf_update_slowness(sf_ctx* ctx, const float* grad, int grad_mem, float scale
  * traveltime tables (nzz x nxx each, as sf_batch_table writes them); the
  * context's slowness is the model. The reference sums the traces with one
  * launch and one atomicAdd per trace; this is one launch that sums each
- * cell's terms in the same order. Host outputs synchronise `stream`. */
+ * cell's terms in the same order. Host outputs synchronise `stream`.
+ * This and the three operators below hold the terms of their tables, 32 bytes
+ * per table and cell, in a workspace of up to 4 GiB that the context keeps.
+ * They work in blocks that fit: of fewer columns, rows or tables where the
+ * allocation fails, down to one column, one row or two tables (SF_ERR_NOMEM
+ * beyond). Any allocation of the context that fails gives the workspace up
+ * first. */
 int sf_adjoint_convolution(sf_ctx* ctx, const float* traces, float* out, int ntr, int nt, float dt, float fmax,
                            int mem, void* stream);
 int sf_kirchhoff_image(sf_ctx* ctx, const float* Ts, const float* Tr, int nsrc, int nrec, const float* xsrc,

@@ -58,6 +58,7 @@ SIGNATURES = {
     "sf_synchronize": (C.c_int, [VP, VP]),
     "sf_set_wait_limit": (C.c_int, [VP, C.c_double]),
     "sf_test_stall_next_batch": (C.c_int, [VP]),
+    "sf_test_workspace_limit": (C.c_int, [VP, C.c_size_t]),
     "sf_set_launch": (C.c_int, [VP, C.c_int, C.c_int]),
     "sf_set_arithmetic": (C.c_int, [VP, C.c_int]),
     "sf_get_arithmetic": (C.c_int, [VP, IP]),

@@ -58,8 +58,17 @@ int sf_dev_reserve(sf_ctx* c, void** p, size_t* cap, size_t bytes)
     *cap = 0;
     size_t want = std::max<size_t>(bytes, 256);
     cudaError_t e = cudaMalloc(p, want);
+    if (e == cudaErrorMemoryAllocation && c->d_kterm) {
+        // the Kirchhoff operators' workspace, which they can do with less of, makes room
+        cudaGetLastError();
+        cudaFree(c->d_kterm);
+        c->d_kterm = nullptr;
+        c->cap_kterm = 0;
+        e = cudaMalloc(p, want);
+    }
     if (e != cudaSuccess) {
         *p = nullptr;
+        if (e == cudaErrorMemoryAllocation) cudaGetLastError();  // reported here, not by the next launch's check
         return sf_cuda_check(c, e, "cudaMalloc");
     }
     *cap = want;
@@ -309,6 +318,13 @@ extern "C" int sf_test_stall_next_batch(sf_ctx* c)
 {
     if (!c) return SF_ERR_ARG;
     c->stall_next = true;
+    return SF_OK;
+}
+
+extern "C" int sf_test_workspace_limit(sf_ctx* c, size_t bytes)
+{
+    if (!c) return SF_ERR_ARG;
+    c->kterm_limit = bytes;
     return SF_OK;
 }
 

@@ -587,14 +587,35 @@ extern "C" int sf_forward_convolution(sf_ctx* c, const float* traces, float* out
     return wavelet_filter(c, traces, out, ntr, nt, dt, fmax, mem, stream, true);
 }
 
+// Bytes of the terms of `tables` tables at `cells` cells.
+static size_t term_bytes(size_t tables, size_t cells) { return 2 * tables * cells * sizeof(float4); }
+
+// The workspace of the terms; it comes after an operator's other buffers,
+// whose allocation may give it up (sf_dev_reserve).
+static int reserve_terms(sf_ctx* c, size_t bytes)
+{
+    if (c->kterm_limit && bytes > c->kterm_limit) return sf_fail(c, SF_ERR_NOMEM, "workspace limit of a test");
+    return sf_dev_reserve(c, &c->d_kterm, &c->cap_kterm, bytes);
+}
+
+// The largest count of `each` bytes, at most `all`, that kTermBytes and the
+// device's memory allow, reserved: halved until its allocation succeeds.
+static int reserve_blocks(sf_ctx* c, int all, size_t each, int* count)
+{
+    int n = (int)std::min<size_t>(all, std::max<size_t>(kTermBytes / each, 1));
+    int rc;
+    while ((rc = reserve_terms(c, n * each)) == SF_ERR_NOMEM && n > 1) n = (n + 1) / 2;
+    *count = n;
+    return rc;
+}
+
 // Terms of the tables at rows iz0 .. iz0+nr-1 of columns jx0 .. jx0+nc-1 into
-// the context's workspace.
+// the workspace, which is large enough.
 static int table_terms(sf_ctx* c, const float* Ts, const float* Tr, int nsrc, int nrec, int iz0, int nr, int jx0, int nc,
                        TermTable* q, cudaStream_t st)
 {
     const size_t ntab = (size_t)nsrc + nrec, n = (size_t)nr * nc;
     int rc = sf_wait_slowness(c, st);  // (the operators' kernels follow this one)
-    if (!rc) rc = sf_dev_reserve(c, (void**)&c->d_kterm, &c->cap_kterm, 2 * ntab * n * sizeof(float4));
     if (rc) return rc;
     q->a = reinterpret_cast<float4*>(c->d_kterm);
     q->b = reinterpret_cast<float2*>(q->a + ntab * n);
@@ -651,8 +672,9 @@ extern "C" int sf_kirchhoff_image(sf_ctx* c, const float* Ts, const float* Tr, i
     p.aperture = aperture;
     p.max_offset = max_offset;
     // blocks of whole columns whose terms fit the workspace
-    const size_t per_column = 2 * ((size_t)nsrc + nrec) * sizeof(float4) * c->nz;
-    const int cols = (int)std::min<size_t>(c->nx, std::max<size_t>(kTermBytes / per_column, 1));
+    int cols;
+    rc = reserve_blocks(c, c->nx, term_bytes((size_t)nsrc + nrec, c->nz), &cols);
+    if (rc) return rc;
     for (int j0 = 0; j0 < c->nx; j0 += cols) {
         const int nc = std::min(cols, c->nx - j0);
         rc = table_terms(c, Ts, Tr, nsrc, nrec, 0, c->nz, j0, nc, &p.tab, st);
@@ -770,8 +792,9 @@ extern "C" int sf_kirchhoff_angle_gathers(sf_ctx* c, const float* Ts, const floa
     p.rda = (da > 1e-6f && da < 1e6f) ? 1.0f / da : 0.0f;
     p.aperture = aperture;
     // blocks of whole rows whose terms fit the workspace
-    const size_t per_row = 2 * ((size_t)nsrc + nrec) * sizeof(float4) * c->nx;
-    const int rows = (int)std::min<size_t>(c->nz, std::max<size_t>(kTermBytes / per_row, 1));
+    int rows;
+    rc = reserve_blocks(c, c->nz, term_bytes((size_t)nsrc + nrec, c->nx), &rows);
+    if (rc) return rc;
     for (int i0 = 0; i0 < c->nz; i0 += rows) {
         rc = table_terms(c, Ts, Tr, nsrc, nrec, i0, std::min(rows, c->nz - i0), 0, c->nx, &p.tab, st);
         if (rc) return rc;
@@ -807,29 +830,35 @@ static int kirchhoff_forward(sf_ctx* c, bool angle, const float* Ts, const float
     // the tables in groups whose terms fit the workspace (a trace needs its
     // source's and its receiver's): one group unless the grid or the survey is
     // large; each trace is summed in one launch whatever the groups
-    const size_t per_table = 2 * sizeof(float4) * (size_t)c->nx * c->nz;
-    const int fit = (int)std::max<size_t>(2, std::min<size_t>(kTermBytes / per_table, (size_t)nsrc + nrec));
-    const int gs = std::max(1, std::min(nsrc, fit - std::min(nrec, fit / 2))), gr = std::max(1, std::min(nrec, fit - gs));
     struct Group { int s0, ns, r0, nr, first, n; };
     std::vector<Group> groups;
     std::vector<int> ids, bins;
-    for (int s0 = 0; s0 < nsrc; s0 += gs)
-        for (int r0 = 0; r0 < nrec; r0 += gr) {
-            Group g{s0, std::min(gs, nsrc - s0), r0, std::min(gr, nrec - r0), (int)ids.size(), 0};
-            for (int s = s0; s < s0 + g.ns; s++)
-                for (int r = r0; r < r0 + g.nr; r++) {
-                    if (!(fabsf(xsrc[s] - xrec[r]) < max_offset)) continue;
-                    if (angle) {
-                        const float cmp = 0.5f * (xsrc[s] + xrec[r]);
-                        const int b = (int)((cmp - mincmp) / dcmp);
-                        if (b < 0 || b >= ncmp) continue;
-                        bins.push_back(b);
+    auto make_groups = [&](int fit) {  // fit >= 2 tables
+        const int gs = std::max(1, std::min(nsrc, fit - std::min(nrec, fit / 2))), gr = std::max(1, std::min(nrec, fit - gs));
+        groups.clear();
+        ids.clear();
+        bins.clear();
+        for (int s0 = 0; s0 < nsrc; s0 += gs)
+            for (int r0 = 0; r0 < nrec; r0 += gr) {
+                Group g{s0, std::min(gs, nsrc - s0), r0, std::min(gr, nrec - r0), (int)ids.size(), 0};
+                for (int s = s0; s < s0 + g.ns; s++)
+                    for (int r = r0; r < r0 + g.nr; r++) {
+                        if (!(fabsf(xsrc[s] - xrec[r]) < max_offset)) continue;
+                        if (angle) {
+                            const float cmp = 0.5f * (xsrc[s] + xrec[r]);
+                            const int b = (int)((cmp - mincmp) / dcmp);
+                            if (b < 0 || b >= ncmp) continue;
+                            bins.push_back(b);
+                        }
+                        ids.push_back(s * nrec + r);
                     }
-                    ids.push_back(s * nrec + r);
-                }
-            g.n = (int)ids.size() - g.first;
-            if (g.n) groups.push_back(g);
-        }
+                g.n = (int)ids.size() - g.first;
+                if (g.n) groups.push_back(g);
+            }
+    };
+    const size_t per_table = term_bytes(1, (size_t)c->nx * c->nz);
+    int fit = (int)std::max<size_t>(2, std::min<size_t>(kTermBytes / per_table, (size_t)nsrc + nrec));
+    make_groups(fit);
     const int ntrace = (int)ids.size();
     const size_t per_warp = (size_t)nt * sizeof(float) + 32 * sizeof(float);
     const int W = (int)std::min<size_t>(8, kFwdSmem / per_warp);
@@ -840,17 +869,22 @@ static int kirchhoff_forward(sf_ctx* c, bool angle, const float* Ts, const float
         1, std::min<long>((kFwdCtas + std::max(ntrace, 1) - 1) / std::max(ntrace, 1), (ncell + 4095) / 4096));
     const int chunk = (int)((ncell + nchunk - 1) / nchunk);
     const size_t nd = (size_t)nsrc * nrec * nt;
-    c->h_kgeo.assign(xsrc, xsrc + nsrc);
-    c->h_kgeo.insert(c->h_kgeo.end(), xrec, xrec + nrec);
-    c->h_kint.assign(ids.begin(), ids.end());
-    c->h_kint.insert(c->h_kint.end(), bins.begin(), bins.end());
-    int rc = sf_dev_reserve(c, (void**)&c->d_kgeo, &c->cap_kgeo, c->h_kgeo.size() * sizeof(float));
-    if (!rc) rc = sf_dev_reserve(c, (void**)&c->d_kint, &c->cap_kint, std::max<size_t>(1, c->h_kint.size()) * sizeof(int));
+    int rc = sf_dev_reserve(c, (void**)&c->d_kgeo, &c->cap_kgeo, ((size_t)nsrc + nrec) * sizeof(float));
+    if (!rc) rc = sf_dev_reserve(c, (void**)&c->d_kint, &c->cap_kint, std::max<size_t>(1, ids.size() + bins.size()) * sizeof(int));
     if (!rc && (model_mem == SF_MEM_HOST || data_mem == SF_MEM_HOST))
         rc = sf_dev_reserve(c, (void**)&c->d_mig, &c->cap_mig, (nd + nmodel) * sizeof(float));
     if (!rc && nchunk > 1)
         rc = sf_dev_reserve(c, (void**)&c->d_kpart, &c->cap_kpart, (size_t)ntrace * nchunk * nt * sizeof(float));
     if (rc) return rc;
+    while (ntrace > 0 && (rc = reserve_terms(c, fit * per_table)) == SF_ERR_NOMEM && fit > 2) {
+        fit = std::max(2, (fit + 1) / 2);
+        make_groups(fit);
+    }
+    if (rc) return rc;
+    c->h_kgeo.assign(xsrc, xsrc + nsrc);
+    c->h_kgeo.insert(c->h_kgeo.end(), xrec, xrec + nrec);
+    c->h_kint.assign(ids.begin(), ids.end());
+    c->h_kint.insert(c->h_kint.end(), bins.begin(), bins.end());
     CK(cudaMemcpyAsync(c->d_kgeo, c->h_kgeo.data(), c->h_kgeo.size() * sizeof(float), cudaMemcpyHostToDevice, st));
     if (!c->h_kint.empty())
         CK(cudaMemcpyAsync(c->d_kint, c->h_kint.data(), c->h_kint.size() * sizeof(int), cudaMemcpyHostToDevice, st));

@@ -430,6 +430,11 @@ class Engine:
         a handoff tag nothing writes (sf_test_stall_next_batch)."""
         self._check(self.L.sf_test_stall_next_batch(self._ctx), "sf_test_stall_next_batch")
 
+    def test_workspace_limit(self, nbytes):
+        """Test of the Kirchhoff operators on a full device: allocations of
+        their workspace of more than nbytes fail (0: none; sf_test_workspace_limit)."""
+        self._check(self.L.sf_test_workspace_limit(self._ctx, int(nbytes)), "sf_test_workspace_limit")
+
     ARITHMETICS = {"reference": _lib.SF_ARITH_REFERENCE, "ieee": _lib.SF_ARITH_IEEE,
                    "compensated": _lib.SF_ARITH_COMPENSATED}
 

@@ -341,12 +341,12 @@ int sf_update_slowness(sf_ctx* ctx, const float* grad, int grad_mem, float scale
  * context's slowness is the model. The reference sums the traces with one
  * launch and one atomicAdd per trace; this is one launch that sums each
  * cell's terms in the same order. Host outputs synchronise `stream`.
- * This and the three operators below hold the terms of their tables, 32 bytes
- * per table and cell, in a workspace of up to 4 GiB that the context keeps.
- * They work in blocks that fit: of fewer columns, rows or tables where the
- * allocation fails, down to one column, one row or two tables (SF_ERR_NOMEM
- * beyond). Any allocation of the context that fails gives the workspace up
- * first. */
+ * This and the three operators below hold the terms of their tables, 24 bytes
+ * per table and cell (32 in the angle domain), in a workspace of up to 4 GiB
+ * that the context keeps. They work in blocks that fit: of fewer columns, rows
+ * or tables where the allocation fails, down to one column, one row or two
+ * tables (SF_ERR_NOMEM beyond). Any allocation of the context that fails gives
+ * the workspace up first. */
 int sf_adjoint_convolution(sf_ctx* ctx, const float* traces, float* out, int ntr, int nt, float dt, float fmax,
                            int mem, void* stream);
 int sf_kirchhoff_image(sf_ctx* ctx, const float* Ts, const float* Tr, int nsrc, int nrec, const float* xsrc,

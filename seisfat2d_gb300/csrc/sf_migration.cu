@@ -54,13 +54,13 @@ struct CellTerms {
 
 // The terms of a call's tables at a block of model cells (rows iz0 .. iz0+nr-1
 // of columns jx0 .., z fastest) are computed once (k_table_terms), 32 bytes per
-// table and cell: a trace then costs a cell the products of two
-// tables' terms instead of both tables' stencils, roots, divisions and arc
-// cosines.
+// table and cell, 24 without the gradient: a trace then costs a cell the
+// products of two tables' terms instead of both tables' stencils, roots,
+// divisions and arc cosines.
 struct TermTable {
     float4* a;         // T, norm, detH, theta; table t, cell q of the block at t * n + q
     float2* b;         // u, R
-    float2* g;         // dx1, dz1 (the angle operators)
+    float2* g;         // dx1, dz1 (the angle operators only)
     size_t n;          // cells of the block
     int iz0, nr, jx0;
 };
@@ -76,7 +76,9 @@ __device__ __forceinline__ CellTerms load_terms(const TermTable& q, size_t t, si
 
 // Centred first and second differences of one table at padded node (i, j),
 // gradient norm, unit direction (migration.cu:418-450). blockIdx.y strides over
-// the tables (the sources' first), blockIdx.x over the cells.
+// the tables (the sources' first), blockIdx.x over the cells. GRAD: the
+// gradients too (the angle operators).
+template <bool GRAD>
 __global__ void k_table_terms(const float* __restrict__ S, const float* __restrict__ Ts, const float* __restrict__ Tr,
                               int nsrc, int ntab, int nxx, int nzz, int nb, float dx, float dz, TermTable out)
 {
@@ -112,7 +114,7 @@ __global__ void k_table_terms(const float* __restrict__ S, const float* __restri
             const size_t o = (size_t)t * out.n + q;
             out.a[o] = make_float4(c, norm, detH, theta);
             out.b[o] = make_float2(u, R);
-            out.g[o] = make_float2(d_dx, d_dz);
+            if (GRAD) out.g[o] = make_float2(d_dx, d_dz);
         }
     }
 }
@@ -587,8 +589,11 @@ extern "C" int sf_forward_convolution(sf_ctx* c, const float* traces, float* out
     return wavelet_filter(c, traces, out, ntr, nt, dt, fmax, mem, stream, true);
 }
 
-// Bytes of the terms of `tables` tables at `cells` cells.
-static size_t term_bytes(size_t tables, size_t cells) { return 2 * tables * cells * sizeof(float4); }
+// Bytes of the terms of `tables` tables at `cells` cells, with the gradients or without.
+static size_t term_bytes(bool grad, size_t tables, size_t cells)
+{
+    return tables * cells * (sizeof(float4) + (grad ? 2 : 1) * sizeof(float2));
+}
 
 // The workspace of the terms; it comes after an operator's other buffers,
 // whose allocation may give it up (sf_dev_reserve).
@@ -610,8 +615,8 @@ static int reserve_blocks(sf_ctx* c, int all, size_t each, int* count)
 }
 
 // Terms of the tables at rows iz0 .. iz0+nr-1 of columns jx0 .. jx0+nc-1 into
-// the workspace, which is large enough.
-static int table_terms(sf_ctx* c, const float* Ts, const float* Tr, int nsrc, int nrec, int iz0, int nr, int jx0, int nc,
+// the workspace, which is large enough. grad: with the gradients.
+static int table_terms(sf_ctx* c, bool grad, const float* Ts, const float* Tr, int nsrc, int nrec, int iz0, int nr, int jx0, int nc,
                        TermTable* q, cudaStream_t st)
 {
     const size_t ntab = (size_t)nsrc + nrec, n = (size_t)nr * nc;
@@ -619,13 +624,13 @@ static int table_terms(sf_ctx* c, const float* Ts, const float* Tr, int nsrc, in
     if (rc) return rc;
     q->a = reinterpret_cast<float4*>(c->d_kterm);
     q->b = reinterpret_cast<float2*>(q->a + ntab * n);
-    q->g = q->b + ntab * n;
+    q->g = grad ? q->b + ntab * n : nullptr;
     q->n = n;
     q->iz0 = iz0;
     q->nr = nr;
     q->jx0 = jx0;
     const unsigned gx = (unsigned)std::min<size_t>((n + 127) / 128, 65535);
-    k_table_terms<<<dim3(gx, (unsigned)std::min<size_t>(ntab, 65535)), 128, 0, st>>>(
+    (grad ? k_table_terms<true> : k_table_terms<false>)<<<dim3(gx, (unsigned)std::min<size_t>(ntab, 65535)), 128, 0, st>>>(
         c->d_S, Ts, Tr, nsrc, (int)ntab, c->nxx, c->nzz, c->nb, c->dx, c->dz, *q);
     CK(cudaGetLastError());
     return SF_OK;
@@ -673,11 +678,11 @@ extern "C" int sf_kirchhoff_image(sf_ctx* c, const float* Ts, const float* Tr, i
     p.max_offset = max_offset;
     // blocks of whole columns whose terms fit the workspace
     int cols;
-    rc = reserve_blocks(c, c->nx, term_bytes((size_t)nsrc + nrec, c->nz), &cols);
+    rc = reserve_blocks(c, c->nx, term_bytes(false, (size_t)nsrc + nrec, c->nz), &cols);
     if (rc) return rc;
     for (int j0 = 0; j0 < c->nx; j0 += cols) {
         const int nc = std::min(cols, c->nx - j0);
-        rc = table_terms(c, Ts, Tr, nsrc, nrec, 0, c->nz, j0, nc, &p.tab, st);
+        rc = table_terms(c, false, Ts, Tr, nsrc, nrec, 0, c->nz, j0, nc, &p.tab, st);
         if (rc) return rc;
         k_kirchhoff_image<<<(unsigned)std::min<size_t>((p.tab.n + 31) / 32, (size_t)1 << 30), 32 * kImageWarps, 0, st>>>(p);
         CK(cudaGetLastError());
@@ -793,10 +798,10 @@ extern "C" int sf_kirchhoff_angle_gathers(sf_ctx* c, const float* Ts, const floa
     p.aperture = aperture;
     // blocks of whole rows whose terms fit the workspace
     int rows;
-    rc = reserve_blocks(c, c->nz, term_bytes((size_t)nsrc + nrec, c->nx), &rows);
+    rc = reserve_blocks(c, c->nz, term_bytes(true, (size_t)nsrc + nrec, c->nx), &rows);
     if (rc) return rc;
     for (int i0 = 0; i0 < c->nz; i0 += rows) {
-        rc = table_terms(c, Ts, Tr, nsrc, nrec, i0, std::min(rows, c->nz - i0), 0, c->nx, &p.tab, st);
+        rc = table_terms(c, true, Ts, Tr, nsrc, nrec, i0, std::min(rows, c->nz - i0), 0, c->nx, &p.tab, st);
         if (rc) return rc;
         const size_t nthr = (size_t)p.tab.nr * ncmp;
         k_kirchhoff_angles<<<(unsigned)std::min<size_t>((nthr + 127) / 128, (size_t)c->sms * 64), 128, 0, st>>>(p);
@@ -856,7 +861,7 @@ static int kirchhoff_forward(sf_ctx* c, bool angle, const float* Ts, const float
                 if (g.n) groups.push_back(g);
             }
     };
-    const size_t per_table = term_bytes(1, (size_t)c->nx * c->nz);
+    const size_t per_table = term_bytes(angle, 1, (size_t)c->nx * c->nz);
     int fit = (int)std::max<size_t>(2, std::min<size_t>(kTermBytes / per_table, (size_t)nsrc + nrec));
     make_groups(fit);
     const int ntrace = (int)ids.size();
@@ -899,7 +904,7 @@ static int kirchhoff_forward(sf_ctx* c, bool angle, const float* Ts, const float
     for (const Group& g : groups) {
         KirchFwdParams p;
         const size_t matsize = (size_t)c->nxx * c->nzz;
-        rc = table_terms(c, Ts + matsize * g.s0, Tr + matsize * g.r0, g.ns, g.nr, 0, c->nz, 0, c->nx, &p.tab, st);
+        rc = table_terms(c, angle, Ts + matsize * g.s0, Tr + matsize * g.r0, g.ns, g.nr, 0, c->nz, 0, c->nx, &p.tab, st);
         if (rc) return rc;
         p.S = c->d_S;
         p.xs = c->d_kgeo;

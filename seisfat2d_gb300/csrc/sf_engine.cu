@@ -257,8 +257,9 @@ extern "C" int sf_ctx_create(sf_ctx** out, int nx, int nz, float dx, float dz, i
     cap = 0;
     if (st == SF_OK) st = sf_dev_reserve(c, (void**)&c->d_flags, &cap, 256);
     if (st == SF_OK) st = sf_cuda_check(c, cudaMemset(c->d_flags, 0, 256), "cudaMemset");
-    if (st == SF_OK)
-        st = sf_cuda_check(c, cudaEventCreateWithFlags(&c->slowness_ev, cudaEventDisableTiming), "cudaEventCreateWithFlags");
+    for (cudaEvent_t* ev : {&c->slowness_ev, &c->kirch_ev})
+        if (st == SF_OK)
+            st = sf_cuda_check(c, cudaEventCreateWithFlags(ev, cudaEventDisableTiming), "cudaEventCreateWithFlags");
     if (st == SF_OK) st = sf_fwd_setup(c);
     if (st != SF_OK) {
         sf_ctx_destroy(c);
@@ -280,7 +281,8 @@ extern "C" int sf_ctx_destroy(sf_ctx* c)
                     c->d_vfac, c->d_gcij, c->d_fuse, c->d_Tl, c->d_srange, c->d_kterm};
     for (void* b : bufs)
         if (b) cudaFree(b);
-    if (c->slowness_ev) cudaEventDestroy(c->slowness_ev);
+    for (cudaEvent_t ev : {c->slowness_ev, c->kirch_ev})
+        if (ev) cudaEventDestroy(ev);
     delete c;
     return SF_OK;
 }

@@ -144,6 +144,7 @@ struct sf_ctx {
     float* d_kgeo = nullptr; size_t cap_kgeo = 0;
     void* d_kterm = nullptr; size_t cap_kterm = 0;  // terms of the call's traveltime tables
     size_t kterm_limit = 0;  // sf_test_workspace_limit
+    cudaEvent_t kirch_ev = nullptr;  // the end of the last operator, which the next one follows
     int* d_kint = nullptr; size_t cap_kint = 0;
     float* d_kpart = nullptr; size_t cap_kpart = 0;  // forward operator chunk partials
 

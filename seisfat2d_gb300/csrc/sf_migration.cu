@@ -595,34 +595,67 @@ static size_t term_bytes(bool grad, size_t tables, size_t cells)
     return tables * cells * (sizeof(float4) + (grad ? 2 : 1) * sizeof(float2));
 }
 
-// The workspace of the terms; it comes after an operator's other buffers,
-// whose allocation may give it up (sf_dev_reserve).
-static int reserve_terms(sf_ctx* c, size_t bytes)
-{
-    if (c->kterm_limit && bytes > c->kterm_limit) return sf_fail(c, SF_ERR_NOMEM, "workspace limit of a test");
-    return sf_dev_reserve(c, &c->d_kterm, &c->cap_kterm, bytes);
-}
+// One operator's use of the context's buffers on its stream, the workspace of
+// the terms among them: after the operator before it, whatever its stream. A
+// captured operator, whose replays no event of the context could order, has a
+// workspace of its graph's.
+class KirchCall {
+public:
+    KirchCall(sf_ctx* c, cudaStream_t st) : c_(c), st_(st) {}
+    KirchCall(const KirchCall&) = delete;
+    KirchCall& operator=(const KirchCall&) = delete;
+    ~KirchCall()
+    {
+        if (own_) cudaFreeAsync(own_, st_);
+        if (open_ && !capturing_) cudaEventRecord(c_->kirch_ev, st_);
+    }
+    int open()
+    {
+        if (st_ && st_ != cudaStreamLegacy) {
+            cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+            int rc = sf_cuda_check(c_, cudaStreamIsCapturing(st_, &cs), "cudaStreamIsCapturing");
+            if (rc) return rc;
+            capturing_ = cs != cudaStreamCaptureStatusNone;
+        }
+        open_ = true;
+        return capturing_ ? SF_OK : sf_cuda_check(c_, cudaStreamWaitEvent(st_, c_->kirch_ev, 0), "cudaStreamWaitEvent");
+    }
+    // The workspace; it comes after the operator's other buffers, whose
+    // allocation may give it up (sf_dev_reserve).
+    int reserve(size_t bytes)
+    {
+        if (c_->kterm_limit && bytes > c_->kterm_limit) return sf_fail(c_, SF_ERR_NOMEM, "workspace limit of a test");
+        if (capturing_) return sf_cuda_check(c_, cudaMallocAsync(&own_, bytes, st_), "cudaMallocAsync");
+        return sf_dev_reserve(c_, &c_->d_kterm, &c_->cap_kterm, bytes);
+    }
+    // The largest count of `each` bytes, at most `all`, that kTermBytes and the
+    // device's memory allow, reserved: halved until its allocation succeeds.
+    int reserve_blocks(int all, size_t each, int* count)
+    {
+        int n = (int)std::min<size_t>(all, std::max<size_t>(kTermBytes / each, 1));
+        int rc;
+        while ((rc = reserve(n * each)) == SF_ERR_NOMEM && n > 1) n = (n + 1) / 2;
+        *count = n;
+        return rc;
+    }
+    void* workspace() const { return capturing_ ? own_ : c_->d_kterm; }
 
-// The largest count of `each` bytes, at most `all`, that kTermBytes and the
-// device's memory allow, reserved: halved until its allocation succeeds.
-static int reserve_blocks(sf_ctx* c, int all, size_t each, int* count)
-{
-    int n = (int)std::min<size_t>(all, std::max<size_t>(kTermBytes / each, 1));
-    int rc;
-    while ((rc = reserve_terms(c, n * each)) == SF_ERR_NOMEM && n > 1) n = (n + 1) / 2;
-    *count = n;
-    return rc;
-}
+private:
+    sf_ctx* c_;
+    cudaStream_t st_;
+    bool capturing_ = false, open_ = false;
+    void* own_ = nullptr;
+};
 
 // Terms of the tables at rows iz0 .. iz0+nr-1 of columns jx0 .. jx0+nc-1 into
-// the workspace, which is large enough. grad: with the gradients.
-static int table_terms(sf_ctx* c, bool grad, const float* Ts, const float* Tr, int nsrc, int nrec, int iz0, int nr, int jx0, int nc,
-                       TermTable* q, cudaStream_t st)
+// the call's workspace, which is large enough. grad: with the gradients.
+static int table_terms(sf_ctx* c, const KirchCall& call, bool grad, const float* Ts, const float* Tr, int nsrc, int nrec,
+                       int iz0, int nr, int jx0, int nc, TermTable* q, cudaStream_t st)
 {
     const size_t ntab = (size_t)nsrc + nrec, n = (size_t)nr * nc;
     int rc = sf_wait_slowness(c, st);  // (the operators' kernels follow this one)
     if (rc) return rc;
-    q->a = reinterpret_cast<float4*>(c->d_kterm);
+    q->a = reinterpret_cast<float4*>(call.workspace());
     q->b = reinterpret_cast<float2*>(q->a + ntab * n);
     q->g = grad ? q->b + ntab * n : nullptr;
     q->n = n;
@@ -644,8 +677,10 @@ extern "C" int sf_kirchhoff_image(sf_ctx* c, const float* Ts, const float* Tr, i
         return sf_fail(c, SF_ERR_ARG, "bad Kirchhoff arguments");
     CK(cudaSetDevice(c->dev));
     cudaStream_t st = (cudaStream_t)stream;
+    KirchCall call(c, st);
     const size_t nd = (size_t)nsrc * nrec * nt, ni = (size_t)c->nx * c->nz;
-    int rc = sf_dev_reserve(c, (void**)&c->d_kgeo, &c->cap_kgeo, (size_t)(nsrc + nrec) * sizeof(float));
+    int rc = call.open();
+    if (!rc) rc = sf_dev_reserve(c, (void**)&c->d_kgeo, &c->cap_kgeo, (size_t)(nsrc + nrec) * sizeof(float));
     if (!rc && (data_mem == SF_MEM_HOST || image_mem == SF_MEM_HOST))
         rc = sf_dev_reserve(c, (void**)&c->d_mig, &c->cap_mig, (nd + ni) * sizeof(float));
     if (rc) return rc;
@@ -678,11 +713,11 @@ extern "C" int sf_kirchhoff_image(sf_ctx* c, const float* Ts, const float* Tr, i
     p.max_offset = max_offset;
     // blocks of whole columns whose terms fit the workspace
     int cols;
-    rc = reserve_blocks(c, c->nx, term_bytes(false, (size_t)nsrc + nrec, c->nz), &cols);
+    rc = call.reserve_blocks(c->nx, term_bytes(false, (size_t)nsrc + nrec, c->nz), &cols);
     if (rc) return rc;
     for (int j0 = 0; j0 < c->nx; j0 += cols) {
         const int nc = std::min(cols, c->nx - j0);
-        rc = table_terms(c, false, Ts, Tr, nsrc, nrec, 0, c->nz, j0, nc, &p.tab, st);
+        rc = table_terms(c, call, false, Ts, Tr, nsrc, nrec, 0, c->nz, j0, nc, &p.tab, st);
         if (rc) return rc;
         k_kirchhoff_image<<<(unsigned)std::min<size_t>((p.tab.n + 31) / 32, (size_t)1 << 30), 32 * kImageWarps, 0, st>>>(p);
         CK(cudaGetLastError());
@@ -759,7 +794,9 @@ extern "C" int sf_kirchhoff_angle_gathers(sf_ctx* c, const float* Ts, const floa
     c->h_kgeo.insert(c->h_kgeo.end(), xrec, xrec + nrec);
     c->h_kint.assign(cnt.begin(), cnt.end());
     c->h_kint.insert(c->h_kint.end(), ids.begin(), ids.end());
-    int rc = sf_dev_reserve(c, (void**)&c->d_kgeo, &c->cap_kgeo, c->h_kgeo.size() * sizeof(float));
+    KirchCall call(c, st);
+    int rc = call.open();
+    if (!rc) rc = sf_dev_reserve(c, (void**)&c->d_kgeo, &c->cap_kgeo, c->h_kgeo.size() * sizeof(float));
     if (!rc) rc = sf_dev_reserve(c, (void**)&c->d_kint, &c->cap_kint, c->h_kint.size() * sizeof(int));
     if (!rc && (data_mem == SF_MEM_HOST || gathers_mem == SF_MEM_HOST))
         rc = sf_dev_reserve(c, (void**)&c->d_mig, &c->cap_mig, (nd + ng) * sizeof(float));
@@ -798,10 +835,10 @@ extern "C" int sf_kirchhoff_angle_gathers(sf_ctx* c, const float* Ts, const floa
     p.aperture = aperture;
     // blocks of whole rows whose terms fit the workspace
     int rows;
-    rc = reserve_blocks(c, c->nz, term_bytes(true, (size_t)nsrc + nrec, c->nx), &rows);
+    rc = call.reserve_blocks(c->nz, term_bytes(true, (size_t)nsrc + nrec, c->nx), &rows);
     if (rc) return rc;
     for (int i0 = 0; i0 < c->nz; i0 += rows) {
-        rc = table_terms(c, true, Ts, Tr, nsrc, nrec, i0, std::min(rows, c->nz - i0), 0, c->nx, &p.tab, st);
+        rc = table_terms(c, call, true, Ts, Tr, nsrc, nrec, i0, std::min(rows, c->nz - i0), 0, c->nx, &p.tab, st);
         if (rc) return rc;
         const size_t nthr = (size_t)p.tab.nr * ncmp;
         k_kirchhoff_angles<<<(unsigned)std::min<size_t>((nthr + 127) / 128, (size_t)c->sms * 64), 128, 0, st>>>(p);
@@ -874,14 +911,16 @@ static int kirchhoff_forward(sf_ctx* c, bool angle, const float* Ts, const float
         1, std::min<long>((kFwdCtas + std::max(ntrace, 1) - 1) / std::max(ntrace, 1), (ncell + 4095) / 4096));
     const int chunk = (int)((ncell + nchunk - 1) / nchunk);
     const size_t nd = (size_t)nsrc * nrec * nt;
-    int rc = sf_dev_reserve(c, (void**)&c->d_kgeo, &c->cap_kgeo, ((size_t)nsrc + nrec) * sizeof(float));
+    KirchCall call(c, st);
+    int rc = call.open();
+    if (!rc) rc = sf_dev_reserve(c, (void**)&c->d_kgeo, &c->cap_kgeo, ((size_t)nsrc + nrec) * sizeof(float));
     if (!rc) rc = sf_dev_reserve(c, (void**)&c->d_kint, &c->cap_kint, std::max<size_t>(1, ids.size() + bins.size()) * sizeof(int));
     if (!rc && (model_mem == SF_MEM_HOST || data_mem == SF_MEM_HOST))
         rc = sf_dev_reserve(c, (void**)&c->d_mig, &c->cap_mig, (nd + nmodel) * sizeof(float));
     if (!rc && nchunk > 1)
         rc = sf_dev_reserve(c, (void**)&c->d_kpart, &c->cap_kpart, (size_t)ntrace * nchunk * nt * sizeof(float));
     if (rc) return rc;
-    while (ntrace > 0 && (rc = reserve_terms(c, fit * per_table)) == SF_ERR_NOMEM && fit > 2) {
+    while (ntrace > 0 && (rc = call.reserve(fit * per_table)) == SF_ERR_NOMEM && fit > 2) {
         fit = std::max(2, (fit + 1) / 2);
         make_groups(fit);
     }
@@ -904,7 +943,7 @@ static int kirchhoff_forward(sf_ctx* c, bool angle, const float* Ts, const float
     for (const Group& g : groups) {
         KirchFwdParams p;
         const size_t matsize = (size_t)c->nxx * c->nzz;
-        rc = table_terms(c, angle, Ts + matsize * g.s0, Tr + matsize * g.r0, g.ns, g.nr, 0, c->nz, 0, c->nx, &p.tab, st);
+        rc = table_terms(c, call, angle, Ts + matsize * g.s0, Tr + matsize * g.r0, g.ns, g.nr, 0, c->nz, 0, c->nx, &p.tab, st);
         if (rc) return rc;
         p.S = c->d_S;
         p.xs = c->d_kgeo;

@@ -65,3 +65,51 @@ def test_smaller_blocks_where_memory_is_short(inputs, name):
     assert err.value.status == 6  # SF_ERR_NOMEM
     e.test_workspace_limit(0)
     assert np.array_equal(run(name, inputs, e), want)
+
+
+# operators of one context on two streams that do not wait for each other, on
+# other tables and inputs, eagerly and from two captured graphs, and many traces
+# so that they are in flight together
+@pytest.mark.parametrize("captured", [False, True])
+def test_operators_on_two_streams(engine_lib, cuda, captured):
+    from seisfat2d_gb300 import Engine
+    nx, nz, ns, nr, nt = 63, 64, 12, 100, 400
+    e = Engine(nx, nz, 10.0, 10.0)
+    e.set_slowness(np.full((nx, nz), 1 / 2000.0, np.float32))
+    xs, xr = np.linspace(105.0, 500.0, ns).astype(np.float32), np.linspace(15.0, 560.0, nr).astype(np.float32)
+    x, z = (cuda.arange(n, device="cuda") * 10.0 - 30.0 for n in (nx + 6, nz + 6))
+    gen = cuda.Generator().manual_seed(6)
+    jobs = []
+    for k in range(2):
+        tab = [cuda.sqrt((x[None, :, None] - cuda.from_numpy(p).cuda()[:, None, None]) ** 2 + (z + 25.0) ** 2) / (1600.0 + 800 * k)
+               for p in (xs, xr)]
+        data, img = cuda.randn(ns, nr, nt, generator=gen).cuda(), cuda.randn(nx, nz, generator=gen).cuda()
+        jobs.append((*[t.contiguous() for t in tab], data, img, cuda.empty_like(img), cuda.empty_like(data)))
+
+    def call(job, stream=None):
+        Ts, Tr, data, img, image, traces = job
+        e.kirchhoff_image(Ts, Tr, xs, xr, data, 0.004, 40.0, 1e4, out=image, stream=stream)
+        e.kirchhoff_image_forward(Ts, Tr, xs, xr, img, nt, 0.004, 40.0, 1e4, out=traces, stream=stream)
+
+    want = []
+    for job in jobs:
+        call(job)
+        cuda.cuda.synchronize()
+        want.append([job[-2].clone(), job[-1].clone()])
+        assert all(w.abs().max() > 0 for w in want[-1])
+    cuda.cuda.synchronize()
+    streams, graphs = [cuda.cuda.Stream() for _ in jobs], [cuda.cuda.CUDAGraph() for _ in jobs]
+    if captured:
+        for job, st, g in zip(jobs, streams, graphs):
+            with cuda.cuda.graph(g, stream=st):
+                call(job, st)
+    for _ in range(20):
+        for job in jobs:
+            job[-2].zero_(), job[-1].zero_()
+        cuda.cuda.synchronize()
+        for job, st, g in zip(jobs, streams, graphs):
+            with cuda.cuda.stream(st):
+                g.replay() if captured else call(job, st)
+        cuda.cuda.synchronize()
+        for job, w in zip(jobs, want):
+            assert cuda.equal(job[-2], w[0]) and cuda.equal(job[-1], w[1])

@@ -851,9 +851,12 @@ extern "C" int sf_kirchhoff_angle_gathers(sf_ctx* c, const float* Ts, const floa
     return SF_OK;
 }
 
-// Shared memory of one forward CTA: per warp a histogram of nt samples and 32
-// staged (sample, term) pairs.
+// The warps of a forward CTA share kFwdSmem bytes, each a histogram of nt
+// samples and kFwdWarp bytes, of which 32 staged terms take half: the count of
+// warps decides the order of a trace's sums, so it does not follow what a warp
+// happens to stage.
 constexpr size_t kFwdSmem = 200 * 1024;
+constexpr size_t kFwdWarp = 64 * sizeof(float);
 // Work traces times chunks the forward aims at when traces are few; a fixed
 // number, so the summation order depends on the sizes only.
 constexpr long kFwdCtas = 2432;
@@ -902,7 +905,7 @@ static int kirchhoff_forward(sf_ctx* c, bool angle, const float* Ts, const float
     int fit = (int)std::max<size_t>(2, std::min<size_t>(kTermBytes / per_table, (size_t)nsrc + nrec));
     make_groups(fit);
     const int ntrace = (int)ids.size();
-    const size_t per_warp = (size_t)nt * sizeof(float) + 32 * sizeof(float);
+    const size_t per_warp = (size_t)nt * sizeof(float) + kFwdWarp;
     const int W = (int)std::min<size_t>(8, kFwdSmem / per_warp);
     if (W < 1) return sf_fail(c, SF_ERR_RANGE, "too many time samples for the forward operator");
     const int nz = c->nzz - 2 * c->nb;

@@ -281,3 +281,15 @@ def test_infinite_pick_gradients(oracle, engine_lib, cuda, arith, big):
     bad = ~np.isfinite(want)
     assert 0 < bad.sum() < 0.5 * bad.size
     assert np.array_equal(g, want, equal_nan=True)
+
+
+def test_forward_operator_sample_limit(engine_lib, cuda):
+    """The most time samples a forward CTA holds, and one more."""
+    from seisfat2d_gb300 import EngineError
+    e = engine(smooth_model(12, 9, 10.0))
+    T = cuda.full((1, e.nxx, e.nzz), 0.1, device="cuda")
+    args = (T, T, np.array([30.0]), np.array([60.0]), cuda.ones(12, 9, device="cuda"))
+    assert e.kirchhoff_image_forward(*args, 51136, 0.002, 40.0, 1e4).shape == (1, 1, 51136)
+    with pytest.raises(EngineError) as err:
+        e.kirchhoff_image_forward(*args, 51137, 0.002, 40.0, 1e4)
+    assert err.value.status == 4  # SF_ERR_RANGE

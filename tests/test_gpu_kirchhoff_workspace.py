@@ -77,14 +77,14 @@ def test_operators_on_two_streams(engine_lib, cuda, captured):
     e = Engine(nx, nz, 10.0, 10.0)
     e.set_slowness(np.full((nx, nz), 1 / 2000.0, np.float32))
     xs, xr = np.linspace(105.0, 500.0, ns).astype(np.float32), np.linspace(15.0, 560.0, nr).astype(np.float32)
-    x, z = (cuda.arange(n, device="cuda") * 10.0 - 30.0 for n in (nx + 6, nz + 6))
+    x, z = (np.arange(n) * 10.0 - 30.0 for n in (nx + 6, nz + 6))
     gen = cuda.Generator().manual_seed(6)
     jobs = []
     for k in range(2):
-        tab = [cuda.sqrt((x[None, :, None] - cuda.from_numpy(p).cuda()[:, None, None]) ** 2 + (z + 25.0) ** 2) / (1600.0 + 800 * k)
-               for p in (xs, xr)]
+        tab = [cuda.from_numpy((np.hypot(x[None, :, None] - p[:, None, None], z + 25.0) / (1600.0 + 800 * k))
+                               .astype(np.float32)).cuda() for p in (xs, xr)]
         data, img = cuda.randn(ns, nr, nt, generator=gen).cuda(), cuda.randn(nx, nz, generator=gen).cuda()
-        jobs.append((*[t.contiguous() for t in tab], data, img, cuda.empty_like(img), cuda.empty_like(data)))
+        jobs.append((*tab, data, img, cuda.empty_like(img), cuda.empty_like(data)))
 
     def call(job, stream=None):
         Ts, Tr, data, img, image, traces = job

@@ -335,8 +335,9 @@ int sf_update_slowness(sf_ctx* ctx, const float* grad, int grad_mem, float scale
  * sf_kirchhoff_image: the image (nz x nx, z fastest; host or device per
  * image_mem) = sum over sources s and receivers r with |xsrc[s] - xrec[r]| <
  * max_offset, in that order, of the reference's image-domain weight times
- * the correlated trace sample at t = Ts + Tr (data: nsrc x nrec x nt, host or
- * device per data_mem). Ts and Tr are device arrays of nsrc and nrec padded
+ * the correlated trace sample at t = Ts + Tr, nothing where that lies before
+ * or past the trace (the reference reads before it). data: nsrc x nrec x nt,
+ * host or device per data_mem. Ts and Tr are device arrays of nsrc and nrec padded
  * traveltime tables (nzz x nxx each, as sf_batch_table writes them); the
  * context's slowness is the model. The reference sums the traces with one
  * launch and one atomicAdd per trace; this is one launch that sums each

@@ -255,7 +255,7 @@ __global__ void __launch_bounds__(32 * kImageWarps) k_kirchhoff_image(KirchParam
                     if (fabsf((xs - xr)) < p.max_offset) {
                         const CellTerms tr = load_terms<false>(p.tab, (size_t)p.nsrc + r, q);
                         const int tId = sample_of(ts.T + tr.T, p.dt, p.rdt);
-                        if (tId < p.nt)
+                        if ((unsigned)tId < (unsigned)p.nt)
                             v = kirchhoff_term(ts, tr, Sc, taper_exponent(x, 0.5f * (xs + xr), width, rwidth),
                                                p.data[((size_t)s * p.nrec + r) * p.nt + tId]);
                     }
@@ -384,7 +384,7 @@ __global__ void k_kirchhoff_angles(AngleParams p)
                 const float x = __int2float_rd(j - p.nb) * p.dx;
                 const float T = ts.T + tr.T;
                 const int tId = sample_of(T, p.dt, p.rdt);
-                if (tId >= p.nt) continue;
+                if ((unsigned)tId >= (unsigned)p.nt) continue;
                 const float Sc = p.S[(size_t)i + (size_t)j * p.nzz];
                 const float term = kirchhoff_term(ts, tr, Sc, taper_exponent(x, cmp, width, rwidth), trace[tId]);
                 const float reflection_angle = 0.5f * acosf(gradient_cosine(ts, tr));

@@ -293,3 +293,24 @@ def test_forward_operator_sample_limit(engine_lib, cuda):
     with pytest.raises(EngineError) as err:
         e.kirchhoff_image_forward(*args, 51137, 0.002, 40.0, 1e4)
     assert err.value.status == 4  # SF_ERR_RANGE
+
+
+def test_negative_times_add_nothing(oracle, engine_lib, cuda):
+    """Tables with times before the traces' first sample: those cells read no
+    sample, as if the traces were zero there."""
+    m = smooth_model(33, 21, 10.0, seed=4)
+    S = oracle.expand_boundary(m)
+    xs, xr = np.array([30.0, 150.0], np.float32), np.array([20.0, 110.0, 290.0], np.float32)
+    tab = lambda xx: np.stack([oracle.solve_f32(S, 10.0, 10.0, float(x), 0.0) for x in xx])
+    Ts, Tr = tab(xs), cuda.from_numpy(tab(xr)).cuda()
+    d = np.random.default_rng(0).standard_normal((2, 3, 300)).astype(np.float32)
+    e = engine(m)
+    zero = d.copy()
+    zero[0] = 0.0
+    for shift in (1.0, 1e6):
+        early = Ts.copy()
+        early[0] -= np.float32(shift)
+        for op, ang in ((e.kirchhoff_image, ()), (e.kirchhoff_angle_gathers, (60.0, 2.0))):
+            want = op(cuda.from_numpy(Ts).cuda(), Tr, xs, xr, zero, 0.002, 40.0, 1e4, *ang)
+            got = op(cuda.from_numpy(early).cuda(), Tr, xs, xr, d, 0.002, 40.0, 1e4, *ang)
+            assert np.abs(want).max() > 0 and np.array_equal(got, want)

@@ -178,12 +178,14 @@ __device__ __forceinline__ float kirchhoff_term(const CellTerms& s, const CellTe
     return __fmul_rn(kirchhoff_weight<false>(s, r, Sc, texp), v);
 }
 
-// floor(T / dt): the sample of a time.
+// floor(T / dt): the sample of a time (rdt: sample_rate's).
 __device__ __forceinline__ int sample_of(float T, float dt, float rdt)
 {
     const float q = fdiv_k<false>(T, dt, rdt);
-    return __float2int_rd((T > 1e-20f && T < 1e20f) ? q : T / dt);
+    return __float2int_rd((rdt > 0.0f && T > 1e-20f && T < 1e20f) ? q : T / dt);
 }
+// RN(1/dt), or 0 for steps so far out that the quotient needs IEEE division.
+float sample_rate(float dt) { return (dt > 1e-15f && dt < 1e15f) ? 1.0f / dt : 0.0f; }
 
 // RN(RN64(180 a / pi)), the angle in degrees as the reference's double
 // expression rounds it, without the GPU's slow FP64 pipe: x / pi as x times a
@@ -211,7 +213,7 @@ struct KirchParams {
     const float* data;  // nsrc x nrec x nt correlated traces
     float* image;       // nz x nx
     int nsrc, nrec, nt, nzz, nb;
-    float dt, rdt, dx, dz, aperture, max_offset;  // rdt: RN(1/dt)
+    float dt, rdt, dx, dz, aperture, max_offset;  // rdt: sample_rate(dt)
 };
 
 // The image cells of the block (whole columns), 32 per CTA. The image is the
@@ -351,7 +353,7 @@ struct AngleParams {
     const int* cmp_tr;      // trace s * nrec + r, trace order within a bin
     float* gathers;         // nz x nang x ncmp
     int nsrc, nrec, nt, nxx, nzz, nb, nang, ncmp;
-    float dt, rdt, dx, dz, da, rda, aperture;  // rdt: RN(1/dt); rda: angle_bin's
+    float dt, rdt, dx, dz, da, rda, aperture;  // rdt: sample_rate(dt); rda: angle_bin's
 };
 
 // ADKDM's angle_domain_adjoint_kernel (migration.cu:572-663) as a gather: one
@@ -407,7 +409,7 @@ struct KirchFwdParams {
     float* part;         // ntrace x nchunk x nt partial traces (nchunk > 1)
     float* data;         // nsrc x nrec x nt
     int nchunk, chunk, s0, r0, nsrc, nrec, nt, nxx, nzz, nb, nang, warps;
-    float dt, rdt, dx, dz, da, rda, aperture;  // rdt: RN(1/dt); rda: angle_bin's
+    float dt, rdt, dx, dz, da, rda, aperture;  // rdt: sample_rate(dt); rda: angle_bin's
 };
 
 // The forward (demigration) operator of the least-squares variants:
@@ -706,7 +708,7 @@ extern "C" int sf_kirchhoff_image(sf_ctx* c, const float* Ts, const float* Tr, i
     p.nzz = c->nzz;
     p.nb = c->nb;
     p.dt = dt;
-    p.rdt = 1.0f / dt;
+    p.rdt = sample_rate(dt);
     p.dx = c->dx;
     p.dz = c->dz;
     p.aperture = aperture;
@@ -827,7 +829,7 @@ extern "C" int sf_kirchhoff_angle_gathers(sf_ctx* c, const float* Ts, const floa
     p.nang = nang;
     p.ncmp = ncmp;
     p.dt = dt;
-    p.rdt = 1.0f / dt;
+    p.rdt = sample_rate(dt);
     p.dx = c->dx;
     p.dz = c->dz;
     p.da = da;
@@ -969,7 +971,7 @@ static int kirchhoff_forward(sf_ctx* c, bool angle, const float* Ts, const float
         p.nang = nang;
         p.warps = W;
         p.dt = dt;
-        p.rdt = 1.0f / dt;
+        p.rdt = sample_rate(dt);
         p.dx = c->dx;
         p.dz = c->dz;
         p.da = da;

@@ -314,3 +314,17 @@ def test_negative_times_add_nothing(oracle, engine_lib, cuda):
             want = op(cuda.from_numpy(Ts).cuda(), Tr, xs, xr, zero, 0.002, 40.0, 1e4, *ang)
             got = op(cuda.from_numpy(early).cuda(), Tr, xs, xr, d, 0.002, 40.0, 1e4, *ang)
             assert np.abs(want).max() > 0 and np.array_equal(got, want)
+
+
+@pytest.mark.parametrize("dt", [1e-37, 1e-30, 1e30])
+def test_extreme_sample_steps(engine_lib, cuda, dt):
+    """Steps at which a time's sample lies past FP32's range, past the trace
+    or is the first one."""
+    e = engine(smooth_model(20, 15, 10.0))
+    T = (500.0 + 1e-3 * cuda.arange(e.nzz, dtype=cuda.float32)).expand(1, e.nxx, -1).contiguous().cuda()
+    d, x = cuda.ones(1, 1, 8).cuda(), np.array([100.0])
+    img = e.kirchhoff_image(T, T, x, x, d, dt, 40.0, 1e4)
+    tr = e.kirchhoff_image_forward(T, T, x, x, np.ones((20, 15), np.float32), 8, dt, 40.0, 1e4)
+    assert np.isfinite(img).all() and np.isfinite(tr).all()
+    assert np.abs(img).max() > 0 if dt > 1 else not img.any()
+    assert np.abs(tr[0, 0, 0]) > 0 if dt > 1 else not tr.any()

@@ -80,7 +80,7 @@ __device__ __forceinline__ CellTerms load_terms(const TermTable& q, size_t t, si
 // gradients too (the angle operators).
 template <bool GRAD>
 __global__ void k_table_terms(const float* __restrict__ S, const float* __restrict__ Ts, const float* __restrict__ Tr,
-                              int nsrc, int ntab, int nxx, int nzz, int nb, float dx, float dz, TermTable out)
+                              int nsrc, int ntab, int nxx, int nzz, int nb, float dx, float dz, bool fast, TermTable out)
 {
     const size_t matsize = (size_t)nzz * nxx;
     for (int t = blockIdx.y; t < ntab; t += gridDim.y) {
@@ -106,9 +106,9 @@ __global__ void k_table_terms(const float* __restrict__ S, const float* __restri
             float R = max(c / Sc, kEps);
             const float detH = fabsf(det) + kEps;
             // every factor well inside FP32's range (their minima are EPS): the
-            // weight's roots and quotients may take the fast form. A negative R
-            // marks a cell where they may not.
-            const bool regular = norm < 1e6f && detH < 1e10f && R < 1e10f && fabsf(u) > 1e-12f && fabsf(u) < 2.0f &&
+            // weight's roots and quotients may take the fast form (fast: it was
+            // found exact, fast_form). A negative R marks a cell where they may not.
+            const bool regular = fast && norm < 1e6f && detH < 1e10f && R < 1e10f && fabsf(u) > 1e-12f && fabsf(u) < 2.0f &&
                                  fabsf(c) < 1e10f && Sc > 1e-9f && Sc < 1e9f;
             if (!regular) R = -R;
             const size_t o = (size_t)t * out.n + q;
@@ -165,17 +165,20 @@ __device__ __forceinline__ float kirchhoff_weight(const CellTerms& s, const Cell
     return scale_const * Jterm * obliquity * G * R * taper;
 }
 
-// weight * v, the term that a trace adds at a cell.
-__device__ __forceinline__ float kirchhoff_term(const CellTerms& s, const CellTerms& r, float Sc, float texp, float v)
+// weight * v, the term that a trace adds at a cell x of aperture width `width`
+// (rwidth: its reciprocal, at a regular cell by the fast form).
+__device__ __forceinline__ float kirchhoff_term(const CellTerms& s, const CellTerms& r, float Sc, float x, float cmp,
+                                                float width, float rwidth, float v)
 {
     if (fminf(s.R, r.R) > 0.0f) {
         // expf underflows to 0 below this exponent (half the smallest subnormal is
         // exp(-103.98)): outside the trace's aperture, most of a shallow row, a
         // finite sample's term is 0
+        const float texp = taper_exponent(x, cmp, width, rwidth);
         if (texp < -106.0f && fabsf(v) < 1e30f) return 0.0f;
         return __fmul_rn(kirchhoff_weight<true>(s, r, Sc, texp), v);
     }
-    return __fmul_rn(kirchhoff_weight<false>(s, r, Sc, texp), v);
+    return __fmul_rn(kirchhoff_weight<false>(s, r, Sc, taper_exponent(x, cmp, width, __frcp_rn(width))), v);
 }
 
 // floor(T / dt): the sample of a time (rdt: sample_rate's).
@@ -258,7 +261,7 @@ __global__ void __launch_bounds__(32 * kImageWarps) k_kirchhoff_image(KirchParam
                         const CellTerms tr = load_terms<false>(p.tab, (size_t)p.nsrc + r, q);
                         const int tId = sample_of(ts.T + tr.T, p.dt, p.rdt);
                         if ((unsigned)tId < (unsigned)p.nt)
-                            v = kirchhoff_term(ts, tr, Sc, taper_exponent(x, 0.5f * (xs + xr), width, rwidth),
+                            v = kirchhoff_term(ts, tr, Sc, x, 0.5f * (xs + xr), width, rwidth,
                                                p.data[((size_t)s * p.nrec + r) * p.nt + tId]);
                     }
                     term[buf][k][lane] = v;
@@ -388,7 +391,7 @@ __global__ void k_kirchhoff_angles(AngleParams p)
                 const int tId = sample_of(T, p.dt, p.rdt);
                 if ((unsigned)tId >= (unsigned)p.nt) continue;
                 const float Sc = p.S[(size_t)i + (size_t)j * p.nzz];
-                const float term = kirchhoff_term(ts, tr, Sc, taper_exponent(x, cmp, width, rwidth), trace[tId]);
+                const float term = kirchhoff_term(ts, tr, Sc, x, cmp, width, rwidth, trace[tId]);
                 const float reflection_angle = 0.5f * acosf(gradient_cosine(ts, tr));
                 const int aId = angle_bin(degrees_of(reflection_angle), p.da, p.rda);
                 if (aId >= 0 && aId < p.nang) acc[aId] = add_ftz(acc[aId], term);
@@ -458,7 +461,6 @@ __global__ void k_kirchhoff_forward(KirchFwdParams p)
                 const float x = __int2float_rd(jx) * p.dx;
                 const float Sc = p.S[(size_t)(iz + p.nb) + (size_t)(jx + p.nb) * p.nzz];
                 const float width = __fadd_rn(__fmul_rn(tan_ap, z), kEps);
-                const float texp = taper_exponent(x, cmp, width, frcp_k(width));
                 size_t mId = (size_t)m;
                 bool in = true;
                 if (ANGLE) {
@@ -468,7 +470,7 @@ __global__ void k_kirchhoff_forward(KirchFwdParams p)
                     mId = (size_t)iz + (size_t)aId * nz + (size_t)cmpId * p.nang * nz;
                 }
                 if (in) {
-                    v = kirchhoff_term(ts, tr, Sc, texp, p.model[mId]);
+                    v = kirchhoff_term(ts, tr, Sc, x, cmp, width, frcp_k(width), p.model[mId]);
                     if (v != 0.0f) tq = tId;  // (NaN is kept)
                 }
             }
@@ -591,6 +593,10 @@ extern "C" int sf_forward_convolution(sf_ctx* c, const float* traces, float* out
     return wavelet_filter(c, traces, out, ntr, nt, dt, fmax, mem, stream, true);
 }
 
+// Whether the roots and reciprocals made from the hardware's approximations
+// are IEEE's on this device (checked at the context's creation).
+static bool fast_form(const sf_ctx* c) { return (c->kc.mflags & 0x30) == 0x30; }
+
 // Bytes of the terms of `tables` tables at `cells` cells, with the gradients or without.
 static size_t term_bytes(bool grad, size_t tables, size_t cells)
 {
@@ -666,7 +672,7 @@ static int table_terms(sf_ctx* c, const KirchCall& call, bool grad, const float*
     q->jx0 = jx0;
     const unsigned gx = (unsigned)std::min<size_t>((n + 127) / 128, 65535);
     (grad ? k_table_terms<true> : k_table_terms<false>)<<<dim3(gx, (unsigned)std::min<size_t>(ntab, 65535)), 128, 0, st>>>(
-        c->d_S, Ts, Tr, nsrc, (int)ntab, c->nxx, c->nzz, c->nb, c->dx, c->dz, *q);
+        c->d_S, Ts, Tr, nsrc, (int)ntab, c->nxx, c->nzz, c->nb, c->dx, c->dz, fast_form(c), *q);
     CK(cudaGetLastError());
     return SF_OK;
 }

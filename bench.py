@@ -47,7 +47,8 @@ def parse():
     ap.add_argument("--cpu-seconds", type=float, default=15.0)
     ap.add_argument("--warps", type=int, default=0, help="warps per CTA (0: engine default)")
     ap.add_argument("--gang", type=int, default=0, help="warps per shot (0: automatic)")
-    ap.add_argument("--no-fused-gather", action="store_true", help="gather in its own launch")
+    ap.add_argument("--fused-gather", action="store_true", help="gather inside the reverse-sweep launch where it fits")
+    ap.add_argument("--no-fused-gather", action="store_true", help="gather in its own launch (the default)")
     ap.add_argument("--strip-loop", default="auto", choices=["auto", "general", "interior"],
                     help="strip-loop form (fixing it, or --warps/--gang, skips the autotuner)")
     ap.add_argument("--arith", default="compensated", choices=["reference", "ieee", "compensated"],
@@ -394,7 +395,7 @@ def measure(cfg, a, env, arith, full, steps, warmup):
     if a.warps or a.gang:
         eng.set_launch(a.warps, a.gang)
     eng.set_strip_loop(a.strip_loop)
-    eng.set_fused_gather(not a.no_fused_gather)
+    eng.set_fused_gather(a.fused_gather and not a.no_fused_gather)
     if ani:
         eng.set_stiffness(w.cij)
     eng.set_slowness(w.slowness)
@@ -582,7 +583,7 @@ def measure(cfg, a, env, arith, full, steps, warmup):
         # reverse sweeps and gather in one launch (sf_set_fused_gather)
         stages["adjoint"] = {"kernel": "sf::k_adjoint_gather (reverse sweeps + gather)", "ms": kt["adjoint"],
                              "algorithmic_bytes": BYTES_PER_CELL_ADJ * cells,
-                             "traffic_file": f"k_adjoint_gather_cfg{cfg}.txt"}
+                             "traffic_file": None}
     if fa:
         stages["residual"] = {"kernel": "sf::k_residual", "ms": kt["residual"],
                               "algorithmic_bytes": 3 * 4 * len(shots) * nrec, "traffic_file": None}

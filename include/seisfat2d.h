@@ -243,10 +243,10 @@ int sf_set_strip_loop(sf_ctx* ctx, int mode);
 int sf_get_strip_loop(const sf_ctx* ctx, int* mode, int* last_interior);
 
 /* Gradient gather inside the reverse-sweep launch (no counterpart in the
- * reference). Asked for with 2 or 4 warps per CTA and an isotropic batch, and
- * when the device holds every reverse-sweep CTA plus two gather CTAs per SM
- * (or one per tile) at once, one launch runs both. Never asked (reported as
- * enable = 1), the gather runs in its own launch, which measured faster.
+ * reference; default off). Asked for with 2 or 4 warps per CTA and an isotropic
+ * batch, and when the device holds every reverse-sweep CTA plus two gather CTAs
+ * per SM (or one per tile) at once, one launch runs both; the gather's own
+ * launch measured faster.
  * In one launch, each gather tile starts as soon as every shot's
  * last reverse sweep has finished its columns in the tile's strip and the
  * next, instead of after the whole reverse pass. Same bits either way.

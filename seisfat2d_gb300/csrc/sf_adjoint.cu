@@ -276,7 +276,7 @@ int sf_adj_configure(sf_ctx* c, cudaStream_t st, AdjLaunch* A)
     // gather CTAs per SM at once (600 windows that left room for 8 gather CTAs
     // took 834 ms in one launch, 26 ms in two).
     A->fused = false;
-    if (c->fuse_gather > 0 && !c->batch_ani && (c->warps == 2 || c->warps == 4)) {
+    if (c->fuse_gather && !c->batch_ani && (c->warps == 2 || c->warps == 4)) {
         const bool in = c->batch_interior;
         const void* fk = (c->warps == 2) ? (in ? (const void*)k_adjoint_gather<true, 2> : (const void*)k_adjoint_gather<false, 2>)
                                          : (in ? (const void*)k_adjoint_gather<true, 4> : (const void*)k_adjoint_gather<false, 4>);
@@ -456,7 +456,7 @@ extern "C" int sf_batch_stiffness_gradient(sf_ctx* c, float* grad_c11, float* gr
 extern "C" int sf_set_fused_gather(sf_ctx* c, int enable)
 {
     if (!c) return SF_ERR_ARG;
-    c->fuse_gather = enable != 0 ? 1 : 0;
+    c->fuse_gather = enable != 0;
     c->plan_dirty = true;
     return SF_OK;
 }

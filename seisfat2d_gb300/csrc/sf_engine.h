@@ -58,7 +58,7 @@ struct sf_ctx {
     int warps = 1;        // warps per CTA
     int gang_warps = 0;   // warps solving one shot (0: chosen per batch)
     int strip_loop = -1;  // strip loops: SF_LOOP_* (sf_set_strip_loop)
-    int fuse_gather = -1;  // gather inside the reverse-sweep launch when it fits (sf_set_fused_gather): 1 yes, 0 no, -1 the default, no
+    bool fuse_gather = false;  // gather inside the reverse-sweep launch when it fits (sf_set_fused_gather)
     bool last_fused = false;  // the last adjoint ran fused
     unsigned* d_fuse = nullptr; size_t cap_fuse = 0;
     bool batch_interior = false;  // the last batch's forward ran the interior-block body

@@ -328,3 +328,17 @@ def test_extreme_sample_steps(engine_lib, cuda, dt):
     assert np.isfinite(img).all() and np.isfinite(tr).all()
     assert np.abs(img).max() > 0 if dt > 1 else not img.any()
     assert np.abs(tr[0, 0, 0]) > 0 if dt > 1 else not tr.any()
+
+
+def test_fused_gather_default(engine_lib, cuda):
+    """An untouched context reports what it does, and setting what it reports
+    changes nothing."""
+    m = smooth_model(150, 60, 10.0, seed=5)
+    rx, rz = receivers(150, 10.0)
+    e = engine(m)
+    e.set_launch(warps=4)
+    for _ in range(2):
+        pk = e.batch_forward([(300.0, 0.0)], rx, rz, keep_tape=True)
+        e.misfit_gradient(pk + np.float32(0.01))
+        assert e.fused_gather() == (False, False)
+        e.set_fused_gather(e.fused_gather()[0])

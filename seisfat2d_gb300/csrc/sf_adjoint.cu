@@ -254,6 +254,7 @@ int sf_adj_configure(sf_ctx* c, cudaStream_t st, AdjLaunch* A)
         if (rc) return rc;
         g.vfac = c->d_vfac;
         g.vfac_total = c->batch_q_cells;
+        g.undef = c->d_srange + c->hshots.size();
         g.grad_c11 = c->d_gcij;
         g.grad_c13 = c->d_gcij + npad;
     }

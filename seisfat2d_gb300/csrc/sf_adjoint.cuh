@@ -465,7 +465,9 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1) k_adjoint(AdjParams p)
 // the tile's columns come from a per-column-block list built on the host,
 // staged in shared memory kGChunk at a time. Runs without a nonzero term (the
 // rays of a shot pass through a part of its window only) are left out: the
-// reverse sweeps mark every 1024 tape entries that hold one (vflag).
+// reverse sweeps mark every 1024 tape entries that hold one (vflag). A shot
+// without a term is then not summed at all, unless a factor of its zero is not
+// finite (undef).
 constexpr int kGSteps = kGT + 32;   // tape steps a tile's strip spans per sweep
 constexpr int kGStages = 3;
 constexpr int kGChunk = 128;
@@ -589,8 +591,11 @@ __device__ bool gather_tile(const GatherParams& p, GatherSmem& sm, int k, int cb
         for (size_t q = lo >> 10; q <= hi >> 10; q++) any |= __ldcg(p.vflag + q);
         return any != 0;
     };
+    // the sum of a shot that may be left out: 0, or none (NaN) as zero times a
+    // factor that is not finite is NaN
+    const float skip = VTI && *p.undef != 0 ? __int_as_float(0x7fc00000) : 0.0f;
     auto wanted = [&](const GatherShot& t, int sw) {
-        if (sw == 3 && has_source(t)) return true;
+        if (sw == 3 && ((VTI && skip != skip) || has_source(t))) return true;
         int fmlo, fmhi;
         fm_range(t, sw, fmlo, fmhi);
         const size_t base = tape_strip_base(t.tape_off, sw, k, p.nstrips, t.ncols);
@@ -653,7 +658,7 @@ __device__ bool gather_tile(const GatherParams& p, GatherSmem& sm, int k, int cb
                     g[q] = fadd(g[q], fmul(FUSED ? __ldcg(li) : *li, __double2float_rn(d)));
                 }
             }
-            if (g[q] != 0.0f && a < p.nzz && bc < p.nxx && bl >= 0 && bl < t.ncols) {
+            if (g[q] != (VTI ? skip : 0.0f) && a < p.nzz && bc < p.nxx && bl >= 0 && bl < t.ncols) {
                 if (VTI) {
                     const float* f = p.vfac + t.q_off + (size_t)a + (size_t)bl * strip_pitch(p.nzz);
                     total[q] += (double)g[q] * (double)f[0];

@@ -65,6 +65,7 @@ struct GatherParams {
     // slowness, times the shot's dSq/dS, dSq/dC11, dSq/dC13 (3 x vfac_total)
     const float* vfac;
     long long vfac_total;
+    const int* undef;        // not 0: a factor is not finite, and no shot's zero sum may be left out
     float* grad_c11;         // nzz x nxx
     float* grad_c13;         // nzz x nxx
     // gather inside the reverse-sweep launch: a shot's initialisation term is

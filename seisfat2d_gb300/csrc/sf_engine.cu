@@ -912,7 +912,8 @@ int sf_qp_launch(sf_ctx* c, bool fact, cudaStream_t st)
     std::memcpy(q.mm, c->mm, sizeof(q.mm));
     q.Sq = c->d_Sq;
     q.srange = c->d_srange;
-    CK(cudaMemsetAsync(c->d_srange, 0, c->hshots.size() * sizeof(int), st));
+    q.undef = c->d_srange + c->hshots.size();
+    CK(cudaMemsetAsync(c->d_srange, 0, (c->hshots.size() + 1) * sizeof(int), st));
     q.vfac = fact ? c->d_vfac : nullptr;
     q.vfac_total = c->batch_q_cells;
     const bool comp = c->arith == SF_ARITH_COMPENSATED, ref = c->arith == SF_ARITH_REFERENCE;
@@ -946,7 +947,7 @@ int sf_launch_shots(sf_ctx* c, int ani, int nrec, float* d_picks, bool keep_tabl
         // eikonal_ani.cu:33-45: solve on S, qP pass, solve on the qP slowness;
         // every shot keeps its window between the launches
         rc = sf_dev_reserve(c, (void**)&c->d_Sq, &c->cap_Sq, (size_t)c->batch_q_cells * sizeof(float));
-        if (!rc) rc = sf_dev_reserve(c, (void**)&c->d_srange, &c->cap_srange, c->hshots.size() * sizeof(int));
+        if (!rc) rc = sf_dev_reserve(c, (void**)&c->d_srange, &c->cap_srange, (c->hshots.size() + 1) * sizeof(int));
         if (!rc && tape)
             rc = sf_dev_reserve(c, (void**)&c->d_vfac, &c->cap_vfac, 3 * (size_t)c->batch_q_cells * sizeof(float));
         FwdLaunch L1, L2;

@@ -151,7 +151,7 @@ struct sf_ctx {
     // anisotropic adjoint: per-shot dSq/d{S, C11, C13} factors and the
     // stiffness gradients of the last adjoint (sf_batch_stiffness_gradient)
     float* d_vfac = nullptr; size_t cap_vfac = 0;
-    int* d_srange = nullptr; size_t cap_srange = 0;  // per shot: qP slowness outside in_fast_range
+    int* d_srange = nullptr; size_t cap_srange = 0;  // per shot: qP slowness outside in_fast_range; then: a factor is not finite
     float* d_gcij = nullptr; size_t cap_gcij = 0;
     bool gcij_valid = false;
     std::vector<int> h_kint;

@@ -266,6 +266,7 @@ struct QpParams {
     float mm[12];
     float* Sq;            // per-shot qP slowness windows at q_off
     int* srange;          // per shot: set when its qP slowness has a value outside in_fast_range
+    int* undef;           // FACT: set when a derivative factor is not finite
     float* vfac;          // FACT: dSq/dS, dSq/dC11, dSq/dC13 per window cell (3 x vfac_total)
     long long vfac_total;
 };
@@ -336,6 +337,7 @@ __global__ void __launch_bounds__(128) k_qp(QpParams p)
                         f[0] = fS;
                         f[p.vfac_total] = f11;
                         f[2 * p.vfac_total] = f13;
+                        if (!(fabsf(fS) + fabsf(f11) + fabsf(f13) < INFINITY)) *p.undef = 1;
                     }
                 }
             }

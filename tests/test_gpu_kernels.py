@@ -342,3 +342,34 @@ def test_fused_gather_default(engine_lib, cuda):
         e.misfit_gradient(pk + np.float32(0.01))
         assert e.fused_gather() == (False, False)
         e.set_fused_gather(e.fused_gather()[0])
+
+
+def test_undefined_stiffness_factors(oracle, engine_lib, cuda, arith):
+    """Cells without a real qP slowness (C33 below zero) have no derivative:
+    their gradients are NaN whether or not a ray passes through them."""
+    from seisfat2d_gb300.synthetic import thomsen_stiffness
+    m = smooth_model(120, 50, 10.0, seed=9)
+    rng = np.random.default_rng(9)
+    vp = 1.0 / m.astype(np.float64)
+    codes, mm = [], []
+    for k, c in enumerate(thomsen_stiffness(vp, vp / np.sqrt(3.0), 1000.0, rng.uniform(0.0, 0.25, m.shape),
+                                            rng.uniform(-0.05, 0.15, m.shape))):
+        if k == 3:
+            c = c.copy()
+            c[5, 45], c[60, 30] = -c[5, 45], -c[60, 30]
+        cd, mn, mx = oracle.compress(oracle.expand_boundary(c.astype(np.float32)))
+        codes.append(cd)
+        mm += [mn, mx]
+    cij = codes, np.array(mm, np.float32)
+    e = engine(m, arith=arith)
+    e.set_stiffness_codes(*cij)
+    rx, rz = receivers(120, 10.0)
+    shots = [(300.0, 0.0), (900.0, 20.0, 30, 90)]
+    pk = e.batch_forward(shots, rx, rz, ani=True, keep_tape=True)
+    tobs = np.zeros_like(pk)
+    J, g = e.misfit_gradient(tobs)
+    o = oracle.batch_misfit_gradient(oracle.expand_boundary(m), 10.0, 10.0, shots, rx, rz, tobs, ani=cij)
+    assert np.array_equal(pk, o[2], equal_nan=True)
+    for got, want in zip((g, *e.stiffness_gradient()), (o[1], o[4], o[5])):
+        assert np.isnan(want).sum() == 2 and np.nanmax(np.abs(want)) > 0
+        assert np.array_equal(got, want, equal_nan=True)

@@ -373,3 +373,43 @@ def test_undefined_stiffness_factors(oracle, engine_lib, cuda, arith):
     for got, want in zip((g, *e.stiffness_gradient()), (o[1], o[4], o[5])):
         assert np.isnan(want).sum() == 2 and np.nanmax(np.abs(want)) > 0
         assert np.array_equal(got, want, equal_nan=True)
+
+
+# cell sizes outside the fast updates' range: too large, too small, too oblong
+@pytest.mark.parametrize("dx,dz", [(2000.0, 2000.0), (0.01, 0.0125), (200.0, 10.0)])
+def test_cells_outside_fast_range(oracle, engine_lib, cuda, arith, dx, dz):
+    m = smooth_model(140, 40, 10.0, seed=8, noise=0.02)
+    shots = [(30 * dx, 0.0), (110 * dx, 2 * dz, 30, 116)]
+    check_gradient(oracle, engine(m, dx, dz, arith), m, dx, dz, shots)
+
+
+def test_windows_of_unequal_size_at_once(oracle, engine_lib, cuda, arith):
+    """More shots than SMs / 2, every one with a gang of its own: no queue, but
+    gangs whose sweeps drift apart share one body for both directions."""
+    nx, nz = 200, 60
+    m = smooth_model(nx, nz, 10.0, seed=5)
+    e = engine(m, arith=arith)
+    rng = np.random.default_rng(1)
+    shots = []
+    for _ in range(100):
+        n = int(rng.integers(128, nx + 7))
+        c0 = int(rng.integers(0, nx + 7 - n))
+        shots.append((float(10 * rng.integers(c0 + 2, c0 + n - 10)), float(rng.integers(0, 300)), c0, n))
+    check_gradient(oracle, e, m, 10.0, 10.0, shots)
+    assert e.strip_loop()[1]
+
+
+@pytest.mark.parametrize("dx,scale", [(10.0, 1.0), (10.0, 1e-6), (2000.0, 1.0)])
+def test_allocation_free_solve_outside_fast_range(oracle, engine_lib, cuda, dx, scale):
+    """The allocation-free solve's own checks of slowness and cell sizes."""
+    import ctypes as C
+    m = smooth_model(140, 70, 10.0, seed=8, noise=0.02)
+    m[70, 20] *= np.float32(scale)
+    e = engine(m, dx, dx, "reference")
+    want = e.time_propagation(30 * dx, 0.0)
+    S = cuda.from_numpy(oracle.expand_boundary(m)).cuda()
+    T = cuda.empty_like(S)
+    for _ in range(2):
+        st = e.L.sf_time_propagation_noalloc(C.c_void_p(S.data_ptr()), 140, 70, dx, dx, 30 * dx, 0.0,
+                                             C.c_void_p(T.data_ptr()), None)
+        assert st == 0 and np.array_equal(T.cpu().numpy(), want)

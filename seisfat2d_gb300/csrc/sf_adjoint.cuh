@@ -337,8 +337,6 @@ __device__ __forceinline__ void adj_strip(const AdjStripArgs& a)
     __syncwarp();
 }
 
-// (kMaxWarps * 32, 1): the block size alone as the bound caps the kernel at
-// 64 registers and spills the strip loop's state.
 // The reverse sweeps of every shot (persistent gangs, as the forward). f:
 // inside a fused launch, count finished column blocks in the last reverse
 // sweep and flag each shot's initialisation term.
@@ -445,6 +443,8 @@ __device__ void adjoint_body(const AdjParams& p, const FuseParams* f)
     }
 }
 
+// (kMaxWarps * 32, 1): the block size alone as the bound caps the kernel at
+// 64 registers and spills the strip loop's state.
 template <bool INTERIOR>
 __global__ void __launch_bounds__(kMaxWarps * 32, 1) k_adjoint(AdjParams p)
 {

@@ -8,9 +8,10 @@
 // once per source-receiver trace over the whole grid and adds each trace's
 // term with atomicAdd; a cell is touched by one thread per launch, so the
 // image is the FP32 sum of the traces' terms in trace order (source outer,
-// receiver inner). Here one thread owns an image cell and walks every trace
-// in that order: the same sum, one launch, no atomics, and the source-table
-// derivatives computed once per source instead of once per trace.
+// receiver inner). Here what a term takes from one table is computed once per
+// table and cell (k_table_terms), and a CTA owns 32 image cells: its warps form
+// the traces' terms side by side and one of them adds them in that order
+// (k_kirchhoff_image): the same sum, without atomics.
 #include <cuda_runtime.h>
 
 #include <algorithm>

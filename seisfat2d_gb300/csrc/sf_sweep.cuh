@@ -87,9 +87,8 @@ constexpr int kMaxWarps = 16;
 // compensated kernels keep a second traveltime ring (the lo parts): at most
 // 8 warps per CTA fit in shared memory
 constexpr int kMaxWarpsComp = 8;
-// the taped interior-block forward kernels bound their CTAs to 8 warps, which
-// lets them keep more of the block's state in registers (measured 2.6%
-// faster on the headline batch; the other kernels measured slower that way)
+// the taped interior-block forward kernels have up to 168 registers a thread
+// (k_shots), of which an SM holds three warps per scheduler: CTAs of 8 warps
 constexpr int kMaxWarpsTapedInterior = 8;
 constexpr long long kSpinLimit = 1ll << 30;          // iterations
 constexpr unsigned kPollNs = 100;                    // pause between two polls of a wait
@@ -176,7 +175,6 @@ __device__ __forceinline__ unsigned long long pack_tag(float v, unsigned tag)
 __device__ __forceinline__ unsigned tag_of(unsigned long long e) { return (unsigned)(e >> 32); }
 __device__ __forceinline__ float val_of(unsigned long long e) { return __uint_as_float((unsigned)e); }
 
-// Everything one warp needs for one strip of one sweep.
 // The ring offset STEP further on in a ring of END words (x < END, STEP <= END).
 template <int STEP, int END>
 __device__ __forceinline__ unsigned ring_next(unsigned x)
@@ -185,6 +183,7 @@ __device__ __forceinline__ unsigned ring_next(unsigned x)
     return min(x, x - END);  // x - END wraps past 2^31 while x < END
 }
 
+// Everything one warp needs for one strip of one sweep.
 struct StripArgs {
     const float* S;   // slowness of the window
     float* T;         // traveltimes of the window

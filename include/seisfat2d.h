@@ -97,7 +97,9 @@ int sf_set_stiffness_codes(sf_ctx* ctx, const uint16_t* const codes[6], const fl
 /* Eikonal_ISO::time_propagation / Eikonal_ANI::time_propagation
  * (eikonal_iso.cu:9-12, eikonal_ani.cu:33-45): initialization() +
  * eikonal_solver() [+ get_quasi_slowness + second solve] for one source on
- * the whole padded grid. T receives nzz x nxx traveltimes. One CTA. */
+ * the whole padded grid. T receives nzz x nxx traveltimes. The solve works on
+ * a window of the context's own (nzz rounded up to whole strips of 32, times
+ * nxx floats; two in the compensated arithmetic). */
 int sf_time_propagation(sf_ctx* ctx, int ani, float sx, float sz, float* T, int T_mem,
                         void* stream);
 
@@ -123,7 +125,8 @@ int sf_batch_forward(sf_ctx* ctx, int ani, const sf_shot* shots, int nshots, con
                      void* stream);
 
 /* Traveltime window of shot `shot` of the last batch run with
- * SF_KEEP_TABLES: nzz x ncols values, z fastest. */
+ * SF_KEEP_TABLES: nzz x ncols values, z fastest. Every shot keeps its window
+ * on the device, its nzz rounded up to whole strips of 32. */
 int sf_batch_table(sf_ctx* ctx, int shot, float* T, int mem, void* stream);
 
 /* Adjoint-state gradient (no counterpart in the reference, whose tomography

@@ -528,6 +528,16 @@ int sf_solver_slowness(sf_ctx* c, const float* model, const float* dS, cudaStrea
     return SF_OK;
 }
 
+int sf_capturing(sf_ctx* c, cudaStream_t st, bool* capturing)
+{
+    *capturing = false;
+    if (!st || st == cudaStreamLegacy) return SF_OK;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    CK(cudaStreamIsCapturing(st, &cs));
+    *capturing = cs != cudaStreamCaptureStatusNone;
+    return SF_OK;
+}
+
 // Orders work on `st` that reads or updates the slowness after the last
 // sf_set_slowness, which returns before its work on the legacy stream is done
 // when its source is a padded device field. Blocking streams follow the legacy
@@ -536,9 +546,10 @@ int sf_solver_slowness(sf_ctx* c, const float* model, const float* dS, cudaStrea
 int sf_wait_slowness(sf_ctx* c, cudaStream_t st)
 {
     if (!st || st == cudaStreamLegacy) return SF_OK;
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    CK(cudaStreamIsCapturing(st, &cs));
-    if (cs != cudaStreamCaptureStatusNone) {
+    bool capturing;
+    int rc = sf_capturing(c, st, &capturing);
+    if (rc) return rc;
+    if (capturing) {
         CK(cudaStreamWaitEvent(st, c->slowness_ev, cudaEventWaitExternal));
         return SF_OK;
     }

@@ -185,6 +185,8 @@ int sf_dev_reserve_zero(sf_ctx* c, void** p, size_t* cap, size_t bytes);
 // Next handoff-tag epoch (never 0 or kGraphEpoch; wraps within 22 bits).
 unsigned sf_next_epoch(sf_ctx* c);
 int sf_check_flags(sf_ctx* c, cudaStream_t st);
+// Whether `st` is being captured (the legacy stream never is).
+int sf_capturing(sf_ctx* c, cudaStream_t st, bool* capturing);
 // The solver's copy and the range check of the context's slowness after it changed.
 int sf_solver_slowness(sf_ctx* c, const float* model, const float* dS, cudaStream_t st);
 // Work on `st` follows the slowness that was set last.

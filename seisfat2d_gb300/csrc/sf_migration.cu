@@ -621,12 +621,8 @@ public:
     }
     int open()
     {
-        if (st_ && st_ != cudaStreamLegacy) {
-            cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-            int rc = sf_cuda_check(c_, cudaStreamIsCapturing(st_, &cs), "cudaStreamIsCapturing");
-            if (rc) return rc;
-            capturing_ = cs != cudaStreamCaptureStatusNone;
-        }
+        int rc = sf_capturing(c_, st_, &capturing_);
+        if (rc) return rc;
         open_ = true;
         return capturing_ ? SF_OK : sf_cuda_check(c_, cudaStreamWaitEvent(st_, c_->kirch_ev, 0), "cudaStreamWaitEvent");
     }

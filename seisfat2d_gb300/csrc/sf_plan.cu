@@ -151,9 +151,9 @@ extern "C" int sf_plan_iteration(sf_ctx* c, const float* t_obs, float* picks, do
     if (rc) return rc;
     CK(cudaSetDevice(c->dev));
     cudaStream_t st = (cudaStream_t)stream;
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    CK(cudaStreamIsCapturing(st, &cs));
-    const bool capturing = cs != cudaStreamCaptureStatusNone;
+    bool capturing;
+    rc = sf_capturing(c, st, &capturing);
+    if (rc) return rc;
     if (c->plan_dirty) {
         if (capturing)
             return sf_fail(c, SF_ERR_STATE, "launch shape changed: run the plan once before capturing it");

@@ -18,11 +18,13 @@ class EikonalPicks(torch.autograd.Function):
         if not S.is_cuda:
             raise ValueError("S must be a CUDA tensor on the engine's device")
         S = S.detach().contiguous()
+        stream = torch.cuda.current_stream(S.device)
+        # set_slowness copies S on the default stream; the forward follows it
+        torch.cuda.default_stream(S.device).wait_stream(stream)
         engine.set_slowness(S, padded=True)
         picks = torch.empty((len(shots), len(rx)), dtype=torch.float32, device=S.device)
-        engine.batch_forward(shots, rx, rz, keep_tape=True, out=picks,
-                             stream=torch.cuda.current_stream(S.device))
-        engine.synchronize(torch.cuda.current_stream(S.device))
+        engine.batch_forward(shots, rx, rz, keep_tape=True, out=picks, stream=stream)
+        engine.synchronize(stream)
         ctx.engine = engine
         ctx.generation = engine.tape_generation
         ctx.shape = S.shape

@@ -114,3 +114,21 @@ def test_slowness_reaches_other_streams(engine_lib, cuda, call):
                 got = e.kirchhoff_image(*args, out=cuda.empty((NX, NZ), device="cuda"), stream=st)
             st.synchronize()
         assert np.array_equal(got.cpu().numpy(), want.cpu().numpy(), equal_nan=True)
+
+
+def test_autograd_on_a_side_stream(engine_lib, cuda):
+    """The slowness is made on a busy side stream, on which the wrapper runs."""
+    from seisfat2d_gb300.autograd import EikonalPicks
+    a, b = models()
+    rx, rz = surface_receivers(NX, 10.0, step=3)
+    want = engine(b).batch_forward(SHOTS, rx, rz)
+    e = engine(a)
+    S, new = (cuda.from_numpy(np.pad(m, 3, mode="edge")).cuda() for m in (a, b))
+    st = cuda.cuda.Stream()
+    cuda.cuda.synchronize()
+    with cuda.cuda.stream(st):
+        cuda.cuda._sleep(100_000_000)
+        S.copy_(new)
+        got = EikonalPicks.apply(S, e, SHOTS, rx, rz)
+        st.synchronize()
+    assert np.array_equal(got.cpu().numpy(), want, equal_nan=True)

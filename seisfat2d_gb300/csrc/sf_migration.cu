@@ -622,6 +622,7 @@ public:
     int open()
     {
         int rc = sf_capturing(c_, st_, &capturing_);
+        if (!rc) rc = sf_wait_slowness(c_, st_);
         if (rc) return rc;
         open_ = true;
         return capturing_ ? SF_OK : sf_cuda_check(c_, cudaStreamWaitEvent(st_, c_->kirch_ev, 0), "cudaStreamWaitEvent");
@@ -659,8 +660,6 @@ static int table_terms(sf_ctx* c, const KirchCall& call, bool grad, const float*
                        int iz0, int nr, int jx0, int nc, TermTable* q, cudaStream_t st)
 {
     const size_t ntab = (size_t)nsrc + nrec, n = (size_t)nr * nc;
-    int rc = sf_wait_slowness(c, st);  // (the operators' kernels follow this one)
-    if (rc) return rc;
     q->a = reinterpret_cast<float4*>(call.workspace());
     q->b = reinterpret_cast<float2*>(q->a + ntab * n);
     q->g = grad ? q->b + ntab * n : nullptr;

@@ -317,7 +317,7 @@ int sf_adj_enqueue(sf_ctx* c, AdjLaunch& A, const float* d_pg, float* d_grad, un
     A.g.grad = d_grad;
     CK(cudaMemsetAsync(A.p.bar, 0, A.nctr * sizeof(unsigned), st));
     CK(cudaMemsetAsync(A.p.vflag, 0, A.nflag, st));
-    if (c->hand_stale_a) {  // the epoch wrapped (sf_next_epoch)
+    if (c->hand_stale_a && epoch != kGraphEpoch) {  // the epoch wrapped (sf_next_epoch)
         CK(cudaMemsetAsync(c->d_hand2, 0, c->cap_hand2, st));
         c->hand_stale_a = false;
     }
@@ -360,7 +360,9 @@ int sf_adjoint_device(sf_ctx* c, const float* d_pg, float* d_grad, cudaStream_t 
 {
     AdjLaunch A;
     int rc = sf_adj_configure(c, st, &A);
-    if (!rc) rc = sf_adj_enqueue(c, A, d_pg, d_grad, sf_next_epoch(c), st);
+    unsigned epoch = 0;
+    if (!rc) rc = sf_launch_epoch(c, A.p.hand, A.hand_bytes, st, &epoch);
+    if (!rc) rc = sf_adj_enqueue(c, A, d_pg, d_grad, epoch, st);
     if (rc) return rc;
     c->tape_valid = false;  // the reverse sweeps overwrite the tape's c2 with their terms
     c->gcij_valid = c->batch_ani != 0;

@@ -538,6 +538,16 @@ int sf_capturing(sf_ctx* c, cudaStream_t st, bool* capturing)
     return SF_OK;
 }
 
+int sf_launch_epoch(sf_ctx* c, void* hand, size_t bytes, cudaStream_t st, unsigned* epoch)
+{
+    bool capturing;
+    int rc = sf_capturing(c, st, &capturing);
+    if (rc) return rc;
+    *epoch = capturing ? kGraphEpoch : sf_next_epoch(c);
+    if (capturing) CK(cudaMemsetAsync(hand, 0, bytes, st));
+    return SF_OK;
+}
+
 // Orders work on `st` that reads or updates the slowness after the last
 // sf_set_slowness, which returns before its work on the legacy stream is done
 // when its source is a padded device field. Blocking streams follow the legacy
@@ -885,7 +895,7 @@ int sf_fwd_launch(sf_ctx* c, FwdLaunch& L, float* d_picks, unsigned epoch, cudaS
     L.p.picks = d_picks;
     L.p.epoch = epoch;
     CK(cudaMemsetAsync(L.p.bar, 0, L.nctr * sizeof(unsigned), st));
-    if (c->hand_stale_f) {
+    if (c->hand_stale_f && epoch != kGraphEpoch) {
         CK(cudaMemsetAsync(c->d_hand, 0, c->cap_hand, st));
         c->hand_stale_f = false;
     }
@@ -953,7 +963,9 @@ int sf_launch_shots(sf_ctx* c, int ani, int nrec, float* d_picks, bool keep_tabl
         FwdLaunch L;
         rc = sf_fwd_configure(c, nrec, keep_tables, tape, gang_warps, st, &L, nullptr);
         L.p.stall_handoff = stall ? 1 : 0;
-        if (!rc) rc = sf_fwd_enqueue(c, L, d_picks, sf_next_epoch(c), st);
+        unsigned epoch = 0;
+        if (!rc) rc = sf_launch_epoch(c, L.p.hand, L.hand_bytes, st, &epoch);
+        if (!rc) rc = sf_fwd_enqueue(c, L, d_picks, epoch, st);
     } else {
         // eikonal_ani.cu:33-45: solve on S, qP pass, solve on the qP slowness;
         // every shot keeps its window between the launches
@@ -972,10 +984,13 @@ int sf_launch_shots(sf_ctx* c, int ani, int nrec, float* d_picks, bool keep_tabl
         L1.p.hand = c->d_hand;
         L1.p.bar = c->d_ctr;
         L1.p.stall_handoff = L2.p.stall_handoff = stall ? 1 : 0;
+        unsigned epoch = 0;
         rc = sf_kt_begin(c, SF_KT_FORWARD, st);
-        if (!rc) rc = sf_fwd_launch(c, L1, nullptr, sf_next_epoch(c), st);
+        if (!rc) rc = sf_launch_epoch(c, L1.p.hand, L1.hand_bytes, st, &epoch);
+        if (!rc) rc = sf_fwd_launch(c, L1, nullptr, epoch, st);
         if (!rc) rc = sf_qp_launch(c, tape, st);
-        if (!rc) rc = sf_fwd_launch(c, L2, d_picks, sf_next_epoch(c), st);
+        if (!rc) rc = sf_launch_epoch(c, L2.p.hand, L2.hand_bytes, st, &epoch);
+        if (!rc) rc = sf_fwd_launch(c, L2, d_picks, epoch, st);
         if (!rc) rc = sf_kt_end(c, SF_KT_FORWARD, st);
     }
     if (rc) return rc;

@@ -184,6 +184,9 @@ int sf_dev_reserve(sf_ctx* c, void** p, size_t* cap, size_t bytes);
 int sf_dev_reserve_zero(sf_ctx* c, void** p, size_t* cap, size_t bytes);
 // Next handoff-tag epoch (never 0 or kGraphEpoch; wraps within 22 bits).
 unsigned sf_next_epoch(sf_ctx* c);
+// Epoch of one launch on `st` with these handoff buffers: the next, or
+// kGraphEpoch with the buffers zeroed first when `st` is being captured.
+int sf_launch_epoch(sf_ctx* c, void* hand, size_t bytes, cudaStream_t st, unsigned* epoch);
 int sf_check_flags(sf_ctx* c, cudaStream_t st);
 // Whether `st` is being captured (the legacy stream never is).
 int sf_capturing(sf_ctx* c, cudaStream_t st, bool* capturing);

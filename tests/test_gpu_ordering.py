@@ -132,3 +132,47 @@ def test_autograd_on_a_side_stream(engine_lib, cuda):
         got = EikonalPicks.apply(S, e, SHOTS, rx, rz)
         st.synchronize()
     assert np.array_equal(got.cpu().numpy(), want, equal_nan=True)
+
+
+# calls captured by the user: each replay follows its own pairs and progress
+# words, not those of the replay before it on another model
+@pytest.mark.parametrize("ani", [False, True])
+def test_captured_calls_replay_on_a_new_model(engine_lib, cuda, ani):
+    from seisfat2d_gb300.synthetic import thomsen_stiffness
+    a, b = models()
+    rx, rz = surface_receivers(NX, 10.0, step=3)
+    obs = np.zeros((len(SHOTS), len(rx)), np.float32)
+
+    def make(m):
+        e = engine(m, "compensated")
+        if ani:
+            vp = 1.0 / models()[0].astype(np.float64)
+            e.set_stiffness([c.astype(np.float32) for c in
+                             thomsen_stiffness(vp, vp / np.sqrt(3.0), 1000.0, 0.1 + 0 * vp, 0.05 + 0 * vp)])
+        return e
+
+    want = []
+    for m in (a, b):
+        e = make(m)
+        pk = e.batch_forward(SHOTS, rx, rz, ani=ani, keep_tape=True)
+        want.append((pk, e.misfit_gradient(obs)[1]))
+    e = make(a)
+    t_obs = cuda.from_numpy(obs).cuda()
+    picks, grad = cuda.empty_like(t_obs), cuda.empty((e.nxx, e.nzz), device="cuda")
+    st, g = cuda.cuda.Stream(), cuda.cuda.CUDAGraph()
+
+    def calls():
+        e.batch_forward(SHOTS, rx, rz, ani=ani, keep_tape=True, out=picks, stream=st)
+        e.misfit_gradient(t_obs, out=grad, stream=st, want_misfit=False)
+
+    calls()
+    e.synchronize(st)
+    with cuda.cuda.graph(g, stream=st):
+        calls()
+    for k in (0, 1, 0, 1, 1):
+        e.set_slowness((a, b)[k])
+        g.replay()
+        cuda.cuda.synchronize()
+        e.synchronize()
+        assert np.array_equal(picks.cpu().numpy(), want[k][0], equal_nan=True)
+        assert np.array_equal(grad.cpu().numpy(), want[k][1])
